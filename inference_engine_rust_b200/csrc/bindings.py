@@ -139,6 +139,7 @@ def _declare(lib) -> None:
         "iert_add_into": [P, P, c_int, c_longlong, S],
         "iert_advance_positions": [P, P, P, c_int, S],
         "iert_gemm_plain": [P, c_int, P, c_int, P, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, S],
+        "iert_gemm_f32_tc": [P, P, P, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, P, S],
         "iert_attention_plain": [P, P, c_int, POINTER(BatchView), POINTER(KvView), c_int, c_float, c_int, c_float, P, P, S],
         "iert_sample_greedy": [P, c_int, c_int, c_longlong, P, P, S],
         "iert_sample_temperature": [P, c_int, c_int, c_longlong, c_float, c_ulonglong, P, P, P, P, S],
@@ -345,6 +346,20 @@ def gemm_plain(x, w, out, M: int, mode: int, stream) -> None:
     check(core().iert_gemm_plain(x.data_ptr(), dtype_code(x.dtype), w.data_ptr(), dtype_code(w.dtype),
                                  out.data_ptr(), dtype_code(out.dtype), M, N, K,
                                  x.stride(0), w.stride(0), out.stride(0), mode, stream), "gemm_plain")
+
+
+def gemm_f32_tc(x, w, out, M: int, mode: int, err, stream) -> bool:
+    """`gemm_plain` of fp32 operands on the tensor cores (each number split into three bf16 parts, sums kept in fp32
+    registers).  False, nothing launched, where the kernel does not take the operands."""
+    if x.dtype != torch.float32 or w.dtype != torch.float32 or out.dtype != torch.float32:
+        return False
+    N, K = w.shape
+    status = core().iert_gemm_f32_tc(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), w.stride(0), out.stride(0),
+                                     mode, err.data_ptr(), stream)
+    if status == 1:
+        return False
+    check(status, "gemm_f32_tc")
+    return True
 
 
 def attention_plain(qkv, out, batch: BatchView, kv: KvView, heads: int, scale: float, paged: bool,

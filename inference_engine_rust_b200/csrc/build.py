@@ -34,7 +34,7 @@ NVCC_FLAGS = [
 # the model's sizes; kernels specialised on a size are separate libraries made on demand.
 CORE_SOURCES = [
     "runtime.cu", "elementwise.cu", "gemm_plain.cu", "attention_plain.cu", "sampling.cu",
-    "gemm_tc.cu", "gemm_rows.cu", "attention_decode.cu",
+    "gemm_tc.cu", "gemm_rows.cu", "gemm_f32_tc.cu", "attention_decode.cu",
     "streams_norm.cu", "recurrent_prep.cu", "latent_attention.cu", "latent_decode_tc.cu", "moe.cu",
     "outnorm.cu", "qk_prep.cu", "rglru.cu", "qkv_prep.cu", "layernorm.cu", "embed_pairs.cu", "latent_decode_umma.cu",
     "selective_scan.cu",

@@ -94,6 +94,8 @@ class Runtime:
         self.device = torch.device(self.device)
         if self.dtype not in (torch.bfloat16, torch.float32):
             raise ValueError(f"run dtype must be bfloat16 or float32, got {self.dtype}")
+        # products of float32 runs may go to the tensor cores in three bf16 parts per number
+        self.split_f32 = self.dtype == torch.float32 and not self.plain_only
         if self.dtype == torch.float32:
             self.plain_only = True
         if self.err is None:

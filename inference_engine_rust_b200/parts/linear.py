@@ -2,8 +2,10 @@
 file has it (reference layout: src/ops/matmul.rs:1-3).  Not a registered part: mixers,
 feed-forwards and the output head use it for their matrix products.
 
-float32 runs use the plain fp32 kernel (every multiply-add in 32-bit).  bfloat16 runs use
-the tcgen05 tensor-core kernel unless the runtime asks for plain kernels only.
+float32 runs use the kernel that splits fp32 numbers into three bf16 parts for the tensor cores (an error no
+larger than that of fp32 multiply-adds: csrc/gemm_f32_tc.cu) or, for short inner axes, the plain fp32 kernel
+(every multiply-add in 32-bit).  bfloat16 runs use the tcgen05 tensor-core kernel.  A runtime that asks for
+plain kernels only gets the plain kernel in both.
 """
 from __future__ import annotations
 
@@ -51,6 +53,8 @@ class Linear:
             from . import fast_linear
             if fast_linear.apply(self, x, out, n_rows, mode, stream, ctx if add_residual else None, epilogue):
                 return
-        B.gemm_plain(as_tensor(x, n_rows), self.weight, out, n_rows, mode, stream)
+        x = as_tensor(x, n_rows)
+        if not (self.rt.split_f32 and B.gemm_f32_tc(x, self.weight, out, n_rows, mode, self.rt.err, stream)):
+            B.gemm_plain(x, self.weight, out, n_rows, mode, stream)
         if epilogue is not None:
             B.epilogue_rows(out, n_rows, epilogue, stream)
