@@ -63,17 +63,24 @@ class Workspace:
     def __init__(self, device):
         self.device = device
         self._bufs: Dict[str, torch.Tensor] = {}
+        self._last: Dict[str, tuple] = {}      # name -> (shape, dtype, the view handed out last)
 
     def take(self, name: str, shape, dtype: torch.dtype) -> torch.Tensor:
+        # steps of one size ask for the same views over and over: making one costs the host about as much as a launch
+        last = self._last.get(name)
+        if last is not None and last[0] == shape and last[1] == dtype:
+            return last[2]
         n = 1
         for s in shape:
             n *= int(s)
-        nbytes = max(n * torch.empty((), dtype=dtype).element_size(), 16)
+        nbytes = n * dtype.itemsize
         buf = self._bufs.get(name)
         if buf is None or buf.numel() < nbytes:
-            buf = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+            buf = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=self.device)
             self._bufs[name] = buf
-        return buf[:n * torch.empty((), dtype=dtype).element_size()].view(dtype).view(*shape)
+        view = buf[:nbytes].view(dtype).view(*shape)
+        self._last[name] = (tuple(shape), dtype, view)
+        return view
 
     def bytes(self) -> int:
         return sum(b.numel() for b in self._bufs.values())
