@@ -21,8 +21,9 @@ LAUNCHERS = ["embed_gather", "rmsnorm", "rope_kv_store", "silu_mul", "gemm_plain
              "latent_attention_decode", "router_topk", "moe_scale", "add_normed", "cast_rows", "scale_values", "qk_prep",
              "rglru_conv", "rglru_gates", "rglru_scan", "qkv_prep", "gate_mul", "router_grouped", "gated_act_mul",
              "token_shift", "wkv_decay", "wkv_recur", "wkv_finish", "latent_prep", "head_gate_mul", "layernorm", "embed_pairs",
-             "rows_begin", "selective_conv", "selective_scan", "epilogue_rows"]
-GEMMS = {"gemm_plain", "gemm_tc", "gemm_rows", "gemm_tc_scaled", "gemm_tc_gated", "gemm_tc_gated_scaled"}
+             "rows_begin", "selective_conv", "selective_scan", "epilogue_rows", "gemm_f32_tc", "moe_sort", "moe_gather", "moe_combine",
+             "gemm_tc_grouped_gated", "gemm_tc_grouped"]
+GEMMS = {"gemm_plain", "gemm_f32_tc", "gemm_tc", "gemm_rows", "gemm_tc_scaled", "gemm_tc_gated", "gemm_tc_gated_scaled"}
 
 
 class KernelClock:
@@ -164,7 +165,7 @@ def _costs(cfg: dict, T: int, n_seqs: int, ctx: int, prompt: bool) -> Dict[str, 
         mlp = next((l["mlp"] for l in cfg["layers"] if l["mlp"] and l["mlp"]["kind"] == "moe"), None)
         if mlp:
             r = mlp["router"]
-            out["moe_scale"] = (0.0, False, T * (r["experts"] * mlp["expert"]["ff"] * 4 + (10 * H if r.get("identity") else 0)))
+            out["moe_scale"] = (0.0, False, T * r["experts"] * mlp["expert"]["ff"] * 4)
             out["router_grouped"] = (0.0, False, T * (r["experts"] + r.get("identity", 0)) * 8)
     elif cfg.get("architecture") == "Vufinex":
         H = cfg["width"]

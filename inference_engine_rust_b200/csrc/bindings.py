@@ -170,8 +170,13 @@ def _declare(lib) -> None:
         "iert_wkv_decay": [P, LL, c_int, P, P, c_int, P, P, c_int, LL, c_int, P, LL, LL, POINTER(BatchView), S],
         "iert_wkv_finish": [P, P, LL, P, c_float, c_float, P, c_int, POINTER(BatchView), c_int, c_int, S],
         "iert_latent_decode_tc_plan": [c_int, c_int, c_int, c_int, c_int, POINTER(c_int), POINTER(c_int)],
-        "iert_router_topk": [P, LL, P, c_int, c_int, c_int, P, P, P, S],
-        "iert_moe_scale": [P, c_int, LL, P, c_int, c_int, c_int, P, P, LL, P, c_int, S],
+        "iert_router_topk": [P, LL, LL, P, c_int, c_int, c_int, P, c_int, P, P, S],
+        "iert_moe_scale": [P, c_int, LL, P, c_int, c_int, c_int, c_int, S],
+        "iert_moe_sort": [P, P, c_int, c_int, c_int, P, P, P, P, S],
+        "iert_moe_gather": [P, LL, P, P, c_int, P, c_int, S],
+        "iert_moe_combine": [P, P, P, c_int, c_int, P, c_int, S],
+        "iert_gemm_tc_grouped_gated": [P, LL, P, LL, P, LL, c_int, c_int, P, c_int, c_int, c_int, c_int, P, POINTER(GatedAct), P, S],
+        "iert_gemm_tc_grouped": [P, LL, P, LL, P, LL, c_int, c_int, P, c_int, c_int, c_int, P, S],
         "iert_router_grouped": [P, LL, LL, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
                                 c_int, c_int, P, c_int, P, P, P, P, c_int, LL, P, c_int, S],
         "iert_qkv_prep": [P, LL, P, P, c_int, POINTER(BatchView), POINTER(KvView), c_int, c_int, c_int, P, c_int, c_float, c_int,
@@ -193,8 +198,8 @@ def _declare(lib) -> None:
     lib.iert_attention_decode.restype = c_int
     lib.iert_attention_decode_scratch_floats.argtypes = [c_int, c_int, c_int, c_int]
     lib.iert_attention_decode_scratch_floats.restype = c_longlong
-    lib.iert_gemm_tc_gated.argtypes = [P, c_longlong, P, c_longlong, P, c_longlong, c_int, c_int, c_int, POINTER(GatedAct),
-                                       c_int, c_int, P, S]
+    lib.iert_gemm_tc_gated.argtypes = [P, c_longlong, P, c_longlong, P, c_longlong, c_int, c_int, c_int, c_int, POINTER(GatedAct),
+                                       POINTER(Epilogue), c_int, c_int, P, S]
     lib.iert_gemm_tc_gated.restype = c_int
     lib.iert_gemm_rows.argtypes = [P, c_longlong, P, c_longlong, P, c_int, c_longlong, c_int, c_int, c_int, c_int,
                                    POINTER(RowScale), POINTER(NormAhead), POINTER(Epilogue), c_int, c_int, P, S]
@@ -624,14 +629,17 @@ def attention_decode_tc_rope(qkv, out, batch: BatchView, kv: KvView, heads: int,
 
 
 def gemm_tc_gated(x, w, act, M: int, err, stream, force_bt: int = 0, force_stages: int = 0,
-                  fn: Optional[GatedAct] = None) -> bool:
+                  fn: Optional[GatedAct] = None, epilogue: Optional[Epilogue] = None, inter: Optional[int] = None,
+                  up_rows: int = 0) -> bool:
     """act[:M] = f(x @ w[:I].T, x @ w[I:].T) for w = [gate; up] with 2 I rows and f of the gated-activation family
-    (`fn`; None: silu(gate) * up), on the tensor cores in one kernel.  Returns False, having launched nothing, when the
-    operands do not meet the kernel's alignment rules."""
+    (`fn`; None: silu(gate) * up), on the tensor cores in one kernel.  `epilogue`: a factor per token and block of columns.
+    `inter`, `up_rows`: w's first `inter` rows are the gate, the up rows start `up_rows` further on (a part of a stack of
+    matrices).  Returns False, having launched nothing, when the operands do not meet the kernel's alignment rules."""
     two_i, K = w.shape
     status = core().iert_gemm_tc_gated(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), act.data_ptr(),
-                                       act.stride(0), M, two_i // 2, K, byref(fn) if fn is not None else None,
-                                       force_bt, force_stages, err.data_ptr(), stream)
+                                       act.stride(0), M, inter or two_i // 2, up_rows, K, byref(fn) if fn is not None else None,
+                                       byref(epilogue) if epilogue is not None else None, force_bt, force_stages, err.data_ptr(),
+                                       stream)
     if status == 1:
         return False
     check(status, "gemm_tc_gated")
@@ -851,8 +859,10 @@ def latent_attention_decode_tc(q, w_uk, w_uv, out, batch: BatchView, kv: KvView,
     return True
 
 
-def router_topk(z, bias, n_tokens: int, E: int, top: int, wt, idx, w, stream) -> None:
-    check(core().iert_router_topk(z.data_ptr(), z.stride(0), _ptr(bias), n_tokens, E, top, wt.data_ptr(), idx.data_ptr(),
+def router_topk(z, bias, n_tokens: int, E: int, top: int, wt, idx, w, stream, by_output: bool = False) -> None:
+    """z: fp32 [T, E], or with `by_output` [E, T]; wt [T, >= E]: columns from E on are set to 1."""
+    ldz, lde = (z.stride(1), z.stride(0)) if by_output else (z.stride(0), z.stride(1))
+    check(core().iert_router_topk(z.data_ptr(), ldz, lde, _ptr(bias), n_tokens, E, top, wt.data_ptr(), wt.stride(0), idx.data_ptr(),
                                   w.data_ptr(), stream), "router_topk")
 
 
@@ -880,11 +890,49 @@ def router_grouped(z, correction, n_tokens: int, E: int, N: int, top: int, group
                                      residual.shape[-1] if residual is not None else 0, stream), "router_grouped")
 
 
-def moe_scale(act, wt, n_tokens: int, E: int, F: int, stream, wid=None, x=None, residual=None) -> None:
-    """act[t, e*F + i] *= wt[t, e]; with `wid`, also residual[t] += wid[t] * x[t]."""
-    check(core().iert_moe_scale(act.data_ptr(), dtype_code(act.dtype), act.stride(0), wt.data_ptr(), n_tokens, E, F,
-                                _ptr(wid), _ptr(x), x.stride(0) if x is not None else 0, _ptr(residual),
-                                residual.shape[-1] if residual is not None else 0, stream), "moe_scale")
+def moe_scale(act, wt, n_tokens: int, E: int, F: int, stream) -> None:
+    """act[t, e*F + i] *= wt[t, e]."""
+    check(core().iert_moe_scale(act.data_ptr(), dtype_code(act.dtype), act.stride(0), wt.data_ptr(), wt.stride(0), n_tokens, E, F,
+                                stream), "moe_scale")
+
+
+def moe_group_ints(n_tokens: int, top: int, E: int) -> int:
+    """Length of `moe_sort`'s table of row tiles."""
+    return 2 + 3 * (n_tokens * top // 128 + E)
+
+
+def moe_sort(idx, w, n_tokens: int, top: int, E: int, groups, pos, row_token, row_w, stream) -> None:
+    """The choices idx, w [T, top] by expert: pos [T * top] the row of a choice (-1: none), row_token / row_w [T * top] the token
+    and weight of a row, groups the table of row tiles for the grouped products."""
+    check(core().iert_moe_sort(idx.data_ptr(), w.data_ptr(), n_tokens, top, E, groups.data_ptr(), pos.data_ptr(), row_token.data_ptr(),
+                               row_w.data_ptr(), stream), "moe_sort")
+
+
+def moe_gather(x, groups, row_token, max_rows: int, xs, stream) -> None:
+    """xs[row] = x[row_token[row]] for the rows of the table (bf16)."""
+    check(core().iert_moe_gather(x.data_ptr(), x.stride(0), groups.data_ptr(), row_token.data_ptr(), max_rows, xs.data_ptr(),
+                                 xs.shape[-1], stream), "moe_gather")
+
+
+def moe_combine(y, pos, w, n_tokens: int, top: int, residual, stream) -> None:
+    """residual[t] += the sum of y[pos[t, k]] over the choices that have a row."""
+    check(core().iert_moe_combine(y.data_ptr(), pos.data_ptr(), w.data_ptr(), n_tokens, top, residual.data_ptr(), residual.shape[-1],
+                                  stream), "moe_combine")
+
+
+def gemm_tc_grouped_gated(x, w, act, groups, max_row_tiles: int, experts: int, F: int, up_rows: int, row_scale, err, stream,
+                          fn: Optional[GatedAct] = None) -> None:
+    """Rows of x sorted by expert (`moe_sort`): act[r, i] = f(x[r] . w[e F + i], x[r] . w[up_rows + e F + i]) * row_scale[r]."""
+    check(core().iert_gemm_tc_grouped_gated(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), act.data_ptr(), act.stride(0), x.shape[0],
+                                            max_row_tiles, groups.data_ptr(), experts, F, up_rows, w.shape[1], _ptr(row_scale),
+                                            byref(fn) if fn is not None else None, err.data_ptr(), stream), "gemm_tc_grouped_gated")
+
+
+def gemm_tc_grouped(x, w, out, groups, max_row_tiles: int, experts: int, K: int, err, stream) -> None:
+    """out[r] = x[r] . w[:, e K : (e + 1) K]^T (fp32) for rows of x sorted by expert."""
+    check(core().iert_gemm_tc_grouped(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), x.shape[0],
+                                      max_row_tiles, groups.data_ptr(), experts, w.shape[0], K, err.data_ptr(), stream),
+          "gemm_tc_grouped")
 
 
 # ---------------------------------------------------------------------------------------

@@ -85,6 +85,12 @@ struct GemmParams {
                         // writes the next norm's first half
   IertEpilogue ep;      // plain stores: activation and column scale of every output (see common.cuh)
   IertGatedAct act;     // gated launches: the activation (see common.cuh)
+  // grouped launches (rows sorted by expert, see moe_sort in moe.cu): groups[0] row tiles, then from groups[2] on per row tile
+  // {expert, first row, end of the expert's rows}; expert e's matrix starts group_w_rows * e rows and group_k * e columns into w;
+  // row_scale (gated): a factor of every output of a row
+  const int* groups;
+  int group_w_rows, group_k;
+  const float* row_scale;
   int trace_seq;        // >= 0: the launch's row in the trace (builds with IERT_GEMM_TRACE only)
   uint32_t poll_limit;  // polls of a tile's counter before a CTA gives up waiting for the other CTAs of its tile
 };
@@ -269,8 +275,8 @@ __device__ __forceinline__ void tile_coords(const GemmParams& p, int tile, int& 
 struct WorkIter {
   const GemmParams& p;
   int work, total_work, n_tail;
-  __device__ WorkIter(const GemmParams& p_) : p(p_) {
-    const int tiles = p.n_tiles * p.t_tiles;
+  __device__ WorkIter(const GemmParams& p_, int t_tiles) : p(p_) {
+    const int tiles = p.n_tiles * t_tiles;
     n_tail = p.tail_parts > 1 ? tiles - p.full_tiles : 0;
     total_work = p.tail_parts > 1 ? p.full_tiles + n_tail * p.tail_parts : tiles * p.splits;
     work = blockIdx.x;
@@ -296,7 +302,33 @@ struct WorkIter {
   }
 };
 
-template <int BT, bool GATED>
+// Where a tile lies: first output column and first token row, the end of the valid rows, and where its weights start in w.
+struct TilePlace { int n_idx, n0, t0, t_end, w_row, w_col; };
+template <int BT, bool GROUPED>
+__device__ __forceinline__ TilePlace tile_place(const GemmParams& p, int tile, int t_tiles) {
+  TilePlace c;
+  if (GROUPED) {                         // the row tiles run fastest: an expert's weights are read by all its row tiles at once
+    c.n_idx = tile / t_tiles;
+    const int* g = p.groups + 2 + 3 * (tile - c.n_idx * t_tiles);
+    const int e = __ldg(g);
+    c.n0 = c.n_idx * p.n_step;
+    c.t0 = __ldg(g + 1);
+    c.t_end = __ldg(g + 2);
+    c.w_row = c.n0 + e * p.group_w_rows;
+    c.w_col = e * p.group_k;
+  } else {
+    int t_idx;
+    tile_coords(p, tile, c.n_idx, t_idx);
+    c.n0 = c.n_idx * p.n_step;
+    c.t0 = t_idx * BT;
+    c.t_end = p.M;
+    c.w_row = c.n0;
+    c.w_col = 0;
+  }
+  return c;
+}
+
+template <int BT, bool GATED, bool GROUPED = false>
 __global__ void __launch_bounds__(THREADS, 2)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                const __grid_constant__ CUtensorMap map_o, const GemmParams p) {
@@ -339,6 +371,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   const uint32_t tmem_base = *tmem_slot;
   if (threadIdx.x == 0) pdl_launch_dependents();
   if (threadIdx.x == 0) IERT_TRACE(0);                       // start
+  if (GROUPED) pdl_wait();                                   // the table of row tiles comes from a kernel in front
+  const int t_tiles = GROUPED ? __ldg(p.groups) : p.t_tiles;
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -348,14 +382,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       // then their token tiles follow.  (With an ordinary launch the wait returns at once.)
       int stage = 0, issued = 0;
       uint32_t phase = 0;
-      bool ok = true, dep_ready = false;
+      bool ok = true, dep_ready = GROUPED;
       int pend_kb[12], pend_t0[12];
-      WorkIter it(p);
+      WorkIter it(p, t_tiles);
       int tile, split, n_parts, kb0, kb1;
       while (ok && it.next(tile, split, n_parts, kb0, kb1)) {
-        int n_idx, t_idx;
-        tile_coords(p, tile, n_idx, t_idx);
-        const int n0 = n_idx * p.n_step, t0 = t_idx * BT;
+        const TilePlace at = tile_place<BT, GROUPED>(p, tile, t_tiles);
+        const int t0 = at.t0, w_row = at.w_row, w_col = at.w_col;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!dep_ready && issued == stages) {
             pdl_wait();
@@ -367,11 +400,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           if (!wait_or_abort(&empty[stage], phase ^ 1, abort_flag)) { ok = false; break; }
           uint8_t* ws_ = smem + (size_t)stage * STAGE_BYTES;
           mbar_expect_tx(&full[stage], STAGE_BYTES);
-          tma_load_2d(ws_, &map_w, &full[stage], kb * TILE_K, n0);
+          tma_load_2d(ws_, &map_w, &full[stage], w_col + kb * TILE_K, w_row);
           if (GATED)   // the second 128 weight rows of the tile: the up rows (gated) or the next rows (plain)
-            tma_load_2d(ws_ + W_STAGE_BYTES, &map_w, &full[stage], kb * TILE_K, n0 + p.second_rows);
+            tma_load_2d(ws_ + W_STAGE_BYTES, &map_w, &full[stage], w_col + kb * TILE_K, w_row + p.second_rows);
           else if (p.mode == MODE_GATED_SILU)   // weight-major gated: 64 gate rows (above), then their 64 up rows
-            tma_load_2d(ws_ + W_STAGE_BYTES / 2, &map_w, &full[stage], kb * TILE_K, n0 + p.second_rows);
+            tma_load_2d(ws_ + W_STAGE_BYTES / 2, &map_w, &full[stage], kb * TILE_K, w_row + p.second_rows);
           if (dep_ready) tma_load_2d(ws_ + X_OFF, &map_x, &full[stage], kb * TILE_K, t0);
           else { pend_kb[issued] = kb; pend_t0[issued] = t0; }
           if (issued == 0) IERT_TRACE(1);                    // first weights asked for
@@ -404,7 +437,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
-      WorkIter it(p);
+      WorkIter it(p, t_tiles);
       int tile, split, n_parts, kb0, kb1;
       while (ok && it.next(tile, split, n_parts, kb0, kb1)) {
         if (!wait_or_abort(&acc_empty[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
@@ -452,14 +485,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
-    WorkIter it(p);
+    WorkIter it(p, t_tiles);
     int tile, split, n_parts, kb0, kb1;
     while (ok && it.next(tile, split, n_parts, kb0, kb1)) {
-      int n_idx, t_idx;
-      tile_coords(p, tile, n_idx, t_idx);
-      const int n0 = n_idx * p.n_step, t0 = t_idx * BT;
+      const TilePlace at = tile_place<BT, GROUPED>(p, tile, t_tiles);
+      const int n_idx = at.n_idx, n0 = at.n0, t0 = at.t0, t_end = at.t_end;
       const int n = n0 + n_local;
-      const int t_valid = min(BT, p.M - t0);
+      const int t_valid = min(BT, t_end - t0);
+      // (weight-major gated tiles: the columns' factors are asked for while the weights stream)
+      constexpr int N_FACTORS = !GATED && BT <= 32 ? BT : 1;
+      float factor[N_FACTORS];
+      const float* factor_col = nullptr;
+      if (!GATED && p.mode == MODE_GATED_SILU && p.ep.scale && q < 2) {
+        factor_col = p.ep.scale + (long long)t0 * p.ep.ld_scale + epilogue_block(n0 + n_local, p.ep);
+#pragma unroll
+        for (int j = 0; j < N_FACTORS; ++j) factor[j] = j < t_valid ? factor_col[(long long)j * p.ep.ld_scale] : 0.f;
+      }
       if (!wait_or_abort(&acc_full[acc], acc_phase, abort_flag)) { ok = false; break; }
       if (threadIdx.x == 64) IERT_TRACE(5);                    // the accumulator is complete
       tc_fence_after();
@@ -481,25 +522,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       if (GATED && p.mode == MODE_GATED_SILU) {
         // lane = token, columns [0, 128) = gate rows, [128, 256) = their up rows
         const int tok = t0 + n_local;
+        const float row_factor = GROUPED && p.row_scale && tok < t_end ? p.row_scale[tok] : 1.0f;
 #pragma unroll 1
         for (int c = 0; c < TILE_N; c += 16) {
           float v[16], u[16];
           tmem_ld16(taddr + c, v);
           tmem_ld16(taddr + TILE_N + c, u);
-          if (tok < p.M) {
+          if (tok < t_end) {
             __nv_bfloat16* o = (__nv_bfloat16*)p.out + (long long)tok * p.ldo + n0 + c;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = GROUPED ? silu_mul(v[j], u[j]) * row_factor : silu_mul(v[j], u[j]);
+            if (!GROUPED && p.ep.scale) epilogue_run<16>(v, tok, n0 + c, p.ep);
             if (n0 + c + 16 <= p.N && (p.ldo & 7) == 0 && ((uintptr_t)p.out & 15) == 0) {
               uint4 w2[2];
               __nv_bfloat162* wp = reinterpret_cast<__nv_bfloat162*>(w2);
 #pragma unroll
-              for (int j = 0; j < 8; ++j)
-                wp[j] = __floats2bfloat162_rn(silu_mul(v[2 * j], u[2 * j]), silu_mul(v[2 * j + 1], u[2 * j + 1]));
+              for (int j = 0; j < 8; ++j) wp[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
               reinterpret_cast<uint4*>(o)[0] = w2[0];
               reinterpret_cast<uint4*>(o)[1] = w2[1];
             } else {
 #pragma unroll
               for (int j = 0; j < 16; ++j)
-                if (n0 + c + j < p.N) o[j] = __float2bfloat16_rn(silu_mul(v[j], u[j]));
+                if (n0 + c + j < p.N) o[j] = __float2bfloat16_rn(v[j]);
             }
           }
         }
@@ -512,7 +556,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           if (n0 + c >= p.N) break;                    // warp-uniform
           float v[16];
           tmem_ld16(taddr + c, v);
-          if (tok >= p.M) continue;
+          if (tok >= t_end) continue;
           if (p.mode == MODE_STORE && epilogue_on(p.ep)) epilogue_run<16>(v, tok, n0 + c, p.ep);
           const bool full16 = n0 + c + 16 <= p.N;
           if (p.out_dtype == IERT_F32) {
@@ -557,7 +601,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         // that belong to them.  The up warps hand their values over through shared memory, the
         // gate warps write silu(gate) * up, 64 consecutive outputs of a token per pair of warps.
         float* xch = reinterpret_cast<float*>(xch_s);                 // [16 tokens][64]
-#pragma unroll 1
+#pragma unroll
         for (int c = 0; c < BT; c += 16) {
           if (c >= t_valid) break;                   // uniform over the four warps
           float v[16];
@@ -574,8 +618,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
               for (int j = 0; j < 16; ++j)
                 if (c + j < t_valid) {
                   const float r = scaled ? rstd_s[c + j] : 1.0f;
-                  ((__nv_bfloat16*)p.out)[(long long)(t0 + c + j) * p.ldo + i] =
-                      __float2bfloat16_rn(silu_mul(v[j] * r, xch[j * 64 + n_local] * r));
+                  float act = silu_mul(v[j] * r, xch[j * 64 + n_local] * r);
+                  if (factor_col) act *= N_FACTORS > 1 ? factor[(c + j) % N_FACTORS] : factor_col[(long long)(c + j) * p.ep.ld_scale];
+                  ((__nv_bfloat16*)p.out)[(long long)(t0 + c + j) * p.ldo + i] = __float2bfloat16_rn(act);
                 }
             }
           }
@@ -902,7 +947,7 @@ int g_trace_next = 0;
 
 uint32_t g_poll_limit = WAIT_LIMIT;
 
-template <int BT, bool GATED>
+template <int BT, bool GATED, bool GROUPED = false>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, GemmParams p, int grid, cudaStream_t stream,
            const CUtensorMap* mo = nullptr) {
   p.trace_seq = -1;
@@ -917,11 +962,11 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, GemmParams p, int grid,
                                          p.scale.sumsq != nullptr);
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(gemm_tc_kernel<BT, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_tc_kernel<BT, GATED, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
       return iert_check_launch("gemm_tc attribute");
     configured = true;
   }
-  launch_dep(gemm_tc_kernel<BT, GATED>, dim3(grid), dim3(THREADS), smem, stream, mw, mx, mo ? *mo : mw, p);
+  launch_dep(gemm_tc_kernel<BT, GATED, GROUPED>, dim3(grid), dim3(THREADS), smem, stream, mw, mx, mo ? *mo : mw, p);
   return iert_check_launch("gemm_tc");
 }
 
@@ -1010,6 +1055,7 @@ int gemm_tc_impl(const void* x, long long ldx, const void* w, long long ldw, voi
   if (bt != 16 && bt != 32 && bt != 64 && bt != 128 && bt != 256) return IERT_BAD_ARGUMENT;
 
   GemmParams p;
+  p.groups = nullptr; p.group_w_rows = p.group_k = 0; p.row_scale = nullptr;
   p.scale = IertRowScale{nullptr, 0, 0, 0.f};
   p.ahead = IertNormAhead{nullptr, 0, nullptr, 0, nullptr, 0};
   if (scale) p.scale = *scale;
@@ -1186,15 +1232,18 @@ IERT_API int iert_gemm_tc_scaled(const void* x, long long ldx, const void* w, lo
 // tiles only; same alignment rules as iert_gemm_tc.
 namespace {
 int gemm_tc_gated_impl(const void* x, long long ldx, const void* w, long long ldw, void* act,
-                       long long ldo, int M, int inter, int K, const IertRowScale* scale, const IertGatedAct* fn, int force_bt,
-                       int force_stages, int* err, cudaStream_t stream) {
+                       long long ldo, int M, int inter, int up_rows, int K, const IertRowScale* scale, const IertGatedAct* fn,
+                       const IertEpilogue* ep, int force_bt, int force_stages, int* err, cudaStream_t stream) {
   if (M <= 0 || inter <= 0) return IERT_OK;
   if (K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15))
     return IERT_BAD_ARGUMENT;
   if (scale && (!scale->sumsq || scale->parts <= 0 || scale->hidden <= 0)) return IERT_BAD_ARGUMENT;
   GemmParams p;
+  p.groups = nullptr; p.group_w_rows = p.group_k = 0; p.row_scale = nullptr;
   p.scale = IertRowScale{nullptr, 0, 0, 0.f};
-  p.ep = IertEpilogue{IERT_ACT_NONE, nullptr, 0, 0, 1};
+  if (ep && (ep->act != IERT_ACT_NONE || !ep->scale || ep->blocks < 0 || ep->block_cols <= 0)) return IERT_BAD_ARGUMENT;
+  if (up_rows < inter) return IERT_BAD_ARGUMENT;
+  p.ep = ep ? *ep : IertEpilogue{IERT_ACT_NONE, nullptr, 0, 0, 1};
   p.tail_parts = 1; p.full_tiles = 0; p.tma_out = 0; p.t_group = 1 << 30;
   p.out = act; p.ldo = ldo; p.out_dtype = IERT_BF16; p.mode = MODE_GATED_SILU;
   p.act = fn ? *fn : IertGatedAct{INFINITY, INFINITY, 0.f, 1.f, 0.f};
@@ -1208,7 +1257,7 @@ int gemm_tc_gated_impl(const void* x, long long ldx, const void* w, long long ld
     // per tile, no split over k.  Chosen when its tiles alone fill the device; for smaller
     // matrices the caller does better with the split product and a separate activation.
     const int wbt = force_bt ? force_bt : (M <= 16 ? 16 : M <= 32 ? 32 : 64);
-    p.n_step = TILE_N / 2; p.second_rows = inter;
+    p.n_step = TILE_N / 2; p.second_rows = up_rows;
     p.n_tiles = (inter + TILE_N / 2 - 1) / (TILE_N / 2);
     p.t_tiles = 1;
     p.kb_total = (K + TILE_K - 1) / TILE_K;
@@ -1221,7 +1270,7 @@ int gemm_tc_gated_impl(const void* x, long long ldx, const void* w, long long ld
     if (stages < 2 || (size_t)stages * stage_bytes + 1280 + XCH_BYTES > 227 * 1024) return IERT_BAD_ARGUMENT;
     p.stages = stages;
     CUtensorMap mw, mx;
-    if (!tensor_map(w, 2ll * inter, K, ldw, TILE_N / 2, &mw) || !tensor_map(x, M, K, ldx, wbt, &mx)) return IERT_BAD_ARGUMENT;
+    if (!tensor_map(w, (long long)up_rows + inter, K, ldw, TILE_N / 2, &mw) || !tensor_map(x, M, K, ldx, wbt, &mx)) return IERT_BAD_ARGUMENT;
     const int slots = 2 * sm_count();
     const int grid = p.n_tiles < slots ? p.n_tiles : slots;
     switch (wbt) {
@@ -1232,7 +1281,7 @@ int gemm_tc_gated_impl(const void* x, long long ldx, const void* w, long long ld
   }
   if (scale) return IERT_BAD_ARGUMENT;                 // only the one-token form scales its rows
   const int bt = 128;                                  // tokens per tile: the MMA's M side
-  p.n_step = TILE_N; p.second_rows = inter;
+  p.n_step = TILE_N; p.second_rows = up_rows;
   p.n_tiles = (inter + TILE_N - 1) / TILE_N;
   p.t_tiles = (M + bt - 1) / bt;
   p.kb_total = (K + TILE_K - 1) / TILE_K;
@@ -1248,16 +1297,16 @@ int gemm_tc_gated_impl(const void* x, long long ldx, const void* w, long long ld
   if (stages < 2 || (size_t)stages * stage_bytes + 1280 > 227 * 1024) return IERT_BAD_ARGUMENT;
   p.stages = stages;
   CUtensorMap mw, mx;
-  if (!tensor_map(w, 2ll * inter, K, ldw, TILE_N, &mw) || !tensor_map(x, M, K, ldx, bt, &mx)) return IERT_BAD_ARGUMENT;
+  if (!tensor_map(w, (long long)up_rows + inter, K, ldw, TILE_N, &mw) || !tensor_map(x, M, K, ldx, bt, &mx)) return IERT_BAD_ARGUMENT;
   const int grid = tiles < slots ? tiles : slots;
   return launch<128, true>(mw, mx, p, grid, stream);
 }
 }  // namespace
 
 IERT_API int iert_gemm_tc_gated(const void* x, long long ldx, const void* w, long long ldw, void* act,
-                                long long ldo, int M, int inter, int K, const IertGatedAct* fn, int force_bt, int force_stages,
-                                int* err, cudaStream_t stream) {
-  return gemm_tc_gated_impl(x, ldx, w, ldw, act, ldo, M, inter, K, nullptr, fn, force_bt, force_stages, err, stream);
+                                long long ldo, int M, int inter, int up_rows, int K, const IertGatedAct* fn, const IertEpilogue* ep,
+                                int force_bt, int force_stages, int* err, cudaStream_t stream) {
+  return gemm_tc_gated_impl(x, ldx, w, ldw, act, ldo, M, inter, up_rows ? up_rows : inter, K, nullptr, fn, ep, force_bt, force_stages, err, stream);
 }
 
 // The one-token form (M <= 64) for an x that is the first half of an RMSNorm (IertNormAhead of the kernel
@@ -1267,5 +1316,60 @@ IERT_API int iert_gemm_tc_gated_scaled(const void* x, long long ldx, const void*
                                        long long ldo, int M, int inter, int K, const IertRowScale* scale,
                                        const IertGatedAct* fn, int force_bt, int* err, cudaStream_t stream) {
   if (!scale) return IERT_BAD_ARGUMENT;
-  return gemm_tc_gated_impl(x, ldx, w, ldw, act, ldo, M, inter, K, scale, fn, force_bt, 0, err, stream);
+  return gemm_tc_gated_impl(x, ldx, w, ldw, act, ldo, M, inter, inter, K, scale, fn, nullptr, force_bt, 0, err, stream);
+}
+
+// Products over rows sorted by expert (moe_sort in moe.cu): a row tile belongs to one expert and meets that expert's matrix
+// alone.  Token-major tiles as above; `groups` is the device table, `max_row_tiles` its bound (the grid's size), `rows` the
+// rows of x at most.
+//   gated   act[r, i] = f(x[r] . w[e F + i], x[r] . w[up_rows + e F + i]) * row_scale[r],  i < F
+//   plain   out[r, n] = x[r] . w[n, e K .. e K + K)   (fp32; experts' matrices side by side)
+IERT_API int iert_gemm_tc_grouped_gated(const void* x, long long ldx, const void* w, long long ldw, void* act, long long ldo,
+                                        int rows, int max_row_tiles, const int* groups, int experts, int F, int up_rows, int K,
+                                        const float* row_scale, const IertGatedAct* fn, int* err, cudaStream_t stream) {
+  if (rows <= 0 || max_row_tiles <= 0) return IERT_OK;
+  if (F <= 0 || K <= 0 || experts <= 0 || up_rows < experts * F || (K & 7) || (ldx & 7) || (ldw & 7) ||
+      (((uintptr_t)x | (uintptr_t)w) & 15) || !groups)
+    return IERT_BAD_ARGUMENT;
+  GemmParams p;
+  memset(&p, 0, sizeof p);
+  p.ep = IertEpilogue{IERT_ACT_NONE, nullptr, 0, 0, 1};
+  p.tail_parts = 1; p.splits = 1; p.t_group = 1 << 30;
+  p.out = act; p.ldo = ldo; p.out_dtype = IERT_BF16; p.mode = MODE_GATED_SILU;
+  p.act = fn ? *fn : IertGatedAct{INFINITY, INFINITY, 0.f, 1.f, 0.f};
+  p.M = rows; p.N = F; p.K = K; p.err = err;
+  p.groups = groups; p.group_w_rows = F; p.row_scale = row_scale;
+  p.n_step = TILE_N; p.second_rows = up_rows;
+  p.n_tiles = (F + TILE_N - 1) / TILE_N; p.t_tiles = max_row_tiles;
+  p.kb_total = p.kb_per_split = (K + TILE_K - 1) / TILE_K;
+  p.stages = (226 * 1024 - 2048) / (2 * W_STAGE_BYTES + 128 * TILE_K * 2);
+  CUtensorMap mw, mx;
+  if (!tensor_map(w, (long long)up_rows + (long long)experts * F, K, ldw, TILE_N, &mw) || !tensor_map(x, rows, K, ldx, 128, &mx))
+    return IERT_BAD_ARGUMENT;
+  const long long tiles = (long long)p.n_tiles * max_row_tiles;
+  return launch<128, true, true>(mw, mx, p, (int)(tiles < sm_count() ? tiles : sm_count()), stream);
+}
+
+IERT_API int iert_gemm_tc_grouped(const void* x, long long ldx, const void* w, long long ldw, float* out, long long ldo, int rows,
+                                  int max_row_tiles, const int* groups, int experts, int N, int K, int* err, cudaStream_t stream) {
+  if (rows <= 0 || max_row_tiles <= 0) return IERT_OK;
+  // (an expert's last block of k must not reach into the next expert's columns)
+  if (N <= 0 || K <= 0 || experts <= 0 || K % TILE_K || ldw < (long long)experts * K || (ldx & 7) || (ldw & 7) ||
+      (((uintptr_t)x | (uintptr_t)w) & 15) || !groups)
+    return IERT_BAD_ARGUMENT;
+  GemmParams p;
+  memset(&p, 0, sizeof p);
+  p.ep = IertEpilogue{IERT_ACT_NONE, nullptr, 0, 0, 1};
+  p.tail_parts = 1; p.splits = 1; p.t_group = 1 << 30;
+  p.out = out; p.ldo = ldo; p.out_dtype = IERT_F32; p.mode = MODE_STORE;
+  p.M = rows; p.N = N; p.K = K; p.err = err;
+  p.groups = groups; p.group_k = K;
+  p.n_step = 2 * TILE_N; p.second_rows = TILE_N;
+  p.n_tiles = (N + 2 * TILE_N - 1) / (2 * TILE_N); p.t_tiles = max_row_tiles;
+  p.kb_total = p.kb_per_split = K / TILE_K;
+  p.stages = (226 * 1024 - 2048) / (2 * W_STAGE_BYTES + 128 * TILE_K * 2);
+  CUtensorMap mw, mx;
+  if (!tensor_map(w, N, (long long)experts * K, ldw, TILE_N, &mw) || !tensor_map(x, rows, K, ldx, 128, &mx)) return IERT_BAD_ARGUMENT;
+  const long long tiles = (long long)p.n_tiles * max_row_tiles;
+  return launch<128, true, true>(mw, mx, p, (int)(tiles < sm_count() ? tiles : sm_count()), stream);
 }

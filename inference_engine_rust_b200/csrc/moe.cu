@@ -11,8 +11,13 @@
 //   wt [T, E] over the experts with tensors, as wid [T] (the sum of the weights of chosen identity experts) and
 //   as lists idx / w [T, top].
 // moe_scale: act[t, e*F + i] *= wt[t, e] for the E routed experts' blocks of F activations; columns
-//   beyond E*F (an expert that every token uses) are left as they are.  With `wid`: also
-//   residual[t, :] += wid[t] * x[t, :] (the identity experts' share; x in the activations' dtype).
+//   beyond E*F (an expert that every token uses) are left as they are.
+//
+// Prompts run the experts' products over the tokens that chose them (gemm_tc.cu, grouped launches):
+// moe_sort: the (token, choice) pairs of a step by expert, in one block: counts, offsets, places.  An expert's rows follow one
+//   another without gaps; `groups` lists its row tiles of 128.
+// moe_gather: xs[row] = x[row_token[row]] (16-byte copies).
+// moe_combine: residual[t, :] += the sum over t's choices of y[pos] (choices in order, so the order of the additions is fixed).
 #include "common.cuh"
 
 using namespace iert;
@@ -21,8 +26,8 @@ namespace {
 
 constexpr int MAX_TOP = 32;
 
-__global__ void router_topk_kernel(const float* __restrict__ z, long long ldz, const float* __restrict__ bias,
-                                   int E, int top, float* __restrict__ wt, int* __restrict__ idx,
+__global__ void router_topk_kernel(const float* __restrict__ z, long long ldz, long long lde, const float* __restrict__ bias,
+                                   int E, int top, float* __restrict__ wt, int ldw, int* __restrict__ idx,
                                    float* __restrict__ w) {
   // one warp per token
   pdl_launch_dependents();     // the next kernel may start its preamble now
@@ -37,7 +42,7 @@ __global__ void router_topk_kernel(const float* __restrict__ z, long long ldz, c
     for (int e = lane; e < E; e += 32) {
       bool taken = false;
       for (int j = 0; j < k; ++j) taken |= chosen[j] == e;
-      const float v = row[e] + (bias ? bias[e] : 0.f);
+      const float v = row[e * lde] + (bias ? bias[e] : 0.f);
       if (!taken && (v > best || (v == best && e < bi))) { best = v; bi = e; }
     }
 #pragma unroll
@@ -52,12 +57,12 @@ __global__ void router_topk_kernel(const float* __restrict__ z, long long ldz, c
   float den = 0.f;
   const float largest = val[0];
   for (int k = 0; k < top; ++k) { val[k] = expf(val[k] - largest); den += val[k]; }
-  for (int e = lane; e < E; e += 32) wt[(size_t)t * E + e] = 0.f;
+  for (int e = lane; e < ldw; e += 32) wt[(size_t)t * ldw + e] = e < E ? 0.f : 1.f;      // (what every token uses has weight 1)
   __syncwarp();
   if (lane == 0)
     for (int k = 0; k < top; ++k) {
       const float p = val[k] / den;
-      if (chosen[k] < E) wt[(size_t)t * E + chosen[k]] = p;
+      if (chosen[k] < E) wt[(size_t)t * ldw + chosen[k]] = p;
       idx[(size_t)t * top + k] = chosen[k];
       w[(size_t)t * top + k] = p;
     }
@@ -223,21 +228,14 @@ __global__ void router_grouped_kernel(RouterArgs a, const TX* __restrict__ x, lo
 }
 
 template <typename T>
-__global__ void moe_scale_kernel(T* __restrict__ act, long long ld, const float* __restrict__ wt, int E, int F,
-                                 const float* __restrict__ wid, const T* __restrict__ x, long long ldx,
-                                 float* __restrict__ residual, int H) {
+__global__ void moe_scale_kernel(T* __restrict__ act, long long ld, const float* __restrict__ wt, int ldw, int E, int F) {
   pdl_launch_dependents();     // the down product may fetch its first weights now
   pdl_wait();
   const int t = blockIdx.x;
   T* row = act + (size_t)t * ld;
-  if (wid) {
-    const float a = wid[t];
-    if (a != 0.f)
-      for (int i = threadIdx.x; i < H; i += blockDim.x) residual[(size_t)t * H + i] += a * to_f32(x[(size_t)t * ldx + i]);
-  }
   if (sizeof(T) == 2 && F % 8 == 0 && ld % 8 == 0 && ((uintptr_t)act & 15) == 0) {      // eight at a time
     for (int i = threadIdx.x * 8; i < E * F; i += blockDim.x * 8) {
-      const float w = wt[(size_t)t * E + i / F];
+      const float w = wt[(size_t)t * ldw + i / F];
       uint4 v = *reinterpret_cast<const uint4*>(row + i);
       __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&v);
 #pragma unroll
@@ -250,16 +248,149 @@ __global__ void moe_scale_kernel(T* __restrict__ act, long long ld, const float*
     return;
   }
   for (int i = threadIdx.x; i < E * F; i += blockDim.x)
-    row[i] = from_f32<T>(to_f32(row[i]) * wt[(size_t)t * E + i / F]);
+    row[i] = from_f32<T>(to_f32(row[i]) * wt[(size_t)t * ldw + i / F]);
+}
+
+constexpr int SORT_THREADS = 1024, ROW_TILE = 128;
+
+__global__ void __launch_bounds__(SORT_THREADS)
+moe_sort_kernel(const int* __restrict__ idx, const float* __restrict__ w, int pairs, int top, int E, int* __restrict__ groups,
+                int* __restrict__ pos, int* __restrict__ row_token, float* __restrict__ row_w) {
+  extern __shared__ int sm_sort[];
+  int* count = sm_sort;                  // [E]
+  int* next = sm_sort + E;               // [E] the expert's next free row
+  int* tile0 = sm_sort + 2 * E;          // [E] its first row tile
+  pdl_launch_dependents();
+  for (int e = threadIdx.x; e < E; e += SORT_THREADS) count[e] = 0;
+  __syncthreads();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int rounds = (pairs + SORT_THREADS - 1) / SORT_THREADS;
+  auto expert_of = [&](int i) {
+    const int e = i < pairs ? idx[i] : -1;
+    return e >= 0 && e < E ? e : -1;     // experts without tensors, and choices that could not be made, have no rows
+  };
+  for (int r = 0; r < rounds; ++r) {
+    const int e = expert_of(r * SORT_THREADS + threadIdx.x);
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    if (e >= 0 && lane == __ffs(same) - 1) atomicAdd(&count[e], __popc(same));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int rows = 0, tiles = 0;
+    for (int e = 0; e < E; ++e) {
+      next[e] = rows;
+      tile0[e] = tiles;
+      rows += count[e];
+      tiles += (count[e] + ROW_TILE - 1) / ROW_TILE;
+    }
+    groups[0] = tiles;
+    groups[1] = rows;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += SORT_THREADS)
+    for (int t = 0; t * ROW_TILE < count[e]; ++t) {
+      int* g = groups + 2 + 3 * (tile0[e] + t);
+      g[0] = e;
+      g[1] = next[e] + t * ROW_TILE;
+      g[2] = next[e] + count[e];
+    }
+  __syncthreads();
+  for (int r = 0; r < rounds; ++r) {
+    const int i = r * SORT_THREADS + threadIdx.x;
+    const int e = expert_of(i);
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    int row = 0;
+    if (e >= 0 && lane == __ffs(same) - 1) row = atomicAdd(&next[e], __popc(same));
+    row = __shfl_sync(0xffffffffu, row, __ffs(same) - 1) + __popc(same & ((1u << lane) - 1u));
+    if (i < pairs) pos[i] = e >= 0 ? row : -1;
+    if (e >= 0) { row_token[row] = i / top; row_w[row] = w[i]; }
+  }
+}
+
+__global__ void __launch_bounds__(256) moe_gather_kernel(const uint4* __restrict__ x, long long ldx16, const int* __restrict__ groups,
+                                                         const int* __restrict__ row_token, uint4* __restrict__ xs, int width16) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int row = blockIdx.x;
+  if (row >= groups[1]) return;
+  const uint4* src = x + (size_t)row_token[row] * ldx16;
+  uint4* dst = xs + (size_t)row * width16;
+  for (int i = threadIdx.x; i < width16; i += 4 * 256) {
+    uint4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) if (i + k * 256 < width16) v[k] = src[i + k * 256];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) if (i + k * 256 < width16) dst[i + k * 256] = v[k];
+  }
+}
+
+__global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ pos, const float* __restrict__ w,
+                                                          int top, float* __restrict__ residual, int H) {
+  __shared__ int pos_s[MAX_TOP];
+  __shared__ float w_s[MAX_TOP];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x;
+  if (threadIdx.x < top) {
+    pos_s[threadIdx.x] = pos[(size_t)t * top + threadIdx.x];
+    w_s[threadIdx.x] = w[(size_t)t * top + threadIdx.x];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x * 4; i < H; i += 256 * 4) {
+    float4* out = reinterpret_cast<float4*>(residual + (size_t)t * H + i);
+    float4 o = *out, a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < top; ++k) {
+      if (pos_s[k] < 0) {                // no rows: an expert without tensors, or no choice for want of a number
+        const float n = w_s[k] != w_s[k] ? w_s[k] : 0.f;
+        a.x += n; a.y += n; a.z += n; a.w += n;
+        continue;
+      }
+      const float4 v = *reinterpret_cast<const float4*>(y + (size_t)pos_s[k] * H + i);
+      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+    }
+    o.x += a.x; o.y += a.y; o.z += a.z; o.w += a.w;
+    *out = o;
+  }
 }
 
 }  // namespace
 
-IERT_API int iert_router_topk(const float* z, long long ldz, const float* bias, int n_tokens, int E, int top,
-                              float* wt, int* idx, float* w, cudaStream_t stream) {
+// idx, w [n_tokens, top] as the routers leave them.  groups: [2 + 3 * (n_tokens * top / 128 + E)] ints; pos [n_tokens * top];
+// row_token, row_w [n_tokens * top].
+IERT_API int iert_moe_sort(const int* idx, const float* w, int n_tokens, int top, int E, int* groups, int* pos, int* row_token,
+                           float* row_w, cudaStream_t stream) {
   if (n_tokens <= 0) return IERT_OK;
-  if (E <= 0 || top <= 0 || top > E || top > MAX_TOP) return IERT_BAD_ARGUMENT;
-  launch_dep(router_topk_kernel, dim3(n_tokens), dim3(32), 0, stream, z, ldz, bias, E, top, wt, idx, w);
+  if (top <= 0 || E <= 0 || E > 1024 || (long long)n_tokens * top > (1 << 24)) return IERT_BAD_ARGUMENT;
+  launch_dep(moe_sort_kernel, dim3(1), dim3(SORT_THREADS), 3 * E * sizeof(int), stream, idx, w, n_tokens * top, top, E, groups, pos,
+             row_token, row_w);
+  return iert_check_launch("moe_sort");
+}
+
+// x [*, width] bf16 with row stride ldx, xs [rows, width] bf16 (width and ldx multiples of 8, rows on 16-byte boundaries).
+IERT_API int iert_moe_gather(const void* x, long long ldx, const int* groups, const int* row_token, int max_rows, void* xs, int width,
+                             cudaStream_t stream) {
+  if (max_rows <= 0) return IERT_OK;
+  if (width <= 0 || width % 8 || ldx % 8 || (((uintptr_t)x | (uintptr_t)xs) & 15)) return IERT_BAD_ARGUMENT;
+  launch_dep(moe_gather_kernel, dim3(max_rows), dim3(256), 0, stream, (const uint4*)x, ldx / 8, groups, row_token, (uint4*)xs, width / 8);
+  return iert_check_launch("moe_gather");
+}
+
+// y fp32 [rows, H]; residual fp32 [n_tokens, H].
+IERT_API int iert_moe_combine(const float* y, const int* pos, const float* w, int n_tokens, int top, float* residual, int H,
+                              cudaStream_t stream) {
+  if (n_tokens <= 0) return IERT_OK;
+  if (top <= 0 || top > MAX_TOP || H <= 0 || H % 4 || (((uintptr_t)y | (uintptr_t)residual) & 15)) return IERT_BAD_ARGUMENT;
+  launch_dep(moe_combine_kernel, dim3(n_tokens), dim3(256), 0, stream, y, pos, w, top, residual, H);
+  return iert_check_launch("moe_combine");
+}
+
+// z: output e of token t at z[t * ldz + e * lde]; wt: row stride ldw >= E, columns from E on are set to 1.
+IERT_API int iert_router_topk(const float* z, long long ldz, long long lde, const float* bias, int n_tokens, int E, int top,
+                              float* wt, int ldw, int* idx, float* w, cudaStream_t stream) {
+  if (n_tokens <= 0) return IERT_OK;
+  if (E <= 0 || top <= 0 || top > E || top > MAX_TOP || ldw < E) return IERT_BAD_ARGUMENT;
+  launch_dep(router_topk_kernel, dim3(n_tokens), dim3(32), 0, stream, z, ldz, lde, bias, E, top, wt, ldw, idx, w);
   return iert_check_launch("router_topk");
 }
 
@@ -287,18 +418,13 @@ IERT_API int iert_router_grouped(const float* z, long long ldz, long long lde, c
   return iert_check_launch("router_grouped");
 }
 
-// wid (optional, fp32 [T]) with x ([T, H], stride ldx, the activations' dtype) and residual (fp32 [T, H]): the share of
-// experts that return their input.
-IERT_API int iert_moe_scale(void* act, int dtype, long long ld, const float* wt, int n_tokens, int E, int F, const float* wid,
-                            const void* x, long long ldx, float* residual, int H, cudaStream_t stream) {
+IERT_API int iert_moe_scale(void* act, int dtype, long long ld, const float* wt, int ldw, int n_tokens, int E, int F, cudaStream_t stream) {
   if (n_tokens <= 0) return IERT_OK;
-  if (E < 0 || F <= 0 || (wid && (!x || !residual || H <= 0))) return IERT_BAD_ARGUMENT;
+  if (E < 0 || F <= 0 || ldw < E) return IERT_BAD_ARGUMENT;
   if (dtype == IERT_F32)
-    launch_dep(moe_scale_kernel<float>, dim3(n_tokens), dim3(256), 0, stream, (float*)act, ld, wt, E, F, wid, (const float*)x, ldx,
-               residual, H);
+    launch_dep(moe_scale_kernel<float>, dim3(n_tokens), dim3(256), 0, stream, (float*)act, ld, wt, ldw, E, F);
   else if (dtype == IERT_BF16)
-    launch_dep(moe_scale_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(256), 0, stream, (__nv_bfloat16*)act, ld, wt, E, F, wid,
-               (const __nv_bfloat16*)x, ldx, residual, H);
+    launch_dep(moe_scale_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(256), 0, stream, (__nv_bfloat16*)act, ld, wt, ldw, E, F);
   else return IERT_BAD_ARGUMENT;
   return iert_check_launch("moe_scale");
 }

@@ -75,9 +75,10 @@ def apply(linear, x, out, n_rows: int, mode: int, stream: int, ctx=None, epilogu
                      epilogue=epilogue)
 
 
-def apply_gated(linear, x, act, n_rows: int, stream: int, fn=None) -> bool:
+def apply_gated(linear, x, act, n_rows: int, stream: int, fn=None, epilogue=None) -> bool:
     """act = silu(x . Wgate^T) * (x . Wup^T) (or another activation of the gated family: `fn`, a
-    `bindings.GatedAct`) in one kernel, for a row-concatenated [gate; up] weight.  False means the caller runs product and activation separately.  An `x`
+    `bindings.GatedAct`) in one kernel, for a row-concatenated [gate; up] weight; `epilogue`: a factor per token and block of
+    columns.  False means the caller runs product and activation separately.  An `x`
     that is the first half of a norm (`ScaledRows`) is taken by the one-token form only."""
     from .norm import ScaledRows
     if linear.weight.dtype != torch.bfloat16 or act.dtype != torch.bfloat16:
@@ -92,8 +93,10 @@ def apply_gated(linear, x, act, n_rows: int, stream: int, fn=None) -> bool:
         if n_rows > GATED_MAX_DECODE_ROWS or -(-(linear.weight.shape[0] // 2) // 64) < B.sm_count():
             return False
         if scaled is not None:
+            if epilogue is not None:
+                return False
             return B.gemm_tc_gated_scaled(scaled.scaled, linear.weight, act, n_rows, scaled.row_scale(), linear.rt.err, stream,
                                           fn=fn)
     elif scaled is not None:
         return False
-    return B.gemm_tc_gated(x, linear.weight, act, n_rows, linear.rt.err, stream, fn=fn)
+    return B.gemm_tc_gated(x, linear.weight, act, n_rows, linear.rt.err, stream, fn=fn, epilogue=epilogue)

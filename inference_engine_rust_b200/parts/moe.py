@@ -10,7 +10,9 @@ Run as two products over all experts at once: the experts' gate and up matrices 
 outputs and the shared one and adds them to the residual.  The products are the same projection kernels
 the dense feed-forward uses, the step stays free of host decisions (CUDA graphs), and the result does
 not depend on what else is in the batch; the price is that every expert's product is computed for every
-token.
+token.  One-token steps and short prompts pay it gladly (all experts' weights are read anyway); longer prompts sort
+their (token, choice) pairs by expert on the device and run each expert's products over its own rows alone
+(`_forward_grouped`), the sums of a token's choices being added to the residual in order.
 
 `GroupedMoE` (kind "grouped_moe") is the same with another router and another expert: scores are the softmax over ALL
 router outputs, the choice is made on score + a stored `correction`, restricted to the `keep` best of `groups` equal
@@ -42,6 +44,12 @@ from .linear import Linear
 # Prompts of more than this many tokens compute a grouped router's logits (at most 32 outputs) with the kernel for few
 # rows against a long matrix, the tokens being the matrix.
 SKINNY_ROUTER_MIN_TOKENS = 32
+# Prompts of at least this many tokens run the experts' products over the tokens that chose them, if that is less than half of
+# the rows that all experts over all tokens would have.  (16 experts at 7B sizes, grouped against all experts, two chosen and a
+# shared one: 256 tokens 149 / 122 us, 384: 143 / 161, 2,048: 273 / 520; four chosen: 384: 129 / 184, 2,048: 324 / 526.)
+GROUPED_MIN_TOKENS = 384
+# ... in portions of this many tokens, which bounds the sorted rows and their results in memory.
+GROUPED_MAX_TOKENS = 8192
 
 
 class MoE(FeedForward):
@@ -86,25 +94,80 @@ class MoE(FeedForward):
     def weight_bytes(self) -> int:
         return self.gate_up.nbytes() + self.down.nbytes() + self.router.nbytes()
 
-    def _route(self, xn, ctx: StepContext):
-        """(wt [T, E] dense routing weights, wid [T] or None: the share of experts that return their input)."""
-        ws, T, E = self.rt.workspace, ctx.n_tokens, self.experts
-        z = ws.take("moe.logits", (T, E), torch.float32)
-        self.router.apply(xn, z, T, ctx.stream)
-        wt = ws.take("moe.weights", (T, E), torch.float32)
+    def _router_logits(self, xn, N: int, T: int, stream: int):
+        """The fp32 product of the step's rows with the router's N rows, and whether it lies by output ([N, T]) or by token."""
+        ws = self.rt.workspace
+        by_output = False
+        if (self.rt.fast and T > SKINNY_ROUTER_MIN_TOKENS and N <= 32 and isinstance(xn, torch.Tensor)
+                and xn.dtype == torch.bfloat16 and self.router.weight.dtype == torch.bfloat16):
+            # A prompt: few router outputs against many tokens.  A token tile of the tensor-core product would carry
+            # N columns and 128-token tiles alone leave most of the device idle; the kernel for few rows against a long
+            # matrix takes the router's rows as its "tokens" and the tokens as the matrix it streams, 16 tokens per
+            # CTA, and leaves the logits with a row per router output.
+            z = ws.take("moe.logits_by_output", (N, T), torch.float32)
+            # the streamed "matrix" is the step's rows, which the norm in front has just written
+            by_output = B.gemm_rows(self.router.weight, xn[:T], z, N, B.GEMM_STORE, self.rt.err, stream, w_dynamic=True)
+        if not by_output:
+            z = ws.take("moe.logits", (T, N), torch.float32)
+            self.router.apply(xn, z, T, stream)
+        return z, by_output
+
+    def _route(self, xn, residual, T: int, stream: int):
+        """(wt [T, E or more] dense routing weights, idx, w [T, top] the choices); the share of experts that return their
+        input is added to `residual`."""
+        ws, E = self.rt.workspace, self.experts
+        z, by_output = self._router_logits(xn, E, T, stream)
+        wt = ws.take("moe.weights", (T, E + (1 if self.shared_ff else 0)), torch.float32)
         idx = ws.take("moe.chosen", (T, self.top), torch.int32)
         w = ws.take("moe.chosen_weights", (T, self.top), torch.float32)
-        B.router_topk(z, self.router_bias, T, E, self.top, wt, idx, w, ctx.stream)
-        return wt, None
+        B.router_topk(z, self.router_bias, T, E, self.top, wt, idx, w, stream, by_output=by_output)
+        return wt, idx, w
+
+    def _takes_grouped(self, xn, T: int) -> bool:
+        E, F, H = self.experts, self.expert_ff, self.hidden_size
+        return (self.rt.fast and T >= GROUPED_MIN_TOKENS and T * E >= 2 * (T * self.top + 64 * E) and E <= 1024
+                and isinstance(xn, torch.Tensor) and xn.dtype == torch.bfloat16 and xn.stride(0) % 8 == 0
+                and xn.data_ptr() % 16 == 0 and F % 64 == 0 and H % 8 == 0 and self.shared_ff % 8 == 0)
+
+    def _forward_grouped(self, xn, residual, T: int, stream: int) -> None:
+        """One portion of a prompt: the choices sorted by expert, each expert's products over its own rows, the shared expert
+        over all rows, then a token's results added to its residual."""
+        rt, ws, E, F, H, top, S = self.rt, self.rt.workspace, self.experts, self.expert_ff, self.hidden_size, self.top, self.shared_ff
+        _, idx, w = self._route(xn, residual, T, stream)
+        rows, tiles = T * top, T * top // 128 + E
+        groups = ws.take("moe.groups", (B.moe_group_ints(T, top, E),), torch.int32)
+        pos = ws.take("moe.pos", (rows,), torch.int32)
+        row_token = ws.take("moe.row_token", (rows,), torch.int32)
+        row_w = ws.take("moe.row_weight", (rows,), torch.float32)
+        B.moe_sort(idx, w, T, top, E, groups, pos, row_token, row_w, stream)
+        xs = ws.take("moe.rows", (rows, H), torch.bfloat16)
+        B.moe_gather(xn, groups, row_token, rows, xs, stream)
+        act = ws.take("moe.act", (rows, F), torch.bfloat16)
+        B.gemm_tc_grouped_gated(xs, self.gate_up.weight, act, groups, tiles, E, F, self.inter, row_w, rt.err, stream, fn=self.act)
+        y = ws.take("moe.results", (rows, H), torch.float32)
+        B.gemm_tc_grouped(act, self.down.weight, y, groups, tiles, E, F, rt.err, stream)
+        if S:
+            act_s = ws.take("ffn.act", (T, S), torch.bfloat16)
+            if not (B.gemm_tc_gated(xn, self.gate_up.weight[E * F:], act_s, T, rt.err, stream, fn=self.act, inter=S, up_rows=self.inter)
+                    and B.gemm_tc(act_s, self.down.weight[:, E * F:], residual, T, B.GEMM_ADD_RESIDUAL, rt.err, stream)):
+                raise B.KernelError("grouped experts: the shared expert's products were refused")
+        B.moe_combine(y, pos, w, T, top, residual, stream)
 
     def forward(self, xn, residual, ctx: StepContext) -> None:
         rt, ws, T, I, E = self.rt, self.rt.workspace, ctx.n_tokens, self.inter, self.experts
-        wt, wid = self._route(xn, ctx)
+        if self._takes_grouped(xn, T):
+            for t in range(0, T, GROUPED_MAX_TOKENS):
+                n = min(GROUPED_MAX_TOKENS, T - t)
+                self._forward_grouped(xn[t:t + n], residual[t:t + n], n, ctx.stream)
+            return
+        wt, _, _ = self._route(xn, residual, T, ctx.stream)
         act = ws.take("ffn.act", (T, I), rt.dtype)
         done = False
         if rt.fast:
             from . import fast_linear
-            done = fast_linear.apply_gated(self.gate_up, xn, act, T, ctx.stream, fn=self.act)
+            # every block of columns times its expert's weight, in the product's own kernel
+            factor = B.epilogue(scale=wt, blocks=wt.shape[1] - 1, block_cols=self.expert_ff)
+            done = fast_linear.apply_gated(self.gate_up, xn, act, T, ctx.stream, fn=self.act, epilogue=factor)
         if not done:
             gu = ws.take("ffn.gate_up", (T, 2 * I), rt.dtype)
             self.gate_up.apply(xn, gu, T, ctx.stream)
@@ -112,10 +175,7 @@ class MoE(FeedForward):
                 B.silu_mul(gu, act, T, I, ctx.stream)
             else:
                 B.gated_act_mul(gu, act, T, I, self.act, ctx.stream)
-        if wid is None:
             B.moe_scale(act, wt, T, E, self.expert_ff, ctx.stream)
-        else:
-            B.moe_scale(act, wt, T, E, self.expert_ff, ctx.stream, wid=wid, x=xn, residual=residual)
         self.down.apply(act, residual, T, ctx.stream, add_residual=True, ctx=ctx)
 
 
@@ -157,35 +217,17 @@ class GroupedMoE(MoE):
         self._load_experts(tensors)
         self.correction = tensors["correction"].to(torch.float32).contiguous()
 
-    def _route(self, xn, ctx: StepContext):
-        ws, T, E, N = self.rt.workspace, ctx.n_tokens, self.experts, self.outputs
+    def _route(self, xn, residual, T: int, stream: int):
+        ws, E, N = self.rt.workspace, self.experts, self.outputs
         wt = ws.take("moe.weights", (T, E), torch.float32)
         wid = ws.take("moe.identity_share", (T,), torch.float32)
         idx = ws.take("moe.chosen", (T, self.top), torch.int32)
         w = ws.take("moe.chosen_weights", (T, self.top), torch.float32)
-        z, by_output = self._router_logits(xn, N, ctx)
-        B.router_grouped(z, self.correction, T, E, N, self.top, self.groups, self.keep, wt, wid, idx, w, ctx.stream,
+        z, by_output = self._router_logits(xn, N, T, stream)
+        B.router_grouped(z, self.correction, T, E, N, self.top, self.groups, self.keep, wt, wid, idx, w, stream,
                          by_output=by_output, score=self.score, group_score=self.group_score, weight_eps=self.weight_eps,
-                         weight_scale=self.weight_scale)
-        return wt, (wid if self.identity else None)
-
-    def _router_logits(self, xn, N: int, ctx: StepContext):
-        """The fp32 product of the step's rows with the router's N rows, and whether it lies by output ([N, T]) or by token."""
-        ws, T = self.rt.workspace, ctx.n_tokens
-        by_output = False
-        if (self.rt.fast and T > SKINNY_ROUTER_MIN_TOKENS and N <= 32 and isinstance(xn, torch.Tensor)
-                and xn.dtype == torch.bfloat16 and self.router.weight.dtype == torch.bfloat16):
-            # A prompt: few router outputs against many tokens.  A token tile of the tensor-core product would carry
-            # N columns and 128-token tiles alone leave most of the device idle; the kernel for few rows against a long
-            # matrix takes the router's rows as its "tokens" and the tokens as the matrix it streams, 16 tokens per
-            # CTA, and leaves the logits with a row per router output.
-            z = ws.take("moe.logits_by_output", (N, T), torch.float32)
-            # the streamed "matrix" is the step's rows, which the norm in front has just written
-            by_output = B.gemm_rows(self.router.weight, xn[:T], z, N, B.GEMM_STORE, self.rt.err, ctx.stream, w_dynamic=True)
-        if not by_output:
-            z = ws.take("moe.logits", (T, N), torch.float32)
-            self.router.apply(xn, z, T, ctx.stream)
-        return z, by_output
+                         weight_scale=self.weight_scale, x=xn if self.identity else None, residual=residual if self.identity else None)
+        return wt, idx, w
 
 
 class UngatedMoE(GroupedMoE):
@@ -225,7 +267,7 @@ class UngatedMoE(GroupedMoE):
 
     def forward(self, xn, residual, ctx: StepContext) -> None:
         rt, ws, T, E = self.rt, self.rt.workspace, ctx.n_tokens, self.experts
-        z, by_output = self._router_logits(xn, self.router_rows, ctx)
+        z, by_output = self._router_logits(xn, self.router_rows, T, ctx.stream)
         wt = ws.take("moe.weights", (T, self.wt_cols), torch.float32)
         wid = ws.take("moe.identity_share", (T,), torch.float32)
         idx = ws.take("moe.chosen", (T, self.top), torch.int32)

@@ -1,0 +1,117 @@
+"""Experts' products over the tokens that chose them: the sort of the choices, and the feed-forward against 64-bit arithmetic at
+the edges of its row tiles (experts without a token, with one, with a tile and one more), for every router and with portions."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("T,top,E", [(1, 1, 1), (256, 2, 5), (257, 3, 16), (1000, 1, 300), (4096, 2, 16)])
+def test_sort(T, top, E):
+    from inference_engine_rust_b200.csrc import bindings as B
+    g = torch.Generator().manual_seed(T)
+    idx = torch.randint(-1, E + 2, (T, top), generator=g, dtype=torch.int32)        # -1 and E, E + 1: no rows
+    idx[T // 2:] = E // 2                                                            # one expert takes half of the tokens
+    w = torch.rand(T, top, generator=g)
+    groups = torch.full((B.moe_group_ints(T, top, E),), -7, dtype=torch.int32, device=DEV)
+    pos, row_token = (torch.full((T * top,), -9, dtype=torch.int32, device=DEV) for _ in range(2))
+    row_w = torch.zeros(T * top, device=DEV)
+    B.moe_sort(idx.to(DEV), w.to(DEV), T, top, E, groups, pos, row_token, row_w, B.stream_ptr())
+    groups, pos, row_token, row_w = groups.tolist(), pos.view(T, top).cpu(), row_token.cpu(), row_w.cpu()
+    valid = (idx >= 0) & (idx < E)
+    assert (pos[~valid] == -1).all() and groups[1] == int(valid.sum())
+    assert sorted(pos[valid].tolist()) == list(range(groups[1]))
+    t_of = torch.arange(T)[:, None].expand(T, top)
+    assert (row_token[pos[valid].long()] == t_of[valid]).all() and (row_w[pos[valid].long()] == w[valid]).all()
+    expert_of_row = torch.empty(groups[1], dtype=torch.int32)
+    expert_of_row[pos[valid].long()] = idx[valid]
+    covered = 0
+    for i in range(groups[0]):
+        e, first, end = groups[2 + 3 * i:5 + 3 * i]
+        last = min(first + 128, end)
+        assert first == covered and last > first and (expert_of_row[first:last] == e).all()
+        assert end == groups[1] or expert_of_row[end] != e
+        covered = last
+    assert covered == groups[1]
+
+
+def part_of(kind, E, top, ff, shared, identity, hidden):
+    from inference_engine_rust_b200.config.specs import PartSpec
+    from inference_engine_rust_b200.parts import Runtime, part_class
+    rt = Runtime(dtype=torch.bfloat16, device=DEV)
+    p = {"hidden_size": hidden, "experts": E, "top": top, "expert_ff": ff}
+    if kind == "moe":
+        p["shared_ff"] = shared
+    else:
+        p.update(identity=identity, groups=1, keep=1, score="softmax", activation="gelu_tanh")
+    part = part_class("ffn", kind)(PartSpec(kind, p), rt)
+    g = torch.Generator(device=DEV).manual_seed(E + top)
+    w = {n: (torch.randn(s.shape, generator=g, device=DEV) * 0.1).to(torch.bfloat16) for n, s in part.tensor_specs().items()}
+    part.load(dict(w))
+    return part, w
+
+
+def exact(kind, part, w, x):
+    x = x.double()
+    z = x @ w["router"].double().t()
+    act = F.silu if kind == "moe" else lambda v: F.gelu(v, approximate="tanh")
+    if kind == "moe":
+        val, idx = torch.topk(z + w["router.b"].double(), part.top)
+        wt = torch.softmax(val, -1)
+    else:
+        s = torch.softmax(z, -1)
+        idx = torch.topk(s + w["correction"].double(), part.top).indices
+        wt = torch.gather(s, 1, idx)
+        wt = wt / wt.sum(-1, keepdim=True)
+    out = torch.zeros_like(x)
+
+    def ff(v, n):
+        return (act(v @ w[n + ".gate"].double().t()) * (v @ w[n + ".up"].double().t())) @ w[n + ".down"].double().t()
+    for e in range(z.shape[1]):
+        t, j = torch.nonzero(idx == e, as_tuple=True)
+        if t.numel():
+            out[t] += wt[t, j, None] * (ff(x[t], f"e{e}") if e < part.experts else x[t])
+    return out + ff(x, "shared") if "shared.gate" in w else out
+
+
+@pytest.mark.parametrize("kind,E,top,ff,shared,identity", [("moe", 8, 2, 64, 96, 0), ("moe", 40, 3, 192, 0, 0), ("moe", 9, 1, 128, 200, 0),
+                                                           ("grouped_moe", 12, 2, 64, 0, 0), ("grouped_moe", 13, 2, 192, 0, 3)])
+@pytest.mark.parametrize("T", [256, 385, 1030])
+def test_against_64_bits(monkeypatch, kind, E, top, ff, shared, identity, T):
+    from inference_engine_rust_b200.parts import StepContext, moe
+    part, w = part_of(kind, E, top, ff, shared, identity, 136)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randn((T, 136), generator=g, device=DEV).to(torch.bfloat16)
+    x[: T // 2] = x[0]                                # one choice takes half of the tokens, some take few or none
+    ctx = StepContext(kind="prompt", batch=None, n_tokens=T, n_seqs=1, q_lens=[T], pos0=[0], slots=[0],
+                      stream=torch.cuda.current_stream().cuda_stream, rt=part.rt)
+    base = torch.randn((T, 136), generator=g, device=DEV)
+    want = base + exact(kind, part, w, x)
+    got = {}
+    for name, least, most in (("grouped", 1, 8192), ("portions", 1, 256), ("all experts", 1 << 30, 8192)):
+        monkeypatch.setattr(moe, "GROUPED_MIN_TOKENS", least)
+        monkeypatch.setattr(moe, "GROUPED_MAX_TOKENS", most)
+        assert part._takes_grouped(x, T) == (least == 1)
+        got[name] = base.clone()
+        part.forward(x, got[name], ctx)
+        torch.cuda.synchronize()
+        assert part.rt.err.item() == 0
+        # bf16 weights and inputs are exact here; an activation is rounded once, by at most 2^-9 of itself
+        assert (got[name] - want).norm() <= 2.0 ** -8 * (want - base).norm(), name
+    if T % 256 == 0:
+        assert torch.equal(got["grouped"], got["portions"])
+
+
+def test_a_row_that_is_no_number_stays_one():
+    from inference_engine_rust_b200.parts import StepContext
+    part, w = part_of("moe", 8, 2, 64, 96, 0, 136)
+    x = torch.randn((400, 136), device=DEV).to(torch.bfloat16)
+    x[7] = float("nan")
+    out = torch.zeros((400, 136), device=DEV)
+    ctx = StepContext(kind="prompt", batch=None, n_tokens=400, n_seqs=1, q_lens=[400], pos0=[0], slots=[0],
+                      stream=torch.cuda.current_stream().cuda_stream, rt=part.rt)
+    assert part._takes_grouped(x, 400)
+    part.forward(x, out, ctx)
+    assert torch.isnan(out[7]).all() and torch.isfinite(out[:7]).all() and torch.isfinite(out[8:]).all()
