@@ -168,6 +168,213 @@ __global__ void __launch_bounds__(256 + LOADERS) delta_recur_kernel(DeltaArgs a,
   }
 }
 
+// ---- prompts: eight tokens at a time ---------------------------------------------------------------------------------
+// Token after token, a step's time is the latency of its chain (dot product, shuffles, update: about 680 cycles a token), not its
+// work.  Over a chunk of c = 8 tokens with decays g and G_i = g_1 .. g_i, the state in front of the chunk S and u_i as above:
+//
+//   S_i = G_i S + sum_{j <= i} (G_i / G_j) k_j u_j      so      u_i = beta_i (v_i - G_i k_i.S - sum_{j < i} (G_i / G_j) (k_i.k_j) u_j)
+//   o_i = G_i q_i.S + sum_{j <= i} (G_i / G_j) (q_i.k_j) u_j
+//
+// The sixteen dot products k_i.S, q_i.S of a column are independent: all their partial sums are formed first and then added
+// over the 16 lanes of the column together, each lane ending with one of them (15 shuffles instead of 64); what is left of
+// the chain is eight steps of one broadcast and one multiply-add, with the tokens' products k_i.k_j, q_i.k_j (the same for all
+// columns) and the ratios (products of the decays between, never quotients) prepared by the loader warps a chunk ahead.  Everything
+// is fp32; the sums of a token's terms run in another order than token after token, no longer ones.
+// A thread owns DIM / 16 rows of FOUR columns, so that a token's k and q, read from shared memory, serve four columns.
+#define IERT_CHUNKED (DIM == 64 || DIM == 128)                // (larger sizes would not fit the registers)
+#if IERT_CHUNKED
+constexpr int CT = 8, CG = 4, CL = 16, CWORK = 128, CCOLS = CWORK / CL * CG, CLOAD = 64;
+constexpr int CR = DIM / CL, CPAD = DIM + 4;                 // rows per lane; row stride in shared memory
+
+// Sum over the 16 lanes of a column of 2 * HALF values per column: the lanes whose bit MASK is set keep the upper half.
+template <int HALF, int MASK>
+__device__ __forceinline__ void halve(float (&v)[16][CG], bool upper) {
+#pragma unroll
+  for (int m = 0; m < HALF; ++m)
+#pragma unroll
+    for (int c = 0; c < CG; ++c) {
+      const float send = upper ? v[m][c] : v[m + HALF][c], keep = upper ? v[m + HALF][c] : v[m][c];
+      v[m][c] = keep + __shfl_xor_sync(0xffffffffu, send, MASK);
+    }
+}
+
+__global__ void __launch_bounds__(CWORK + CLOAD) delta_chunk_kernel(DeltaArgs a, IertBatchView b) {
+  __shared__ __align__(16) float k_s[3][CT][CPAD], q_s[3][CT][CPAD], v_s[3][CT][CCOLS], bg_s[3][CT][2];
+  __shared__ __align__(16) float coef_s[2][2 * CT][CT];       // row i: of u_i; row 8 + i: of o_i
+  __shared__ float scale_s[2][3][CT];                          // G_i, G_8 / G_i, beta_i
+  pdl_wait();
+  const int s = blockIdx.x, head = blockIdx.y, c0 = blockIdx.z * CCOLS;
+  const int slot = b.slot_ids[s];
+  const int t0 = b.cu_q[s], t1 = b.cu_q[s + 1];
+  if (slot < 0 || t1 <= t0) return;
+  const int n_chunks = (t1 - t0 + CT - 1) / CT;
+  const int g = head / (a.H / a.G), GD = a.G * DIM, C = 2 * GD + a.H * a.V;
+  float* Sg = a.state + (size_t)slot * a.state_stride + a.s_off + (size_t)head * DIM * a.V;
+
+  if (threadIdx.x >= CWORK) {
+    // ---------------- loaders ----------------
+    const int tid = threadIdx.x - CWORK;
+    constexpr int ROW4 = DIM / 4, KQ = CT * ROW4 / CLOAD;       // float4 of a row; of k (and q) per thread
+    float4 kr[KQ], qr[KQ], vr;
+    float br, gr;
+    auto ask = [&](int n) {                                      // a token beyond the sequence: zeros, decay 1
+      const int tc = t0 + n * CT;
+#pragma unroll
+      for (int i = 0; i < KQ; ++i) {
+        const int x = tid + i * CLOAD, tt = x / ROW4, d = 4 * (x % ROW4);
+        const bool in = tc + tt < t1;
+        const float* row = a.qkv + (size_t)(in ? tc + tt : t0) * C + g * DIM + d;
+        qr[i] = in ? *reinterpret_cast<const float4*>(row) : make_float4(0.f, 0.f, 0.f, 0.f);
+        kr[i] = in ? *reinterpret_cast<const float4*>(row + GD) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      const int tt = tid / (CCOLS / 4), col = c0 + 4 * (tid % (CCOLS / 4));
+      const bool in = tc + tt < t1 && col < a.V;
+      vr = in ? *reinterpret_cast<const float4*>(a.qkv + (size_t)(tc + tt) * C + 2 * GD + head * a.V + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (tid < CT) {
+        const bool live = tc + tid < t1;
+        br = live ? a.beta[(size_t)(tc + tid) * a.H + head] : 0.f;
+        gr = live ? a.decay[(size_t)(tc + tid) * a.H + head] : 1.f;
+      }
+    };
+    auto put = [&](int buf) {
+#pragma unroll
+      for (int i = 0; i < KQ; ++i) {
+        const int x = tid + i * CLOAD, tt = x / ROW4, d = 4 * (x % ROW4);
+        *reinterpret_cast<float4*>(&q_s[buf][tt][d]) = qr[i];
+        *reinterpret_cast<float4*>(&k_s[buf][tt][d]) = kr[i];
+      }
+      *reinterpret_cast<float4*>(&v_s[buf][tid / (CCOLS / 4)][4 * (tid % (CCOLS / 4))]) = vr;
+      if (tid < CT) { bg_s[buf][tid][0] = br; bg_s[buf][tid][1] = gr; }
+    };
+    // this thread's pair of tokens: rows 1 .. 7 of u (j < i), then rows 0 .. 7 of o (j <= i)
+    int pi = 0, pj = 0;
+    const bool of_o = tid >= 28;
+    for (int x = 0, i = 0; i < CT; ++i)
+      for (int j = 0; j < i + (of_o ? 1 : 0); ++j, ++x)
+        if (x == tid - (of_o ? 28 : 0)) { pi = i; pj = j; }
+    auto prepare = [&](int n, int buf) {                         // the coefficients of chunk n
+      const float* x = of_o ? q_s[buf][pi] : k_s[buf][pi];
+      const float* y = k_s[buf][pj];
+      float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
+#pragma unroll 8
+      for (int d = 0; d < DIM; d += 4) {
+        const float4 u = *reinterpret_cast<const float4*>(x + d), v = *reinterpret_cast<const float4*>(y + d);
+        d0 = fmaf(u.x, v.x, d0); d1 = fmaf(u.y, v.y, d1); d2 = fmaf(u.z, v.z, d2); d3 = fmaf(u.w, v.w, d3);
+      }
+      float ratio = 1.f;
+      for (int m = pj + 1; m <= pi; ++m) ratio *= bg_s[buf][m][1];
+      const float dot = ((d0 + d1) + (d2 + d3)) * ratio;
+      coef_s[n & 1][(of_o ? CT : 0) + pi][pj] = of_o ? dot : -bg_s[buf][pi][0] * dot;
+      if (tid < CT) {
+        float to = 1.f, from = 1.f;
+        for (int m = 0; m <= tid; ++m) to *= bg_s[buf][m][1];
+        for (int m = tid + 1; m < CT; ++m) from *= bg_s[buf][m][1];
+        scale_s[n & 1][0][tid] = to;
+        scale_s[n & 1][1][tid] = from;
+        scale_s[n & 1][2][tid] = bg_s[buf][tid][0];
+      }
+    };
+    ask(0);
+    put(0);
+    if (n_chunks > 1) { ask(1); put(1); }
+    asm volatile("bar.sync 1, %0;" ::"n"(CLOAD) : "memory");
+    prepare(0, 0);
+    __syncthreads();
+    for (int n = 0; n < n_chunks; ++n) {
+      const bool more = n + 2 < n_chunks;
+      if (more) ask(n + 2);
+      if (n + 1 < n_chunks) prepare(n + 1, (n + 1) % 3);
+      if (more) put((n + 2) % 3);
+      __syncthreads();
+    }
+    return;
+  }
+
+  // ---------------- workers: lane r of a column's 16 owns rows 64 x + 4 r .. + 3 ----------------
+  const int r = threadIdx.x % CL, grp = threadIdx.x / CL, j0 = c0 + grp * CG;
+  const bool live = j0 < a.V;
+  const int i_own = r & (CT - 1), limit = r < CT ? r : i_own + 1;
+  float S[CR][CG];
+#pragma unroll
+  for (int i = 0; i < CR; ++i) {
+    const int d = (i / 4) * 64 + 4 * r + i % 4;
+    const float4 v = live ? *reinterpret_cast<const float4*>(Sg + (size_t)d * a.V + j0) : make_float4(0.f, 0.f, 0.f, 0.f);
+    S[i][0] = v.x; S[i][1] = v.y; S[i][2] = v.z; S[i][3] = v.w;
+  }
+  __syncthreads();
+  for (int n = 0; n < n_chunks; ++n) {
+    const int buf = n % 3;
+    float kk[CT][CR], v[16][CG];
+#pragma unroll
+    for (int t = 0; t < CT; ++t) {
+#pragma unroll
+      for (int x = 0; x < CR / 4; ++x) {
+        const float4 f = *reinterpret_cast<const float4*>(&k_s[buf][t][64 * x + 4 * r]);
+        kk[t][4 * x] = f.x; kk[t][4 * x + 1] = f.y; kk[t][4 * x + 2] = f.z; kk[t][4 * x + 3] = f.w;
+      }
+      float qq[CR];
+#pragma unroll
+      for (int x = 0; x < CR / 4; ++x) {
+        const float4 f = *reinterpret_cast<const float4*>(&q_s[buf][t][64 * x + 4 * r]);
+        qq[4 * x] = f.x; qq[4 * x + 1] = f.y; qq[4 * x + 2] = f.z; qq[4 * x + 3] = f.w;
+      }
+#pragma unroll
+      for (int c = 0; c < CG; ++c) {
+        float dk = 0.f, dq = 0.f;
+#pragma unroll
+        for (int i = 0; i < CR; ++i) { dk = fmaf(S[i][c], kk[t][i], dk); dq = fmaf(S[i][c], qq[i], dq); }
+        v[t][c] = dk;
+        v[CT + t][c] = dq;
+      }
+    }
+    halve<8, 8>(v, r & 8);
+    halve<4, 4>(v, r & 4);
+    halve<2, 2>(v, r & 2);
+    halve<1, 1>(v, r & 1);               // lane r: k_r.S (r < 8) or q_(r - 8).S of the four columns
+    const float G = scale_s[n & 1][0][i_own], beta = scale_s[n & 1][2][i_own];
+    const float4 vt = *reinterpret_cast<const float4*>(&v_s[buf][i_own][grp * CG]);
+    const float vv[CG] = {vt.x, vt.y, vt.z, vt.w};
+    float co[CT], x[CG], u[CT][CG];
+    *reinterpret_cast<float4*>(co) = *reinterpret_cast<const float4*>(&coef_s[n & 1][r][0]);
+    *reinterpret_cast<float4*>(co + 4) = *reinterpret_cast<const float4*>(&coef_s[n & 1][r][4]);
+#pragma unroll
+    for (int c = 0; c < CG; ++c) x[c] = r < CT ? beta * (vv[c] - G * v[0][c]) : G * v[0][c];
+#pragma unroll
+    for (int j = 0; j < CT; ++j)
+#pragma unroll
+      for (int c = 0; c < CG; ++c) {
+        u[j][c] = __shfl_sync(0xffffffffu, x[c], j, CL);
+        if (j < limit) x[c] = fmaf(co[j], u[j][c], x[c]);
+      }
+    if (live && r >= CT && t0 + n * CT + i_own < t1)
+      *reinterpret_cast<float4*>(a.o + (size_t)(t0 + n * CT + i_own) * a.H * a.V + (size_t)head * a.V + j0) = make_float4(x[0], x[1], x[2], x[3]);
+    const float G8 = scale_s[n & 1][0][CT - 1];
+#pragma unroll
+    for (int i = 0; i < CR; ++i)
+#pragma unroll
+      for (int c = 0; c < CG; ++c) S[i][c] *= G8;
+#pragma unroll
+    for (int j = 0; j < CT; ++j) {
+      const float f = scale_s[n & 1][1][j];
+#pragma unroll
+      for (int c = 0; c < CG; ++c) {
+        const float uw = f * u[j][c];
+#pragma unroll
+        for (int i = 0; i < CR; ++i) S[i][c] = fmaf(kk[j][i], uw, S[i][c]);
+      }
+    }
+    __syncthreads();
+  }
+  if (live) {
+#pragma unroll
+    for (int i = 0; i < CR; ++i) {
+      const int d = (i / 4) * 64 + 4 * r + i % 4;
+      *reinterpret_cast<float4*>(Sg + (size_t)d * a.V + j0) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+    }
+  }
+}
+#endif
+
 struct MlstmArgs {
   const void* proj;      // [T, ld] run dtype: q [H*DIM] | k [H*DIM] | v [H*V] | ...
   long long ld;
@@ -509,9 +716,203 @@ __global__ void __launch_bounds__(256 + LOADERS) wkv_recur_kernel(WkvArgs a, Ier
   }
 }
 
+#if IERT_CHUNKED
+// Prompts, eight tokens at a time, as for the delta rule above.  With W_i = w_1 .. w_i (per row of S) the state in front of the
+// chunk S gives
+//   o_i = (W_(i-1) r_i).S + sum_{j < i} (sum_d r_i k_j w_(j+1) .. w_(i-1)) v_j + (r_i.(u k_i)) v_i
+//   S  <- W_8 S + sum_j (w_(j+1) .. w_8 k_j) v_j^T
+// There is no chain inside a chunk at all.  A loader thread per row of S forms the rows scaled by the decays and its share of
+// the 36 products of two tokens (decays multiplied, never divided), which are then added over the rows.
+constexpr int WLOAD = DIM;
+
+__global__ void __launch_bounds__(CWORK + WLOAD) wkv_chunk_kernel(WkvArgs a, IertBatchView b) {
+  __shared__ __align__(16) float rt_s[2][CT][DIM], kt_s[2][CT][DIM], v_s[2][CT][CCOLS], wc_s[2][DIM], p_s[2][CT][CT];
+  __shared__ float sum_s[WLOAD / 32][36];
+  pdl_wait();
+  const int s = blockIdx.x, head = blockIdx.y, c0 = blockIdx.z * CCOLS;
+  const int slot = b.slot_ids[s];
+  const int t0 = b.cu_q[s], t1 = b.cu_q[s + 1];
+  if (slot < 0 || t1 <= t0) return;
+  const int n_chunks = (t1 - t0 + CT - 1) / CT, HD = a.H * DIM;
+  float* Sg = a.state + (size_t)slot * a.state_stride + a.s_off + (size_t)head * DIM * a.V;
+
+  if (threadIdx.x >= CWORK) {
+    // ---------------- loaders: thread d looks after row d ----------------
+    const int d = threadIdx.x - CWORK, lane = d & 31;
+    const float bonus = a.u[head * DIM + d];
+    struct Raw { float r[CT], k[CT], w[CT]; float4 v; };
+    auto ask = [&](int n, Raw& x) {                              // a token beyond the sequence: zeros, decay 1
+      const int tc = t0 + n * CT;
+#pragma unroll
+      for (int t = 0; t < CT; ++t) {
+        const bool in = tc + t < t1;
+        const size_t tok = in ? tc + t : t0;
+        const float* row = a.x + tok * a.ld + head * DIM + d;
+        x.r[t] = in ? row[0] : 0.f;
+        x.k[t] = in ? row[HD] : 0.f;
+        x.w[t] = in ? a.decay[tok * HD + head * DIM + d] : 1.f;
+      }
+      const int tt = d / (CCOLS / 4), col = c0 + 4 * (d % (CCOLS / 4));
+      x.v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (tt < CT && tc + tt < t1 && col < a.V)
+        x.v = *reinterpret_cast<const float4*>(a.x + (size_t)(tc + tt) * a.ld + 2 * HD + head * a.V + col);
+    };
+    auto put = [&](int n, const Raw& x) {
+      const int buf = n & 1;
+      float pw = 1.f;
+#pragma unroll
+      for (int t = 0; t < CT; ++t) { rt_s[buf][t][d] = x.r[t] * pw; pw *= x.w[t]; }
+      wc_s[buf][d] = pw;
+      float sw = 1.f;
+#pragma unroll
+      for (int t = CT - 1; t >= 0; --t) { kt_s[buf][t][d] = x.k[t] * sw; sw *= x.w[t]; }
+      if (d < CT * CCOLS / 4) *reinterpret_cast<float4*>(&v_s[buf][d / (CCOLS / 4)][4 * (d % (CCOLS / 4))]) = x.v;
+      float p[36];                                               // pair (i, j <= i) at i (i + 1) / 2 + j
+#pragma unroll
+      for (int j = 0; j < CT; ++j) {
+        p[j * (j + 1) / 2 + j] = x.r[j] * (bonus * x.k[j]);
+        float e = x.k[j];
+#pragma unroll
+        for (int i = j + 1; i < CT; ++i) {
+          p[i * (i + 1) / 2 + j] = x.r[i] * e;
+          e *= x.w[i];
+        }
+      }
+      // over the warp's rows: 32 of the sums spread over the lanes, the other four by full butterflies
+#pragma unroll
+      for (int half = 16; half > 0; half >>= 1) {
+        const bool upper = lane & half;
+#pragma unroll
+        for (int m = 0; m < half; ++m) {
+          const float send = upper ? p[m] : p[m + half], keep = upper ? p[m + half] : p[m];
+          p[m] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+        }
+      }
+#pragma unroll
+      for (int m = 32; m < 36; ++m) p[m] = warp_sum(p[m]);
+      sum_s[d / 32][lane] = p[0];
+      if (lane < 4) sum_s[d / 32][32 + lane] = lane == 0 ? p[32] : lane == 1 ? p[33] : lane == 2 ? p[34] : p[35];
+      asm volatile("bar.sync 1, %0;" ::"n"(WLOAD) : "memory");
+      if (d < 36) {
+        float t = sum_s[0][d];
+#pragma unroll
+        for (int x2 = 1; x2 < WLOAD / 32; ++x2) t += sum_s[x2][d];
+        int i = 0;
+        while ((i + 1) * (i + 2) / 2 <= d) ++i;
+        p_s[buf][i][d - i * (i + 1) / 2] = t;
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(WLOAD) : "memory");
+    };
+    Raw cur, nxt;
+    ask(0, cur);
+    if (n_chunks > 1) ask(1, nxt);
+    put(0, cur);
+    __syncthreads();
+    for (int n = 0; n < n_chunks; ++n) {
+      cur = nxt;
+      if (n + 2 < n_chunks) ask(n + 2, nxt);
+      if (n + 1 < n_chunks) put(n + 1, cur);
+      __syncthreads();
+    }
+    return;
+  }
+
+  // ---------------- workers: lane r of a column's 16 owns rows 64 x + 4 r .. + 3 ----------------
+  const int r = threadIdx.x % CL, grp = threadIdx.x / CL, j0 = c0 + grp * CG;
+  const bool live = j0 < a.V;
+  const int i_own = r >> 1, col2 = 2 * (r & 1);      // the token and the two columns whose read-out this lane ends with
+  float S[CR][CG];
+#pragma unroll
+  for (int i = 0; i < CR; ++i) {
+    const int d = (i / 4) * 64 + 4 * r + i % 4;
+    const float4 v = live ? *reinterpret_cast<const float4*>(Sg + (size_t)d * a.V + j0) : make_float4(0.f, 0.f, 0.f, 0.f);
+    S[i][0] = v.x; S[i][1] = v.y; S[i][2] = v.z; S[i][3] = v.w;
+  }
+  __syncthreads();
+  for (int n = 0; n < n_chunks; ++n) {
+    const int buf = n & 1;
+    float v[16][CG];                                  // [8] used
+#pragma unroll
+    for (int t = 0; t < CT; ++t) {
+      float rr[CR];
+#pragma unroll
+      for (int x = 0; x < CR / 4; ++x) {
+        const float4 f = *reinterpret_cast<const float4*>(&rt_s[buf][t][64 * x + 4 * r]);
+        rr[4 * x] = f.x; rr[4 * x + 1] = f.y; rr[4 * x + 2] = f.z; rr[4 * x + 3] = f.w;
+      }
+#pragma unroll
+      for (int c = 0; c < CG; ++c) {
+        float o = 0.f;
+#pragma unroll
+        for (int i = 0; i < CR; ++i) o = fmaf(S[i][c], rr[i], o);
+        v[t][c] = o;
+      }
+    }
+    halve<4, 8>(v, r & 8);
+    halve<2, 4>(v, r & 4);
+    halve<1, 2>(v, r & 2);
+    const bool odd = r & 1;
+    float o[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const float send = odd ? v[0][c] : v[0][c + 2], keep = odd ? v[0][c + 2] : v[0][c];
+      o[c] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+    }
+    float pr[CT];
+    *reinterpret_cast<float4*>(pr) = *reinterpret_cast<const float4*>(&p_s[buf][i_own][0]);
+    *reinterpret_cast<float4*>(pr + 4) = *reinterpret_cast<const float4*>(&p_s[buf][i_own][4]);
+#pragma unroll
+    for (int i = 0; i < CR; i += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(&wc_s[buf][(i / 4) * 64 + 4 * r]);
+#pragma unroll
+      for (int c = 0; c < CG; ++c) { S[i][c] *= f.x; S[i + 1][c] *= f.y; S[i + 2][c] *= f.z; S[i + 3][c] *= f.w; }
+    }
+#pragma unroll
+    for (int j = 0; j < CT; ++j) {
+      const float4 f = *reinterpret_cast<const float4*>(&v_s[buf][j][grp * CG]);
+      const float vv[CG] = {f.x, f.y, f.z, f.w};
+      if (j <= i_own) {
+        o[0] = fmaf(pr[j], odd ? vv[2] : vv[0], o[0]);
+        o[1] = fmaf(pr[j], odd ? vv[3] : vv[1], o[1]);
+      }
+#pragma unroll
+      for (int i = 0; i < CR; i += 4) {
+        const float4 kt = *reinterpret_cast<const float4*>(&kt_s[buf][j][(i / 4) * 64 + 4 * r]);
+#pragma unroll
+        for (int c = 0; c < CG; ++c) {
+          S[i][c] = fmaf(kt.x, vv[c], S[i][c]);
+          S[i + 1][c] = fmaf(kt.y, vv[c], S[i + 1][c]);
+          S[i + 2][c] = fmaf(kt.z, vv[c], S[i + 2][c]);
+          S[i + 3][c] = fmaf(kt.w, vv[c], S[i + 3][c]);
+        }
+      }
+    }
+    if (live && t0 + n * CT + i_own < t1)
+      *reinterpret_cast<float2*>(a.o + (size_t)(t0 + n * CT + i_own) * a.H * a.V + (size_t)head * a.V + j0 + col2) = make_float2(o[0], o[1]);
+    __syncthreads();
+  }
+  if (live) {
+#pragma unroll
+    for (int i = 0; i < CR; ++i) {
+      const int d = (i / 4) * 64 + 4 * r + i % 4;
+      *reinterpret_cast<float4*>(Sg + (size_t)d * a.V + j0) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+    }
+  }
+}
+#endif
+
 // Lanes per column: the fewest that give the device about eight warps per SM (at most 32), and columns per
 // CTA so that a CTA has up to 256 computing threads.  (Measured at 32 heads of 128 x 128, one prompt of 2,048
 // tokens: 8 lanes per column 1.08 ms, 16 lanes 0.91 ms, 32 lanes 1.42 ms per layer.)
+#if IERT_CHUNKED
+// Prompts go eight tokens at a time; a step of one token (or about as few) per sequence token after token: a chunk costs what
+// eight tokens cost, and such a step is bound by reading and writing the state.
+bool chunked(const IertBatchView* b) {
+  const char* off = getenv("IERT_RECURRENT_LANES");                  // (a forced number of lanes asks for the other kernels)
+  return !(off && atoi(off) >= 1) && b->n_tokens >= 4 * b->n_seqs;
+}
+#endif
+
 struct Split { int lanes, cols; };
 Split pick_split(int n_seqs, int H, int V) {
   const long long want = 8LL * 32 * iert_sm_count_cached();          // threads
@@ -545,6 +946,14 @@ IERT_API int iert_delta_recur(const float* qkv, const float* beta, const float* 
                               const IertBatchView* batch, cudaStream_t stream) {
   if (batch->n_seqs <= 0 || batch->n_tokens <= 0) return IERT_OK;
   if (G <= 0 || H <= 0 || H % G || V <= 0 || H > 65535) return IERT_BAD_ARGUMENT;
+#if IERT_CHUNKED
+  if (chunked(batch) && V % 4 == 0 && (2 * G * DIM + H * V) % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
+      (((uintptr_t)qkv | (uintptr_t)state | (uintptr_t)o) & 15) == 0) {
+    DeltaArgs a = {qkv, beta, decay, state, state_stride, s_off, o, G, H, V, CCOLS};
+    launch_dep(delta_chunk_kernel, dim3(batch->n_seqs, H, (V + CCOLS - 1) / CCOLS), dim3(CWORK + CLOAD), 0, stream, a, *batch);
+    return iert_check_launch("delta_recur");
+  }
+#endif
   const Split sp = pick_split(batch->n_seqs, H, V);
   DeltaArgs a = {qkv, beta, decay, state, state_stride, s_off, o, G, H, V, sp.cols};
   dim3 grid(batch->n_seqs, H, (V + sp.cols - 1) / sp.cols);
@@ -559,6 +968,14 @@ IERT_API int iert_wkv_recur(const float* x, long long ld, const float* decay, co
                             cudaStream_t stream) {
   if (batch->n_seqs <= 0 || batch->n_tokens <= 0) return IERT_OK;
   if (H <= 0 || V <= 0 || H > 65535 || ld < (long long)2 * H * DIM + (long long)H * V) return IERT_BAD_ARGUMENT;
+#if IERT_CHUNKED
+  if (chunked(batch) && V % 4 == 0 && ld % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
+      (((uintptr_t)x | (uintptr_t)state | (uintptr_t)o) & 15) == 0) {
+    WkvArgs a = {x, ld, decay, u, state, state_stride, s_off, o, H, V, CCOLS};
+    launch_dep(wkv_chunk_kernel, dim3(batch->n_seqs, H, (V + CCOLS - 1) / CCOLS), dim3(CWORK + WLOAD), 0, stream, a, *batch);
+    return iert_check_launch("wkv_recur");
+  }
+#endif
   const Split sp = pick_split(batch->n_seqs, H, V);
   WkvArgs a = {x, ld, decay, u, state, state_stride, s_off, o, H, V, sp.cols};
   dim3 grid(batch->n_seqs, H, (V + sp.cols - 1) / sp.cols);
