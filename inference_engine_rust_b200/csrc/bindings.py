@@ -706,12 +706,14 @@ def _recurrent_lib(dim: int):
     if lib is None:
         lib = build.load_library(*build.recurrent_library(dim))
         P, LL = c_void_p, c_longlong
-        lib.iert_delta_recur.argtypes = [P, P, P, P, LL, LL, P, c_int, c_int, c_int, POINTER(BatchView), P]
+        lib.iert_delta_recur.argtypes = [P, P, P, P, LL, LL, P, P, c_int, c_int, c_int, POINTER(BatchView), P]
         lib.iert_delta_recur.restype = c_int
         lib.iert_mlstm_recur.argtypes = [P, c_int, LL, P, LL, P, P, c_float, P, LL, LL, LL, LL, P, P, c_int, c_int,
                                          POINTER(BatchView), P]
         lib.iert_mlstm_recur.restype = c_int
-        lib.iert_wkv_recur.argtypes = [P, LL, P, P, P, LL, LL, P, c_int, c_int, POINTER(BatchView), P]
+        lib.iert_recurrent_scratch_floats.argtypes = [c_int, c_int]
+        lib.iert_recurrent_scratch_floats.restype = LL
+        lib.iert_wkv_recur.argtypes = [P, LL, P, P, P, LL, LL, P, P, c_int, c_int, POINTER(BatchView), P]
         lib.iert_wkv_recur.restype = c_int
         if os.environ.get("IERT_PDL", "1") == "0":
             lib.iert_set_pdl(0)
@@ -728,11 +730,17 @@ def _check_lib(status: int, what: str, launches: int = 1) -> None:
     launch_count += launches
 
 
-def delta_recur(qkv, beta, decay, state, s_off: int, o, G: int, D: int, H: int, V: int, batch: BatchView, stream) -> None:
-    """The gated delta rule over the step's tokens, state [slots, floats] read and written at `s_off`."""
+def recurrent_scratch_floats(D: int, n_tokens: int, H: int) -> int:
+    """Scratch that lets `delta_recur` and `wkv_recur` take a prompt several tokens at a time (fp32)."""
+    return _recurrent_lib(D).iert_recurrent_scratch_floats(n_tokens, H)
+
+
+def delta_recur(qkv, beta, decay, state, s_off: int, o, G: int, D: int, H: int, V: int, batch: BatchView, stream, scratch=None) -> None:
+    """The gated delta rule over the step's tokens, state [slots, floats] read and written at `s_off`.  `scratch`
+    (`recurrent_scratch_floats`): prompts may go several tokens at a time."""
     _check_lib(_recurrent_lib(D).iert_delta_recur(qkv.data_ptr(), beta.data_ptr(), decay.data_ptr(), state.data_ptr(),
-                                                  state.stride(0), s_off, o.data_ptr(), G, H, V, byref(batch), stream),
-               "delta_recur")
+                                                  state.stride(0), s_off, o.data_ptr(), _ptr(scratch), G, H, V, byref(batch), stream),
+               "delta_recur", 2 if scratch is not None and batch.n_tokens >= 4 * batch.n_seqs and D in (64, 128) else 1)
 
 
 def mlstm_recur(proj, gates, bi, bf, cap: float, state, s_off: int, n_off: int, m_off: int, coef, o, D: int, H: int, V: int,
@@ -761,11 +769,13 @@ def wkv_decay(z, L: int, w2t, w0, decay, h, state, prev_off: int, batch: BatchVi
                                 prev_off, byref(batch), stream), "wkv_decay")
 
 
-def wkv_recur(x, decay, u, state, s_off: int, o, D: int, H: int, V: int, batch: BatchView, stream) -> None:
+def wkv_recur(x, decay, u, state, s_off: int, o, D: int, H: int, V: int, batch: BatchView, stream, scratch=None) -> None:
     """o_t = (S + diag(u) k_t v_t^T)^T r_t; S <- diag(w_t) S + k_t v_t^T over the step's tokens, from the fp32
-    projections x = [r | k | v | ...] and the decays w; S [H, D, V] per slot in `state` at `s_off`."""
+    projections x = [r | k | v | ...] and the decays w; S [H, D, V] per slot in `state` at `s_off`.  `scratch` as for
+    `delta_recur`."""
     _check_lib(_recurrent_lib(D).iert_wkv_recur(x.data_ptr(), x.stride(0), decay.data_ptr(), u.data_ptr(), state.data_ptr(),
-                                                state.stride(0), s_off, o.data_ptr(), H, V, byref(batch), stream), "wkv_recur")
+                                                state.stride(0), s_off, o.data_ptr(), _ptr(scratch), H, V, byref(batch), stream),
+               "wkv_recur", 2 if scratch is not None and batch.n_tokens >= 4 * batch.n_seqs and D == 64 else 1)
 
 
 def wkv_finish(o, gate, w, eps: float, out_scale: float, out, batch: BatchView, H: int, V: int, stream) -> None:

@@ -177,14 +177,135 @@ __global__ void __launch_bounds__(256 + LOADERS) delta_recur_kernel(DeltaArgs a,
 //
 // The sixteen dot products k_i.S, q_i.S of a column are independent: all their partial sums are formed first and then added
 // over the 16 lanes of the column together, each lane ending with one of them (15 shuffles instead of 64); what is left of
-// the chain is eight steps of one broadcast and one multiply-add, with the tokens' products k_i.k_j, q_i.k_j (the same for all
-// columns) and the ratios (products of the decays between, never quotients) prepared by the loader warps a chunk ahead.  Everything
-// is fp32; the sums of a token's terms run in another order than token after token, no longer ones.
-// A thread owns DIM / 16 rows of FOUR columns, so that a token's k and q, read from shared memory, serve four columns.
+// the chain is eight steps of one broadcast and one multiply-add.  The tokens' products k_i.k_j, q_i.k_j (the same for all
+// columns) with the ratios (products of the decays between, never quotients) come from a kernel in front, which has a block per
+// chunk and key head; a loader warp brings everything through a ring of four chunks.  Everything is fp32.
+// A thread owns DIM / 16 rows of FOUR columns, so that a token's k and q, read from shared memory, serve four columns (with two
+// columns and twice the warps: 448 us against 404 over 2,048 tokens, 32 heads of 128 x 128).  Two rows share an instruction.
 #define IERT_CHUNKED (DIM == 64 || DIM == 128)                // (larger sizes would not fit the registers)
 #if IERT_CHUNKED
-constexpr int CT = 8, CG = 4, CL = 16, CWORK = 128, CCOLS = CWORK / CL * CG, CLOAD = 64;
-constexpr int CR = DIM / CL, CPAD = DIM + 4;                 // rows per lane; row stride in shared memory
+constexpr int CT = 8, CG = 4, CL = 16, CWORK = 128, CCOLS = CWORK / CL * CG;
+constexpr int CP = DIM / CL / 2;                              // pairs of rows per lane
+constexpr int RING = 4;                                       // chunks in shared memory
+// per token and head: 8 coefficients of earlier u in u_i, 8 in o_i, then G_i, G_8 / G_i, beta_i, G_8
+constexpr int COEF = 20;
+
+// Two fp32 numbers side by side: one instruction, each rounded as by fmaf.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
+        "l"(reinterpret_cast<const unsigned long long&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return d;
+}
+// A lane's rows 64 x + 4 r .. + 3 of a vector in shared memory.
+__device__ __forceinline__ void own_rows(float2 (&v)[CP], const float* src, int r) {
+#pragma unroll
+  for (int x = 0; x < CP / 2; ++x) {
+    const float4 f = *reinterpret_cast<const float4*>(src + 64 * x + 4 * r);
+    v[2 * x] = make_float2(f.x, f.y);
+    v[2 * x + 1] = make_float2(f.z, f.w);
+  }
+}
+// The rows 64 x + 4 r .. + 3 of four columns of the state, from memory and back.
+__device__ __forceinline__ void load_rows(float2 (&S)[CP][CG], const float* Sg, int V, int r, bool live) {
+#pragma unroll
+  for (int i = 0; i < CP; ++i) {
+    const float* p = Sg + (size_t)((i / 2) * 64 + 4 * r + (i % 2) * 2) * V;
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 u = live ? *reinterpret_cast<const float4*>(p) : z, v = live ? *reinterpret_cast<const float4*>(p + V) : z;
+    S[i][0] = make_float2(u.x, v.x); S[i][1] = make_float2(u.y, v.y); S[i][2] = make_float2(u.z, v.z); S[i][3] = make_float2(u.w, v.w);
+  }
+}
+__device__ __forceinline__ void store_rows(const float2 (&S)[CP][CG], float* Sg, int V, int r) {
+#pragma unroll
+  for (int i = 0; i < CP; ++i) {
+    float* p = Sg + (size_t)((i / 2) * 64 + 4 * r + (i % 2) * 2) * V;
+    *reinterpret_cast<float4*>(p) = make_float4(S[i][0].x, S[i][1].x, S[i][2].x, S[i][3].x);
+    *reinterpret_cast<float4*>(p + V) = make_float4(S[i][0].y, S[i][1].y, S[i][2].y, S[i][3].y);
+  }
+}
+
+__device__ __forceinline__ void copy16(void* dst, const void* src, bool in) {      // zeros where there is nothing to read
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+// The chunk that block `x` of a grid over all sequences' chunks looks after: first token and end of the sequence; false: none.
+__device__ __forceinline__ bool chunk_of(const IertBatchView& b, int x, int& tc, int& t1) {
+  for (int s = 0; s < b.n_seqs; ++s) {
+    const int lo = b.cu_q[s], hi = b.cu_q[s + 1], n = (hi - lo + CT - 1) / CT;
+    if (x < n) {
+      tc = lo + x * CT;
+      t1 = hi;
+      return b.slot_ids[s] >= 0;
+    }
+    x -= n;
+  }
+  return false;
+}
+
+// Block (chunk, key head): a thread per product of two of the chunk's tokens, then per coefficient of each head that shares them.
+// (No early start for the kernel behind: its blocks want an SM each, and would be packed in pairs beside this kernel's.)
+__global__ void __launch_bounds__(128) delta_coef_kernel(DeltaArgs a, float* __restrict__ coef, IertBatchView b) {
+  __shared__ __align__(16) float k_s[CT][DIM + 4], q_s[CT][DIM + 4];
+  __shared__ float dot_s[2 * CT][CT], g_s[CT], beta_s[CT];
+  pdl_wait();
+  int tc, t1;
+  if (!chunk_of(b, blockIdx.x, tc, t1)) return;
+  const int g = blockIdx.y, GD = a.G * DIM, C = 2 * GD + a.H * a.V, n = min(CT, t1 - tc), rep = a.H / a.G;
+  for (int x = threadIdx.x; x < CT * DIM / 4; x += 128) {
+    const int t = x / (DIM / 4), d = 4 * (x % (DIM / 4));
+    const float* row = a.qkv + (size_t)(tc + min(t, n - 1)) * C + g * DIM + d;
+    *reinterpret_cast<float4*>(&q_s[t][d]) = *reinterpret_cast<const float4*>(row);
+    *reinterpret_cast<float4*>(&k_s[t][d]) = *reinterpret_cast<const float4*>(row + GD);
+  }
+  __syncthreads();
+  const int row = threadIdx.x / CT, j = threadIdx.x % CT, i = row % CT;      // row i of u, or row 8 + i of o
+  const bool used = j < i + (row >= CT ? 1 : 0);
+  if (used) {
+    const float* x = row < CT ? k_s[i] : q_s[i];
+    const float* y = k_s[j];
+    float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
+#pragma unroll 8
+    for (int d = 0; d < DIM; d += 4) {
+      const float4 u = *reinterpret_cast<const float4*>(x + d), v = *reinterpret_cast<const float4*>(y + d);
+      d0 = fmaf(u.x, v.x, d0); d1 = fmaf(u.y, v.y, d1); d2 = fmaf(u.z, v.z, d2); d3 = fmaf(u.w, v.w, d3);
+    }
+    dot_s[row][j] = (d0 + d1) + (d2 + d3);
+  }
+  for (int h = g * rep; h < (g + 1) * rep; ++h) {
+    __syncthreads();
+    if (threadIdx.x < CT) {
+      const bool in = (int)threadIdx.x < n;
+      beta_s[threadIdx.x] = in ? a.beta[(size_t)(tc + threadIdx.x) * a.H + h] : 0.f;
+      g_s[threadIdx.x] = in ? a.decay[(size_t)(tc + threadIdx.x) * a.H + h] : 1.f;
+    }
+    __syncthreads();
+    if (i < n) {
+      float* out = coef + ((size_t)(tc + i) * a.H + h) * COEF;
+      float ratio = 1.f;
+      for (int m = j + 1; m <= i; ++m) ratio *= g_s[m];
+      const float v = used ? dot_s[row][j] * ratio : 0.f;
+      out[(row >= CT ? CT : 0) + j] = row < CT ? -beta_s[i] * v : v;
+      if (row < CT && j < 4) {
+        float to = 1.f, from = 1.f;
+        for (int m = 0; m <= i; ++m) to *= g_s[m];
+        for (int m = i + 1; m < CT; ++m) from *= g_s[m];
+        out[2 * CT + j] = j == 0 ? to : j == 1 ? from : j == 2 ? beta_s[i] : to * from;
+      }
+    }
+  }
+}
 
 // Sum over the 16 lanes of a column of 2 * HALF values per column: the lanes whose bit MASK is set keep the upper half.
 template <int HALF, int MASK>
@@ -198,145 +319,89 @@ __device__ __forceinline__ void halve(float (&v)[16][CG], bool upper) {
     }
 }
 
-__global__ void __launch_bounds__(CWORK + CLOAD) delta_chunk_kernel(DeltaArgs a, IertBatchView b) {
-  __shared__ __align__(16) float k_s[3][CT][CPAD], q_s[3][CT][CPAD], v_s[3][CT][CCOLS], bg_s[3][CT][2];
-  __shared__ __align__(16) float coef_s[2][2 * CT][CT];       // row i: of u_i; row 8 + i: of o_i
-  __shared__ float scale_s[2][3][CT];                          // G_i, G_8 / G_i, beta_i
+__global__ void __launch_bounds__(CWORK + 32) delta_chunk_kernel(DeltaArgs a, const float* __restrict__ coef, IertBatchView b) {
+  __shared__ __align__(16) float k_s[RING][CT][DIM], q_s[RING][CT][DIM], v_s[RING][CT][CCOLS], c_s[RING][CT][COEF];
   pdl_wait();
   const int s = blockIdx.x, head = blockIdx.y, c0 = blockIdx.z * CCOLS;
   const int slot = b.slot_ids[s];
   const int t0 = b.cu_q[s], t1 = b.cu_q[s + 1];
   if (slot < 0 || t1 <= t0) return;
   const int n_chunks = (t1 - t0 + CT - 1) / CT;
-  const int g = head / (a.H / a.G), GD = a.G * DIM, C = 2 * GD + a.H * a.V;
-  float* Sg = a.state + (size_t)slot * a.state_stride + a.s_off + (size_t)head * DIM * a.V;
 
   if (threadIdx.x >= CWORK) {
-    // ---------------- loaders ----------------
-    const int tid = threadIdx.x - CWORK;
-    constexpr int ROW4 = DIM / 4, KQ = CT * ROW4 / CLOAD;       // float4 of a row; of k (and q) per thread
-    float4 kr[KQ], qr[KQ], vr;
-    float br, gr;
-    auto ask = [&](int n) {                                      // a token beyond the sequence: zeros, decay 1
-      const int tc = t0 + n * CT;
+    // ---------------- loader: one warp, three chunks ahead ----------------
+    const int lane = threadIdx.x - CWORK, g = head / (a.H / a.G), GD = a.G * DIM, C = 2 * GD + a.H * a.V;
+    auto ask = [&](int n) {
+      if (n < n_chunks) {
+        const int tc = t0 + n * CT, buf = n % RING;
 #pragma unroll
-      for (int i = 0; i < KQ; ++i) {
-        const int x = tid + i * CLOAD, tt = x / ROW4, d = 4 * (x % ROW4);
-        const bool in = tc + tt < t1;
-        const float* row = a.qkv + (size_t)(in ? tc + tt : t0) * C + g * DIM + d;
-        qr[i] = in ? *reinterpret_cast<const float4*>(row) : make_float4(0.f, 0.f, 0.f, 0.f);
-        kr[i] = in ? *reinterpret_cast<const float4*>(row + GD) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int t = 0; t < CT; ++t) {
+          const bool in = tc + t < t1;
+          const size_t tok = in ? tc + t : t0;
+          const float* row = a.qkv + tok * C;
+          if (lane < DIM / 4) {
+            copy16(&q_s[buf][t][4 * lane], row + g * DIM + 4 * lane, in);
+            copy16(&k_s[buf][t][4 * lane], row + GD + g * DIM + 4 * lane, in);
+          }
+          if (lane < CCOLS / 4) {
+            const bool col = c0 + 4 * lane < a.V;
+            copy16(&v_s[buf][t][4 * lane], row + 2 * GD + (col ? head * a.V + c0 + 4 * lane : 0), in && col);
+          } else if (lane < CCOLS / 4 + COEF / 4) {
+            const int x = 4 * (lane - CCOLS / 4);
+            copy16(&c_s[buf][t][x], coef + (tok * a.H + head) * COEF + x, in);
+          }
+        }
       }
-      const int tt = tid / (CCOLS / 4), col = c0 + 4 * (tid % (CCOLS / 4));
-      const bool in = tc + tt < t1 && col < a.V;
-      vr = in ? *reinterpret_cast<const float4*>(a.qkv + (size_t)(tc + tt) * C + 2 * GD + head * a.V + col) : make_float4(0.f, 0.f, 0.f, 0.f);
-      if (tid < CT) {
-        const bool live = tc + tid < t1;
-        br = live ? a.beta[(size_t)(tc + tid) * a.H + head] : 0.f;
-        gr = live ? a.decay[(size_t)(tc + tid) * a.H + head] : 1.f;
-      }
+      copies_commit();
     };
-    auto put = [&](int buf) {
-#pragma unroll
-      for (int i = 0; i < KQ; ++i) {
-        const int x = tid + i * CLOAD, tt = x / ROW4, d = 4 * (x % ROW4);
-        *reinterpret_cast<float4*>(&q_s[buf][tt][d]) = qr[i];
-        *reinterpret_cast<float4*>(&k_s[buf][tt][d]) = kr[i];
-      }
-      *reinterpret_cast<float4*>(&v_s[buf][tid / (CCOLS / 4)][4 * (tid % (CCOLS / 4))]) = vr;
-      if (tid < CT) { bg_s[buf][tid][0] = br; bg_s[buf][tid][1] = gr; }
-    };
-    // this thread's pair of tokens: rows 1 .. 7 of u (j < i), then rows 0 .. 7 of o (j <= i)
-    int pi = 0, pj = 0;
-    const bool of_o = tid >= 28;
-    for (int x = 0, i = 0; i < CT; ++i)
-      for (int j = 0; j < i + (of_o ? 1 : 0); ++j, ++x)
-        if (x == tid - (of_o ? 28 : 0)) { pi = i; pj = j; }
-    auto prepare = [&](int n, int buf) {                         // the coefficients of chunk n
-      const float* x = of_o ? q_s[buf][pi] : k_s[buf][pi];
-      const float* y = k_s[buf][pj];
-      float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
-#pragma unroll 8
-      for (int d = 0; d < DIM; d += 4) {
-        const float4 u = *reinterpret_cast<const float4*>(x + d), v = *reinterpret_cast<const float4*>(y + d);
-        d0 = fmaf(u.x, v.x, d0); d1 = fmaf(u.y, v.y, d1); d2 = fmaf(u.z, v.z, d2); d3 = fmaf(u.w, v.w, d3);
-      }
-      float ratio = 1.f;
-      for (int m = pj + 1; m <= pi; ++m) ratio *= bg_s[buf][m][1];
-      const float dot = ((d0 + d1) + (d2 + d3)) * ratio;
-      coef_s[n & 1][(of_o ? CT : 0) + pi][pj] = of_o ? dot : -bg_s[buf][pi][0] * dot;
-      if (tid < CT) {
-        float to = 1.f, from = 1.f;
-        for (int m = 0; m <= tid; ++m) to *= bg_s[buf][m][1];
-        for (int m = tid + 1; m < CT; ++m) from *= bg_s[buf][m][1];
-        scale_s[n & 1][0][tid] = to;
-        scale_s[n & 1][1][tid] = from;
-        scale_s[n & 1][2][tid] = bg_s[buf][tid][0];
-      }
-    };
-    ask(0);
-    put(0);
-    if (n_chunks > 1) { ask(1); put(1); }
-    asm volatile("bar.sync 1, %0;" ::"n"(CLOAD) : "memory");
-    prepare(0, 0);
+    for (int n = 0; n < RING - 1; ++n) ask(n);
+    copies_wait<RING - 2>();
     __syncthreads();
     for (int n = 0; n < n_chunks; ++n) {
-      const bool more = n + 2 < n_chunks;
-      if (more) ask(n + 2);
-      if (n + 1 < n_chunks) prepare(n + 1, (n + 1) % 3);
-      if (more) put((n + 2) % 3);
+      ask(n + RING - 1);                 // its place was read before the last barrier
+      copies_wait<RING - 2>();           // chunk n + 1 has arrived
       __syncthreads();
     }
     return;
   }
 
-  // ---------------- workers: lane r of a column's 16 owns rows 64 x + 4 r .. + 3 ----------------
+  // ---------------- workers ----------------
   const int r = threadIdx.x % CL, grp = threadIdx.x / CL, j0 = c0 + grp * CG;
   const bool live = j0 < a.V;
   const int i_own = r & (CT - 1), limit = r < CT ? r : i_own + 1;
-  float S[CR][CG];
-#pragma unroll
-  for (int i = 0; i < CR; ++i) {
-    const int d = (i / 4) * 64 + 4 * r + i % 4;
-    const float4 v = live ? *reinterpret_cast<const float4*>(Sg + (size_t)d * a.V + j0) : make_float4(0.f, 0.f, 0.f, 0.f);
-    S[i][0] = v.x; S[i][1] = v.y; S[i][2] = v.z; S[i][3] = v.w;
-  }
+  float* Sg = a.state + (size_t)slot * a.state_stride + a.s_off + (size_t)head * DIM * a.V + j0;
+  float2 S[CP][CG];
+  load_rows(S, Sg, a.V, r, live);
   __syncthreads();
   for (int n = 0; n < n_chunks; ++n) {
-    const int buf = n % 3;
-    float kk[CT][CR], v[16][CG];
+    const int buf = n % RING;
+    float2 kk[CT][CP];
+    float v[16][CG];
 #pragma unroll
     for (int t = 0; t < CT; ++t) {
-#pragma unroll
-      for (int x = 0; x < CR / 4; ++x) {
-        const float4 f = *reinterpret_cast<const float4*>(&k_s[buf][t][64 * x + 4 * r]);
-        kk[t][4 * x] = f.x; kk[t][4 * x + 1] = f.y; kk[t][4 * x + 2] = f.z; kk[t][4 * x + 3] = f.w;
-      }
-      float qq[CR];
-#pragma unroll
-      for (int x = 0; x < CR / 4; ++x) {
-        const float4 f = *reinterpret_cast<const float4*>(&q_s[buf][t][64 * x + 4 * r]);
-        qq[4 * x] = f.x; qq[4 * x + 1] = f.y; qq[4 * x + 2] = f.z; qq[4 * x + 3] = f.w;
-      }
+      float2 qq[CP];
+      own_rows(kk[t], k_s[buf][t], r);
+      own_rows(qq, q_s[buf][t], r);
 #pragma unroll
       for (int c = 0; c < CG; ++c) {
-        float dk = 0.f, dq = 0.f;
+        float2 dk = make_float2(0.f, 0.f), dq = dk;
 #pragma unroll
-        for (int i = 0; i < CR; ++i) { dk = fmaf(S[i][c], kk[t][i], dk); dq = fmaf(S[i][c], qq[i], dq); }
-        v[t][c] = dk;
-        v[CT + t][c] = dq;
+        for (int i = 0; i < CP; ++i) { dk = fma2(S[i][c], kk[t][i], dk); dq = fma2(S[i][c], qq[i], dq); }
+        v[t][c] = dk.x + dk.y;
+        v[CT + t][c] = dq.x + dq.y;
       }
     }
     halve<8, 8>(v, r & 8);
     halve<4, 4>(v, r & 4);
     halve<2, 2>(v, r & 2);
     halve<1, 1>(v, r & 1);               // lane r: k_r.S (r < 8) or q_(r - 8).S of the four columns
-    const float G = scale_s[n & 1][0][i_own], beta = scale_s[n & 1][2][i_own];
+    const float4 sc = *reinterpret_cast<const float4*>(&c_s[buf][i_own][2 * CT]);
+    const float G = sc.x, beta = sc.z;
     const float4 vt = *reinterpret_cast<const float4*>(&v_s[buf][i_own][grp * CG]);
     const float vv[CG] = {vt.x, vt.y, vt.z, vt.w};
     float co[CT], x[CG], u[CT][CG];
-    *reinterpret_cast<float4*>(co) = *reinterpret_cast<const float4*>(&coef_s[n & 1][r][0]);
-    *reinterpret_cast<float4*>(co + 4) = *reinterpret_cast<const float4*>(&coef_s[n & 1][r][4]);
+    *reinterpret_cast<float4*>(co) = *reinterpret_cast<const float4*>(&c_s[buf][i_own][r & CT]);
+    *reinterpret_cast<float4*>(co + 4) = *reinterpret_cast<const float4*>(&c_s[buf][i_own][(r & CT) + 4]);
 #pragma unroll
     for (int c = 0; c < CG; ++c) x[c] = r < CT ? beta * (vv[c] - G * v[0][c]) : G * v[0][c];
 #pragma unroll
@@ -348,30 +413,24 @@ __global__ void __launch_bounds__(CWORK + CLOAD) delta_chunk_kernel(DeltaArgs a,
       }
     if (live && r >= CT && t0 + n * CT + i_own < t1)
       *reinterpret_cast<float4*>(a.o + (size_t)(t0 + n * CT + i_own) * a.H * a.V + (size_t)head * a.V + j0) = make_float4(x[0], x[1], x[2], x[3]);
-    const float G8 = scale_s[n & 1][0][CT - 1];
+    const float2 G8 = make_float2(c_s[buf][0][2 * CT + 3], c_s[buf][0][2 * CT + 3]);
 #pragma unroll
-    for (int i = 0; i < CR; ++i)
+    for (int i = 0; i < CP; ++i)
 #pragma unroll
-      for (int c = 0; c < CG; ++c) S[i][c] *= G8;
+      for (int c = 0; c < CG; ++c) S[i][c] = mul2(S[i][c], G8);
 #pragma unroll
     for (int j = 0; j < CT; ++j) {
-      const float f = scale_s[n & 1][1][j];
+      const float f = c_s[buf][j][2 * CT + 1];
 #pragma unroll
       for (int c = 0; c < CG; ++c) {
-        const float uw = f * u[j][c];
+        const float2 uw = make_float2(f * u[j][c], f * u[j][c]);
 #pragma unroll
-        for (int i = 0; i < CR; ++i) S[i][c] = fmaf(kk[j][i], uw, S[i][c]);
+        for (int i = 0; i < CP; ++i) S[i][c] = fma2(kk[j][i], uw, S[i][c]);
       }
     }
     __syncthreads();
   }
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < CR; ++i) {
-      const int d = (i / 4) * 64 + 4 * r + i % 4;
-      *reinterpret_cast<float4*>(Sg + (size_t)d * a.V + j0) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
-    }
-  }
+  if (live) store_rows(S, Sg, a.V, r);
 }
 #endif
 
@@ -716,136 +775,151 @@ __global__ void __launch_bounds__(256 + LOADERS) wkv_recur_kernel(WkvArgs a, Ier
   }
 }
 
-#if IERT_CHUNKED
+#if DIM == 64               // (at 128 the ring would not fit beside the scaled rows in the shared memory that needs no opt-in)
 // Prompts, eight tokens at a time, as for the delta rule above.  With W_i = w_1 .. w_i (per row of S) the state in front of the
 // chunk S gives
 //   o_i = (W_(i-1) r_i).S + sum_{j < i} (sum_d r_i k_j w_(j+1) .. w_(i-1)) v_j + (r_i.(u k_i)) v_i
 //   S  <- W_8 S + sum_j (w_(j+1) .. w_8 k_j) v_j^T
-// There is no chain inside a chunk at all.  A loader thread per row of S forms the rows scaled by the decays and its share of
-// the 36 products of two tokens (decays multiplied, never divided), which are then added over the rows.
+// There is no chain inside a chunk at all.  The products of two tokens (decays multiplied, never divided) come from a kernel in
+// front with a block per chunk and head; here a loader thread per row of S brings the rows through a ring and scales them.
 constexpr int WLOAD = DIM;
 
-__global__ void __launch_bounds__(CWORK + WLOAD) wkv_chunk_kernel(WkvArgs a, IertBatchView b) {
-  __shared__ __align__(16) float rt_s[2][CT][DIM], kt_s[2][CT][DIM], v_s[2][CT][CCOLS], wc_s[2][DIM], p_s[2][CT][CT];
-  __shared__ float sum_s[WLOAD / 32][36];
+// pairs[token][head][8]: row i of the chunk's products with the tokens j <= i.  Thread d: row d's share, then summed over the rows.
+__global__ void __launch_bounds__(DIM) wkv_pairs_kernel(WkvArgs a, float* __restrict__ pairs, IertBatchView b) {
+  __shared__ float sum_s[DIM / 32][36];
+  pdl_wait();                                                    // (no early start for the kernel behind, as above)
+  int tc, t1;
+  if (!chunk_of(b, blockIdx.x, tc, t1)) return;
+  const int head = blockIdx.y, d = threadIdx.x, lane = d & 31, HD = a.H * DIM, n = min(CT, t1 - tc);
+  const float bonus = a.u[head * DIM + d];
+  float r[CT], k[CT], w[CT];
+#pragma unroll
+  for (int t = 0; t < CT; ++t) {
+    const size_t tok = tc + min(t, n - 1);
+    const float* row = a.x + tok * a.ld + head * DIM + d;
+    r[t] = row[0];
+    k[t] = row[HD];
+    w[t] = a.decay[tok * HD + head * DIM + d];
+  }
+  float p[36];                                                   // pair (i, j <= i) at i (i + 1) / 2 + j
+#pragma unroll
+  for (int j = 0; j < CT; ++j) {
+    p[j * (j + 1) / 2 + j] = r[j] * (bonus * k[j]);
+    float e = k[j];
+#pragma unroll
+    for (int i = j + 1; i < CT; ++i) {
+      p[i * (i + 1) / 2 + j] = r[i] * e;
+      e *= w[i];
+    }
+  }
+  // over the warp's rows: 32 of the sums spread over the lanes, the other four by full butterflies
+#pragma unroll
+  for (int half = 16; half > 0; half >>= 1) {
+    const bool upper = lane & half;
+#pragma unroll
+    for (int m = 0; m < half; ++m) {
+      const float send = upper ? p[m] : p[m + half], keep = upper ? p[m + half] : p[m];
+      p[m] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+    }
+  }
+#pragma unroll
+  for (int m = 32; m < 36; ++m) p[m] = warp_sum(p[m]);
+  sum_s[d / 32][lane] = p[0];
+  if (lane < 4) sum_s[d / 32][32 + lane] = lane == 0 ? p[32] : lane == 1 ? p[33] : lane == 2 ? p[34] : p[35];
+  __syncthreads();
+  const int i = d / CT, j = d % CT;                              // (64 threads: one per entry)
+  if (i < n) {
+    float t = 0.f;
+    if (j <= i) {
+      t = sum_s[0][i * (i + 1) / 2 + j];
+#pragma unroll
+      for (int x = 1; x < DIM / 32; ++x) t += sum_s[x][i * (i + 1) / 2 + j];
+    }
+    pairs[((size_t)(tc + i) * a.H + head) * CT + j] = t;
+  }
+}
+
+__global__ void __launch_bounds__(CWORK + WLOAD) wkv_chunk_kernel(WkvArgs a, const float* __restrict__ pairs, IertBatchView b) {
+  __shared__ __align__(16) float raw_s[RING][3][CT][DIM];        // r, k, w as they are in memory
+  __shared__ __align__(16) float v_s[RING][CT][CCOLS], p_s[RING][CT][CT], rt_s[2][CT][DIM], kt_s[2][CT][DIM], wc_s[2][DIM];
   pdl_wait();
   const int s = blockIdx.x, head = blockIdx.y, c0 = blockIdx.z * CCOLS;
   const int slot = b.slot_ids[s];
   const int t0 = b.cu_q[s], t1 = b.cu_q[s + 1];
   if (slot < 0 || t1 <= t0) return;
   const int n_chunks = (t1 - t0 + CT - 1) / CT, HD = a.H * DIM;
-  float* Sg = a.state + (size_t)slot * a.state_stride + a.s_off + (size_t)head * DIM * a.V;
 
   if (threadIdx.x >= CWORK) {
-    // ---------------- loaders: thread d looks after row d ----------------
-    const int d = threadIdx.x - CWORK, lane = d & 31;
-    const float bonus = a.u[head * DIM + d];
-    struct Raw { float r[CT], k[CT], w[CT]; float4 v; };
-    auto ask = [&](int n, Raw& x) {                              // a token beyond the sequence: zeros, decay 1
-      const int tc = t0 + n * CT;
-#pragma unroll
-      for (int t = 0; t < CT; ++t) {
-        const bool in = tc + t < t1;
-        const size_t tok = in ? tc + t : t0;
-        const float* row = a.x + tok * a.ld + head * DIM + d;
-        x.r[t] = in ? row[0] : 0.f;
-        x.k[t] = in ? row[HD] : 0.f;
-        x.w[t] = in ? a.decay[tok * HD + head * DIM + d] : 1.f;
-      }
-      const int tt = d / (CCOLS / 4), col = c0 + 4 * (d % (CCOLS / 4));
-      x.v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (tt < CT && tc + tt < t1 && col < a.V)
-        x.v = *reinterpret_cast<const float4*>(a.x + (size_t)(tc + tt) * a.ld + 2 * HD + head * a.V + col);
-    };
-    auto put = [&](int n, const Raw& x) {
-      const int buf = n & 1;
-      float pw = 1.f;
-#pragma unroll
-      for (int t = 0; t < CT; ++t) { rt_s[buf][t][d] = x.r[t] * pw; pw *= x.w[t]; }
-      wc_s[buf][d] = pw;
-      float sw = 1.f;
-#pragma unroll
-      for (int t = CT - 1; t >= 0; --t) { kt_s[buf][t][d] = x.k[t] * sw; sw *= x.w[t]; }
-      if (d < CT * CCOLS / 4) *reinterpret_cast<float4*>(&v_s[buf][d / (CCOLS / 4)][4 * (d % (CCOLS / 4))]) = x.v;
-      float p[36];                                               // pair (i, j <= i) at i (i + 1) / 2 + j
-#pragma unroll
-      for (int j = 0; j < CT; ++j) {
-        p[j * (j + 1) / 2 + j] = x.r[j] * (bonus * x.k[j]);
-        float e = x.k[j];
-#pragma unroll
-        for (int i = j + 1; i < CT; ++i) {
-          p[i * (i + 1) / 2 + j] = x.r[i] * e;
-          e *= x.w[i];
+    // ---------------- loaders: three chunks ahead; thread d scales row d ----------------
+    const int d = threadIdx.x - CWORK;
+    auto ask = [&](int n) {
+      if (n < n_chunks) {
+        const int tc = t0 + n * CT, buf = n % RING;
+        for (int x = d; x < 3 * CT * DIM / 4; x += WLOAD) {
+          const int which = x / (CT * DIM / 4), t = x / (DIM / 4) % CT, e = 4 * (x % (DIM / 4));
+          const bool in = tc + t < t1;
+          const size_t tok = in ? tc + t : t0;
+          copy16(&raw_s[buf][which][t][e], which < 2 ? a.x + tok * a.ld + which * HD + head * DIM + e : a.decay + tok * HD + head * DIM + e, in);
+        }
+        for (int x = d; x < CT * (CCOLS + CT) / 4; x += WLOAD) {
+          const bool of_v = x < CT * CCOLS / 4;
+          const int y = of_v ? x : x - CT * CCOLS / 4;
+          const int t = of_v ? y / (CCOLS / 4) : y / (CT / 4), e = 4 * (of_v ? y % (CCOLS / 4) : y % (CT / 4));
+          const bool in = tc + t < t1, col = c0 + e < a.V;
+          const size_t tok = in ? tc + t : t0;
+          if (of_v) copy16(&v_s[buf][t][e], a.x + tok * a.ld + 2 * HD + (col ? head * a.V + c0 + e : 0), in && col);
+          else copy16(&p_s[buf][t][e], pairs + (tok * a.H + head) * CT + e, in);
         }
       }
-      // over the warp's rows: 32 of the sums spread over the lanes, the other four by full butterflies
-#pragma unroll
-      for (int half = 16; half > 0; half >>= 1) {
-        const bool upper = lane & half;
-#pragma unroll
-        for (int m = 0; m < half; ++m) {
-          const float send = upper ? p[m] : p[m + half], keep = upper ? p[m + half] : p[m];
-          p[m] = keep + __shfl_xor_sync(0xffffffffu, send, half);
-        }
-      }
-#pragma unroll
-      for (int m = 32; m < 36; ++m) p[m] = warp_sum(p[m]);
-      sum_s[d / 32][lane] = p[0];
-      if (lane < 4) sum_s[d / 32][32 + lane] = lane == 0 ? p[32] : lane == 1 ? p[33] : lane == 2 ? p[34] : p[35];
-      asm volatile("bar.sync 1, %0;" ::"n"(WLOAD) : "memory");
-      if (d < 36) {
-        float t = sum_s[0][d];
-#pragma unroll
-        for (int x2 = 1; x2 < WLOAD / 32; ++x2) t += sum_s[x2][d];
-        int i = 0;
-        while ((i + 1) * (i + 2) / 2 <= d) ++i;
-        p_s[buf][i][d - i * (i + 1) / 2] = t;
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(WLOAD) : "memory");
+      copies_commit();
     };
-    Raw cur, nxt;
-    ask(0, cur);
-    if (n_chunks > 1) ask(1, nxt);
-    put(0, cur);
+    auto scale = [&](int n) {                                    // a token beyond the sequence: zeros, decay 1
+      const int buf = n % RING, out = n & 1, left = t1 - (t0 + n * CT);
+      float w[CT], pw = 1.f, sw = 1.f;
+#pragma unroll
+      for (int t = 0; t < CT; ++t) w[t] = t < left ? raw_s[buf][2][t][d] : 1.f;
+#pragma unroll
+      for (int t = 0; t < CT; ++t) { rt_s[out][t][d] = raw_s[buf][0][t][d] * pw; pw *= w[t]; }
+      wc_s[out][d] = pw;
+#pragma unroll
+      for (int t = CT - 1; t >= 0; --t) { kt_s[out][t][d] = raw_s[buf][1][t][d] * sw; sw *= w[t]; }
+    };
+    for (int n = 0; n < RING - 1; ++n) ask(n);
+    copies_wait<RING - 2>();
+    asm volatile("bar.sync 1, %0;" ::"n"(WLOAD) : "memory");     // every loader's copies of chunk 0
+    scale(0);
     __syncthreads();
     for (int n = 0; n < n_chunks; ++n) {
-      cur = nxt;
-      if (n + 2 < n_chunks) ask(n + 2, nxt);
-      if (n + 1 < n_chunks) put(n + 1, cur);
+      copies_wait<RING - 3>();                                   // chunk n + 1 has arrived ...
+      asm volatile("bar.sync 1, %0;" ::"n"(WLOAD) : "memory");   // ... for all loaders
+      if (n + 1 < n_chunks) scale(n + 1);
+      ask(n + RING - 1);                 // its place: read by the workers before the last barrier, scaled from two chunks ago
       __syncthreads();
     }
     return;
   }
 
-  // ---------------- workers: lane r of a column's 16 owns rows 64 x + 4 r .. + 3 ----------------
+  // ---------------- workers ----------------
   const int r = threadIdx.x % CL, grp = threadIdx.x / CL, j0 = c0 + grp * CG;
   const bool live = j0 < a.V;
   const int i_own = r >> 1, col2 = 2 * (r & 1);      // the token and the two columns whose read-out this lane ends with
-  float S[CR][CG];
-#pragma unroll
-  for (int i = 0; i < CR; ++i) {
-    const int d = (i / 4) * 64 + 4 * r + i % 4;
-    const float4 v = live ? *reinterpret_cast<const float4*>(Sg + (size_t)d * a.V + j0) : make_float4(0.f, 0.f, 0.f, 0.f);
-    S[i][0] = v.x; S[i][1] = v.y; S[i][2] = v.z; S[i][3] = v.w;
-  }
+  float* Sg = a.state + (size_t)slot * a.state_stride + a.s_off + (size_t)head * DIM * a.V + j0;
+  float2 S[CP][CG];
+  load_rows(S, Sg, a.V, r, live);
   __syncthreads();
   for (int n = 0; n < n_chunks; ++n) {
-    const int buf = n & 1;
+    const int buf = n & 1, ring = n % RING;
     float v[16][CG];                                  // [8] used
 #pragma unroll
     for (int t = 0; t < CT; ++t) {
-      float rr[CR];
-#pragma unroll
-      for (int x = 0; x < CR / 4; ++x) {
-        const float4 f = *reinterpret_cast<const float4*>(&rt_s[buf][t][64 * x + 4 * r]);
-        rr[4 * x] = f.x; rr[4 * x + 1] = f.y; rr[4 * x + 2] = f.z; rr[4 * x + 3] = f.w;
-      }
+      float2 rr[CP];
+      own_rows(rr, rt_s[buf][t], r);
 #pragma unroll
       for (int c = 0; c < CG; ++c) {
-        float o = 0.f;
+        float2 o = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int i = 0; i < CR; ++i) o = fmaf(S[i][c], rr[i], o);
-        v[t][c] = o;
+        for (int i = 0; i < CP; ++i) o = fma2(S[i][c], rr[i], o);
+        v[t][c] = o.x + o.y;
       }
     }
     halve<4, 8>(v, r & 8);
@@ -859,45 +933,36 @@ __global__ void __launch_bounds__(CWORK + WLOAD) wkv_chunk_kernel(WkvArgs a, Ier
       o[c] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
     }
     float pr[CT];
-    *reinterpret_cast<float4*>(pr) = *reinterpret_cast<const float4*>(&p_s[buf][i_own][0]);
-    *reinterpret_cast<float4*>(pr + 4) = *reinterpret_cast<const float4*>(&p_s[buf][i_own][4]);
+    *reinterpret_cast<float4*>(pr) = *reinterpret_cast<const float4*>(&p_s[ring][i_own][0]);
+    *reinterpret_cast<float4*>(pr + 4) = *reinterpret_cast<const float4*>(&p_s[ring][i_own][4]);
+    float2 wc[CP];
+    own_rows(wc, wc_s[buf], r);
 #pragma unroll
-    for (int i = 0; i < CR; i += 4) {
-      const float4 f = *reinterpret_cast<const float4*>(&wc_s[buf][(i / 4) * 64 + 4 * r]);
+    for (int i = 0; i < CP; ++i)
 #pragma unroll
-      for (int c = 0; c < CG; ++c) { S[i][c] *= f.x; S[i + 1][c] *= f.y; S[i + 2][c] *= f.z; S[i + 3][c] *= f.w; }
-    }
+      for (int c = 0; c < CG; ++c) S[i][c] = mul2(S[i][c], wc[i]);
 #pragma unroll
     for (int j = 0; j < CT; ++j) {
-      const float4 f = *reinterpret_cast<const float4*>(&v_s[buf][j][grp * CG]);
-      const float vv[CG] = {f.x, f.y, f.z, f.w};
+      const float4 f = *reinterpret_cast<const float4*>(&v_s[ring][j][grp * CG]);
       if (j <= i_own) {
-        o[0] = fmaf(pr[j], odd ? vv[2] : vv[0], o[0]);
-        o[1] = fmaf(pr[j], odd ? vv[3] : vv[1], o[1]);
+        o[0] = fmaf(pr[j], odd ? f.z : f.x, o[0]);
+        o[1] = fmaf(pr[j], odd ? f.w : f.y, o[1]);
       }
+      const float vv[CG] = {f.x, f.y, f.z, f.w};
+      float2 kt[CP];
+      own_rows(kt, kt_s[buf][j], r);
 #pragma unroll
-      for (int i = 0; i < CR; i += 4) {
-        const float4 kt = *reinterpret_cast<const float4*>(&kt_s[buf][j][(i / 4) * 64 + 4 * r]);
+      for (int c = 0; c < CG; ++c) {
+        const float2 v2 = make_float2(vv[c], vv[c]);
 #pragma unroll
-        for (int c = 0; c < CG; ++c) {
-          S[i][c] = fmaf(kt.x, vv[c], S[i][c]);
-          S[i + 1][c] = fmaf(kt.y, vv[c], S[i + 1][c]);
-          S[i + 2][c] = fmaf(kt.z, vv[c], S[i + 2][c]);
-          S[i + 3][c] = fmaf(kt.w, vv[c], S[i + 3][c]);
-        }
+        for (int i = 0; i < CP; ++i) S[i][c] = fma2(kt[i], v2, S[i][c]);
       }
     }
     if (live && t0 + n * CT + i_own < t1)
       *reinterpret_cast<float2*>(a.o + (size_t)(t0 + n * CT + i_own) * a.H * a.V + (size_t)head * a.V + j0 + col2) = make_float2(o[0], o[1]);
     __syncthreads();
   }
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < CR; ++i) {
-      const int d = (i / 4) * 64 + 4 * r + i % 4;
-      *reinterpret_cast<float4*>(Sg + (size_t)d * a.V + j0) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
-    }
-  }
+  if (live) store_rows(S, Sg, a.V, r);
 }
 #endif
 
@@ -941,16 +1006,21 @@ IERT_API int iert_recurrent_dim() { return DIM; }
     default: { constexpr int RR = 32; CALL; } break;                 \
   }
 
+// Scratch (floats) of the recurrences over n_tokens tokens and H heads: the products of tokens with one another.
+IERT_API long long iert_recurrent_scratch_floats(int n_tokens, int H) { return (long long)n_tokens * H * 20; }
+
+// scratch: as many floats as above, or null (then tokens go one after another)
 IERT_API int iert_delta_recur(const float* qkv, const float* beta, const float* decay, float* state,
-                              long long state_stride, long long s_off, float* o, int G, int H, int V,
+                              long long state_stride, long long s_off, float* o, float* scratch, int G, int H, int V,
                               const IertBatchView* batch, cudaStream_t stream) {
   if (batch->n_seqs <= 0 || batch->n_tokens <= 0) return IERT_OK;
   if (G <= 0 || H <= 0 || H % G || V <= 0 || H > 65535) return IERT_BAD_ARGUMENT;
 #if IERT_CHUNKED
-  if (chunked(batch) && V % 4 == 0 && (2 * G * DIM + H * V) % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
-      (((uintptr_t)qkv | (uintptr_t)state | (uintptr_t)o) & 15) == 0) {
+  if (scratch && chunked(batch) && V % 4 == 0 && (2 * G * DIM + H * V) % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
+      (((uintptr_t)qkv | (uintptr_t)state | (uintptr_t)o | (uintptr_t)scratch) & 15) == 0) {
     DeltaArgs a = {qkv, beta, decay, state, state_stride, s_off, o, G, H, V, CCOLS};
-    launch_dep(delta_chunk_kernel, dim3(batch->n_seqs, H, (V + CCOLS - 1) / CCOLS), dim3(CWORK + CLOAD), 0, stream, a, *batch);
+    launch_dep(delta_coef_kernel, dim3(batch->n_tokens / CT + batch->n_seqs, G), dim3(128), 0, stream, a, scratch, *batch);
+    launch_dep(delta_chunk_kernel, dim3(batch->n_seqs, H, (V + CCOLS - 1) / CCOLS), dim3(CWORK + 32), 0, stream, a, (const float*)scratch, *batch);
     return iert_check_launch("delta_recur");
   }
 #endif
@@ -964,15 +1034,16 @@ IERT_API int iert_delta_recur(const float* qkv, const float* beta, const float* 
 
 // x: fp32 [T, ld] = r [H*DIM] | k [H*DIM] | v [H*V] | ...; decay fp32 [T, H*DIM]; u fp32 [H, DIM]; o fp32 [T, H*V].
 IERT_API int iert_wkv_recur(const float* x, long long ld, const float* decay, const float* u, float* state,
-                            long long state_stride, long long s_off, float* o, int H, int V, const IertBatchView* batch,
+                            long long state_stride, long long s_off, float* o, float* scratch, int H, int V, const IertBatchView* batch,
                             cudaStream_t stream) {
   if (batch->n_seqs <= 0 || batch->n_tokens <= 0) return IERT_OK;
   if (H <= 0 || V <= 0 || H > 65535 || ld < (long long)2 * H * DIM + (long long)H * V) return IERT_BAD_ARGUMENT;
-#if IERT_CHUNKED
-  if (chunked(batch) && V % 4 == 0 && ld % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
-      (((uintptr_t)x | (uintptr_t)state | (uintptr_t)o) & 15) == 0) {
+#if DIM == 64
+  if (scratch && chunked(batch) && V % 4 == 0 && ld % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
+      (((uintptr_t)x | (uintptr_t)decay | (uintptr_t)state | (uintptr_t)o | (uintptr_t)scratch) & 15) == 0) {
     WkvArgs a = {x, ld, decay, u, state, state_stride, s_off, o, H, V, CCOLS};
-    launch_dep(wkv_chunk_kernel, dim3(batch->n_seqs, H, (V + CCOLS - 1) / CCOLS), dim3(CWORK + WLOAD), 0, stream, a, *batch);
+    launch_dep(wkv_pairs_kernel, dim3(batch->n_tokens / CT + batch->n_seqs, H), dim3(DIM), 0, stream, a, scratch, *batch);
+    launch_dep(wkv_chunk_kernel, dim3(batch->n_seqs, H, (V + CCOLS - 1) / CCOLS), dim3(CWORK + WLOAD), 0, stream, a, (const float*)scratch, *batch);
     return iert_check_launch("wkv_recur");
   }
 #endif

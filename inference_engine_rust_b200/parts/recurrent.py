@@ -91,7 +91,8 @@ class GatedDelta(Mixer):
         B.delta_prep(proj, gates, self.conv_w, self.A_log, self.dt_bias, state, self.s_floats, qkv, beta, decay,
                      self.G, self.D, H, V, self.taps, ctx.batch, ctx.stream)
         o = ws.take("delta.readout", (T, H * V), torch.float32)
-        B.delta_recur(qkv, beta, decay, state, 0, o, self.G, self.D, H, V, ctx.batch, ctx.stream)
+        scratch = ws.take("delta.pairs", (B.recurrent_scratch_floats(self.D, T, H),), torch.float32)
+        B.delta_recur(qkv, beta, decay, state, 0, o, self.G, self.D, H, V, ctx.batch, ctx.stream, scratch=scratch)
         out = ws.take("delta.out", (T, H * V), rt.dtype)
         B.gated_head_norm(o, proj, self.C, self.norm, True, 0, self.eps, out, T, H, V, ctx.stream)
         self.o.apply(out, residual, T, ctx.stream, add_residual=True)
@@ -215,7 +216,8 @@ class Wkv(Mixer):
         decay = ws.take("wkv.decay", (T, hd), torch.float32)
         B.wkv_decay(z, self.L, self.w2t, self.w0, decay, xn, state, self.s_floats, ctx.batch, ctx.stream)
         o = ws.take("wkv.readout", (T, hd), torch.float32)
-        B.wkv_recur(x, decay, self.u, state, 0, o, D, H, D, ctx.batch, ctx.stream)
+        scratch = ws.take("wkv.pairs", (B.recurrent_scratch_floats(D, T, H),), torch.float32)
+        B.wkv_recur(x, decay, self.u, state, 0, o, D, H, D, ctx.batch, ctx.stream, scratch=scratch)
         out = ws.take("wkv.out", (T, hd), rt.dtype)
         B.wkv_finish(o, x[:, 3 * hd:], self.norm, self.eps, self.out_scale, out, ctx.batch, H, D, ctx.stream)
         self.o.apply(out, residual, T, ctx.stream, add_residual=True, ctx=ctx)

@@ -57,7 +57,8 @@ def test_delta_rule(monkeypatch, D, V, H, G, lens):
 
     def call(s):
         o = torch.zeros((T, H * V), device=DEV)
-        B.delta_recur(qkv, beta, decay, s, 0, o, G, D, H, V, view, B.stream_ptr())
+        scratch = torch.full((B.recurrent_scratch_floats(D, T, H),), float("nan"), device=DEV)
+        B.delta_recur(qkv, beta, decay, s, 0, o, G, D, H, V, view, B.stream_ptr(), scratch=scratch)
         return o
     (o, s), (o1, s1) = both_ways(monkeypatch, call, state)
     q, k, v = (x.double() for x in (qkv[:, :G * D].view(T, G, D), qkv[:, G * D:2 * G * D].view(T, G, D), qkv[:, 2 * G * D:].view(T, H, V)))
@@ -96,7 +97,8 @@ def test_decay_per_key_channel(monkeypatch, D, V, H, lens):
 
     def call(s):
         o = torch.zeros((T, H * V), device=DEV)
-        B.wkv_recur(x, decay, u, s, 0, o, D, H, V, view, B.stream_ptr())
+        scratch = torch.full((B.recurrent_scratch_floats(D, T, H),), float("nan"), device=DEV)
+        B.wkv_recur(x, decay, u, s, 0, o, D, H, V, view, B.stream_ptr(), scratch=scratch)
         return o
     (o, s), (o1, s1) = both_ways(monkeypatch, call, state)
     r, k, v = (x[:, a:b].double().view(T, H, -1) for a, b in ((0, H * D), (H * D, 2 * H * D), (2 * H * D, 2 * H * D + H * V)))
