@@ -116,3 +116,25 @@ def test_decay_per_key_channel(monkeypatch, D, V, H, lens):
     for got, plain, want in ((o, o1, want_o.flatten(1)), (s, s1, want_s)):
         assert off(got, want) <= 2.0 ** -20
         assert off(got, want) <= 1.25 * off(plain, want) + 2.0 ** -25
+
+
+@pytest.mark.parametrize("V", [8, 64, 128, 24, 256])
+@pytest.mark.parametrize("H,n_tokens", [(3, 1), (5, 7), (64, 300)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_norm_of_the_read_out_and_gate(dtype, H, n_tokens, V):
+    """A norm per head, a weight per number (shared by the heads or not) and a gate: at the edges of a block's (token, head)
+    pairs, for head sizes that the vector form takes and for others."""
+    from inference_engine_rust_b200.csrc import bindings as B
+    g = torch.Generator(device=DEV).manual_seed(V + H)
+    o = torch.randn((n_tokens, H, V), generator=g, device=DEV)
+    proj = (torch.randn((n_tokens, H * V + 16), generator=g, device=DEV) * 3).to(dtype)
+    for shared in (True, False):
+        w = torch.randn((V if shared else H * V,), generator=g, device=DEV)
+        out = torch.empty((n_tokens, H * V), dtype=dtype, device=DEV)
+        B.gated_head_norm(o, proj, 16, w, shared, 0 if shared else 1, 1e-5, out, n_tokens, H, V, B.stream_ptr())
+        z = proj[:, 16:].double()
+        gate = torch.sigmoid(z) * (z if shared else 1.0)
+        x = o.double()
+        want = (x / torch.sqrt(x.square().mean(-1, keepdim=True) + 1e-5) * (w.double() if shared else w.double().view(H, V))).flatten(1) * gate
+        # a few fp32 roundings, and one to the result's type
+        assert ((out.double() - want).abs() <= want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -19) + 1e-7).all()
