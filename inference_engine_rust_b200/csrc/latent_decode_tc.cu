@@ -421,8 +421,259 @@ latent_decode_merge_kernel(const float* __restrict__ part_m, const float* __rest
   }
 }
 
+// ---- more than 16 sequences: a head's matrix in shared memory, TT sequences a block ------------------------------------------
+// The two kernels around read a head's 128 KB of weights once per four sequences and wait for each load; with many sequences it
+// is worth bringing the matrix into shared memory whole (before the wait for the kernel in front: weights do not depend on it) and
+// giving a thread a tile of outputs.  64 sequences, 32 heads of 128, rank 512: absorption 23 -> WIDE_A us, merge 56 -> WIDE_M us.
+constexpr int WIDE_THREADS = 256;
+
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
+  const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { const float2 two = __bfloat1622float2(p[i]); f[2 * i] = two.x; f[2 * i + 1] = two.y; }
+}
+size_t absorb_wide_smem(int tt, int D, int rank) { return (size_t)D * rank * 2 + (size_t)tt * (D + 4) * 4; }
+size_t merge_wide_smem(int tt, int rank) { return (size_t)128 * (rank + 8) * 2 + (size_t)tt * (rank + 4) * 4 + (size_t)tt * 64 * 4; }
+
+// qa[t, h, :] = sum_d q[t, h, d] W_uk[h*D + d, :] and the rotated part, as above.  64 threads across the rank (eight columns each), four
+// groups of TT / 4 tokens.
+template <typename TQ, int TT>
+__global__ void __launch_bounds__(WIDE_THREADS)
+latent_absorb_wide_kernel(const TQ* __restrict__ q, long long ldq, const __nv_bfloat16* __restrict__ w_uk, __nv_bfloat16* __restrict__ qa,
+                          int H, int Hpad, int D, int R, int rank, const float* __restrict__ inv_freq, float rot_mul, int pairing,
+                          IertBatchView b) {
+  extern __shared__ __align__(16) uint8_t wide_smem[];
+  __nv_bfloat16* w_s = reinterpret_cast<__nv_bfloat16*>(wide_smem);            // [D][rank]
+  float* q_s = reinterpret_cast<float*>(wide_smem + (size_t)D * rank * 2);     // [TT][D + 4]
+  pdl_launch_dependents();
+  const int t0 = blockIdx.x * TT, h = blockIdx.y, n_t = min(TT, b.n_tokens - t0), tid = threadIdx.x, width = rank + R;
+  if (h < H) {
+    const __nv_bfloat16* src = w_uk + (size_t)h * D * rank;
+    for (int i = tid; i < D * rank / 8; i += WIDE_THREADS) copy16_async(w_s + 8 * i, src + 8 * i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  pdl_wait();
+  if (h >= H) {                         // heads that only fill the MMA tile
+    for (int i = tid; i < n_t * width; i += WIDE_THREADS)
+      qa[((size_t)(t0 + i / width) * Hpad + h) * width + i % width] = __float2bfloat16_rn(0.f);
+    return;
+  }
+  for (int i = tid; i < TT * D; i += WIDE_THREADS) {
+    const int t = i / D, d = i - t * D;
+    q_s[t * (D + 4) + d] = t < n_t ? to_f32(q[(size_t)(t0 + t) * ldq + (size_t)h * (D + R) + d]) : 0.f;
+  }
+  if (sizeof(TQ) == 4) {                // one token per sequence: token t is sequence t's
+    const int half = R / 2;
+    for (int i = tid; i < n_t * half; i += WIDE_THREADS) {
+      const int t = t0 + i / half, k = i % half, pos = b.pos0[t];
+      const TQ* v = q + (size_t)t * ldq + (size_t)h * (D + R) + D;
+      __nv_bfloat16* dst = qa + ((size_t)t * Hpad + h) * width + rank;
+      const int i0 = pairing == IERT_PAIR_INTERLEAVED ? 2 * k : k, i1 = pairing == IERT_PAIR_INTERLEAVED ? 2 * k + 1 : k + half;
+      const float x = to_f32(v[i0]), y = to_f32(v[i1]);
+      float sn, co;
+      sincosf((float)pos * inv_freq[k], &sn, &co);
+      sn *= rot_mul;
+      co *= rot_mul;
+      dst[i0] = __float2bfloat16_rn(x * co - y * sn);
+      dst[i1] = __float2bfloat16_rn(y * co + x * sn);
+    }
+  } else {
+    for (int i = tid; i < n_t * R; i += WIDE_THREADS) {                        // turned already
+      const int t = t0 + i / R, k = i % R;
+      qa[((size_t)t * Hpad + h) * width + rank + k] = __float2bfloat16_rn(to_f32(q[(size_t)t * ldq + (size_t)h * (D + R) + D + k]));
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  constexpr int PT = TT / 4;
+  const int tg = (tid >> 6) * PT;
+  for (int r0 = 8 * (tid & 63); r0 < rank; r0 += 512) {
+    float a[PT][8];
+#pragma unroll
+    for (int t = 0; t < PT; ++t)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a[t][e] = 0.f;
+    for (int d = 0; d < D; d += 4) {                                            // (D a multiple of 4)
+      float4 x[PT];
+#pragma unroll
+      for (int t = 0; t < PT; ++t) x[t] = *reinterpret_cast<const float4*>(q_s + (tg + t) * (D + 4) + d);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float f[8];
+        unpack8(*reinterpret_cast<const uint4*>(w_s + (size_t)(d + k) * rank + r0), f);
+#pragma unroll
+        for (int t = 0; t < PT; ++t) {
+          const float xd = k == 0 ? x[t].x : k == 1 ? x[t].y : k == 2 ? x[t].z : x[t].w;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) a[t][e] = fmaf(xd, f[e], a[t][e]);
+        }
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < PT; ++t)
+      if (tg + t < n_t) {
+        __nv_bfloat162 o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[e] = __floats2bfloat162_rn(a[t][2 * e], a[t][2 * e + 1]);
+        *reinterpret_cast<uint4*>(qa + ((size_t)(t0 + tg + t) * Hpad + h) * width + r0) = *reinterpret_cast<uint4*>(o);
+      }
+  }
+}
+
+// Merge of the runs and product with W_uv: 128 output columns a block (blockIdx.z), a thread four of them (32 apart) for TT / 2
+// sequences over a quarter of the rank; the quarters are added through shared memory in order.
+template <int TT>
+__global__ void __launch_bounds__(WIDE_THREADS)
+latent_merge_wide_kernel(const float* __restrict__ part_m, const float* __restrict__ part_l, const float* __restrict__ part_acc, int splits,
+                         int Hpad, int rank, const float* __restrict__ sink, const float* __restrict__ gate,
+                         const __nv_bfloat16* __restrict__ w_uv, __nv_bfloat16* __restrict__ out, IertBatchView b, int H, int V) {
+  extern __shared__ __align__(16) uint8_t wide_smem[];
+  const int ldw = rank + 8, ldl = rank + 4;
+  __nv_bfloat16* w_s = reinterpret_cast<__nv_bfloat16*>(wide_smem);            // [128][ldw]
+  float* lat = reinterpret_cast<float*>(wide_smem + (size_t)128 * ldw * 2);    // [TT][ldl]
+  float* wgt = lat + TT * ldl;                                                 // [TT][64]
+  pdl_launch_dependents();
+  const int t0 = blockIdx.x * TT, h = blockIdx.y, e0 = blockIdx.z * 128, n_t = min(TT, b.n_seqs - t0), n_e = min(128, V - e0);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r8 = rank / 8;
+  for (int i = tid; i < n_e * r8; i += WIDE_THREADS) {
+    const int e = i / r8, r = 8 * (i - e * r8);
+    copy16_async(w_s + e * ldw + r, w_uv + ((size_t)h * V + e0 + e) * rank + r);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  pdl_wait();
+  for (int t = warp; t < TT; t += WIDE_THREADS / 32) {           // splits <= 64: two runs per lane
+    const bool live = t < n_t && b.slot_ids[t0 + t] >= 0;        // a padding sequence: weights of zero
+    float mi[2], li[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int i = lane + 32 * k;
+      const size_t row = ((size_t)(live ? t0 + t : 0) * splits + (i < splits ? i : 0)) * Hpad + h;
+      mi[k] = live && i < splits ? part_m[row] : -INFINITY;
+      li[k] = live && i < splits ? part_l[row] : 0.f;
+    }
+    const float snk = sink ? sink[h] : -INFINITY;
+    const float M = fmaxf(warp_max(fmaxf(mi[0], mi[1])), snk);
+    float w[2], part = 0.f;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      w[k] = mi[k] == -INFINITY ? 0.f : expf(mi[k] - M);
+      part += w[k] * li[k];
+    }
+    const float L = warp_sum(part) + (sink ? expf(snk - M) : 0.f);
+    const float inv = L > 0.f ? 1.0f / L : 0.f;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) wgt[t * 64 + lane + 32 * k] = lane + 32 * k < splits ? w[k] * inv : 0.f;
+  }
+  __syncthreads();
+  // the runs' partial sums: four numbers of two rows per thread, two runs' loads in flight; an empty run's row (weight 0) is never read
+  const int r4 = rank >> 2;
+  for (int j0 = tid; j0 < TT * r4; j0 += 4 * WIDE_THREADS) {
+    float4 a[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) a[x] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i0 = 0; i0 < splits; i0 += 2) {
+      float4 v[4][2];
+      float w[4][2];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int j = j0 + x * WIDE_THREADS, t = j / r4;
+        const float* src = part_acc + (((size_t)(t0 + t) * splits) * Hpad + h) * rank + 4 * (j - t * r4);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          w[x][k] = j < TT * r4 ? wgt[t * 64 + ((i0 + k) & 63)] : 0.f;         // zero beyond the last run
+          v[x][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (w[x][k] != 0.f) v[x][k] = *reinterpret_cast<const float4*>(src + (size_t)(i0 + k) * Hpad * rank);
+        }
+      }
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          a[x].x = fmaf(w[x][k], v[x][k].x, a[x].x); a[x].y = fmaf(w[x][k], v[x][k].y, a[x].y);
+          a[x].z = fmaf(w[x][k], v[x][k].z, a[x].z); a[x].w = fmaf(w[x][k], v[x][k].w, a[x].w);
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int j = j0 + x * WIDE_THREADS, t = j / r4;
+      if (j < TT * r4) *reinterpret_cast<float4*>(lat + t * ldl + 4 * (j - t * r4)) = a[x];
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  constexpr int PT = TT / 2;
+  const int quarter = tid >> 6, tg = ((tid >> 5) & 1) * PT;
+  float acc[4][PT];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int t = 0; t < PT; ++t) acc[i][t] = 0.f;
+  for (int r = 8 * quarter; r < rank; r += 32) {
+    float f[4][8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) unpack8(*reinterpret_cast<const uint4*>(w_s + (lane + 32 * i) * ldw + r), f[i]);
+#pragma unroll
+    for (int t = 0; t < PT; ++t) {
+      const float4 x0 = *reinterpret_cast<const float4*>(lat + (tg + t) * ldl + r), x1 = *reinterpret_cast<const float4*>(lat + (tg + t) * ldl + r + 4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        acc[i][t] = fmaf(f[i][0], x0.x, acc[i][t]); acc[i][t] = fmaf(f[i][1], x0.y, acc[i][t]);
+        acc[i][t] = fmaf(f[i][2], x0.z, acc[i][t]); acc[i][t] = fmaf(f[i][3], x0.w, acc[i][t]);
+        acc[i][t] = fmaf(f[i][4], x1.x, acc[i][t]); acc[i][t] = fmaf(f[i][5], x1.y, acc[i][t]);
+        acc[i][t] = fmaf(f[i][6], x1.z, acc[i][t]); acc[i][t] = fmaf(f[i][7], x1.w, acc[i][t]);
+      }
+    }
+  }
+  __syncthreads();                                               // nobody reads the weights any more
+  float* red = reinterpret_cast<float*>(wide_smem);              // [3][TT][128], where they were
+  if (quarter > 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int t = 0; t < PT; ++t) red[((quarter - 1) * TT + tg + t) * 128 + lane + 32 * i] = acc[i][t];
+  }
+  __syncthreads();
+  if (quarter == 0) {
+#pragma unroll
+    for (int t = 0; t < PT; ++t) {
+      if (tg + t >= n_t) continue;
+      const float g = gate ? gate[(size_t)(t0 + tg + t) * H + h] : 1.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int e = lane + 32 * i;
+        if (e >= n_e) continue;
+        const float* p = red + (tg + t) * 128 + e;
+        const float sum = ((acc[i][t] + p[0]) + p[TT * 128]) + p[2 * TT * 128];
+        out[((size_t)(t0 + tg + t) * H + h) * V + e0 + e] = __float2bfloat16_rn(gate ? sum * g : sum);
+      }
+    }
+  }
+}
+
 size_t decode_smem(int mt, int width) {
   return (size_t)(mt * 16 + BK) * (width + 8) * 2 + (size_t)mt * 16 * PLD * 2 + (size_t)8 * mt * 16 * 4;
+}
+
+constexpr size_t WIDE_SMEM = 220 * 1024;
+
+// The dynamic shared memory of the wide kernels, asked for once.
+bool wide_configured() {
+  static const bool ok = [] {
+    bool good = true;
+    auto ask = [&](auto* k) { good = good && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WIDE_SMEM) == cudaSuccess; };
+    ask(latent_absorb_wide_kernel<float, 8>);
+    ask(latent_absorb_wide_kernel<float, 16>);
+    ask(latent_absorb_wide_kernel<__nv_bfloat16, 8>);
+    ask(latent_absorb_wide_kernel<__nv_bfloat16, 16>);
+    ask(latent_merge_wide_kernel<8>);
+    ask(latent_merge_wide_kernel<16>);
+    if (!good) cudaGetLastError();
+    return good;
+  }();
+  return ok;
 }
 
 bool umma_enabled() {
@@ -495,14 +746,28 @@ IERT_API int iert_latent_attention_decode_tc(const void* q, int q_f32, long long
     }
     configured = true;
   }
-  // tokens that share a head's weights in the kernels around: one when there are few, so that there are blocks enough
+  // few sequences: tokens that share a head's weights in the kernels around, one when there are fewest, so that there are blocks enough
   const int tt = T <= 4 ? 1 : T <= 8 ? 2 : 4;
+  // many sequences: a head's matrix whole in shared memory, eight or sixteen sequences a block (about one block per SM or more
+  // at 32 heads); padded rows of queries must keep 16-byte stores aligned
+  const int wide = T > 32 ? 16 : 8;
+  const bool wide_absorb = T > 16 && D % 4 == 0 && R % 8 == 0 && ((uintptr_t)w_uk & 15) == 0 && ((uintptr_t)qa & 15) == 0 &&
+                           absorb_wide_smem(wide, D, rank) <= WIDE_SMEM;
+  const bool wide_merge = T > 16 && ((uintptr_t)w_uv & 15) == 0 && merge_wide_smem(wide, rank) <= WIDE_SMEM;
+  if (!wide_configured()) return IERT_CUDA_ERROR;
+#define ABSORB_WIDE(TQ, TT)                                                                                                        \
+  launch_dep(latent_absorb_wide_kernel<TQ, TT>, dim3((T + TT - 1) / TT, Hpad), dim3(WIDE_THREADS), absorb_wide_smem(TT, D, rank), stream, (const TQ*)q, \
+             ldq, (const __nv_bfloat16*)w_uk, (__nv_bfloat16*)qa, H, Hpad, D, R, rank, inv_freq, rot_mul, pairing, *batch)
 #define ABSORB(TQ, TT)                                                                                                             \
   launch_dep(latent_absorb_q_kernel<TQ, TT>, dim3((T + TT - 1) / TT, Hpad), dim3(ABSORB_THREADS), (size_t)TT * (D + 4 * rank) * sizeof(float), \
              stream, (const TQ*)q, ldq, (const __nv_bfloat16*)w_uk, (__nv_bfloat16*)qa, H, Hpad, D, R, rank, inv_freq, rot_mul, pairing, *batch)
-  if (q_f32) { if (tt == 1) ABSORB(float, 1); else if (tt == 2) ABSORB(float, 2); else ABSORB(float, 4); }
+  if (wide_absorb) {
+    if (q_f32) { if (wide == 8) ABSORB_WIDE(float, 8); else ABSORB_WIDE(float, 16); }
+    else { if (wide == 8) ABSORB_WIDE(__nv_bfloat16, 8); else ABSORB_WIDE(__nv_bfloat16, 16); }
+  } else if (q_f32) { if (tt == 1) ABSORB(float, 1); else if (tt == 2) ABSORB(float, 2); else ABSORB(float, 4); }
   else { if (tt == 1) ABSORB(__nv_bfloat16, 1); else if (tt == 2) ABSORB(__nv_bfloat16, 2); else ABSORB(__nv_bfloat16, 4); }
 #undef ABSORB
+#undef ABSORB_WIDE
   dim3 grid(T, splits, Hpad / (mt * 16));
   if (umma) {
     const int st = launch_latent_decode_umma(qa, batch, kv, H, Hpad, R, scale, splits, part_m, part_l, part_acc, err, stream);
@@ -517,9 +782,16 @@ IERT_API int iert_latent_attention_decode_tc(const void* q, int q_f32, long long
   launch_dep(latent_decode_merge_kernel<__nv_bfloat16, TT>, dim3((T + TT - 1) / TT, H, V >= 64 && T <= 8 ? 2 : 1), dim3(MERGE_THREADS),                       \
              (size_t)TT * (rank + 64) * sizeof(float), stream, (const float*)part_m, (const float*)part_l, (const float*)part_acc, splits, \
              Hpad, rank, sink, gate, (const __nv_bfloat16*)w_uv, (__nv_bfloat16*)out, *batch, H, V)
-  if (tt == 1) MERGE(1);
+#define MERGE_WIDE(TT)                                                                                                             \
+  launch_dep(latent_merge_wide_kernel<TT>, dim3((T + TT - 1) / TT, H, (V + 127) / 128), dim3(WIDE_THREADS), merge_wide_smem(TT, rank), stream, \
+             (const float*)part_m, (const float*)part_l, (const float*)part_acc, splits, Hpad, rank, sink, gate, (const __nv_bfloat16*)w_uv, \
+             (__nv_bfloat16*)out, *batch, H, V)
+  if (wide_merge && wide == 8) MERGE_WIDE(8);
+  else if (wide_merge) MERGE_WIDE(16);
+  else if (tt == 1) MERGE(1);
   else if (tt == 2) MERGE(2);
   else MERGE(4);
 #undef MERGE
+#undef MERGE_WIDE
   return iert_check_launch("latent_attention_decode_tc");
 }
