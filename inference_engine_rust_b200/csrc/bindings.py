@@ -172,6 +172,8 @@ def _declare(lib) -> None:
         "iert_latent_decode_tc_plan": [c_int, c_int, c_int, c_int, c_int, POINTER(c_int), POINTER(c_int)],
         "iert_router_topk": [P, LL, LL, P, c_int, c_int, c_int, P, c_int, P, P, S],
         "iert_moe_scale": [P, c_int, LL, P, c_int, c_int, c_int, c_int, S],
+        "iert_router_step": [P, LL, P, LL, c_int, c_int, c_int, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
+                             c_int, c_int, P, c_int, P, P, P, P, S],
         "iert_moe_sort": [P, P, c_int, c_int, c_int, P, P, P, P, S],
         "iert_moe_gather": [P, LL, P, P, c_int, P, c_int, S],
         "iert_moe_combine": [P, P, P, c_int, c_int, P, c_int, S],
@@ -898,6 +900,26 @@ def router_grouped(z, correction, n_tokens: int, E: int, N: int, top: int, group
                                      idx.data_ptr(), w.data_ptr(), _ptr(x), dtype_code(x.dtype) if x is not None else F32,
                                      x.stride(0) if x is not None else 0, _ptr(residual),
                                      residual.shape[-1] if residual is not None else 0, stream), "router_grouped")
+
+
+def router_step(x, w_r, n_tokens: int, E: int, top: int, wt, idx, w, stream, *, bias=None, grouped: Optional[dict] = None, N: int = 0,
+                wid=None, residual=None) -> bool:
+    """The router's product and the routing in one kernel (bf16 rows and weights; one-token steps).  `grouped` None: as
+    `router_topk` with `bias`; else as `router_grouped` with these options (correction, groups, keep, score, group_score, weight_eps,
+    weight_scale, renormalize, shared_gate) over N outputs, `wid` and, for identity experts, `residual`.  False: nothing launched."""
+    if x.dtype != torch.bfloat16 or w_r.dtype != torch.bfloat16:
+        return False
+    g = grouped or {}
+    status = core().iert_router_step(x.data_ptr(), x.stride(0), w_r.data_ptr(), w_r.stride(0), w_r.shape[1], w_r.shape[0], 1 if grouped else 0,
+                                     _ptr(g.get("correction") if grouped else bias), n_tokens, E, N if grouped else E, top,
+                                     g.get("groups", 1), g.get("keep", 1), ROUTER_SCORES[g.get("score", "softmax")],
+                                     ROUTER_GROUP_SCORES[g.get("group_score", "max")], g.get("weight_eps", 1e-20), g.get("weight_scale", 1.0),
+                                     1 if g.get("renormalize", True) else 0, 1 if g.get("shared_gate") else 0, wt.data_ptr(), wt.stride(0),
+                                     _ptr(wid), idx.data_ptr(), w.data_ptr(), _ptr(residual), stream)
+    if status == 1:
+        return False
+    check(status, "router_step")
+    return True
 
 
 def moe_scale(act, wt, n_tokens: int, E: int, F: int, stream) -> None:

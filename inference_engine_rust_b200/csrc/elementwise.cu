@@ -57,7 +57,7 @@ __global__ void embed_gather_kernel(const TW* __restrict__ table, const int* __r
 
 // The same with the row held in registers: V runs of four consecutive numbers per thread, all of them asked for before the first
 // is written, the norm's scale before the wait for the kernel in front.  A one-token step has few rows, and the kernel above takes 16 us
-// for any number up to a few hundred (a chain of sixteen two-byte loads): this one 4 us; 15,308 rows of 4,096 141 -> 67 us (0.84 of a copy).
+// for any number up to a few hundred (a chain of sixteen two-byte loads): this one 5 us; 14,767 rows of 4,096 139 -> 55 us (363 MB).
 template <typename TW, int V>
 __global__ void __launch_bounds__(256) embed_gather_vec_kernel(const TW* __restrict__ table, const int* __restrict__ ids, float* __restrict__ x,
                                                                int hidden, int vocab, float scale, int* __restrict__ err, IertNormAhead ahead) {

@@ -424,7 +424,7 @@ latent_decode_merge_kernel(const float* __restrict__ part_m, const float* __rest
 // ---- more than 16 sequences: a head's matrix in shared memory, TT sequences a block ------------------------------------------
 // The two kernels around read a head's 128 KB of weights once per four sequences and wait for each load; with many sequences it
 // is worth bringing the matrix into shared memory whole (before the wait for the kernel in front: weights do not depend on it) and
-// giving a thread a tile of outputs.  64 sequences, 32 heads of 128, rank 512: absorption 23 -> WIDE_A us, merge 56 -> WIDE_M us.
+// giving a thread a tile of outputs.  64 sequences, 32 heads of 128, rank 512: absorption 23 -> 18 us, merge 56 -> 24 us.
 constexpr int WIDE_THREADS = 256;
 
 __device__ __forceinline__ void copy16_async(void* dst, const void* src) {

@@ -26,14 +26,9 @@ namespace {
 
 constexpr int MAX_TOP = 32;
 
-__global__ void router_topk_kernel(const float* __restrict__ z, long long ldz, long long lde, const float* __restrict__ bias,
-                                   int E, int top, float* __restrict__ wt, int ldw, int* __restrict__ idx,
-                                   float* __restrict__ w) {
-  // one warp per token
-  pdl_launch_dependents();     // the next kernel may start its preamble now
-  pdl_wait();                  // everything below may depend on the kernel before
-  const int t = blockIdx.x, lane = threadIdx.x;
-  const float* row = z + (size_t)t * ldz;
+// The routing of token t by one warp from its logits (output e at row[e * lde]).
+__device__ __forceinline__ void topk_token(const float* __restrict__ row, long long lde, const float* __restrict__ bias, int E, int top,
+                                           float* __restrict__ wt, int ldw, int* __restrict__ idx, float* __restrict__ w, int t, int lane) {
   int chosen[MAX_TOP];
   float val[MAX_TOP];
   for (int k = 0; k < top; ++k) {
@@ -66,6 +61,15 @@ __global__ void router_topk_kernel(const float* __restrict__ z, long long ldz, l
       idx[(size_t)t * top + k] = chosen[k];
       w[(size_t)t * top + k] = p;
     }
+}
+
+__global__ void router_topk_kernel(const float* __restrict__ z, long long ldz, long long lde, const float* __restrict__ bias,
+                                   int E, int top, float* __restrict__ wt, int ldw, int* __restrict__ idx,
+                                   float* __restrict__ w) {
+  // one warp per token
+  pdl_launch_dependents();     // the next kernel may start its preamble now
+  pdl_wait();                  // everything below may depend on the kernel before
+  topk_token(z + (size_t)blockIdx.x * ldz, lde, bias, E, top, wt, ldw, idx, w, blockIdx.x, threadIdx.x);
 }
 
 // A block per token, whose first warp routes; shared memory: s[N], c[N], group score [groups], flags [N] (bytes).  Output e of token t is
@@ -251,6 +255,69 @@ __global__ void moe_scale_kernel(T* __restrict__ act, long long ld, const float*
     row[i] = from_f32<T>(to_f32(row[i]) * wt[(size_t)t * ldw + i / F]);
 }
 
+// One-token steps: the router's product and the routing in one kernel, a block per token.  A warp takes every eighth output, a lane
+// eight numbers of the row at a time; fp32 sums.  The tensor-core product has one tile of up to 32 columns to give to 148 SMs, splits it
+// over k and adds the parts through memory: 20 us and 8 more for the routing at 32 tokens x 16 outputs x 4,096; this kernel 16.
+// GROUPED: route_token with `a`, else topk_token with the fields of `a` it needs (`correction` is the bias then).
+constexpr int ROUTER_THREADS = 256;
+
+template <bool GROUPED>
+__global__ void __launch_bounds__(ROUTER_THREADS)
+router_step_kernel(RouterArgs a, const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w_r, long long ldr, int K,
+                   int rows, float* __restrict__ residual, int H) {
+  extern __shared__ float rsm[];
+  __shared__ float share_s;
+  float* z_s = rsm;                        // [rows] logits, then the routing's own
+  pdl_launch_dependents();
+  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const __nv_bfloat16* xr = x + (size_t)t * ldx;
+  for (size_t i = (size_t)threadIdx.x * 64; t == 0 && i < (size_t)rows * K; i += ROUTER_THREADS * 64)      // (weights: ahead of the wait)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(w_r + i / K * ldr + i % K));
+  pdl_wait();
+  for (int e = warp; e < rows; e += 2 * (ROUTER_THREADS / 32)) {
+    const int e2 = e + ROUTER_THREADS / 32;
+    const __nv_bfloat16* w0 = w_r + (size_t)e * ldr;
+    const __nv_bfloat16* w1 = w_r + (size_t)(e2 < rows ? e2 : e) * ldr;
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll 4
+    for (int k = lane * 8; k < K; k += 256) {
+      const uint4 xv = *reinterpret_cast<const uint4*>(xr + k), u = *reinterpret_cast<const uint4*>(w0 + k), v = *reinterpret_cast<const uint4*>(w1 + k);
+      const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&xv);
+      const __nv_bfloat162* up = reinterpret_cast<const __nv_bfloat162*>(&u);
+      const __nv_bfloat162* vp = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 xf = __bfloat1622float2(xp[i]), uf = __bfloat1622float2(up[i]), vf = __bfloat1622float2(vp[i]);
+        s0 = fmaf(xf.x, uf.x, s0); s0 = fmaf(xf.y, uf.y, s0);
+        s1 = fmaf(xf.x, vf.x, s1); s1 = fmaf(xf.y, vf.y, s1);
+      }
+    }
+    s0 = warp_sum(s0);
+    s1 = warp_sum(s1);
+    if (lane == 0) {
+      z_s[e] = s0;
+      if (e2 < rows) z_s[e2] = s1;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    if (GROUPED) {
+      a.z = z_s;
+      a.ldz = 0;
+      a.lde = 1;
+      const float share = route_token(a, t, lane, rsm + rows);
+      if (lane == 0) share_s = share;
+    } else {
+      topk_token(z_s, 1, a.correction, a.E, a.top, a.wt, a.ldw, a.idx, a.w, t, lane);
+    }
+  }
+  if (!GROUPED || !residual) return;
+  __syncthreads();
+  const float share = share_s;
+  if (share == 0.f) return;
+  for (int i = threadIdx.x; i < H; i += ROUTER_THREADS) residual[(size_t)t * H + i] += share * __bfloat162float(xr[i]);
+}
+
 constexpr int SORT_THREADS = 1024, ROW_TILE = 128;
 
 __global__ void __launch_bounds__(SORT_THREADS)
@@ -427,4 +494,31 @@ IERT_API int iert_moe_scale(void* act, int dtype, long long ld, const float* wt,
     launch_dep(moe_scale_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(256), 0, stream, (__nv_bfloat16*)act, ld, wt, ldw, E, F);
   else return IERT_BAD_ARGUMENT;
   return iert_check_launch("moe_scale");
+}
+
+// The product of x [n_tokens, K] with the router's `rows` rows w_r (bf16) and the routing, in one kernel.  grouped != 0: as
+// iert_router_grouped (rows = N, or N + 1 with shared_gate), `residual` (optional, fp32 [n_tokens, K]) receives the identity experts'
+// share; else as iert_router_topk (`correction` is the bias, rows = E = N).  K and the strides multiples of 8, rows on 16-byte boundaries.
+IERT_API int iert_router_step(const void* x, long long ldx, const void* w_r, long long ldr, int K, int rows, int grouped, const float* correction,
+                              int n_tokens, int E, int N, int top, int groups, int keep, int score_mode, int group_mode, float weight_eps,
+                              float weight_scale, int renorm, int shared_gate, float* wt, int ldw, float* wid, int* idx, float* w,
+                              float* residual, cudaStream_t stream) {
+  if (n_tokens <= 0) return IERT_OK;
+  if (K <= 0 || K % 8 || ldx % 8 || ldr % 8 || (((uintptr_t)x | (uintptr_t)w_r) & 15) || E <= 0 || N < E || top <= 0 || top > MAX_TOP)
+    return IERT_BAD_ARGUMENT;
+  if (grouped ? (score_mode < 0 || score_mode > 1 || group_mode < 0 || group_mode > 1 || groups <= 0 || N % groups || keep <= 0 || keep > groups ||
+                 top > keep * (N / groups) || ldw < E + (shared_gate ? 1 : 0) || rows != N + (shared_gate ? 1 : 0) || !wid)
+              : (top > E || ldw < E || rows != E || residual))
+    return IERT_BAD_ARGUMENT;
+  const size_t smem = (size_t)(rows + 2 * N + groups) * sizeof(float) + (size_t)N;
+  if (smem > 47 * 1024) return IERT_BAD_ARGUMENT;
+  const RouterArgs a = {nullptr, 0, 1, correction, E, N, top, groups, keep, score_mode, group_mode, weight_eps, weight_scale, renorm,
+                        shared_gate, ldw, wt, wid, idx, w};
+  if (grouped)
+    launch_dep(router_step_kernel<true>, dim3(n_tokens), dim3(ROUTER_THREADS), smem, stream, a, (const __nv_bfloat16*)x, ldx,
+               (const __nv_bfloat16*)w_r, ldr, K, rows, residual, K);
+  else
+    launch_dep(router_step_kernel<false>, dim3(n_tokens), dim3(ROUTER_THREADS), smem, stream, a, (const __nv_bfloat16*)x, ldx,
+               (const __nv_bfloat16*)w_r, ldr, K, rows, (float*)nullptr, K);
+  return iert_check_launch("router_step");
 }

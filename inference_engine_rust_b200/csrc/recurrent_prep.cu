@@ -224,7 +224,7 @@ __device__ __forceinline__ void head_store4(__nv_bfloat16* p, float4 v) {
 
 // Read-outs normed per head and gated, four numbers a lane: V / 4 lanes a head (V a power of two from 8 to 128), ROWS tokens per lane
 // with all their loads in flight.  A warp per head with a few loads each, as below, leaves the memory waiting (2,048 tokens: 32 heads
-// of 128 33 us, 64 heads of 64 57 us; here 14 and 19).
+// of 128 33 us, 64 heads of 64 57 us; here 24 and 29).
 //   y = x * r * w * act(gate),  r = factor / sqrt(mean(x^2) + eps)
 template <typename T, typename TG, int ROWS>
 __global__ void __launch_bounds__(128) head_norm_vec_kernel(const float* __restrict__ o, const TG* __restrict__ gate, long long ldg,
@@ -233,20 +233,18 @@ __global__ void __launch_bounds__(128) head_norm_vec_kernel(const float* __restr
   pdl_wait();
   const int lanes = V >> 2, heads = 128 / lanes;                  // lanes per head; (token, head) pairs of a block and round
   const int e = 4 * (threadIdx.x % lanes);
-  const long long first = (long long)blockIdx.x * heads * ROWS + threadIdx.x / lanes, all = (long long)n_tokens * H;
+  const unsigned first = blockIdx.x * heads * ROWS + threadIdx.x / lanes, all = (unsigned)n_tokens * H;
   float4 x[ROWS], g[ROWS], wv[ROWS];
 #pragma unroll
   for (int k = 0; k < ROWS; ++k) {
-    const long long p = first + (long long)k * heads;
-    const long long q = p < all ? p : 0;
-    const int t = (int)(q / H), h = (int)(q - (long long)t * H);
+    const unsigned p = first + k * heads, q = p < all ? p : 0, t = q / (unsigned)H, h = q - t * H;
     x[k] = *reinterpret_cast<const float4*>(o + (size_t)q * V + e);
     g[k] = head_load4(gate + (size_t)t * ldg + (size_t)h * V + e);
     wv[k] = *reinterpret_cast<const float4*>(w + (per_head ? 0 : h * V) + e);
   }
 #pragma unroll
   for (int k = 0; k < ROWS; ++k) {
-    const long long p = first + (long long)k * heads;
+    const unsigned p = first + k * heads;
     float ss = fmaf(x[k].x, x[k].x, fmaf(x[k].y, x[k].y, fmaf(x[k].z, x[k].z, x[k].w * x[k].w)));
     for (int m = lanes >> 1; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
     if (p >= all) continue;
@@ -254,7 +252,7 @@ __global__ void __launch_bounds__(128) head_norm_vec_kernel(const float* __restr
     float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
     bool padding = false;                                          // (nobody wrote a padding token's read-out)
     if (check) {
-      const int s = sequence_of_token(b, (int)(p / H));
+      const int s = sequence_of_token(b, (int)(p / (unsigned)H));
       padding = s < 0 || b.slot_ids[s] < 0;
     }
     if (!padding) {
@@ -275,6 +273,7 @@ bool launch_head_norm_vec(const float* o, const TG* gate, long long ldg, const f
       ((uintptr_t)out % (4 * sizeof(T))))
     return false;
   const long long pairs = (long long)n_tokens * H;
+  if (pairs > (1ll << 30)) return false;
   const int per_round = 512 / V;
   const IertBatchView none = {};
   if (pairs >= 16384)
@@ -439,6 +438,67 @@ wkv_decay_kernel(const float* __restrict__ z, long long ldz, int L, const float*
   }
 }
 
+// The same for prompts: 16 tokens a block and four channels a thread, so that a token's numbers, read from shared memory, serve four
+// channels and the matrix is read once per 16 tokens (2,048 tokens, 64 x 4,096: 70 -> 48 us).  C and L multiples of 4.
+constexpr int DECAY_WIDE = 16;
+
+template <typename T>
+__global__ void __launch_bounds__(128)
+wkv_decay_wide_kernel(const float* __restrict__ z, long long ldz, int L, const float* __restrict__ w2t, const float* __restrict__ w0,
+                      int C, float* __restrict__ decay, const T* __restrict__ h, long long ldh, int width,
+                      float* __restrict__ state, long long state_stride, long long prev_off, IertBatchView b) {
+  extern __shared__ float lora[];          // [DECAY_WIDE][L]
+  __shared__ int keep_slot[DECAY_WIDE];    // the slot whose kept row token tt becomes (-1: none)
+  pdl_wait();
+  const int t0 = blockIdx.x * DECAY_WIDE, n = min(DECAY_WIDE, b.n_tokens - t0);
+  if (threadIdx.x < DECAY_WIDE) {
+    int slot = -1;
+    if ((int)threadIdx.x < n) {
+      const int t = t0 + threadIdx.x, s = sequence_of_token(b, t);
+      if (s >= 0 && t == b.cu_q[s + 1] - 1) slot = b.slot_ids[s];
+    }
+    keep_slot[threadIdx.x] = slot;
+  }
+  for (int i = threadIdx.x; i < DECAY_WIDE * L; i += 128) {
+    const int tt = i / L, l = i - tt * L;
+    lora[i] = tt < n ? tanhf(z[(size_t)(t0 + tt) * ldz + l]) : 0.f;
+  }
+  __syncthreads();
+  const int c = 4 * (blockIdx.y * 128 + threadIdx.x);
+  if (c < C) {
+    const float4 bias = *reinterpret_cast<const float4*>(w0 + c);
+    float4 a[DECAY_WIDE];
+#pragma unroll
+    for (int tt = 0; tt < DECAY_WIDE; ++tt) a[tt] = bias;
+    for (int l = 0; l < L; l += 4) {
+      float4 w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) w[k] = *reinterpret_cast<const float4*>(w2t + (size_t)(l + k) * C + c);
+#pragma unroll
+      for (int tt = 0; tt < DECAY_WIDE; ++tt) {
+        const float4 x = *reinterpret_cast<const float4*>(lora + tt * L + l);
+        const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          a[tt].x = fmaf(w[k].x, xs[k], a[tt].x); a[tt].y = fmaf(w[k].y, xs[k], a[tt].y);
+          a[tt].z = fmaf(w[k].z, xs[k], a[tt].z); a[tt].w = fmaf(w[k].w, xs[k], a[tt].w);
+        }
+      }
+    }
+#pragma unroll
+    for (int tt = 0; tt < DECAY_WIDE; ++tt)
+      if (tt < n)
+        *reinterpret_cast<float4*>(decay + (size_t)(t0 + tt) * C + c) =
+            make_float4(expf(-expf(a[tt].x)), expf(-expf(a[tt].y)), expf(-expf(a[tt].z)), expf(-expf(a[tt].w)));
+  }
+  // the kept rows: every block of the token group takes a slice of the width
+  const int per = (width + gridDim.y - 1) / gridDim.y, i1 = min(width, ((int)blockIdx.y + 1) * per);
+  for (int tt = 0; tt < n; ++tt)
+    if (keep_slot[tt] >= 0)
+      for (int i = blockIdx.y * per + threadIdx.x; i < i1; i += 128)
+        state[(size_t)keep_slot[tt] * state_stride + prev_off + i] = to_f32(h[(size_t)(t0 + tt) * ldh + i]);
+}
+
 template <typename T>
 __global__ void wkv_finish_kernel(const float* __restrict__ o, const float* __restrict__ gate, long long ldg,
                                   const float* __restrict__ w, float eps, float out_scale, T* __restrict__ out,
@@ -518,6 +578,18 @@ IERT_API int iert_wkv_decay(const float* z, long long ldz, int L, const float* w
                             long long prev_off, const IertBatchView* batch, cudaStream_t stream) {
   if (batch->n_tokens <= 0) return IERT_OK;
   if (L <= 0 || L > 1024 || C <= 0 || width <= 0) return IERT_BAD_ARGUMENT;
+  if (batch->n_tokens >= 256 && C % 4 == 0 && L % 4 == 0 && L <= 512 && (((uintptr_t)w2t | (uintptr_t)w0 | (uintptr_t)decay) & 15) == 0 &&
+      (dtype == IERT_F32 || dtype == IERT_BF16)) {
+    const size_t bytes = (size_t)DECAY_WIDE * L * sizeof(float);
+    const dim3 blocks((batch->n_tokens + DECAY_WIDE - 1) / DECAY_WIDE, (C + 511) / 512);
+    if (dtype == IERT_F32)
+      launch_dep(wkv_decay_wide_kernel<float>, blocks, dim3(128), bytes, stream, z, ldz, L, w2t, w0, C, decay, (const float*)h, ldh, width,
+                 state, state_stride, prev_off, *batch);
+    else
+      launch_dep(wkv_decay_wide_kernel<__nv_bfloat16>, blocks, dim3(128), bytes, stream, z, ldz, L, w2t, w0, C, decay, (const __nv_bfloat16*)h, ldh,
+                 width, state, state_stride, prev_off, *batch);
+    return iert_check_launch("wkv_decay");
+  }
   const size_t smem = (size_t)DECAY_TOKENS * L * sizeof(float);
   const dim3 grid((batch->n_tokens + DECAY_TOKENS - 1) / DECAY_TOKENS, (C + 255) / 256);
   if (dtype == IERT_F32)

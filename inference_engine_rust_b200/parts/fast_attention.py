@@ -16,6 +16,7 @@ def _slots(head_dim: int) -> int:
 
 
 _MAX_SPLITS = 16
+CUT_SAVES_LOADS = 16         # page loads in a row that cutting a batch that fills the device must save (see wants_length_cut)
 
 
 def decode_splits(n_tokens: int, kv_heads: int, group: int, head_dim: int) -> int:
@@ -30,11 +31,13 @@ def decode_splits(n_tokens: int, kv_heads: int, group: int, head_dim: int) -> in
 def wants_length_cut(pos0, kv_heads: int, group: int, window, page_tokens: int, head_dim: int, chunk=None,
                      keep: int = 0) -> bool:
     """Should a one-token step over sequences at these positions be cut by length (see
-    `decode_parts`) rather than evenly?  Yes if the longest sequence reads over 1.3 times the
-    average number of pages (an even cut ends when its CTAs do).  And yes if the batch alone
-    fills the device and a cut by length is predicted to take at least 15 % fewer page loads
-    in a row: 48 sequences of 33 pages with 8 kv heads are 384 CTAs on 296 slots, two rounds
-    of 33 pages; cut in two they are 768 CTAs, three rounds of 17."""
+    `decode_parts`) rather than evenly?  Where the batch leaves the device room for several parts per sequence: yes
+    if the longest sequence reads over 1.3 times the average number of pages (an even cut ends when its CTAs do).
+    Where the batch alone fills the device, an even step needs neither parts nor a merge, and a cut costs about 20 us
+    (a grid of eight parts per sequence, most of them empty, and the merge): yes if the cut is predicted to take at
+    least 15 % and 16 fewer page loads in a row.  Measured at 32 heads over 8, even / cut, us a layer:
+    64 sequences of 200 to 256 positions 90 / 111, of 100 to 400 90 / 112, of 512 to 1,024 110 / 129, 48 of 500 92 / 109 (all even by
+    this rule); between 16 and 25 loads saved the two are within 6 % (64 of 100 to 2,048 132 / 136, 48 of 2,100 144 / 153)."""
     n = len(pos0)
     if n < 2:
         return False
@@ -45,17 +48,15 @@ def wants_length_cut(pos0, kv_heads: int, group: int, window, page_tokens: int, 
     else:
         pages = [p // page_tokens + 1 for p in pos0]
     longest, total = max(pages), sum(pages)
-    if longest * n > 1.3 * total:
-        return True
     per_sequence = kv_heads * -(-group // 8)
     slots = _slots(head_dim)
-    if n * per_sequence <= slots:
-        return False
+    if 2 * n * per_sequence <= slots:
+        return longest * n > 1.3 * total
     even = -(-n * per_sequence // slots) * longest
     per_part = max(1, -(-total * per_sequence // (2 * slots)))                 # as the kernel works it out
     parts = [min(8, -(-p // per_part)) for p in pages]
     cut = -(-sum(parts) * per_sequence // slots) * max(-(-p // k) for p, k in zip(pages, parts))
-    return even >= 1.15 * cut
+    return even >= 1.15 * cut and even - cut >= CUT_SAVES_LOADS
 
 
 def decode_parts(n_tokens: int, kv_heads: int, group: int, unequal: bool, head_dim: int):

@@ -44,6 +44,8 @@ from .linear import Linear
 # Prompts of more than this many tokens compute a grouped router's logits (at most 32 outputs) with the kernel for few
 # rows against a long matrix, the tokens being the matrix.
 SKINNY_ROUTER_MIN_TOKENS = 32
+# Up to this many tokens the router's product and the routing are one kernel, a block per token.
+ROUTER_STEP_MAX_TOKENS = 64
 # Prompts of at least this many tokens run the experts' products over the tokens that chose them, if that is less than half of
 # the rows that all experts over all tokens would have.  (16 experts at 7B sizes, grouped against all experts, two chosen and a
 # shared one: 256 tokens 149 / 122 us, 384: 143 / 161, 2,048: 273 / 520; four chosen: 384: 129 / 184, 2,048: 324 / 526.)
@@ -112,14 +114,20 @@ class MoE(FeedForward):
             self.router.apply(xn, z, T, stream)
         return z, by_output
 
+    def _routes_in_one(self, xn, T: int) -> bool:
+        """Steps of few tokens: one kernel for the router's product and the routing."""
+        return (self.rt.fast and T <= ROUTER_STEP_MAX_TOKENS and isinstance(xn, torch.Tensor) and xn.dtype == torch.bfloat16)
+
     def _route(self, xn, residual, T: int, stream: int):
         """(wt [T, E or more] dense routing weights, idx, w [T, top] the choices); the share of experts that return their
         input is added to `residual`."""
         ws, E = self.rt.workspace, self.experts
-        z, by_output = self._router_logits(xn, E, T, stream)
         wt = ws.take("moe.weights", (T, E + (1 if self.shared_ff else 0)), torch.float32)
         idx = ws.take("moe.chosen", (T, self.top), torch.int32)
         w = ws.take("moe.chosen_weights", (T, self.top), torch.float32)
+        if self._routes_in_one(xn, T) and B.router_step(xn, self.router.weight, T, E, self.top, wt, idx, w, stream, bias=self.router_bias):
+            return wt, idx, w
+        z, by_output = self._router_logits(xn, E, T, stream)
         B.router_topk(z, self.router_bias, T, E, self.top, wt, idx, w, stream, by_output=by_output)
         return wt, idx, w
 
@@ -223,6 +231,11 @@ class GroupedMoE(MoE):
         wid = ws.take("moe.identity_share", (T,), torch.float32)
         idx = ws.take("moe.chosen", (T, self.top), torch.int32)
         w = ws.take("moe.chosen_weights", (T, self.top), torch.float32)
+        if self._routes_in_one(xn, T) and B.router_step(
+                xn, self.router.weight, T, E, self.top, wt, idx, w, stream, N=N, wid=wid, residual=residual if self.identity else None,
+                grouped=dict(correction=self.correction, groups=self.groups, keep=self.keep, score=self.score, group_score=self.group_score,
+                             weight_eps=self.weight_eps, weight_scale=self.weight_scale)):
+            return wt, idx, w
         z, by_output = self._router_logits(xn, N, T, stream)
         B.router_grouped(z, self.correction, T, E, N, self.top, self.groups, self.keep, wt, wid, idx, w, stream,
                          by_output=by_output, score=self.score, group_score=self.group_score, weight_eps=self.weight_eps,

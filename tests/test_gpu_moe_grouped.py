@@ -115,3 +115,31 @@ def test_a_row_that_is_no_number_stays_one():
     assert part._takes_grouped(x, 400)
     part.forward(x, out, ctx)
     assert torch.isnan(out[7]).all() and torch.isfinite(out[:7]).all() and torch.isfinite(out[8:]).all()
+
+
+@pytest.mark.parametrize("T,E,top,K,shared", [(1, 1, 1, 8, False), (3, 5, 2, 264, True), (64, 16, 4, 4096, False), (33, 70, 3, 1000, True)])
+def test_router_in_one_kernel(T, E, top, K, shared):
+    """The product with the routing behind it, against the two kernels apart on the same 32-bit logits."""
+    from inference_engine_rust_b200.csrc import bindings as B
+    g = torch.Generator(device=DEV).manual_seed(E)
+    x = torch.randn((T, K), generator=g, device=DEV).to(torch.bfloat16)
+    w_r = (torch.randn((E, K), generator=g, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    bias = torch.randn(E, generator=g, device=DEV) * 0.1
+    z = (x.double() @ w_r.double().t()).float()
+
+    def empty():
+        return (torch.full((T, E + shared), 9.0, device=DEV), torch.empty((T, top), dtype=torch.int32, device=DEV), torch.empty((T, top), device=DEV))
+    for grouped in (None, dict(correction=bias, groups=1, keep=1, score="sigmoid", group_score="top2_sum", weight_scale=2.5)):
+        a, b = empty(), empty()
+        wid = torch.empty(T, device=DEV)
+        if grouped is None:
+            assert B.router_step(x, w_r, T, E, top, *a, B.stream_ptr(), bias=bias)
+            B.router_topk(z, bias, T, E, top, *b, B.stream_ptr())
+        else:
+            assert B.router_step(x, w_r, T, E, top, *a, B.stream_ptr(), N=E, wid=wid, grouped=grouped)
+            opts = dict(grouped)
+            B.router_grouped(z, opts.pop("correction"), T, E, E, top, opts.pop("groups"), opts.pop("keep"), b[0], wid, b[1], b[2], B.stream_ptr(), **opts)
+        assert torch.equal(a[1], b[1])
+        for p, q in ((a[0], b[0]), (a[2], b[2])):
+            assert ((p - q).abs() <= 2.0 ** -16).all()            # logits of size 1 summed in another order, K terms of 2^-24
+    assert not B.router_step(x[:, 1:], w_r[:, 1:], T, E, top, *empty(), B.stream_ptr(), bias=bias)
