@@ -75,6 +75,7 @@ struct GemmParams {
   int coop_reduce;    // splits > 1: every split adds its share of the rows (the grid is co-resident)
   int t_group;        // token tiles per group in the order of the tiles (see tile_coords); t_tiles = one group
   int tma_out;        // residual add through TMA reduce (map_o), weight-major tiles of >= 128 tokens
+  int tma_store;      // token-major tiles: outputs leave through shared memory and TMA (map_o; see StageStore)
   int tail_parts;     // > 1: the tiles from full_tiles on are cut into this many parts of k (see WorkIter)
   int full_tiles;
   int* err;
@@ -328,6 +329,34 @@ __device__ __forceinline__ TilePlace tile_place(const GemmParams& p, int tile, i
   return c;
 }
 
+// Token-major epilogue: a lane holds a token's row, so its stores go to rows apart; a warp's 32 rows of 128 bytes are gathered in shared
+// memory (128-byte swizzle: no two lanes meet in a bank) and leave as one TMA store, two buffers in turn.  Whole rows of a box leave in
+// full lines, and nobody waits for them.  (16-byte stores by lanes took 12.7 us a tile of 128 x 256 fp32, which short inner axes cannot
+// hide: 4,096 tokens x 8,192 x 256 63 -> 42 us, experts' down product of 2,048 tokens 55 -> 44 us,
+// four products of 4,096 x 2,048 x 2,048 66 -> 61 us.)
+struct StageStore {
+  const CUtensorMap* map;
+  uint8_t* buf;              // this warp's two buffers of 4 KB
+  int lane, row0, turn;
+  // `piece`: which 16 bytes of the row's 128; the first of a box waits until the buffer's last store has read it
+  __device__ __forceinline__ void begin() {
+    if (lane == 0) bulk_wait_group_read<1>();
+    __syncwarp();
+  }
+  __device__ __forceinline__ void put(int piece, const uint4& v) {
+    *reinterpret_cast<uint4*>(buf + turn * 4096 + lane * 128 + ((piece ^ (lane & 7)) << 4)) = v;
+  }
+  __device__ __forceinline__ void end(int col0) {
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_2d(map, buf + turn * 4096, col0, row0);
+      bulk_commit_group();
+    }
+    turn ^= 1;
+  }
+};
+
 template <int BT, bool GATED, bool GROUPED = false>
 __global__ void __launch_bounds__(THREADS, 2)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
@@ -353,7 +382,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   int* ticket_s = (int*)(tmem_slot + 2);
   uint8_t* xch_s = (uint8_t*)(((uintptr_t)(tmem_slot + 4) + 15) & ~(uintptr_t)15);   // 4 KB, weight-major gated only
-  uint8_t* out_s = (uint8_t*)(((uintptr_t)(tmem_slot + 4) + 127) & ~(uintptr_t)127);  // 2 x 16 KB, residual add by TMA only
+  // 2 x 16 KB: staging of the residual add by TMA, or of the token-major stores (four warps, two boxes of 4 KB each)
+  uint8_t* out_s = GATED ? (uint8_t*)(((uintptr_t)(tmem_slot + 4) + 1023) & ~(uintptr_t)1023)
+                         : (uint8_t*)(((uintptr_t)(tmem_slot + 4) + 127) & ~(uintptr_t)127);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -485,6 +516,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
+    StageStore stage_out{&map_o, out_s + q * 8192, lane, 0, 0};
+    if (GATED && p.tma_store && threadIdx.x == 64) tma_prefetch_desc(&map_o);
     WorkIter it(p, t_tiles);
     int tile, split, n_parts, kb0, kb1;
     while (ok && it.next(tile, split, n_parts, kb0, kb1)) {
@@ -523,12 +556,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         // lane = token, columns [0, 128) = gate rows, [128, 256) = their up rows
         const int tok = t0 + n_local;
         const float row_factor = GROUPED && p.row_scale && tok < t_end ? p.row_scale[tok] : 1.0f;
+        // (rows behind an expert's last belong to the next expert: such a warp stores by lanes)
+        const bool staged = p.tma_store && (GROUPED ? t0 + q * 32 + 32 <= t_end : t0 + q * 32 < t_end);
+        stage_out.row0 = t0 + q * 32;
 #pragma unroll 1
         for (int c = 0; c < TILE_N; c += 16) {
+          if (staged && n0 + c >= p.N) break;          // warp-uniform
           float v[16], u[16];
           tmem_ld16(taddr + c, v);
           tmem_ld16(taddr + TILE_N + c, u);
-          if (tok < t_end) {
+          if (staged) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = GROUPED ? silu_mul(v[j], u[j]) * row_factor : silu_mul(v[j], u[j]);
+            if (!GROUPED && p.ep.scale && tok < t_end) epilogue_run<16>(v, tok, n0 + c, p.ep);
+            uint4 w2[2];
+            __nv_bfloat162* wp = reinterpret_cast<__nv_bfloat162*>(w2);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) wp[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+            if (c % 64 == 0) stage_out.begin();
+            stage_out.put((c % 64) / 8, w2[0]);
+            stage_out.put((c % 64) / 8 + 1, w2[1]);
+            if (c % 64 == 48 || n0 + c + 16 >= p.N) stage_out.end(n0 + c - c % 64);
+          } else if (tok < t_end) {
             __nv_bfloat16* o = (__nv_bfloat16*)p.out + (long long)tok * p.ldo + n0 + c;
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = GROUPED ? silu_mul(v[j], u[j]) * row_factor : silu_mul(v[j], u[j]);
@@ -551,11 +600,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         // token-major plain product: lane = token, 256 output columns per tile; a thread's 16
         // values of a chunk are contiguous in memory (vector loads and stores)
         const int tok = t0 + n_local;
+        const bool staged = p.tma_store && (GROUPED ? t0 + q * 32 + 32 <= t_end : t0 + q * 32 < t_end);
+        stage_out.row0 = t0 + q * 32;
 #pragma unroll 1
         for (int c = 0; c < 2 * TILE_N; c += 16) {
           if (n0 + c >= p.N) break;                    // warp-uniform
           float v[16];
           tmem_ld16(taddr + c, v);
+          if (staged) {
+            if (epilogue_on(p.ep) && tok < t_end) epilogue_run<16>(v, tok, n0 + c, p.ep);
+            if (p.out_dtype == IERT_F32) {
+              if (c % 32 == 0) stage_out.begin();
+#pragma unroll
+              for (int j = 0; j < 4; ++j) stage_out.put((c % 32) / 4 + j, *reinterpret_cast<const uint4*>(v + 4 * j));
+              if (c % 32 == 16 || n0 + c + 16 >= p.N) stage_out.end(n0 + c - c % 32);
+            } else {
+              uint4 w2[2];
+              __nv_bfloat162* wp = reinterpret_cast<__nv_bfloat162*>(w2);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) wp[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+              if (c % 64 == 0) stage_out.begin();
+              stage_out.put((c % 64) / 8, w2[0]);
+              stage_out.put((c % 64) / 8 + 1, w2[1]);
+              if (c % 64 == 48 || n0 + c + 16 >= p.N) stage_out.end(n0 + c - c % 64);
+            }
+            continue;
+          }
           if (tok >= t_end) continue;
           if (p.mode == MODE_STORE && epilogue_on(p.ep)) epilogue_run<16>(v, tok, n0 + c, p.ep);
           const bool full16 = n0 + c + 16 <= p.N;
@@ -782,6 +852,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
       }
     }
+    if (GATED && lane == 0) bulk_wait_group<0>();                // the staged stores are done before the shared memory goes
     if (!ok && lane == 0) {
       if (!*abort_flag) atomicOr(p.err, IERT_ERR_WAIT_EXPIRED);
       *abort_flag = 1;
@@ -882,6 +953,33 @@ bool tensor_map_out(const void* ptr, long long rows, long long cols, long long l
   return true;
 }
 
+// An output [rows, cols] with row stride ld (fp32 or bf16), stored in boxes of 32 rows x 128 bytes under the 128-byte swizzle.  Rows have
+// to end on a 16-byte boundary: a store writes whole pieces of 16 bytes, zeros behind the last column.
+bool tensor_map_store(const void* ptr, long long rows, long long cols, long long ld, int dtype, CUtensorMap* out) {
+  static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
+  static std::mutex mu;
+  const int elt = dtype == IERT_F32 ? 4 : 2;
+  EncodeTiledFn fn = encode_fn();
+  if (!fn || (cols * elt) % 16 || (ld * elt) % 16 || ((uintptr_t)ptr & 15)) return false;
+  MapKey key{ptr, rows, cols, ld, elt};
+  std::lock_guard<std::mutex> g(mu);
+  auto it = cache.find(key);
+  if (it != cache.end()) { *out = it->second; return true; }
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * elt};
+  cuuint32_t box[2] = {(cuuint32_t)(128 / elt), 32};
+  cuuint32_t estr[2] = {1, 1};
+  CUtensorMap m;
+  CUresult r = fn(&m, dtype == IERT_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims,
+                  strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return false;
+  if (cache.size() > 4096) cache.clear();
+  cache.emplace(key, m);
+  *out = m;
+  return true;
+}
+
 // How many token tiles make a group in the order of the tiles (see tile_coords).  With one group
 // (all token tiles) the whole activation matrix is read once per weight-row tile unless it stays
 // in the L2; with smaller groups the weight matrix is read once per group instead.  A group's
@@ -937,8 +1035,11 @@ int sm_count() {
 // the launch and for the estimate of how many CTAs an SM holds (ctas_per_sm_of).
 constexpr size_t dynamic_smem_bytes(int stages, int stage_bytes, bool gated_weight_major, bool tma_out, bool row_scales = false) {
   return (size_t)stages * stage_bytes + 1024 + 256 + (gated_weight_major ? XCH_BYTES : row_scales ? 256 + 16 : 0) +
-         (tma_out ? 2 * OUT_STAGE_BYTES + 128 : 0);
+         (tma_out ? 2 * OUT_STAGE_BYTES + 1024 : 0);
 }
+
+// Is there shared memory beside the ring for the token-major stores' staging?
+bool room_for_staging(int stages, int stage_bytes) { return dynamic_smem_bytes(stages, stage_bytes, false, true) <= 227 * 1024; }
 
 #ifdef IERT_GEMM_TRACE
 int g_trace_meta[TRACE_LAUNCHES][8];
@@ -958,7 +1059,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, GemmParams p, int grid,
   tm[0] = g_trace_next++; tm[1] = p.M; tm[2] = p.N; tm[3] = p.K; tm[4] = grid; tm[5] = BT; tm[6] = p.splits; tm[7] = p.mode;
 #endif
   constexpr int STAGE_BYTES = (GATED ? 2 : 1) * W_STAGE_BYTES + BT * TILE_K * 2;
-  const size_t smem = dynamic_smem_bytes(p.stages, STAGE_BYTES, !GATED && p.mode == MODE_GATED_SILU, p.tma_out != 0,
+  const size_t smem = dynamic_smem_bytes(p.stages, STAGE_BYTES, !GATED && p.mode == MODE_GATED_SILU, p.tma_out != 0 || p.tma_store != 0,
                                          p.scale.sumsq != nullptr);
   static bool configured = false;
   if (!configured) {
@@ -1055,7 +1156,7 @@ int gemm_tc_impl(const void* x, long long ldx, const void* w, long long ldw, voi
   if (bt != 16 && bt != 32 && bt != 64 && bt != 128 && bt != 256) return IERT_BAD_ARGUMENT;
 
   GemmParams p;
-  p.groups = nullptr; p.group_w_rows = p.group_k = 0; p.row_scale = nullptr;
+  p.tma_store = 0; p.groups = nullptr; p.group_w_rows = p.group_k = 0; p.row_scale = nullptr;
   p.scale = IertRowScale{nullptr, 0, 0, 0.f};
   p.ahead = IertNormAhead{nullptr, 0, nullptr, 0, nullptr, 0};
   if (scale) p.scale = *scale;
@@ -1082,7 +1183,9 @@ int gemm_tc_impl(const void* x, long long ldx, const void* w, long long ldw, voi
     CUtensorMap mw, mx;
     if (!tensor_map(w, N, K, ldw, TILE_N, &mw) || !tensor_map(x, M, K, ldx, 128, &mx)) return IERT_BAD_ARGUMENT;
     const int tiles = p.n_tiles * p.t_tiles;
-    return launch<128, true>(mw, mx, p, tiles < sm_count() ? tiles : sm_count(), stream);
+    CUtensorMap ms;
+    if (mode == MODE_STORE && room_for_staging(p.stages, stage_bytes) && tensor_map_store(out, M, N, ldo, out_dtype, &ms)) p.tma_store = 1;
+    return launch<128, true>(mw, mx, p, tiles < sm_count() ? tiles : sm_count(), stream, p.tma_store ? &ms : nullptr);
   }
   p.n_step = TILE_N; p.second_rows = 0;
   p.n_tiles = (N + TILE_N - 1) / TILE_N;
@@ -1146,7 +1249,7 @@ int gemm_tc_impl(const void* x, long long ldx, const void* w, long long ldw, voi
   // (no read of the residual by the SM).  Needs two staging buffers beside the ring.
   if (mode == MODE_ADD_RESIDUAL && bt >= 128 && splits == 1 && !no_tma_out() && tensor_map_out(out, M, N, ldo, &mo)) {
     int st = stages;
-    while (st >= 2 && (size_t)st * stage_bytes + 1280 + 2 * OUT_STAGE_BYTES + 128 > 227 * 1024) --st;
+    while (st >= 2 && (size_t)st * stage_bytes + 1280 + 2 * OUT_STAGE_BYTES + 1024 > 227 * 1024) --st;
     if (st >= 2 && (force_stages <= 0 || st == stages)) { p.tma_out = 1; stages = st; p.stages = st; }
   }
   int grid = total_work < slots ? total_work : slots;
@@ -1239,7 +1342,7 @@ int gemm_tc_gated_impl(const void* x, long long ldx, const void* w, long long ld
     return IERT_BAD_ARGUMENT;
   if (scale && (!scale->sumsq || scale->parts <= 0 || scale->hidden <= 0)) return IERT_BAD_ARGUMENT;
   GemmParams p;
-  p.groups = nullptr; p.group_w_rows = p.group_k = 0; p.row_scale = nullptr;
+  p.tma_store = 0; p.groups = nullptr; p.group_w_rows = p.group_k = 0; p.row_scale = nullptr;
   p.scale = IertRowScale{nullptr, 0, 0, 0.f};
   if (ep && (ep->act != IERT_ACT_NONE || !ep->scale || ep->blocks < 0 || ep->block_cols <= 0)) return IERT_BAD_ARGUMENT;
   if (up_rows < inter) return IERT_BAD_ARGUMENT;
@@ -1299,7 +1402,9 @@ int gemm_tc_gated_impl(const void* x, long long ldx, const void* w, long long ld
   CUtensorMap mw, mx;
   if (!tensor_map(w, (long long)up_rows + inter, K, ldw, TILE_N, &mw) || !tensor_map(x, M, K, ldx, bt, &mx)) return IERT_BAD_ARGUMENT;
   const int grid = tiles < slots ? tiles : slots;
-  return launch<128, true>(mw, mx, p, grid, stream);
+  CUtensorMap ms;
+  if (room_for_staging(p.stages, stage_bytes) && tensor_map_store(act, M, inter, ldo, IERT_BF16, &ms)) p.tma_store = 1;
+  return launch<128, true>(mw, mx, p, grid, stream, p.tma_store ? &ms : nullptr);
 }
 }  // namespace
 
@@ -1347,7 +1452,9 @@ IERT_API int iert_gemm_tc_grouped_gated(const void* x, long long ldx, const void
   if (!tensor_map(w, (long long)up_rows + (long long)experts * F, K, ldw, TILE_N, &mw) || !tensor_map(x, rows, K, ldx, 128, &mx))
     return IERT_BAD_ARGUMENT;
   const long long tiles = (long long)p.n_tiles * max_row_tiles;
-  return launch<128, true, true>(mw, mx, p, (int)(tiles < sm_count() ? tiles : sm_count()), stream);
+  CUtensorMap ms;
+  if (tensor_map_store(act, rows, F, ldo, IERT_BF16, &ms)) p.tma_store = 1;
+  return launch<128, true, true>(mw, mx, p, (int)(tiles < sm_count() ? tiles : sm_count()), stream, p.tma_store ? &ms : nullptr);
 }
 
 IERT_API int iert_gemm_tc_grouped(const void* x, long long ldx, const void* w, long long ldw, float* out, long long ldo, int rows,
@@ -1371,5 +1478,7 @@ IERT_API int iert_gemm_tc_grouped(const void* x, long long ldx, const void* w, l
   CUtensorMap mw, mx;
   if (!tensor_map(w, N, (long long)experts * K, ldw, TILE_N, &mw) || !tensor_map(x, rows, K, ldx, 128, &mx)) return IERT_BAD_ARGUMENT;
   const long long tiles = (long long)p.n_tiles * max_row_tiles;
-  return launch<128, true, true>(mw, mx, p, (int)(tiles < sm_count() ? tiles : sm_count()), stream);
+  CUtensorMap ms;
+  if (tensor_map_store(out, rows, N, ldo, IERT_F32, &ms)) p.tma_store = 1;
+  return launch<128, true, true>(mw, mx, p, (int)(tiles < sm_count() ? tiles : sm_count()), stream, p.tma_store ? &ms : nullptr);
 }

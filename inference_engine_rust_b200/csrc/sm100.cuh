@@ -91,6 +91,12 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, const 
                ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_addr(smem_src)), "r"(c0), "r"(c1)
                : "memory");
 }
+// The same as a plain store.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int c0, int c1) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_addr(smem_src)), "r"(c0), "r"(c1)
+               : "memory");
+}
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // At most N of this thread's bulk groups still read their shared-memory source.
 template <int N> __device__ __forceinline__ void bulk_wait_group_read() {

@@ -143,6 +143,34 @@ def test_token_major_kernel_in_every_mode(M, N, K):
     run(M, N, K, B.GEMM_ADD_RESIDUAL, torch.float32, force_stages=-1)
 
 
+@pytest.mark.parametrize("M,N", [(257, 16), (290, 331), (290, 336), (288, 1000), (385, 250), (1000, 2080)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_token_major_stores_by_tma_and_by_lanes_are_the_same_and_stay_inside(M, N, dtype):
+    """Rows that begin and end on 16 bytes leave in boxes through shared memory, others by lanes."""
+    from inference_engine_rust_b200.csrc import bindings as B
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x = torch.randn((M, 136), device=DEV, generator=g).bfloat16()
+    w = torch.randn((2 * N, 136), device=DEV, generator=g).bfloat16()
+    fac = torch.rand((M, 1), device=DEV, generator=g)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ep = B.epilogue("gelu", scale=fac)
+    for gated in (False, True):
+        if gated and dtype != torch.bfloat16:
+            continue
+        got = []
+        for ld in ((N + 15) // 8 * 8, (N + 15) // 8 * 8 + 1):
+            buf = torch.full((M + 40, ld), 7.0, dtype=dtype, device=DEV)
+            out = buf[:M, :N]
+            if gated:
+                assert B.gemm_tc_gated(x, w, out, M, err, B.stream_ptr(), force_bt=128)
+            else:
+                assert B.gemm_tc(x, w[:N], out, M, B.GEMM_STORE, err, B.stream_ptr(), epilogue=ep)
+            torch.cuda.synchronize()
+            assert err.item() == 0 and (buf[M:] == 7).all() and (buf[:, N:] == 7).all()
+            got.append(out.clone())
+        assert torch.equal(*got)
+
+
 @pytest.mark.parametrize("M", [65, 96, 128, 129, 200, 256, 257, 300, 384, 385, 512, 513])
 def test_between_decoding_and_prompts_at_layer_sizes(M):
     """65 to 513 tokens at the widths of a 7B layer, with the tile and the splits the kernel
