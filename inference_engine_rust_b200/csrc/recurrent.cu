@@ -190,22 +190,6 @@ constexpr int RING = 4;                                       // chunks in share
 // per token and head: 8 coefficients of earlier u in u_i, 8 in o_i, then G_i, G_8 / G_i, beta_i, G_8
 constexpr int COEF = 20;
 
-// Two fp32 numbers side by side: one instruction, each rounded as by fmaf.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(reinterpret_cast<unsigned long long&>(d))
-      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
-        "l"(reinterpret_cast<const unsigned long long&>(c)));
-  return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;"
-      : "=l"(reinterpret_cast<unsigned long long&>(d))
-      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
-  return d;
-}
 // A lane's rows 64 x + 4 r .. + 3 of a vector in shared memory.
 __device__ __forceinline__ void own_rows(float2 (&v)[CP], const float* src, int r) {
 #pragma unroll

@@ -18,6 +18,14 @@
 // two buffers in shared memory (as fp32, softplus applied): one barrier per chunk.  The lanes' partial sums of L tokens are added by a transposing reduction (L - 1 shuffles for
 // L tokens), after which lane r holds token r's sum and applies D, the gate and the rounding.  A short last chunk is
 // filled up with dt = 0, which changes no state.
+// With more CTAs than two per SM (DENSE; bfloat16, the usual 16 states or 8) others' warps hide what the batches ahead hide otherwise:
+// chunks of 16 tokens and 72 registers leave room for seven CTAs on an SM instead of four, so that 8,192 channels of four prompts run at
+// once instead of in two waves of which the second is not full; B and C stay bfloat16 in shared memory, whose reads (14 wavefronts a
+// warp and token as fp32, 10 so) were next to bound it.  8,192 channels, prompts of 1,024 tokens, before / chunks of 32 / dense:
+// one 100 / 97 / 98 us, two 169 / 158 / 152, four 287 / 266 / 244, sixteen 1,081 / 993 / 870; six prompts of 2,048 channels
+// (384 CTAs) 132 / 125 / 123, four of unequal lengths (256 CTAs) 164 / 154 / 162: hence two per SM.  At four prompts it issues in
+// 75 % of all cycles and the special-function unit is busy in 63 %.
+// States two by two (f32x2) and padded rows of u and z took 4 to 8 % off the other form (128 states: 611 -> 453 us).
 // L is chosen at the launch: what bounds a prompt is the rate of exponentials (one per token, channel and state), so
 // all that matters is enough warps per SM to keep that unit busy.
 //
@@ -25,6 +33,7 @@
 #include "common.cuh"
 
 #include <stdlib.h>
+#include <type_traits>
 
 using namespace iert;
 
@@ -32,7 +41,6 @@ namespace {
 
 constexpr int MAX_TAPS = 16;
 constexpr int THREADS = 128;
-constexpr int CHUNK = 32;
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
 // For results that are rounded to bfloat16.
@@ -58,6 +66,23 @@ template <typename T>
 __device__ __forceinline__ float decay_of(float dt, float A) {
   return sizeof(T) == 2 ? exp2_fast(dt * A) : 1.0f + expm1f(dt * A);
 }
+
+// States two by two (one instruction for both) where a lane holds an even number of them.
+__device__ __forceinline__ float times(float a, float b) { return a * b; }
+__device__ __forceinline__ float2 times(float a, float2 b) { return mul2(make_float2(a, a), b); }
+__device__ __forceinline__ float plus_times(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ float2 plus_times(float2 a, float2 b, float2 c) { return fma2(a, b, c); }
+__device__ __forceinline__ float both(float a) { return a; }
+__device__ __forceinline__ float both(float2 a) { return a.x + a.y; }
+template <typename T> __device__ __forceinline__ float decays_of(float dt, float A) { return decay_of<T>(dt, A); }
+template <typename T> __device__ __forceinline__ float2 decays_of(float dt, float2 A) {
+  if (sizeof(T) != 2) return make_float2(decay_of<T>(dt, A.x), decay_of<T>(dt, A.y));
+  const float2 x = times(dt, A);
+  return make_float2(exp2_fast(x.x), exp2_fast(x.y));
+}
+template <int SPL> struct StatesOf { typedef float2 type; static constexpr int N = SPL / 2; };
+template <> struct StatesOf<1> { typedef float type; static constexpr int N = 1; };
+template <> struct StatesOf<3> { typedef float type; static constexpr int N = 3; };
 
 // Four consecutive numbers; `vec`: aligned, else one by one below `n` (zeros beyond).
 __device__ __forceinline__ float4 load4(const float* p, bool vec, int n) {
@@ -223,29 +248,38 @@ struct ScanArgs {
   int C, N, vec, vec_bc;
 };
 
-constexpr size_t scan_smem_bytes(int L, int SPL) { return (size_t)2 * CHUNK * (4 * (THREADS / L) + 2 * L * SPL) * sizeof(float); }
+constexpr int scan_chunk(bool dense) { return dense ? 16 : 32; }
+// (u and z are read by lanes whose tokens differ: their rows are padded so that those meet in different banks)
+constexpr int scan_pad(int L) { return L == 4 ? 8 : L == 32 ? 0 : 4; }
+constexpr size_t scan_smem_bytes(int L, int SPL, bool dense) {
+  return (size_t)2 * scan_chunk(dense) * (4 * (THREADS / L) + 2 * scan_pad(L) + 2 * L * SPL) * sizeof(float);
+}
 
-template <typename T, int L, int SPL>
-__global__ void __launch_bounds__(THREADS) selective_scan_kernel(ScanArgs a, IertBatchView b) {
+template <typename T, int L, int SPL, bool DENSE>
+__global__ void __launch_bounds__(THREADS, DENSE ? 7 : sizeof(T) == 2 && L * SPL <= 64 ? 4 : 2) selective_scan_kernel(ScanArgs a, IertBatchView b) {
+  constexpr int CHUNK = scan_chunk(DENSE);
   constexpr int CH = THREADS / L;                      // channels of the CTA
+  constexpr int CHP = CH + scan_pad(L);
   constexpr int NP = L * SPL;                          // states, padded
   constexpr int Q = CH / 4;                            // runs of four channels in a row
   constexpr int ROWS_PT = CHUNK * Q / THREADS > 0 ? CHUNK * Q / THREADS : 1;      // such runs a thread fetches
   constexpr int BC_RUNS = CHUNK * 2 * NP / 4;          // runs of four numbers of B and C
   constexpr bool BC_AHEAD = NP <= 64;                  // small enough to fetch into registers ahead of time
   constexpr int BC_PT = BC_AHEAD ? (BC_RUNS + THREADS - 1) / THREADS : 1;
-  extern __shared__ __align__(16) float sm[];          // scan_smem_bytes(L, SPL)
+  extern __shared__ __align__(16) float sm[];          // scan_smem_bytes(L, SPL, DENSE)
   // two buffers of [dt and dt u | u | z, then the results | B | C], each CHUNK rows
-  constexpr int BUF = CHUNK * (4 * CH + 2 * NP);
+  constexpr int BUF = CHUNK * (2 * CH + 2 * CHP + 2 * NP);
   float2 (*d_s)[CH];
-  float (*u_s)[CH], (*z_s)[CH], (*b_s)[NP], (*c_s)[NP];
+  typedef typename std::conditional<DENSE, T, float>::type BC;     // B and C in shared memory (see own)
+  float (*u_s)[CHP], (*z_s)[CHP];
+  BC (*b_s)[NP], (*c_s)[NP];
   auto use = [&](int buf) {
     float* base = sm + buf * BUF;
     d_s = reinterpret_cast<float2 (*)[CH]>(base);
-    u_s = reinterpret_cast<float (*)[CH]>(base + 2 * CHUNK * CH);
-    z_s = reinterpret_cast<float (*)[CH]>(base + 3 * CHUNK * CH);
-    b_s = reinterpret_cast<float (*)[NP]>(base + 4 * CHUNK * CH);
-    c_s = reinterpret_cast<float (*)[NP]>(base + 4 * CHUNK * CH + CHUNK * NP);
+    u_s = reinterpret_cast<float (*)[CHP]>(base + 2 * CHUNK * CH);
+    z_s = reinterpret_cast<float (*)[CHP]>(base + 2 * CHUNK * CH + CHUNK * CHP);
+    b_s = reinterpret_cast<BC (*)[NP]>(base + 2 * CHUNK * (CH + CHP));
+    c_s = b_s + CHUNK;
   };
   pdl_launch_dependents();
   const int s = blockIdx.y;
@@ -255,11 +289,13 @@ __global__ void __launch_bounds__(THREADS) selective_scan_kernel(ScanArgs a, Ier
   const int tid = threadIdx.x, r = tid % L, ch = tid / L;
   const int c0 = blockIdx.x * CH, c = c0 + ch;
   const bool live = c < a.C;
-  float A2[SPL], S[SPL];
+  typedef typename StatesOf<SPL>::type V;
+  constexpr int NV = StatesOf<SPL>::N, W = SPL / NV;    // W: states of a V
+  V A[NV], S[NV];
 #pragma unroll
   for (int i = 0; i < SPL; ++i) {
     const int n = r * SPL + i;
-    A2[i] = live && n < a.N ? a.A2[(size_t)c * a.N + n] : 0.f;
+    reinterpret_cast<float*>(A)[i] = live && n < a.N ? a.A2[(size_t)c * a.N + n] : 0.f;
   }
   const float Dc = live ? a.D[c] : 0.f;
   // the channels whose numbers this thread brings in are the same for all tokens
@@ -271,7 +307,7 @@ __global__ void __launch_bounds__(THREADS) selective_scan_kernel(ScanArgs a, Ier
 #pragma unroll
   for (int i = 0; i < SPL; ++i) {
     const int n = r * SPL + i;
-    S[i] = live && n < a.N ? Sg[n] : 0.f;
+    reinterpret_cast<float*>(S)[i] = live && n < a.N ? Sg[n] : 0.f;
   }
   const T* u = (const T*)a.u;
   const T* z = (const T*)a.z;
@@ -329,10 +365,10 @@ __global__ void __launch_bounds__(THREADS) selective_scan_kernel(ScanArgs a, Ier
       }
     }
     auto put_bc = [&](int x, const Raw& raw) {
-      const float4 v = widen(raw);
       const int tt = x / (2 * NP / 4), q = x - tt * (2 * NP / 4);
-      if (q >= NP / 4) *reinterpret_cast<float4*>(&c_s[tt][4 * (q - NP / 4)]) = v;
-      else *reinterpret_cast<float4*>(&b_s[tt][4 * q]) = v;
+      BC* to = q >= NP / 4 ? &c_s[tt][4 * (q - NP / 4)] : &b_s[tt][4 * q];
+      if constexpr (DENSE) *reinterpret_cast<Raw*>(to) = raw;
+      else *reinterpret_cast<float4*>(to) = widen(raw);
     };
     if (BC_AHEAD) {
 #pragma unroll
@@ -345,20 +381,40 @@ __global__ void __launch_bounds__(THREADS) selective_scan_kernel(ScanArgs a, Ier
     }
   };
   static_assert(NP % 4 == 0, "L is a multiple of 4");
-  // What the chain of J tokens needs and no state enters: made one batch of tokens ahead of the chain, so that the shared
-  // memory and the exponentials answer while the chain of the batch in front runs.
+  // A lane's numbers of a row of B or C.
+  auto own = [&](V (&v)[NV], const BC (&row)[NP]) {
+    if constexpr (DENSE) {
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(&row[r * SPL]);
+      uint32_t x[NV];
+      if constexpr (NV == 2) *reinterpret_cast<uint2*>(x) = *reinterpret_cast<const uint2*>(w);
+      else x[0] = w[0];
+#pragma unroll
+      for (int i = 0; i < NV; ++i) v[i] = make_float2(__uint_as_float(x[i] << 16), __uint_as_float(x[i] & 0xffff0000u));
+    } else if constexpr (SPL % 4 == 0) {
+#pragma unroll
+      for (int i = 0; i < SPL / 4; ++i) *reinterpret_cast<float4*>(&v[2 * i]) = *reinterpret_cast<const float4*>(&row[r * SPL + 4 * i]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) v[i] = *reinterpret_cast<const V*>(&row[r * SPL + W * i]);
+    }
+  };
+  // What the chain of J tokens needs and no state enters: with few warps on an SM made one batch of tokens ahead of the chain, so
+  // that the shared memory and the exponentials answer while the chain of the batch in front runs.
   constexpr int WANT = SPL >= 6 ? 2 : SPL >= 3 ? 4 : SPL == 2 ? 8 : 16;
-  constexpr int J = WANT < L ? WANT : L;
-  struct Ahead { float decay[J][SPL], in[J][SPL], out[J][SPL]; };
+  constexpr int J = DENSE ? 1 : WANT < L ? WANT : L;
+  struct alignas(16) Ahead { V decay[J][NV], in[J][NV], out[J][NV]; };
   auto prepare = [&](Ahead& x, int row) {
 #pragma unroll
     for (int j = 0; j < J; ++j) {
       const float2 d = d_s[row + j][ch];
+      alignas(16) V in[NV], to[NV];
+      own(in, b_s[row + j]);
+      own(to, c_s[row + j]);
 #pragma unroll
-      for (int i = 0; i < SPL; ++i) {
-        x.decay[j][i] = decay_of<T>(d.x, A2[i]);
-        x.in[j][i] = d.y * b_s[row + j][r * SPL + i];
-        x.out[j][i] = c_s[row + j][r * SPL + i];
+      for (int i = 0; i < NV; ++i) {
+        x.decay[j][i] = decays_of<T>(d.x, A[i]);
+        x.in[j][i] = times(d.y, in[i]);
+        x.out[j][i] = to[i];
       }
     }
   };
@@ -382,25 +438,26 @@ __global__ void __launch_bounds__(THREADS) selective_scan_kernel(ScanArgs a, Ier
     if (tc + CHUNK < t1) fetch(tc + CHUNK);
     use(buf);
     Ahead cur;
-    prepare(cur, 0);
-#pragma unroll 2
+    if (!DENSE) prepare(cur, 0);
+#pragma unroll (DENSE ? 1 : 2)
     for (int g = 0; g < CHUNK; g += L) {
       float y[L];
 #pragma unroll
       for (int h = 0; h < L; h += J) {
         Ahead nxt;
-        prepare(nxt, min(g + h + J, CHUNK - J));       // (behind the chunk's last tokens: again those, for nothing)
+        if (DENSE) prepare(cur, g + h);
+        else prepare(nxt, min(g + h + J, CHUNK - J));  // (behind the chunk's last tokens: again those, for nothing)
 #pragma unroll
         for (int j = 0; j < J; ++j) {
-          float acc = 0.f;
+          V acc{};
 #pragma unroll
-          for (int i = 0; i < SPL; ++i) {
-            S[i] = fmaf(cur.decay[j][i], S[i], cur.in[j][i]);
-            acc = fmaf(S[i], cur.out[j][i], acc);
+          for (int i = 0; i < NV; ++i) {
+            S[i] = plus_times(cur.decay[j][i], S[i], cur.in[j][i]);
+            acc = plus_times(S[i], cur.out[j][i], acc);
           }
-          y[h + j] = acc;
+          y[h + j] = both(acc);
         }
-        cur = nxt;
+        if (!DENSE) cur = nxt;
       }
 #pragma unroll
       for (int o = L / 2; o > 0; o >>= 1) {
@@ -427,7 +484,7 @@ __global__ void __launch_bounds__(THREADS) selective_scan_kernel(ScanArgs a, Ier
 #pragma unroll
     for (int i = 0; i < SPL; ++i) {
       const int n = r * SPL + i;
-      if (n < a.N) Sg[n] = S[i];
+      if (n < a.N) Sg[n] = reinterpret_cast<const float*>(S)[i];
     }
   }
 }
@@ -481,16 +538,19 @@ int states_per_lane(int N, int L) {
   return 0;
 }
 
-template <typename T, int L, int SPL>
+template <typename T, int L, int SPL, bool DENSE = false>
 bool launch_scan_as(dim3 grid, cudaStream_t stream, const ScanArgs& a, const IertBatchView& b) {
-  constexpr size_t smem = scan_smem_bytes(L, SPL);
+  if constexpr (!DENSE && sizeof(T) == 2 && L == 4 && (SPL == 2 || SPL == 4)) {
+    if ((long long)grid.x * grid.y > 2LL * iert_sm_count_cached()) return launch_scan_as<T, L, SPL, true>(grid, stream, a, b);
+  }
+  constexpr size_t smem = scan_smem_bytes(L, SPL, DENSE);
   if (smem > 48 * 1024) {
     static bool configured = false;
-    if (!configured && cudaFuncSetAttribute(selective_scan_kernel<T, L, SPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (!configured && cudaFuncSetAttribute(selective_scan_kernel<T, L, SPL, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return false;
     configured = true;
   }
-  launch_dep(selective_scan_kernel<T, L, SPL>, grid, dim3(THREADS), smem, stream, a, b);
+  launch_dep(selective_scan_kernel<T, L, SPL, DENSE>, grid, dim3(THREADS), smem, stream, a, b);
   return true;
 }
 

@@ -363,6 +363,37 @@ def test_selective_convolution_and_scan(monkeypatch, C, N, K, lanes):
                 torch.testing.assert_close(S / want[s][1].abs().max(), want[s][1] / want[s][1].abs().max(), rtol=2e-2 if dtype == torch.bfloat16 else 1e-4, atol=2e-3 if dtype == torch.bfloat16 else 1e-5)
 
 
+@pytest.mark.parametrize("C,N", [(4800, 16), (4801, 13), (4802, 7)])
+def test_selective_scan_of_many_channels(C, N):
+    """So many channels that an SM holds more than two blocks: lengths around the chunk of 16 tokens, channels and states that
+    fill no run of four, a second call that goes on."""
+    b = B()
+    g = torch.Generator().manual_seed(C)
+    slots, plans = [1, 0, 2], ([16, 1, 33], [17, 2, 15])
+    A, D, db = -torch.exp(torch.randn(C, N, generator=g)), torch.randn(C, generator=g), torch.linspace(-8, 2, C)
+    state = torch.zeros(3, C * N, device=DEV)
+    S = [None] * 3
+    past = [[] for _ in slots]
+    for plan in plans:
+        bt = Batch(plan, [0] * 3, slots)
+        T = sum(plan)
+        u, z, bc, raw = (torch.randn(T, w, generator=g) for w in (C, C + 4, 2 * N + 8, C))
+        u, z, bc = (t.to(torch.bfloat16) for t in (u, z, bc))
+        out = torch.full((bt.n_tokens, C), float("nan"), dtype=torch.bfloat16, device=DEV)
+        b.selective_scan(u.to(DEV), raw.to(DEV), db.to(DEV), bc.to(DEV), z.to(DEV), (A * math.log2(math.e)).to(DEV), D.to(DEV), state, 0, out,
+                         C, N, False, bt.view, stream())
+        at = 0
+        for i, n in enumerate(plan):
+            past[i].append(tuple(t[at:at + n] for t in (u.float(), P.softplus(raw + db), bc.float())))
+            cu, cd, cb = (torch.cat(t) for t in zip(*past[i]))
+            y, S[i] = P.selective_scan(cu, cd, A, cb[:, :N], cb[:, N:2 * N], D)
+            ref = y[-n:] * P.silu(z[at:at + n, :C].float())
+            torch.testing.assert_close(out[at:at + n].float().cpu() / ref.abs().max(), ref / ref.abs().max(), rtol=2.0 ** -8, atol=1e-4)
+            at += n
+    for i, slot in enumerate(slots):
+        torch.testing.assert_close(state[slot].view(C, N).cpu(), S[i], rtol=1e-4, atol=1e-4)
+
+
 @pytest.mark.parametrize("D", [48, 64, 128, 192])
 @pytest.mark.parametrize("softness", [1.0, 4.0])
 def test_prompt_attention_with_sinks(D, softness):
