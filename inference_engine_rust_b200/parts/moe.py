@@ -48,7 +48,8 @@ SKINNY_ROUTER_MIN_TOKENS = 32
 ROUTER_STEP_MAX_TOKENS = 64
 # Prompts of at least this many tokens run the experts' products over the tokens that chose them, if that is less than half of
 # the rows that all experts over all tokens would have.  (16 experts at 7B sizes, grouped against all experts, two chosen and a
-# shared one: 256 tokens 149 / 122 us, 384: 143 / 161, 2,048: 273 / 520; four chosen: 384: 129 / 184, 2,048: 324 / 526.)
+# shared one: 256 tokens 149 / 122 us, 384: 143 / 161, 2,048: 273 / 520; four chosen: 384: 129 / 184, 2,048: 324 / 526.
+# All before the grouped products stored by TMA, which takes 15 us off them at 2,048 tokens.)
 GROUPED_MIN_TOKENS = 384
 # ... in portions of this many tokens, which bounds the sorted rows and their results in memory.
 GROUPED_MAX_TOKENS = 8192
