@@ -436,7 +436,14 @@ __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
   for (int i = 0; i < 4; ++i) { const float2 two = __bfloat1622float2(p[i]); f[2 * i] = two.x; f[2 * i + 1] = two.y; }
 }
 size_t absorb_wide_smem(int tt, int D, int rank) { return (size_t)D * rank * 2 + (size_t)tt * (D + 4) * 4; }
-size_t merge_wide_smem(int tt, int rank) { return (size_t)128 * (rank + 8) * 2 + (size_t)tt * (rank + 4) * 4 + (size_t)tt * 64 * 4; }
+// Of the merge, in bytes: the head's weights [128][rank + 8] from 0 on, then the merged rows [tt][rank + 4] at `lat` and the runs' weights
+// [tt][64] at `wgt`.  At the end the sums of three quarters of the rank, [3][tt][128], take the place of all of them; below a rank of
+// about 64 they are what needs the most.
+struct MergeWideSmem { int lat, wgt, total; };
+__host__ __device__ constexpr MergeWideSmem merge_wide_smem(int tt, int rank) {
+  const int lat = 128 * (rank + 8) * 2, wgt = lat + tt * (rank + 4) * 4, end = wgt + tt * 64 * 4, sums = 3 * tt * 128 * 4;
+  return {lat, wgt, end > sums ? end : sums};
+}
 
 // qa[t, h, :] = sum_d q[t, h, d] W_uk[h*D + d, :] and the rotated part, as above.  64 threads across the rank (eight columns each), four
 // groups of TT / 4 tokens.
@@ -532,9 +539,10 @@ latent_merge_wide_kernel(const float* __restrict__ part_m, const float* __restri
                          const __nv_bfloat16* __restrict__ w_uv, __nv_bfloat16* __restrict__ out, IertBatchView b, int H, int V) {
   extern __shared__ __align__(16) uint8_t wide_smem[];
   const int ldw = rank + 8, ldl = rank + 4;
+  const MergeWideSmem at = merge_wide_smem(TT, rank);
   __nv_bfloat16* w_s = reinterpret_cast<__nv_bfloat16*>(wide_smem);            // [128][ldw]
-  float* lat = reinterpret_cast<float*>(wide_smem + (size_t)128 * ldw * 2);    // [TT][ldl]
-  float* wgt = lat + TT * ldl;                                                 // [TT][64]
+  float* lat = reinterpret_cast<float*>(wide_smem + at.lat);                   // [TT][ldl]
+  float* wgt = reinterpret_cast<float*>(wide_smem + at.wgt);                   // [TT][64]
   pdl_launch_dependents();
   const int t0 = blockIdx.x * TT, h = blockIdx.y, e0 = blockIdx.z * 128, n_t = min(TT, b.n_seqs - t0), n_e = min(128, V - e0);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r8 = rank / 8;
@@ -628,7 +636,7 @@ latent_merge_wide_kernel(const float* __restrict__ part_m, const float* __restri
     }
   }
   __syncthreads();                                               // nobody reads the weights any more
-  float* red = reinterpret_cast<float*>(wide_smem);              // [3][TT][128], where they were
+  float* red = reinterpret_cast<float*>(wide_smem);              // [3][TT][128], where all of it was (merge_wide_smem has room)
   if (quarter > 0) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -716,6 +724,9 @@ IERT_API int iert_latent_decode_tc_plan(int n_seqs, int H, int rank, int R, int 
   return IERT_OK;
 }
 
+// The wide merge's shared memory for `tt` sequences a block (bytes).
+IERT_API int iert_latent_merge_wide_smem(int tt, int rank) { return merge_wide_smem(tt, rank).total; }
+
 // q [T, ldq] (H*(D+R) per token, one token per sequence: per head D unrotated and R rotated numbers), bf16 with the rotated
 // numbers turned already, or with q_f32 != 0 fp32 as projected (turned here by inv_freq, rot_mul and pairing); the cache's
 // rows are rank + R wide (latent | rotated key part); w_uk [H*D, rank], w_uv [H*V, rank] bf16 row-major; gate: fp32 [T, H]
@@ -753,7 +764,7 @@ IERT_API int iert_latent_attention_decode_tc(const void* q, int q_f32, long long
   const int wide = T > 32 ? 16 : 8;
   const bool wide_absorb = T > 16 && D % 4 == 0 && R % 8 == 0 && ((uintptr_t)w_uk & 15) == 0 && ((uintptr_t)qa & 15) == 0 &&
                            absorb_wide_smem(wide, D, rank) <= WIDE_SMEM;
-  const bool wide_merge = T > 16 && ((uintptr_t)w_uv & 15) == 0 && merge_wide_smem(wide, rank) <= WIDE_SMEM;
+  const bool wide_merge = T > 16 && ((uintptr_t)w_uv & 15) == 0 && (size_t)merge_wide_smem(wide, rank).total <= WIDE_SMEM;
   if (!wide_configured()) return IERT_CUDA_ERROR;
 #define ABSORB_WIDE(TQ, TT)                                                                                                        \
   launch_dep(latent_absorb_wide_kernel<TQ, TT>, dim3((T + TT - 1) / TT, Hpad), dim3(WIDE_THREADS), absorb_wide_smem(TT, D, rank), stream, (const TQ*)q, \
@@ -783,7 +794,7 @@ IERT_API int iert_latent_attention_decode_tc(const void* q, int q_f32, long long
              (size_t)TT * (rank + 64) * sizeof(float), stream, (const float*)part_m, (const float*)part_l, (const float*)part_acc, splits, \
              Hpad, rank, sink, gate, (const __nv_bfloat16*)w_uv, (__nv_bfloat16*)out, *batch, H, V)
 #define MERGE_WIDE(TT)                                                                                                             \
-  launch_dep(latent_merge_wide_kernel<TT>, dim3((T + TT - 1) / TT, H, (V + 127) / 128), dim3(WIDE_THREADS), merge_wide_smem(TT, rank), stream, \
+  launch_dep(latent_merge_wide_kernel<TT>, dim3((T + TT - 1) / TT, H, (V + 127) / 128), dim3(WIDE_THREADS), (size_t)merge_wide_smem(TT, rank).total, stream, \
              (const float*)part_m, (const float*)part_l, (const float*)part_acc, splits, Hpad, rank, sink, gate, (const __nv_bfloat16*)w_uv, \
              (__nv_bfloat16*)out, *batch, H, V)
   if (wide_merge && wide == 8) MERGE_WIDE(8);
