@@ -1,18 +1,20 @@
-// Projection of a 32-bit run on the tensor cores: out[t, n] = sum_k x[t, k] w[n, k], all fp32, with an error against
-// exact arithmetic no larger than that of the one-accumulator fp32 sum of gemm_plain.cu (which stays for what this
+// Projection of a 32-bit run on the tensor cores: out[t, n] = sum_k x[t, k] w[n, k], all fp32, for the inner axes at which
+// its error against exact arithmetic is well below that of the one-accumulator fp32 sum of gemm_plain.cu (which stays for what this
 // kernel does not take).
 //
-// An fp32 number is the exact sum of three bf16 numbers of 8 mantissa bits each (its bits cut off after 8, then the
-// remainder's, then what is left: no rounding anywhere), so x w is the exact sum of nine bf16 products.  Six are formed on
-// tcgen05 (the other three are below 2^-23 of the product).  The tensor core adds with a few bits less care than an fp32
+// An fp32 number is the sum of three bf16 numbers: the nearest one, the nearest to the remainder, and what is left (exactly, unless it
+// falls below 2^-133, bf16's smallest number), so x w is the sum of nine bf16 products.  Six are formed on tcgen05; the other three come to
+// 2^-24 of the product at most, of either sign.  (Parts cut off instead of rounded left up to 2^-21, always of the product's sign: rows with
+// one number among zeros had 2.5 times the plain kernel's error.)  The tensor core adds with a few bits less care than an fp32
 // addition, so no sum stays there for long: the products of 64 k are summed in tensor memory and then added to fp32 registers
 // by ordinary rounded additions, K / 64 of them per output; the main product (first part times first part) has a tensor-memory
 // sum of its own, so that few additions there meet a sum as large as the result.  Relative error (2-norm) against 64 bits, this
-// kernel / gemm_plain.cu: K of 1,024: 1.3e-7 / 5.7e-7 (1.2e-7 / 4.6e-7 where all numbers are positive); 4,096: 1.9e-7 / 1.2e-6;
-// 14,336: 1.8e-7 / 2.2e-6.
+// kernel / gemm_plain.cu: K of 1,024: 9.0e-8 / 5.8e-7 (8.9e-8 / 5.0e-7 where all numbers are positive); 4,096: 1.1e-7 / 1.2e-6;
+// 14,336: 1.6e-7 / 2.2e-6.  Sums that are short because nearly all of a row is zero have the same error in both: one number in a row
+// 2.6e-8 / 2.5e-8, eight 5.5e-8 / 5.3e-8 (with the two next products as well 2.5e-8 and 5.5e-8, and a tenth more time).
 //
-// Measured (gemm_plain.cu in brackets): 333 tokens x 28,672 x 4,096 0.79 ms (4.42), 333 x 4,096 x 14,336 0.43 ms (2.47), one token
-// x 28,672 x 4,096 0.27 ms (0.97), x 4,096 x 14,336 0.12 ms (2.39).  What bounds it is the chain of a block (copy, split, MMAs, read
+// Measured (gemm_plain.cu in brackets): 333 tokens x 28,672 x 4,096 0.81 ms (4.43), 333 x 4,096 x 14,336 0.43 ms (2.46), one token
+// x 28,672 x 4,096 0.27 ms (0.96), x 4,096 x 14,336 0.12 ms (2.38).  What bounds it is the chain of a block (copy, split, MMAs, read
 // back: about 2,400 cycles for 128 tokens); the six products alone are 768.  An 8 x 8 register tile of fp32 multiply-adds reached
 // 2.1 ms on the first of these sizes: shared memory returns one operand word per lane and cycle, which that tile needs in full.
 //
@@ -61,20 +63,23 @@ __device__ __forceinline__ float ld_cluster(uint32_t addr, int rank) {
   return v;
 }
 
-// Eight fp32 numbers into three 16-byte runs of bf16: parts by truncation, each remainder exact.
+// Eight fp32 numbers into three 16-byte runs of bf16: every part the nearest to what is left, every remainder exact.
 __device__ __forceinline__ void split8(const float4& a, const float4& b, uint4& p0, uint4& p1, uint4& p2) {
   const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
   uint32_t* o0 = reinterpret_cast<uint32_t*>(&p0);
   uint32_t* o1 = reinterpret_cast<uint32_t*>(&p1);
   uint32_t* o2 = reinterpret_cast<uint32_t*>(&p2);
+  auto nearest = [](float x, float y) {
+    const __nv_bfloat162 two = __floats2bfloat162_rn(x, y);
+    return *reinterpret_cast<const uint32_t*>(&two);
+  };
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float x = v[2 * i], y = v[2 * i + 1];
-    const float xr = x - __uint_as_float(__float_as_uint(x) & 0xffff0000u), yr = y - __uint_as_float(__float_as_uint(y) & 0xffff0000u);
-    const float xs = xr - __uint_as_float(__float_as_uint(xr) & 0xffff0000u), ys = yr - __uint_as_float(__float_as_uint(yr) & 0xffff0000u);
-    o0[i] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
-    o1[i] = __byte_perm(__float_as_uint(xr), __float_as_uint(yr), 0x7632);
-    o2[i] = __byte_perm(__float_as_uint(xs), __float_as_uint(ys), 0x7632);
+    o0[i] = nearest(x, y);
+    const float xr = x - __uint_as_float(o0[i] << 16), yr = y - __uint_as_float(o0[i] & 0xffff0000u);
+    o1[i] = nearest(xr, yr);
+    o2[i] = nearest(xr - __uint_as_float(o1[i] << 16), yr - __uint_as_float(o1[i] & 0xffff0000u));
   }
 }
 

@@ -62,3 +62,40 @@ def test_infinities_and_nan():
         assert torch.equal(same(a), same(b))
     fine = torch.isfinite(a)
     assert ((a - b)[fine].abs() <= 1e-4 * a[fine].abs().max()).all()
+
+
+@pytest.mark.parametrize("K", [1024, 4100])
+@pytest.mark.parametrize("kind", ["one number", "eight numbers", "one large number", "positive", "cut remainders", "rounded remainders"])
+def test_error_beside_the_plain_kernel(kind, K):
+    """Sums in which one product counts, or all have one sign: no further from 64 bits than one fp32 sum is."""
+    from inference_engine_rust_b200.csrc import bindings as B
+    torch.manual_seed(K)
+    M, N = 40, 300
+    x, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    # mantissas that parts cut off instead of rounded would serve worst
+    odd = torch.tensor([0x3f80ffff, 0x3f807fff, 0x3f8080ff, 0x3f817f7f], dtype=torch.int32, device=DEV).view(torch.float32)
+    if kind.endswith("numbers") or kind == "one number":
+        n = 1 if kind == "one number" else 8
+        keep = torch.zeros(M, K, device=DEV).scatter_(1, torch.rand(M, K, device=DEV).topk(n, dim=1).indices, 1.0)
+        x = x * keep
+        w[::2] = odd[torch.randint(0, 4, (N // 2, K), device=DEV)]
+        x[::2] = keep[::2] * odd[torch.randint(0, 4, (M // 2, K), device=DEV)]
+    elif kind == "one large number":
+        x *= 1e-4
+        x[:, 17] = 50.0 + torch.randn(M, device=DEV)
+    elif kind == "positive":
+        x, w = x.abs(), w.abs()
+    elif kind == "cut remainders":
+        x, w = odd[torch.randint(0, 4, (M, K), device=DEV)], odd[torch.randint(0, 4, (N, K), device=DEV)]
+    else:            # the largest remainders after rounding: 1 + 2^-8 - 2^-16 + 2^-17 - 2^-23, alone in its row
+        x, w = torch.zeros(M, K, device=DEV), torch.full((N, K), 0x3f807f3f, dtype=torch.int32, device=DEV).view(torch.float32)
+        x[:, 70] = w[0, 0]
+    tc, plain = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    assert run(x, w, tc, M)
+    B.gemm_plain(x, w, plain, M, 0, B.stream_ptr())
+    ref = x.double() @ w.double().t()
+    off, beside = (tc - ref).norm(), (plain - ref).norm()
+    # one product: a rounding of 2^-24 in both kernels, and here the products left out: 2^-24 at most, mostly far less
+    assert off <= (beside + 2.0 ** -24 * ref.norm() if kind == "rounded remainders" else 1.1 * beside)
+    if kind in ("one number", "rounded remainders"):
+        assert ((tc - ref).abs() <= 2.0 ** -23 * ref.abs()).all()
