@@ -306,11 +306,11 @@ struct WorkIter {
 // Where a tile lies: first output column and first token row, the end of the valid rows, and where its weights start in w.
 struct TilePlace { int n_idx, n0, t0, t_end, w_row, w_col; };
 template <int BT, bool GROUPED>
-__device__ __forceinline__ TilePlace tile_place(const GemmParams& p, int tile, int t_tiles) {
+__device__ __forceinline__ TilePlace tile_place(const GemmParams& p, int tile, int group_tiles) {
   TilePlace c;
   if (GROUPED) {                         // the row tiles run fastest: an expert's weights are read by all its row tiles at once
-    c.n_idx = tile / t_tiles;
-    const int* g = p.groups + 2 + 3 * (tile - c.n_idx * t_tiles);
+    c.n_idx = tile / group_tiles;
+    const int* g = p.groups + 2 + 3 * (tile - c.n_idx * group_tiles);
     const int e = __ldg(g);
     c.n0 = c.n_idx * p.n_step;
     c.t0 = __ldg(g + 1);
@@ -357,7 +357,10 @@ struct StageStore {
   }
 };
 
-template <int BT, bool GATED, bool GROUPED = false>
+// FACTORS (gated launches): a factor per token and block of columns (p.ep).  A form of its own, since the dense feed-forwards have none:
+// with the factors' loads and the unrolled epilogue in their kernel, and the number of token tiles in a register instead of the parameters,
+// they took up to 1.7 us longer (64 tokens x 28,672 x 4,096 45.7 us, so 47.4).
+template <int BT, bool GATED, bool GROUPED = false, bool FACTORS = false>
 __global__ void __launch_bounds__(THREADS, 2)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                const __grid_constant__ CUtensorMap map_o, const GemmParams p) {
@@ -403,7 +406,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   if (threadIdx.x == 0) pdl_launch_dependents();
   if (threadIdx.x == 0) IERT_TRACE(0);                       // start
   if (GROUPED) pdl_wait();                                   // the table of row tiles comes from a kernel in front
-  const int t_tiles = GROUPED ? __ldg(p.groups) : p.t_tiles;
+  const int group_tiles = GROUPED ? __ldg(p.groups) : 0;
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -415,10 +418,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       uint32_t phase = 0;
       bool ok = true, dep_ready = GROUPED;
       int pend_kb[12], pend_t0[12];
-      WorkIter it(p, t_tiles);
+      WorkIter it(p, GROUPED ? group_tiles : p.t_tiles);
       int tile, split, n_parts, kb0, kb1;
       while (ok && it.next(tile, split, n_parts, kb0, kb1)) {
-        const TilePlace at = tile_place<BT, GROUPED>(p, tile, t_tiles);
+        const TilePlace at = tile_place<BT, GROUPED>(p, tile, group_tiles);
         const int t0 = at.t0, w_row = at.w_row, w_col = at.w_col;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!dep_ready && issued == stages) {
@@ -468,7 +471,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
-      WorkIter it(p, t_tiles);
+      WorkIter it(p, GROUPED ? group_tiles : p.t_tiles);
       int tile, split, n_parts, kb0, kb1;
       while (ok && it.next(tile, split, n_parts, kb0, kb1)) {
         if (!wait_or_abort(&acc_empty[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
@@ -518,18 +521,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     bool ok = true;
     StageStore stage_out{&map_o, out_s + q * 8192, lane, 0, 0};
     if (GATED && p.tma_store && threadIdx.x == 64) tma_prefetch_desc(&map_o);
-    WorkIter it(p, t_tiles);
+    WorkIter it(p, GROUPED ? group_tiles : p.t_tiles);
     int tile, split, n_parts, kb0, kb1;
     while (ok && it.next(tile, split, n_parts, kb0, kb1)) {
-      const TilePlace at = tile_place<BT, GROUPED>(p, tile, t_tiles);
+      const TilePlace at = tile_place<BT, GROUPED>(p, tile, group_tiles);
       const int n_idx = at.n_idx, n0 = at.n0, t0 = at.t0, t_end = at.t_end;
       const int n = n0 + n_local;
       const int t_valid = min(BT, t_end - t0);
       // (weight-major gated tiles: the columns' factors are asked for while the weights stream)
-      constexpr int N_FACTORS = !GATED && BT <= 32 ? BT : 1;
+      constexpr int N_FACTORS = FACTORS && !GATED && BT <= 32 ? BT : 1;
       float factor[N_FACTORS];
       const float* factor_col = nullptr;
-      if (!GATED && p.mode == MODE_GATED_SILU && p.ep.scale && q < 2) {
+      if (FACTORS && !GATED && q < 2) {
         factor_col = p.ep.scale + (long long)t0 * p.ep.ld_scale + epilogue_block(n0 + n_local, p.ep);
 #pragma unroll
         for (int j = 0; j < N_FACTORS; ++j) factor[j] = j < t_valid ? factor_col[(long long)j * p.ep.ld_scale] : 0.f;
@@ -568,7 +571,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           if (staged) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = GROUPED ? silu_mul(v[j], u[j]) * row_factor : silu_mul(v[j], u[j]);
-            if (!GROUPED && p.ep.scale && tok < t_end) epilogue_run<16>(v, tok, n0 + c, p.ep);
+            if (FACTORS && tok < t_end) epilogue_run<16>(v, tok, n0 + c, p.ep);
             uint4 w2[2];
             __nv_bfloat162* wp = reinterpret_cast<__nv_bfloat162*>(w2);
 #pragma unroll
@@ -581,7 +584,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             __nv_bfloat16* o = (__nv_bfloat16*)p.out + (long long)tok * p.ldo + n0 + c;
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = GROUPED ? silu_mul(v[j], u[j]) * row_factor : silu_mul(v[j], u[j]);
-            if (!GROUPED && p.ep.scale) epilogue_run<16>(v, tok, n0 + c, p.ep);
+            if (FACTORS) epilogue_run<16>(v, tok, n0 + c, p.ep);
             if (n0 + c + 16 <= p.N && (p.ldo & 7) == 0 && ((uintptr_t)p.out & 15) == 0) {
               uint4 w2[2];
               __nv_bfloat162* wp = reinterpret_cast<__nv_bfloat162*>(w2);
@@ -671,9 +674,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         // that belong to them.  The up warps hand their values over through shared memory, the
         // gate warps write silu(gate) * up, 64 consecutive outputs of a token per pair of warps.
         float* xch = reinterpret_cast<float*>(xch_s);                 // [16 tokens][64]
-#pragma unroll
-        for (int c = 0; c < BT; c += 16) {
-          if (c >= t_valid) break;                   // uniform over the four warps
+        auto sixteen = [&](int c) {
           float v[16];
           tmem_ld16(taddr + c, v);
           if (q >= 2) {
@@ -689,12 +690,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 if (c + j < t_valid) {
                   const float r = scaled ? rstd_s[c + j] : 1.0f;
                   float act = silu_mul(v[j] * r, xch[j * 64 + n_local] * r);
-                  if (factor_col) act *= N_FACTORS > 1 ? factor[(c + j) % N_FACTORS] : factor_col[(long long)(c + j) * p.ep.ld_scale];
+                  if (FACTORS) act *= N_FACTORS > 1 ? factor[(c + j) % N_FACTORS] : factor_col[(long long)(c + j) * p.ep.ld_scale];
                   ((__nv_bfloat16*)p.out)[(long long)(t0 + c + j) * p.ldo + i] = __float2bfloat16_rn(act);
                 }
             }
           }
           asm volatile("bar.sync 1, 128;" ::: "memory");
+        };
+        if constexpr (FACTORS) {                     // unrolled: the factors are in registers
+#pragma unroll
+          for (int c = 0; c < BT; c += 16)
+            if (c < t_valid) sixteen(c);             // uniform over the four warps
+        } else {
+#pragma unroll 1
+          for (int c = 0; c < t_valid; c += 16) sixteen(c);
         }
       }
       // Many tokens, residual add, whole tile: 32 tokens per pass, so that twice as many reads of
@@ -1048,7 +1057,7 @@ int g_trace_next = 0;
 
 uint32_t g_poll_limit = WAIT_LIMIT;
 
-template <int BT, bool GATED, bool GROUPED = false>
+template <int BT, bool GATED, bool GROUPED = false, bool FACTORS = false>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, GemmParams p, int grid, cudaStream_t stream,
            const CUtensorMap* mo = nullptr) {
   p.trace_seq = -1;
@@ -1063,11 +1072,11 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, GemmParams p, int grid,
                                          p.scale.sumsq != nullptr);
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(gemm_tc_kernel<BT, GATED, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_tc_kernel<BT, GATED, GROUPED, FACTORS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
       return iert_check_launch("gemm_tc attribute");
     configured = true;
   }
-  launch_dep(gemm_tc_kernel<BT, GATED, GROUPED>, dim3(grid), dim3(THREADS), smem, stream, mw, mx, mo ? *mo : mw, p);
+  launch_dep(gemm_tc_kernel<BT, GATED, GROUPED, FACTORS>, dim3(grid), dim3(THREADS), smem, stream, mw, mx, mo ? *mo : mw, p);
   return iert_check_launch("gemm_tc");
 }
 
@@ -1377,9 +1386,9 @@ int gemm_tc_gated_impl(const void* x, long long ldx, const void* w, long long ld
     const int slots = 2 * sm_count();
     const int grid = p.n_tiles < slots ? p.n_tiles : slots;
     switch (wbt) {
-      case 16: return launch<16, false>(mw, mx, p, grid, stream);
-      case 32: return launch<32, false>(mw, mx, p, grid, stream);
-      default: return launch<64, false>(mw, mx, p, grid, stream);
+      case 16: return ep ? launch<16, false, false, true>(mw, mx, p, grid, stream) : launch<16, false>(mw, mx, p, grid, stream);
+      case 32: return ep ? launch<32, false, false, true>(mw, mx, p, grid, stream) : launch<32, false>(mw, mx, p, grid, stream);
+      default: return ep ? launch<64, false, false, true>(mw, mx, p, grid, stream) : launch<64, false>(mw, mx, p, grid, stream);
     }
   }
   if (scale) return IERT_BAD_ARGUMENT;                 // only the one-token form scales its rows
@@ -1404,7 +1413,8 @@ int gemm_tc_gated_impl(const void* x, long long ldx, const void* w, long long ld
   const int grid = tiles < slots ? tiles : slots;
   CUtensorMap ms;
   if (room_for_staging(p.stages, stage_bytes) && tensor_map_store(act, M, inter, ldo, IERT_BF16, &ms)) p.tma_store = 1;
-  return launch<128, true>(mw, mx, p, grid, stream, p.tma_store ? &ms : nullptr);
+  return ep ? launch<128, true, false, true>(mw, mx, p, grid, stream, p.tma_store ? &ms : nullptr)
+            : launch<128, true>(mw, mx, p, grid, stream, p.tma_store ? &ms : nullptr);
 }
 }  // namespace
 

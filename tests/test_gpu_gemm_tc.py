@@ -233,6 +233,27 @@ def test_gated_product_is_silu_gate_times_up(M, I, K):
         assert torch.isfinite(act).all() and bool((diff <= bound).all()), f"{force}: max diff {diff.max().item():.4g}"
 
 
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 49, 64, 65, 200])
+@pytest.mark.parametrize("I,K", [(200, 136), (9600, 128)])
+def test_gated_product_with_factors(M, I, K):
+    """A factor per token and block of columns, in the forms' own kernels: powers of two scale the results to the bit."""
+    from inference_engine_rust_b200.csrc import bindings as B
+    g = torch.Generator(device=DEV).manual_seed(M + I)
+    x = torch.randn(M, K, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(2 * I, K, device=DEV, generator=g) * (2.0 / K ** 0.5)).bfloat16()
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    fac = torch.tensor([0.0, 0.5, 1.0, 2.0], device=DEV)[torch.randint(0, 4, (M, 4), device=DEV, generator=g)]
+    ep = B.epilogue(scale=fac, blocks=3, block_cols=48)                  # columns from 144 on: the fourth factor
+    cols = torch.clamp(torch.arange(I, device=DEV) // 48, max=3)
+    for bt in [0, 128] + [b for b in (16, 32, 64) if M <= b]:
+        plain, got = (torch.full((M, I), float("nan"), device=DEV, dtype=torch.bfloat16) for _ in range(2))
+        assert B.gemm_tc_gated(x, w, plain, M, err, B.stream_ptr(), force_bt=bt)
+        assert B.gemm_tc_gated(x, w, got, M, err, B.stream_ptr(), force_bt=bt, epilogue=ep)
+        torch.cuda.synchronize()
+        assert err.item() == 0
+        assert torch.equal(got, (plain.float() * fac[:, cols]).bfloat16()), bt
+
+
 # ---- one-token steps of 17 to 64 tokens: an RMSNorm split around the kernel boundary ---------------
 
 
