@@ -173,14 +173,14 @@ def _declare(lib) -> None:
         "iert_router_topk": [P, LL, LL, P, c_int, c_int, c_int, P, c_int, P, P, S],
         "iert_moe_scale": [P, c_int, LL, P, c_int, c_int, c_int, c_int, S],
         "iert_router_step": [P, LL, P, LL, c_int, c_int, c_int, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
-                             c_int, c_int, P, c_int, P, P, P, P, S],
+                             c_int, c_int, P, c_int, P, P, P, P, LL, S],
         "iert_moe_sort": [P, P, c_int, c_int, c_int, P, P, P, P, S],
         "iert_moe_gather": [P, LL, P, P, c_int, P, c_int, S],
-        "iert_moe_combine": [P, P, P, c_int, c_int, P, c_int, S],
+        "iert_moe_combine": [P, P, P, c_int, c_int, P, LL, c_int, S],
         "iert_gemm_tc_grouped_gated": [P, LL, P, LL, P, LL, c_int, c_int, P, c_int, c_int, c_int, c_int, P, POINTER(GatedAct), P, S],
         "iert_gemm_tc_grouped": [P, LL, P, LL, P, LL, c_int, c_int, P, c_int, c_int, c_int, P, S],
         "iert_router_grouped": [P, LL, LL, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
-                                c_int, c_int, P, c_int, P, P, P, P, c_int, LL, P, c_int, S],
+                                c_int, c_int, P, c_int, P, P, P, P, c_int, LL, P, LL, c_int, S],
         "iert_qkv_prep": [P, LL, P, P, c_int, POINTER(BatchView), POINTER(KvView), c_int, c_int, c_int, P, c_int, c_float, c_int,
                           P, P, c_float, P, LL, c_float, c_float, c_float, c_int, P, S],
         "iert_gate_mul": [P, P, LL, c_int, P, c_int, c_int, c_int, c_int, c_int, S],
@@ -898,7 +898,7 @@ def router_grouped(z, correction, n_tokens: int, E: int, N: int, top: int, group
                                      ROUTER_SCORES[score], ROUTER_GROUP_SCORES[group_score], weight_eps, weight_scale,
                                      1 if renormalize else 0, 1 if shared_gate else 0, wt.data_ptr(), wt.stride(0), wid.data_ptr(),
                                      idx.data_ptr(), w.data_ptr(), _ptr(x), dtype_code(x.dtype) if x is not None else F32,
-                                     x.stride(0) if x is not None else 0, _ptr(residual),
+                                     x.stride(0) if x is not None else 0, _ptr(residual), residual.stride(0) if residual is not None else 0,
                                      residual.shape[-1] if residual is not None else 0, stream), "router_grouped")
 
 
@@ -915,7 +915,8 @@ def router_step(x, w_r, n_tokens: int, E: int, top: int, wt, idx, w, stream, *, 
                                      g.get("groups", 1), g.get("keep", 1), ROUTER_SCORES[g.get("score", "softmax")],
                                      ROUTER_GROUP_SCORES[g.get("group_score", "max")], g.get("weight_eps", 1e-20), g.get("weight_scale", 1.0),
                                      1 if g.get("renormalize", True) else 0, 1 if g.get("shared_gate") else 0, wt.data_ptr(), wt.stride(0),
-                                     _ptr(wid), idx.data_ptr(), w.data_ptr(), _ptr(residual), stream)
+                                     _ptr(wid), idx.data_ptr(), w.data_ptr(), _ptr(residual),
+                                     residual.stride(0) if residual is not None else 0, stream)
     if status == 1:
         return False
     check(status, "router_step")
@@ -948,8 +949,8 @@ def moe_gather(x, groups, row_token, max_rows: int, xs, stream) -> None:
 
 def moe_combine(y, pos, w, n_tokens: int, top: int, residual, stream) -> None:
     """residual[t] += the sum of y[pos[t, k]] over the choices that have a row."""
-    check(core().iert_moe_combine(y.data_ptr(), pos.data_ptr(), w.data_ptr(), n_tokens, top, residual.data_ptr(), residual.shape[-1],
-                                  stream), "moe_combine")
+    check(core().iert_moe_combine(y.data_ptr(), pos.data_ptr(), w.data_ptr(), n_tokens, top, residual.data_ptr(), residual.stride(0),
+                                  residual.shape[-1], stream), "moe_combine")
 
 
 def gemm_tc_grouped_gated(x, w, act, groups, max_row_tiles: int, experts: int, F: int, up_rows: int, row_scale, err, stream,

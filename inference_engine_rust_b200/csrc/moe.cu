@@ -194,7 +194,7 @@ __device__ __forceinline__ float route_token(const RouterArgs& a, int t, int lan
 }
 
 template <typename TX>
-__global__ void router_grouped_kernel(RouterArgs a, const TX* __restrict__ x, long long ldx, float* __restrict__ residual, int H) {
+__global__ void router_grouped_kernel(RouterArgs a, const TX* __restrict__ x, long long ldx, float* __restrict__ residual, long long ldres, int H) {
   extern __shared__ float rsm[];
   __shared__ float share_s;
   pdl_launch_dependents();     // the next kernel (the experts' product) may fetch its first weights now
@@ -208,9 +208,9 @@ __global__ void router_grouped_kernel(RouterArgs a, const TX* __restrict__ x, lo
   __syncthreads();
   const float share = share_s;
   if (share == 0.f) return;
-  float* out = residual + (size_t)t * H;
+  float* out = residual + (size_t)t * ldres;
   const TX* in = x + (size_t)t * ldx;
-  if (H % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)residual | (uintptr_t)x) & 15) == 0) {
+  if (H % 4 == 0 && ldx % 4 == 0 && ldres % 4 == 0 && (((uintptr_t)residual | (uintptr_t)x) & 15) == 0) {
     for (int i = threadIdx.x * 4; i < H; i += blockDim.x * 4) {
       float4 o = *reinterpret_cast<const float4*>(out + i);
       float v[4];
@@ -264,7 +264,7 @@ constexpr int ROUTER_THREADS = 256;
 template <bool GROUPED>
 __global__ void __launch_bounds__(ROUTER_THREADS)
 router_step_kernel(RouterArgs a, const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w_r, long long ldr, int K,
-                   int rows, float* __restrict__ residual, int H) {
+                   int rows, float* __restrict__ residual, long long ldres, int H) {
   extern __shared__ float rsm[];
   __shared__ float share_s;
   float* z_s = rsm;                        // [rows] logits, then the routing's own
@@ -315,7 +315,7 @@ router_step_kernel(RouterArgs a, const __nv_bfloat16* __restrict__ x, long long 
   __syncthreads();
   const float share = share_s;
   if (share == 0.f) return;
-  for (int i = threadIdx.x; i < H; i += ROUTER_THREADS) residual[(size_t)t * H + i] += share * __bfloat162float(xr[i]);
+  for (int i = threadIdx.x; i < H; i += ROUTER_THREADS) residual[(size_t)t * ldres + i] += share * __bfloat162float(xr[i]);
 }
 
 constexpr int SORT_THREADS = 1024, ROW_TILE = 128;
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const uint4* __restrict
 }
 
 __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ pos, const float* __restrict__ w,
-                                                          int top, float* __restrict__ residual, int H) {
+                                                          int top, float* __restrict__ residual, long long ldres, int H) {
   __shared__ int pos_s[MAX_TOP];
   __shared__ float w_s[MAX_TOP];
   pdl_launch_dependents();
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
   }
   __syncthreads();
   for (int i = threadIdx.x * 4; i < H; i += 256 * 4) {
-    float4* out = reinterpret_cast<float4*>(residual + (size_t)t * H + i);
+    float4* out = reinterpret_cast<float4*>(residual + (size_t)t * ldres + i);
     float4 o = *out, a = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int k = 0; k < top; ++k) {
       if (pos_s[k] < 0) {                // no rows: an expert without tensors, or no choice for want of a number
@@ -443,12 +443,12 @@ IERT_API int iert_moe_gather(const void* x, long long ldx, const int* groups, co
   return iert_check_launch("moe_gather");
 }
 
-// y fp32 [rows, H]; residual fp32 [n_tokens, H].
-IERT_API int iert_moe_combine(const float* y, const int* pos, const float* w, int n_tokens, int top, float* residual, int H,
-                              cudaStream_t stream) {
+// y fp32 [rows, H]; residual fp32 [n_tokens, H] with row stride ldres (H and ldres multiples of 4, rows on 16-byte boundaries).
+IERT_API int iert_moe_combine(const float* y, const int* pos, const float* w, int n_tokens, int top, float* residual, long long ldres,
+                              int H, cudaStream_t stream) {
   if (n_tokens <= 0) return IERT_OK;
-  if (top <= 0 || top > MAX_TOP || H <= 0 || H % 4 || (((uintptr_t)y | (uintptr_t)residual) & 15)) return IERT_BAD_ARGUMENT;
-  launch_dep(moe_combine_kernel, dim3(n_tokens), dim3(256), 0, stream, y, pos, w, top, residual, H);
+  if (top <= 0 || top > MAX_TOP || H <= 0 || H % 4 || ldres % 4 || (((uintptr_t)y | (uintptr_t)residual) & 15)) return IERT_BAD_ARGUMENT;
+  launch_dep(moe_combine_kernel, dim3(n_tokens), dim3(256), 0, stream, y, pos, w, top, residual, ldres, H);
   return iert_check_launch("moe_combine");
 }
 
@@ -466,7 +466,7 @@ IERT_API int iert_router_topk(const float* z, long long ldz, long long lde, cons
 IERT_API int iert_router_grouped(const float* z, long long ldz, long long lde, const float* correction, int n_tokens, int E, int N, int top,
                                  int groups, int keep, int score_mode, int group_mode, float weight_eps, float weight_scale,
                                  int renorm, int shared_gate, float* wt, int ldw, float* wid, int* idx, float* w, const void* x,
-                                 int x_dtype, long long ldx, float* residual, int H, cudaStream_t stream) {
+                                 int x_dtype, long long ldx, float* residual, long long ldres, int H, cudaStream_t stream) {
   if (n_tokens <= 0) return IERT_OK;
   if (score_mode < 0 || score_mode > 1 || group_mode < 0 || group_mode > 1) return IERT_BAD_ARGUMENT;
   if (ldw < E + (shared_gate ? 1 : 0) || (x && (!residual || H <= 0 || (x_dtype != IERT_F32 && x_dtype != IERT_BF16)))) return IERT_BAD_ARGUMENT;
@@ -479,9 +479,9 @@ IERT_API int iert_router_grouped(const float* z, long long ldz, long long lde, c
                         shared_gate, ldw, wt, wid, idx, w};
   const dim3 threads(x ? 256 : 32);
   if (x && x_dtype == IERT_F32)
-    launch_dep(router_grouped_kernel<float>, dim3(n_tokens), threads, smem, stream, a, (const float*)x, ldx, residual, H);
+    launch_dep(router_grouped_kernel<float>, dim3(n_tokens), threads, smem, stream, a, (const float*)x, ldx, residual, ldres, H);
   else
-    launch_dep(router_grouped_kernel<__nv_bfloat16>, dim3(n_tokens), threads, smem, stream, a, (const __nv_bfloat16*)x, ldx, residual, H);
+    launch_dep(router_grouped_kernel<__nv_bfloat16>, dim3(n_tokens), threads, smem, stream, a, (const __nv_bfloat16*)x, ldx, residual, ldres, H);
   return iert_check_launch("router_grouped");
 }
 
@@ -502,7 +502,7 @@ IERT_API int iert_moe_scale(void* act, int dtype, long long ld, const float* wt,
 IERT_API int iert_router_step(const void* x, long long ldx, const void* w_r, long long ldr, int K, int rows, int grouped, const float* correction,
                               int n_tokens, int E, int N, int top, int groups, int keep, int score_mode, int group_mode, float weight_eps,
                               float weight_scale, int renorm, int shared_gate, float* wt, int ldw, float* wid, int* idx, float* w,
-                              float* residual, cudaStream_t stream) {
+                              float* residual, long long ldres, cudaStream_t stream) {
   if (n_tokens <= 0) return IERT_OK;
   if (K <= 0 || K % 8 || ldx % 8 || ldr % 8 || (((uintptr_t)x | (uintptr_t)w_r) & 15) || E <= 0 || N < E || top <= 0 || top > MAX_TOP)
     return IERT_BAD_ARGUMENT;
@@ -516,9 +516,9 @@ IERT_API int iert_router_step(const void* x, long long ldx, const void* w_r, lon
                         shared_gate, ldw, wt, wid, idx, w};
   if (grouped)
     launch_dep(router_step_kernel<true>, dim3(n_tokens), dim3(ROUTER_THREADS), smem, stream, a, (const __nv_bfloat16*)x, ldx,
-               (const __nv_bfloat16*)w_r, ldr, K, rows, residual, K);
+               (const __nv_bfloat16*)w_r, ldr, K, rows, residual, ldres, K);
   else
     launch_dep(router_step_kernel<false>, dim3(n_tokens), dim3(ROUTER_THREADS), smem, stream, a, (const __nv_bfloat16*)x, ldx,
-               (const __nv_bfloat16*)w_r, ldr, K, rows, (float*)nullptr, K);
+               (const __nv_bfloat16*)w_r, ldr, K, rows, (float*)nullptr, 0, K);
   return iert_check_launch("router_step");
 }

@@ -132,11 +132,13 @@ class MoE(FeedForward):
         B.router_topk(z, self.router_bias, T, E, self.top, wt, idx, w, stream, by_output=by_output)
         return wt, idx, w
 
-    def _takes_grouped(self, xn, T: int) -> bool:
+    def _takes_grouped(self, xn, T: int, residual=None) -> bool:
         E, F, H = self.experts, self.expert_ff, self.hidden_size
         return (self.rt.fast and T >= GROUPED_MIN_TOKENS and T * E >= 2 * (T * self.top + 64 * E) and E <= 1024
                 and isinstance(xn, torch.Tensor) and xn.dtype == torch.bfloat16 and xn.stride(0) % 8 == 0
-                and xn.data_ptr() % 16 == 0 and F % 64 == 0 and H % 8 == 0 and self.shared_ff % 8 == 0)
+                and xn.data_ptr() % 16 == 0 and F % 64 == 0 and H % 8 == 0 and self.shared_ff % 8 == 0
+                # (a token's results are added to its residual by 16-byte accesses)
+                and (residual is None or (residual.stride(0) % 4 == 0 and residual.data_ptr() % 16 == 0)))
 
     def _forward_grouped(self, xn, residual, T: int, stream: int) -> None:
         """One portion of a prompt: the choices sorted by expert, each expert's products over its own rows, the shared expert
@@ -164,7 +166,7 @@ class MoE(FeedForward):
 
     def forward(self, xn, residual, ctx: StepContext) -> None:
         rt, ws, T, I, E = self.rt, self.rt.workspace, ctx.n_tokens, self.inter, self.experts
-        if self._takes_grouped(xn, T):
+        if self._takes_grouped(xn, T, residual):
             for t in range(0, T, GROUPED_MAX_TOKENS):
                 n = min(GROUPED_MAX_TOKENS, T - t)
                 self._forward_grouped(xn[t:t + n], residual[t:t + n], n, ctx.stream)

@@ -143,3 +143,29 @@ def test_router_in_one_kernel(T, E, top, K, shared):
         for p, q in ((a[0], b[0]), (a[2], b[2])):
             assert ((p - q).abs() <= 2.0 ** -16).all()            # logits of size 1 summed in another order, K terms of 2^-24
     assert not B.router_step(x[:, 1:], w_r[:, 1:], T, E, top, *empty(), B.stream_ptr(), bias=bias)
+
+
+@pytest.mark.parametrize("kind,E,top,ff,shared,identity", [("moe", 8, 2, 64, 96, 0), ("grouped_moe", 13, 2, 192, 0, 3)])
+@pytest.mark.parametrize("T", [1, 40, 200, 400])
+def test_residual_that_is_a_view(kind, E, top, ff, shared, identity, T):
+    """Rows wider than the layer, and rows off the 16-byte boundaries: the same results, and nothing beside them written."""
+    from inference_engine_rust_b200.parts import StepContext
+    part, w = part_of(kind, E, top, ff, shared, identity, 136)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randn((T, 136), generator=g, device=DEV).to(torch.bfloat16)
+    step = dict(kind="prompt", batch=None, n_tokens=T, n_seqs=1, q_lens=[T], pos0=[0], slots=[0], rt=part.rt)
+    base = torch.randn((T, 136), generator=g, device=DEV)
+    exactly = exact(kind, part, w, x)
+    for width, first in ((136, 0), (160, 0), (160, 8), (139, 0), (160, 1)):
+        wide = torch.full((T, width), 5.0, device=DEV)
+        res = wide[:, first:first + 136]
+        res.copy_(base)
+        part.forward(x, res, StepContext(stream=torch.cuda.current_stream().cuda_stream, **step))
+        torch.cuda.synchronize()
+        assert part.rt.err.item() == 0
+        assert (res - base - exactly).norm() <= 2.0 ** -8 * exactly.norm(), (width, first)
+        assert (wide[:, :first] == 5.0).all() and (wide[:, first + 136:] == 5.0).all()
+    if T == 400:
+        assert part._takes_grouped(x, T, base) and part._takes_grouped(x, T, torch.zeros((T, 160), device=DEV)[:, 8:144])
+        assert not part._takes_grouped(x, T, torch.zeros((T, 139), device=DEV)[:, :136])
+        assert not part._takes_grouped(x, T, torch.zeros((T, 160), device=DEV)[:, 1:137])
