@@ -51,8 +51,12 @@ ROUTER_STEP_MAX_TOKENS = 64
 # shared one: 256 tokens 149 / 122 us, 384: 143 / 161, 2,048: 273 / 520; four chosen: 384: 129 / 184, 2,048: 324 / 526.
 # All before the grouped products stored by TMA, which takes 15 us off them at 2,048 tokens.)
 GROUPED_MIN_TOKENS = 384
-# ... in portions of this many tokens, which bounds the sorted rows and their results in memory.
+# ... in equal portions of at most this many tokens, and of at most this many bytes for the sorted rows, their activations and their
+# results: top x (4 H + 2 F) a token, 36 KB for two experts of 768 chosen at a width of 4,096 and 140 KB for eight of 512.  Every portion
+# reads the experts' weights again: 8,192 tokens in portions of 8,192 / 4,096 / 2,048 take 522 / 540 / 659 us at the first of these sizes,
+# 1,570 / 1,670 / 2,004 at the second.
 GROUPED_MAX_TOKENS = 8192
+GROUPED_MAX_BYTES = 512 << 20
 
 
 class MoE(FeedForward):
@@ -132,9 +136,13 @@ class MoE(FeedForward):
         B.router_topk(z, self.router_bias, T, E, self.top, wt, idx, w, stream, by_output=by_output)
         return wt, idx, w
 
+    def _portion(self) -> int:
+        """Tokens of a grouped portion at most."""
+        return min(GROUPED_MAX_TOKENS, GROUPED_MAX_BYTES // (self.top * (4 * self.hidden_size + 2 * self.expert_ff)))
+
     def _takes_grouped(self, xn, T: int, residual=None) -> bool:
         E, F, H = self.experts, self.expert_ff, self.hidden_size
-        return (self.rt.fast and T >= GROUPED_MIN_TOKENS and T * E >= 2 * (T * self.top + 64 * E) and E <= 1024
+        return (self.rt.fast and min(T, self._portion()) >= GROUPED_MIN_TOKENS and T * E >= 2 * (T * self.top + 64 * E) and E <= 1024
                 and isinstance(xn, torch.Tensor) and xn.dtype == torch.bfloat16 and xn.stride(0) % 8 == 0
                 and xn.data_ptr() % 16 == 0 and F % 64 == 0 and H % 8 == 0 and self.shared_ff % 8 == 0
                 # (a token's results are added to its residual by 16-byte accesses)
@@ -151,11 +159,11 @@ class MoE(FeedForward):
         row_token = ws.take("moe.row_token", (rows,), torch.int32)
         row_w = ws.take("moe.row_weight", (rows,), torch.float32)
         B.moe_sort(idx, w, T, top, E, groups, pos, row_token, row_w, stream)
-        xs = ws.take("moe.rows", (rows, H), torch.bfloat16)
+        y = ws.take("moe.results", (rows, H), torch.float32)
+        xs = y.view(torch.bfloat16).flatten()[:rows * H].view(rows, H)       # the sorted rows are done with when their results are written
         B.moe_gather(xn, groups, row_token, rows, xs, stream)
         act = ws.take("moe.act", (rows, F), torch.bfloat16)
         B.gemm_tc_grouped_gated(xs, self.gate_up.weight, act, groups, tiles, E, F, self.inter, row_w, rt.err, stream, fn=self.act)
-        y = ws.take("moe.results", (rows, H), torch.float32)
         B.gemm_tc_grouped(act, self.down.weight, y, groups, tiles, E, F, rt.err, stream)
         if S:
             act_s = ws.take("ffn.act", (T, S), torch.bfloat16)
@@ -167,8 +175,9 @@ class MoE(FeedForward):
     def forward(self, xn, residual, ctx: StepContext) -> None:
         rt, ws, T, I, E = self.rt, self.rt.workspace, ctx.n_tokens, self.inter, self.experts
         if self._takes_grouped(xn, T, residual):
-            for t in range(0, T, GROUPED_MAX_TOKENS):
-                n = min(GROUPED_MAX_TOKENS, T - t)
+            size = -(-T // -(-T // self._portion()))
+            for t in range(0, T, size):
+                n = min(size, T - t)
                 self._forward_grouped(xn[t:t + n], residual[t:t + n], n, ctx.stream)
             return
         wt, _, _ = self._route(xn, residual, T, ctx.stream)

@@ -169,3 +169,45 @@ def test_residual_that_is_a_view(kind, E, top, ff, shared, identity, T):
         assert part._takes_grouped(x, T, base) and part._takes_grouped(x, T, torch.zeros((T, 160), device=DEV)[:, 8:144])
         assert not part._takes_grouped(x, T, torch.zeros((T, 139), device=DEV)[:, :136])
         assert not part._takes_grouped(x, T, torch.zeros((T, 160), device=DEV)[:, 1:137])
+
+
+@pytest.mark.parametrize("kind,E,top,ff,shared,identity", [("moe", 8, 2, 64, 96, 0), ("grouped_moe", 13, 2, 192, 0, 3)])
+@pytest.mark.parametrize("T", [512, 513, 768])
+def test_portions(monkeypatch, kind, E, top, ff, shared, identity, T):
+    """A prompt in two, three or four portions, bounded by tokens or by bytes: the bits of one portion, and no more workspace than said."""
+    from inference_engine_rust_b200.parts import StepContext, Workspace, moe
+    part, w = part_of(kind, E, top, ff, shared, identity, 136)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randn((T, 136), generator=g, device=DEV).to(torch.bfloat16)
+    base = torch.randn((T, 136), generator=g, device=DEV)
+    a_token = top * (4 * 136 + 2 * ff)
+    monkeypatch.setattr(moe, "GROUPED_MIN_TOKENS", 128)
+    got = {}
+    for most, room, size in ((8192, 1 << 40, T), (256, 1 << 40, 256), (8192, 200 * a_token + 5, 200), (200, 300 * a_token, 200)):
+        monkeypatch.setattr(moe, "GROUPED_MAX_TOKENS", most)
+        monkeypatch.setattr(moe, "GROUPED_MAX_BYTES", room)
+        part.rt.workspace = Workspace(DEV)
+        assert part._takes_grouped(x, T) and part._portion() == min(most, room // a_token)
+        got[most, room] = base.clone()
+        part.forward(x, got[most, room], StepContext(kind="prompt", batch=None, n_tokens=T, n_seqs=1, q_lens=[T], pos0=[0], slots=[0],
+                                                     stream=torch.cuda.current_stream().cuda_stream, rt=part.rt))
+        torch.cuda.synchronize()
+        assert part.rt.err.item() == 0
+        per_row = sum(b.numel() for n, b in part.rt.workspace._bufs.items() if n in ("moe.act", "moe.results", "moe.rows"))
+        assert per_row <= size * a_token
+    first, *others = got.values()
+    assert all(torch.equal(first, o) for o in others)
+    monkeypatch.setattr(moe, "GROUPED_MAX_BYTES", 127 * a_token)             # portions too small to be worth it
+    assert not part._takes_grouped(x, T)
+
+
+def test_portions_of_one_token():
+    """Every kernel of the grouped form at its smallest."""
+    part, w = part_of("moe", 8, 2, 64, 96, 0, 136)
+    x = torch.randn((5, 136), device=DEV).to(torch.bfloat16)
+    out = torch.zeros((5, 136), device=DEV)
+    for t in range(5):
+        part._forward_grouped(x[t:t + 1], out[t:t + 1], 1, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    want = exact("moe", part, w, x)
+    assert part.rt.err.item() == 0 and (out - want).norm() <= 2.0 ** -8 * want.norm()
