@@ -44,8 +44,12 @@ from .linear import Linear
 # Prompts of more than this many tokens compute a grouped router's logits (at most 32 outputs) with the kernel for few
 # rows against a long matrix, the tokens being the matrix.
 SKINNY_ROUTER_MIN_TOKENS = 32
-# Up to this many tokens the router's product and the routing are one kernel, a block per token.
+# Up to this many tokens and router outputs the router's product and the routing are one kernel, a block per token whose eight warps take
+# two outputs each.  More outputs are further rounds of them in every block, one kernel / two, us a mixture at a width of 4,096 with 8, 32 and 64
+# tokens: 16 outputs 19.8 / 21.5, 30.4 / 37.1, 32.2 / 33.8; 32 outputs 24.8 / 22.2, 35.7 / 39.1, 39.2 / 37.2; 64 outputs 48 / 29, 68 / 51, 71 / 57; 128 outputs
+# 98 / 54, 114 / 75, 114 / 82.
 ROUTER_STEP_MAX_TOKENS = 64
+ROUTER_STEP_MAX_OUTPUTS = 16
 # Prompts of at least this many tokens run the experts' products over the tokens that chose them, if that is less than half of
 # the rows that all experts over all tokens would have.  (16 experts at 7B sizes, grouped against all experts, two chosen and a
 # shared one: 256 tokens 149 / 122 us, 384: 143 / 161, 2,048: 273 / 520; four chosen: 384: 129 / 184, 2,048: 324 / 526.
@@ -120,8 +124,9 @@ class MoE(FeedForward):
         return z, by_output
 
     def _routes_in_one(self, xn, T: int) -> bool:
-        """Steps of few tokens: one kernel for the router's product and the routing."""
-        return (self.rt.fast and T <= ROUTER_STEP_MAX_TOKENS and isinstance(xn, torch.Tensor) and xn.dtype == torch.bfloat16)
+        """Steps of few tokens over few outputs: one kernel for the router's product and the routing."""
+        return (self.rt.fast and T <= ROUTER_STEP_MAX_TOKENS and self.router.out_features <= ROUTER_STEP_MAX_OUTPUTS
+                and isinstance(xn, torch.Tensor) and xn.dtype == torch.bfloat16)
 
     def _route(self, xn, residual, T: int, stream: int):
         """(wt [T, E or more] dense routing weights, idx, w [T, top] the choices); the share of experts that return their

@@ -211,3 +211,29 @@ def test_portions_of_one_token():
     torch.cuda.synchronize()
     want = exact("moe", part, w, x)
     assert part.rt.err.item() == 0 and (out - want).norm() <= 2.0 ** -8 * want.norm()
+
+
+@pytest.mark.parametrize("kind", ["moe", "grouped_moe"])
+@pytest.mark.parametrize("E,one", [(16, True), (17, False), (40, False)])
+def test_which_steps_route_in_one_kernel(monkeypatch, kind, E, one):
+    from inference_engine_rust_b200.csrc import bindings as B
+    from inference_engine_rust_b200.parts import StepContext, moe
+    part, w = part_of(kind, E, 2, 64, 0, 0, 136)
+    taken = []
+    real = B.router_step
+    monkeypatch.setattr(B, "router_step", lambda *a, **k: taken.append(real(*a, **k)) or taken[-1])
+    for T in (1, 33, 64, 65):
+        g = torch.Generator(device=DEV).manual_seed(T)
+        x, out = torch.randn((T, 136), generator=g, device=DEV).to(torch.bfloat16), torch.zeros((T, 136), device=DEV)
+        taken.clear()
+        step = StepContext(kind="decode", batch=None, n_tokens=T, n_seqs=T, q_lens=[1] * T, pos0=[0] * T, slots=list(range(T)),
+                           stream=torch.cuda.current_stream().cuda_stream, rt=part.rt)
+        part.forward(x, out, step)
+        torch.cuda.synchronize()
+        assert part.rt.err.item() == 0 and taken == ([True] if one and T <= 64 else [])
+        apart = torch.zeros((T, 136), device=DEV)
+        with monkeypatch.context() as m:
+            m.setattr(moe, "ROUTER_STEP_MAX_TOKENS", 0)
+            part.forward(x, apart, step)
+        # weights from logits summed in another order (2^-16 at most), behind which an activation may round the other way (2^-8)
+        assert (out - apart).norm() <= 2.0 ** -8 * apart.norm()
