@@ -51,10 +51,22 @@ SKINNY_ROUTER_MIN_TOKENS = 32
 ROUTER_STEP_MAX_TOKENS = 64
 ROUTER_STEP_MAX_OUTPUTS = 16
 # Prompts of at least this many tokens run the experts' products over the tokens that chose them, if that is less than half of
-# the rows that all experts over all tokens would have.  (16 experts at 7B sizes, grouped against all experts, two chosen and a
-# shared one: 256 tokens 149 / 122 us, 384: 143 / 161, 2,048: 273 / 520; four chosen: 384: 129 / 184, 2,048: 324 / 526.
-# All before the grouped products stored by TMA, which takes 15 us off them at 2,048 tokens.)
+# the rows that all experts over all tokens would have, and where two costs of the sorted form are outweighed:
+#   a row's way through the sort, the gather and the sum: the experts left out must hold enough work, E F >= 2,048 top;
+#   a row tile that an expert does not fill, above all where its width does not fill a tile's columns either: T F >= 48 K.
+# Up to 2 M numbers in the sorted rows (T top H) both forms take their launches' time and the rows' way costs nothing.
+# Grouped / all experts, us a mixture (T of 256, 384, 1,024, 2,048), E x F, chosen, width H:
+#   16 x 768, 2, 4,096   112 / 139   115 / 162   136 / 247   168 / 447        8 x 1,792, 2, 4,096    98 / 117   101 / 156   146 / 285   234 / 525
+#   16 x 896, 4, 4,096   126 / 146   119 / 172   170 / 289   289 / 531        64 x 512, 6, 2,048    136 / 145   136 / 186   160 / 343   230 / 617
+#   32 x 384, 4, 4,096   108 / 121   111 / 132   137 / 251   220 / 457        128 x 256, 8, 2,048   145 / 144   152 / 186   188 / 345   266 / 621
+#   256 x 64, 8, 4,096   245 / 154   264 / 209   327 / 345   418 / 618 (768 tokens 299 / 311: the second cost)
+#   64 x 128, 8, 4,096   145 / 106   157 / 146   215 / 201   337 / 330        128 x 64, 8, 2,048    110 / 81    114 / 95    144 / 135   223 / 185 (the first)
+# and at T of 384, 1,024, 4,096: 16 x 128, 4, 4,096   76 / 56   105 / 65   276 / 187        32 x 64, 8, 2,048    65 / 46   102 / 57   308 / 115
+#   8 x 256, 2, 4,096    60 / 55   81 / 62   184 / 184                                      8 x 64, 2, 1,024     32 / 33   36 / 38    68 / 39
 GROUPED_MIN_TOKENS = 384
+GROUPED_ANY_NUMBERS = 2 << 20
+GROUPED_MIN_LEFT_OUT = 2048
+GROUPED_MIN_TILE_WORK = 48 << 10
 # ... in equal portions of at most this many tokens, and of at most this many bytes for the sorted rows, their activations and their
 # results: top x (4 H + 2 F) a token, 36 KB for two experts of 768 chosen at a width of 4,096 and 140 KB for eight of 512.  Every portion
 # reads the experts' weights again: 8,192 tokens in portions of 8,192 / 4,096 / 2,048 take 522 / 540 / 659 us at the first of these sizes,
@@ -148,6 +160,8 @@ class MoE(FeedForward):
     def _takes_grouped(self, xn, T: int, residual=None) -> bool:
         E, F, H = self.experts, self.expert_ff, self.hidden_size
         return (self.rt.fast and min(T, self._portion()) >= GROUPED_MIN_TOKENS and T * E >= 2 * (T * self.top + 64 * E) and E <= 1024
+                and (T * self.top * H <= GROUPED_ANY_NUMBERS
+                     or (E * F >= GROUPED_MIN_LEFT_OUT * self.top and T * F >= GROUPED_MIN_TILE_WORK))
                 and isinstance(xn, torch.Tensor) and xn.dtype == torch.bfloat16 and xn.stride(0) % 8 == 0
                 and xn.data_ptr() % 16 == 0 and F % 64 == 0 and H % 8 == 0 and self.shared_ff % 8 == 0
                 # (a token's results are added to its residual by 16-byte accesses)

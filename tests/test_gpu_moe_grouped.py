@@ -237,3 +237,21 @@ def test_which_steps_route_in_one_kernel(monkeypatch, kind, E, one):
             part.forward(x, apart, step)
         # weights from logits summed in another order (2^-16 at most), behind which an activation may round the other way (2^-8)
         assert (out - apart).norm() <= 2.0 ** -8 * apart.norm()
+
+
+@pytest.mark.parametrize("E,top,ff,hidden,T,takes", [(48, 6, 256, 1024, 384, True), (48, 7, 256, 1024, 384, False), (48, 6, 256, 1024, 383, False),
+                                                     (40, 1, 64, 4096, 767, False), (40, 1, 64, 4096, 768, True),
+                                                     (8, 2, 64, 1024, 1024, True), (8, 2, 64, 1024, 1025, False)])
+def test_thin_experts_stay_with_all_tokens(E, top, ff, hidden, T, takes):
+    from inference_engine_rust_b200.parts import StepContext
+    part, w = part_of("moe", E, top, ff, 0, 0, hidden)
+    w = {n: t * (136 / hidden) ** 0.5 for n, t in w.items()}
+    part.load(dict(w))
+    x = torch.randn((T, hidden), generator=torch.Generator(device=DEV).manual_seed(T), device=DEV).to(torch.bfloat16)
+    out = torch.zeros((T, hidden), device=DEV)
+    assert part._takes_grouped(x, T, out) == takes
+    part.forward(x, out, StepContext(kind="prompt", batch=None, n_tokens=T, n_seqs=1, q_lens=[T], pos0=[0], slots=[0],
+                                     stream=torch.cuda.current_stream().cuda_stream, rt=part.rt))
+    torch.cuda.synchronize()
+    want = exact("moe", part, w, x)
+    assert part.rt.err.item() == 0 and (out - want).norm() <= 2.0 ** -8 * want.norm()
