@@ -955,11 +955,16 @@ __global__ void __launch_bounds__(CWORK + WLOAD) wkv_chunk_kernel(WkvArgs a, con
 // CTA so that a CTA has up to 256 computing threads.  (Measured at 32 heads of 128 x 128, one prompt of 2,048
 // tokens: 8 lanes per column 1.08 ms, 16 lanes 0.91 ms, 32 lanes 1.42 ms per layer.)
 #if IERT_CHUNKED
-// Prompts go eight tokens at a time; a step of one token (or about as few) per sequence token after token: a chunk costs what
-// eight tokens cost, and such a step is bound by reading and writing the state.
-bool chunked(const IertBatchView* b) {
+// Prompts go eight tokens at a time; steps of few tokens per sequence token after token: a chunk costs what eight tokens cost, the kernel
+// in front is one launch more, and such a step is bound by reading and writing the state.  Where the line lies (layers at 4,096, sequences of
+// equal length, chunks / token after token, us):
+//   delta rule, 16 tokens a sequence: one sequence 56 / 54, eight 133 / 132, 32 314 / 313, 128 930 / 961; four tokens 51 / 46, 93 / 85,
+//   201 / 173, 577 / 493; twelve 55 / 52, 124 / 117, 280 / 255, 882 / 817; 64 87 / 93, 254 / 282, 693 / 763;
+//   decays per channel: one sequence of 4 to 32 tokens 71 / 70 to 109 / 110, two of 8 82 / 81, four of 8 110 / 113, eight of 4 114 / 118 and of
+//   16 138 / 165, 32 of 4 170 / 185.
+bool chunked(const IertBatchView* b, int tokens_a_sequence, int tokens) {
   const char* off = getenv("IERT_RECURRENT_LANES");                  // (a forced number of lanes asks for the other kernels)
-  return !(off && atoi(off) >= 1) && b->n_tokens >= 4 * b->n_seqs;
+  return !(off && atoi(off) >= 1) && b->n_tokens >= tokens && b->n_tokens >= (long long)tokens_a_sequence * b->n_seqs;
 }
 #endif
 
@@ -1001,7 +1006,7 @@ IERT_API int iert_delta_recur(const float* qkv, const float* beta, const float* 
   if (batch->n_seqs <= 0 || batch->n_tokens <= 0) return IERT_OK;
   if (G <= 0 || H <= 0 || H % G || V <= 0 || H > 65535) return IERT_BAD_ARGUMENT;
 #if IERT_CHUNKED
-  if (scratch && chunked(batch) && V % 4 == 0 && (2 * G * DIM + H * V) % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
+  if (scratch && chunked(batch, 16, 16) && V % 4 == 0 && (2 * G * DIM + H * V) % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
       (((uintptr_t)qkv | (uintptr_t)state | (uintptr_t)o | (uintptr_t)scratch) & 15) == 0) {
     DeltaArgs a = {qkv, beta, decay, state, state_stride, s_off, o, G, H, V, CCOLS};
     launch_dep(delta_coef_kernel, dim3(batch->n_tokens / CT + batch->n_seqs, G), dim3(128), 0, stream, a, scratch, *batch);
@@ -1024,7 +1029,7 @@ IERT_API int iert_wkv_recur(const float* x, long long ld, const float* decay, co
   if (batch->n_seqs <= 0 || batch->n_tokens <= 0) return IERT_OK;
   if (H <= 0 || V <= 0 || H > 65535 || ld < (long long)2 * H * DIM + (long long)H * V) return IERT_BAD_ARGUMENT;
 #if DIM == 64
-  if (scratch && chunked(batch) && V % 4 == 0 && ld % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
+  if (scratch && chunked(batch, 4, 32) && V % 4 == 0 && ld % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
       (((uintptr_t)x | (uintptr_t)decay | (uintptr_t)state | (uintptr_t)o | (uintptr_t)scratch) & 15) == 0) {
     WkvArgs a = {x, ld, decay, u, state, state_stride, s_off, o, H, V, CCOLS};
     launch_dep(wkv_pairs_kernel, dim3(batch->n_tokens / CT + batch->n_seqs, H), dim3(DIM), 0, stream, a, scratch, *batch);

@@ -39,7 +39,7 @@ def both_ways(monkeypatch, call, state):
 
 
 @pytest.mark.parametrize("D,V,H,G", [(128, 128, 4, 2), (64, 64, 3, 3), (128, 36, 2, 1), (64, 100, 4, 1)])
-@pytest.mark.parametrize("lens", [LENS, [5], [2048]])
+@pytest.mark.parametrize("lens", [LENS, [5], [2048], LENS + [100], [16], [15]])
 def test_delta_rule(monkeypatch, D, V, H, G, lens):
     from inference_engine_rust_b200.csrc import bindings as B
     g = torch.Generator(device=DEV).manual_seed(D + V + len(lens))
@@ -81,7 +81,7 @@ def test_delta_rule(monkeypatch, D, V, H, G, lens):
 
 
 @pytest.mark.parametrize("D,V,H", [(64, 64, 5), (128, 128, 2), (64, 36, 2), (128, 4, 1)])
-@pytest.mark.parametrize("lens", [LENS, [5], [2048]])
+@pytest.mark.parametrize("lens", [LENS, [5], [2048], [4] * 8, [31]])
 def test_decay_per_key_channel(monkeypatch, D, V, H, lens):
     from inference_engine_rust_b200.csrc import bindings as B
     g = torch.Generator(device=DEV).manual_seed(D + V + len(lens))
