@@ -23,7 +23,9 @@
 // block's sums (64 k) to their registers while the next one's MMAs run.  A matrix with few rows is split over k between the
 // CTAs of a cluster (by the matrix's shape alone, so that a row's result does not depend on how many rows the call has), which
 // add their parts in order through distributed shared memory: no scratch, no counters.  An output that is not finite (an
-// infinity or NaN among its inputs, or an overflow) is computed again as gemm_plain.cu does.
+// infinity or NaN among its inputs, or an overflow) is computed again as gemm_plain.cu does, and so is one below 2^-60, whose inputs may
+// have lost bits below 2^-133 (a loss of K 2^-134 |w| at most, under 2^-24 of a larger output for weights up to 2^36); a zero, as rows of
+// zeros give by the thousand, stays.
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -95,7 +97,7 @@ __device__ __noinline__ float plain_dot(const float* x, const float* w, int K) {
 
 __device__ __forceinline__ void put(const F32Params& p, int t, int n, float v) {
   if (t >= p.M || n >= p.N) return;
-  if (!isfinite(v)) v = plain_dot(p.x + (long long)t * p.ldx, p.w + (long long)n * p.ldw, p.K);
+  if (!isfinite(v) || (v != 0.f && fabsf(v) < 0x1p-60f)) v = plain_dot(p.x + (long long)t * p.ldx, p.w + (long long)n * p.ldw, p.K);
   float* o = p.out + (long long)t * p.ldo + n;
   *o = p.add ? *o + v : v;
 }

@@ -99,3 +99,28 @@ def test_error_beside_the_plain_kernel(kind, K):
     assert off <= (beside + 2.0 ** -24 * ref.norm() if kind == "rounded remainders" else 1.1 * beside)
     if kind in ("one number", "rounded remainders"):
         assert ((tc - ref).abs() <= 2.0 ** -23 * ref.abs()).all()
+
+
+@pytest.mark.parametrize("exponent", [-40, -58, -80, -100, -112, -122])
+@pytest.mark.parametrize("M,N", [(1, 140), (40, 300), (130, 9300)])
+def test_small_numbers(exponent, M, N):
+    """Rows whose numbers lose bits below bf16's smallest number: what comes out is as precise as the plain kernel's."""
+    from inference_engine_rust_b200.csrc import bindings as B
+    torch.manual_seed(M)
+    x, w = torch.randn(M, 1024, device=DEV) * 2.0 ** exponent, torch.randn(N, 1024, device=DEV)
+    x[M // 2] = 0.0
+    tc, plain = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    assert run(x, w, tc, M)
+    B.gemm_plain(x, w, plain, M, 0, B.stream_ptr())
+    ref = x.double() @ w.double().t()
+    # every single output: K rounded additions, each at most 2^-24 of the sum of magnitudes (and 2^-149 where that is subnormal)
+    bound = 1024 * (2.0 ** -24 * (x.double().abs() @ w.double().abs().t()) + 2.0 ** -149)
+    assert ((tc - ref).abs() <= bound).all()
+    assert (tc - ref).norm() <= 1.1 * (plain - ref).norm()
+    assert (tc[M // 2] == 0).all()
+    if exponent <= -80:
+        assert ((tc == plain) | (tc == 0)).all() and (tc == 0).sum() <= N + 10       # (a sum may cancel to 0, which stays)
+        both = torch.randn(M, N, device=DEV) * 2.0 ** exponent
+        total = both.clone()
+        assert run(x, w, total, M, mode=1)
+        assert torch.equal(total, both + tc)
