@@ -16,7 +16,8 @@ def _slots(head_dim: int) -> int:
 
 
 _MAX_SPLITS = 16
-CUT_SAVES_LOADS = 16         # page loads in a row that cutting a batch that fills the device must save (see wants_length_cut)
+# what a cut by length costs a batch that fills the device, in page loads: at all, and for every round of the even step's CTAs
+CUT_COSTS, CUT_COSTS_A_ROUND = 24, 11
 
 
 def decode_splits(n_tokens: int, kv_heads: int, group: int, head_dim: int) -> int:
@@ -33,11 +34,12 @@ def wants_length_cut(pos0, kv_heads: int, group: int, window, page_tokens: int, 
     """Should a one-token step over sequences at these positions be cut by length (see
     `decode_parts`) rather than evenly?  Where the batch leaves the device room for several parts per sequence: yes
     if the longest sequence reads over 1.3 times the average number of pages (an even cut ends when its CTAs do).
-    Where the batch alone fills the device, an even step needs neither parts nor a merge, and a cut costs about 20 us
-    (a grid of eight parts per sequence, most of them empty, and the merge): yes if the cut is predicted to take at
-    least 15 % and 16 fewer page loads in a row.  Measured at 32 heads over 8, even / cut, us a layer:
-    64 sequences of 200 to 256 positions 90 / 111, of 100 to 400 90 / 112, of 512 to 1,024 110 / 129, 48 of 500 92 / 109 (all even by
-    this rule); between 16 and 25 loads saved the two are within 6 % (64 of 100 to 2,048 132 / 136, 48 of 2,100 144 / 153)."""
+    Where the batch alone fills the device, an even step needs neither parts nor a merge and takes about as long as its longest
+    sequence or its share of all pages, whichever is more; a cut takes the share, a grid of eight parts per sequence (most of them empty)
+    and the merge: yes if the longest sequence has more pages beyond the share than that costs.  Measured at 32 heads over 8, even / cut,
+    us a layer: 64 sequences of 200 to 256 positions 55 / 77, of 100 to 2,048 90 / 102, of 100 to 8,192 242 / 224, one of 8,000 among 63 of 200
+    126 / 91, two of 3,000 77 / 84; 48 of 2,100 111 / 114, of 100 to 4,096 125 / 115 (even by this rule), two of 3,000 among 46 of 200 75 / 72; 128 of 100 to
+    4,096 214 / 232, four of 1,500 among 124 of 500 95 / 135; 20 of 100 to 2,048 56 / 60, of 100 to 8,192 132 / 107."""
     n = len(pos0)
     if n < 2:
         return False
@@ -52,11 +54,8 @@ def wants_length_cut(pos0, kv_heads: int, group: int, window, page_tokens: int, 
     slots = _slots(head_dim)
     if 2 * n * per_sequence <= slots:
         return longest * n > 1.3 * total
-    even = -(-n * per_sequence // slots) * longest
-    per_part = max(1, -(-total * per_sequence // (2 * slots)))                 # as the kernel works it out
-    parts = [min(8, -(-p // per_part)) for p in pages]
-    cut = -(-sum(parts) * per_sequence // slots) * max(-(-p // k) for p, k in zip(pages, parts))
-    return even >= 1.15 * cut and even - cut >= CUT_SAVES_LOADS
+    rounds = n * per_sequence / slots
+    return longest - total * per_sequence / slots >= CUT_COSTS + CUT_COSTS_A_ROUND * rounds
 
 
 def decode_parts(n_tokens: int, kv_heads: int, group: int, unequal: bool, head_dim: int):
