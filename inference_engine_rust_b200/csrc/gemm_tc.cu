@@ -311,10 +311,10 @@ __device__ __forceinline__ TilePlace tile_place(const GemmParams& p, int tile, i
   if (GROUPED) {                         // the row tiles run fastest: an expert's weights are read by all its row tiles at once
     c.n_idx = tile / group_tiles;
     const int* g = p.groups + 2 + 3 * (tile - c.n_idx * group_tiles);
-    const int e = __ldg(g);
+    const int e = g[0];
     c.n0 = c.n_idx * p.n_step;
-    c.t0 = __ldg(g + 1);
-    c.t_end = __ldg(g + 2);
+    c.t0 = g[1];
+    c.t_end = g[2];
     c.w_row = c.n0 + e * p.group_w_rows;
     c.w_col = e * p.group_k;
   } else {
@@ -406,7 +406,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   if (threadIdx.x == 0) pdl_launch_dependents();
   if (threadIdx.x == 0) IERT_TRACE(0);                       // start
   if (GROUPED) pdl_wait();                                   // the table of row tiles comes from a kernel in front
-  const int group_tiles = GROUPED ? __ldg(p.groups) : 0;
+  const int group_tiles = GROUPED ? p.groups[0] : 0;
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
