@@ -173,7 +173,7 @@ def _declare(lib) -> None:
         "iert_router_topk": [P, LL, LL, P, c_int, c_int, c_int, P, c_int, P, P, S],
         "iert_moe_scale": [P, c_int, LL, P, c_int, c_int, c_int, c_int, S],
         "iert_router_step": [P, LL, P, LL, c_int, c_int, c_int, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
-                             c_int, c_int, P, c_int, P, P, P, P, LL, S],
+                             P, c_int, P, P, P, P, LL, S],
         "iert_moe_sort": [P, P, c_int, c_int, c_int, P, P, P, P, S],
         "iert_moe_gather": [P, LL, P, P, c_int, P, c_int, S],
         "iert_moe_combine": [P, P, P, c_int, c_int, P, LL, c_int, S],
@@ -906,7 +906,7 @@ def router_step(x, w_r, n_tokens: int, E: int, top: int, wt, idx, w, stream, *, 
                 wid=None, residual=None) -> bool:
     """The router's product and the routing in one kernel (bf16 rows and weights; one-token steps).  `grouped` None: as
     `router_topk` with `bias`; else as `router_grouped` with these options (correction, groups, keep, score, group_score, weight_eps,
-    weight_scale, renormalize, shared_gate) over N outputs, `wid` and, for identity experts, `residual`.  False: nothing launched."""
+    weight_scale) over N outputs, `wid` and, for identity experts, `residual`.  False: nothing launched."""
     if x.dtype != torch.bfloat16 or w_r.dtype != torch.bfloat16:
         return False
     g = grouped or {}
@@ -914,7 +914,7 @@ def router_step(x, w_r, n_tokens: int, E: int, top: int, wt, idx, w, stream, *, 
                                      _ptr(g.get("correction") if grouped else bias), n_tokens, E, N if grouped else E, top,
                                      g.get("groups", 1), g.get("keep", 1), ROUTER_SCORES[g.get("score", "softmax")],
                                      ROUTER_GROUP_SCORES[g.get("group_score", "max")], g.get("weight_eps", 1e-20), g.get("weight_scale", 1.0),
-                                     1 if g.get("renormalize", True) else 0, 1 if g.get("shared_gate") else 0, wt.data_ptr(), wt.stride(0),
+                                     wt.data_ptr(), wt.stride(0),
                                      _ptr(wid), idx.data_ptr(), w.data_ptr(), _ptr(residual),
                                      residual.stride(0) if residual is not None else 0, stream)
     if status == 1:

@@ -497,23 +497,22 @@ IERT_API int iert_moe_scale(void* act, int dtype, long long ld, const float* wt,
 }
 
 // The product of x [n_tokens, K] with the router's `rows` rows w_r (bf16) and the routing, in one kernel.  grouped != 0: as
-// iert_router_grouped (rows = N, or N + 1 with shared_gate), `residual` (optional, fp32 [n_tokens, K]) receives the identity experts'
+// iert_router_grouped with weights renormalised and no shared gate (rows = N), `residual` (optional, fp32 [n_tokens, K]) receives the identity experts'
 // share; else as iert_router_topk (`correction` is the bias, rows = E = N).  K and the strides multiples of 8, rows on 16-byte boundaries.
 IERT_API int iert_router_step(const void* x, long long ldx, const void* w_r, long long ldr, int K, int rows, int grouped, const float* correction,
                               int n_tokens, int E, int N, int top, int groups, int keep, int score_mode, int group_mode, float weight_eps,
-                              float weight_scale, int renorm, int shared_gate, float* wt, int ldw, float* wid, int* idx, float* w,
-                              float* residual, long long ldres, cudaStream_t stream) {
+                              float weight_scale, float* wt, int ldw, float* wid, int* idx, float* w, float* residual, long long ldres, cudaStream_t stream) {
   if (n_tokens <= 0) return IERT_OK;
   if (K <= 0 || K % 8 || ldx % 8 || ldr % 8 || (((uintptr_t)x | (uintptr_t)w_r) & 15) || E <= 0 || N < E || top <= 0 || top > MAX_TOP)
     return IERT_BAD_ARGUMENT;
   if (grouped ? (score_mode < 0 || score_mode > 1 || group_mode < 0 || group_mode > 1 || groups <= 0 || N % groups || keep <= 0 || keep > groups ||
-                 top > keep * (N / groups) || ldw < E + (shared_gate ? 1 : 0) || rows != N + (shared_gate ? 1 : 0) || !wid)
+                 top > keep * (N / groups) || ldw < E || rows != N || !wid)
               : (top > E || ldw < E || rows != E || residual))
     return IERT_BAD_ARGUMENT;
   const size_t smem = (size_t)(rows + 2 * N + groups) * sizeof(float) + (size_t)N;
   if (smem > 47 * 1024) return IERT_BAD_ARGUMENT;
-  const RouterArgs a = {nullptr, 0, 1, correction, E, N, top, groups, keep, score_mode, group_mode, weight_eps, weight_scale, renorm,
-                        shared_gate, ldw, wt, wid, idx, w};
+  const RouterArgs a = {nullptr, 0, 1, correction, E, N, top, groups, keep, score_mode, group_mode, weight_eps, weight_scale, 1,
+                        0, ldw, wt, wid, idx, w};
   if (grouped)
     launch_dep(router_step_kernel<true>, dim3(n_tokens), dim3(ROUTER_THREADS), smem, stream, a, (const __nv_bfloat16*)x, ldx,
                (const __nv_bfloat16*)w_r, ldr, K, rows, residual, ldres, K);
