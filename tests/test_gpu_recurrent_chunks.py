@@ -138,3 +138,38 @@ def test_norm_of_the_read_out_and_gate(dtype, H, n_tokens, V):
         want = (x / torch.sqrt(x.square().mean(-1, keepdim=True) + 1e-5) * (w.double() if shared else w.double().view(H, V))).flatten(1) * gate
         # a few fp32 roundings, and one to the result's type
         assert ((out.double() - want).abs() <= want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -19) + 1e-7).all()
+
+
+@pytest.mark.parametrize("L,C,width", [(64, 4096, 4096), (12, 516, 100), (4, 4, 7), (24, 1020, 520), (500, 640, 64)])
+@pytest.mark.parametrize("lens", [[256], [5, 0, 3, 1, 290, 4, 17], [255 + 1, 1], [1] * 300])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_decays_of_a_prompt(dtype, lens, L, C, width):
+    """The product with the decays' matrix, sixteen tokens a block (256 tokens and more), and the rows it keeps: sequences that end
+    inside a block, an empty one and one of padding, channels that leave a rest in a block."""
+    from inference_engine_rust_b200.csrc import bindings as B
+    g = torch.Generator(device=DEV).manual_seed(L + C + len(lens))
+    T, n = sum(lens), len(lens)
+    slots = list(range(n, 0, -1))
+    if n > 1:
+        slots[n // 2] = -1
+    z = torch.randn((T, L + 4), generator=g, device=DEV) * 2
+    w2t = torch.randn((L, C), generator=g, device=DEV) * L ** -0.5
+    w0 = torch.rand((C,), generator=g, device=DEV) * 5 - 6
+    h = torch.randn((T, width + 3), generator=g, device=DEV).to(dtype)[:, :width]
+    state = torch.full((n + 2, width + 9), 7.0, device=DEV)
+    decay = torch.full((T + 1, C), 7.0, device=DEV)
+    view, keep = batch(lens, slots)
+    B.wkv_decay(z, L, w2t, w0, decay, h, state, 5, view, B.stream_ptr())
+    torch.cuda.synchronize()
+    exponent = torch.exp(w0.double() + torch.tanh(z[:, :L].double()) @ w2t.double())
+    want = torch.exp(-exponent)
+    # L + 1 rounded additions in the inner exponent (magnitudes of up to |w0| + sum |w2t|), then two exponentials
+    off_inner = (L + 4) * 2.0 ** -24 * (w0.double().abs() + w2t.double().abs().sum(0))
+    assert ((decay[:T] - want).abs() <= want * (exponent * off_inner * 1.1 + exponent * 2.0 ** -21 + 2.0 ** -21) + 2.0 ** -149).all()
+    assert (decay[T] == 7.0).all()
+    kept, at = torch.full_like(state, 7.0), 0
+    for i, m in enumerate(lens):
+        at += m
+        if m and slots[i] >= 0:
+            kept[slots[i], 5:5 + width] = h[at - 1].float()
+    assert torch.equal(state, kept)
