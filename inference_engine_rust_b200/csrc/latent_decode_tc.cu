@@ -667,6 +667,24 @@ size_t decode_smem(int mt, int width) {
 
 constexpr size_t WIDE_SMEM = 220 * 1024;
 
+// Sequences a block of the wide kernels takes where a head's matrix has `bytes`; 0: the kernels for few sequences.  Bringing a matrix into
+// shared memory pays where it is large or where the other kernels' blocks (four sequences each) would run in rounds; sixteen sequences a
+// block halve how often it is brought, but take longer by themselves, until the blocks of eight are more than the SMs.  One-token layers, other kernels /
+// eight / sixteen a block, us:
+//   128 KB: 4 heads, 17 and 64 sequences  57 / 53 / 64   72 / 58 / 68;   16 heads, 64 and 128  82 / 61 / 70   118 / 90 / 81;   32 heads, 17, 33 and 64
+//           79 / 65 / 76   91 / 87 / 79   127 / 100 / 89
+//   64 KB (rank 256):  16 heads, 17 and 64  51 / 47 / 56   64 / 60 / 65;   32 heads, 48, 64 and 128  78 / 71 / 85   99 / 74 / 85   140 / 102 / 97
+//   32 KB (rank 128):  4 heads, 17 and 128  47 / 43 / 49   57 / 61 / 67;   16 heads, 32 and 128  51 / 46 / 53   77 / 68 / 74;   32 heads, 32 and 64
+//           63 / 66 / 68   85 / 74 / 80
+//   16 KB (rank 128):  16 heads, 17, 64 and 128  42 / 46 / 50   47 / 51 / 54   58 / 49 / 55;   32 heads, 48 and 128  48 / 53 / 56   78 / 65 / 67
+int wide_sequences(int T, int H, size_t bytes) {
+  if (T <= 16) return 0;
+  const long long eights = (long long)((T + 7) / 8) * H;
+  if (bytes >= 64 * 1024) return eights > iert_sm_count_cached() && (bytes >= 128 * 1024 || eights >= 512) ? 16 : 8;
+  if (eights >= 256) return 8;
+  return bytes >= 32 * 1024 && eights <= 64 ? 8 : 0;
+}
+
 // The dynamic shared memory of the wide kernels, asked for once.
 bool wide_configured() {
   static const bool ok = [] {
@@ -759,12 +777,11 @@ IERT_API int iert_latent_attention_decode_tc(const void* q, int q_f32, long long
   }
   // few sequences: tokens that share a head's weights in the kernels around, one when there are fewest, so that there are blocks enough
   const int tt = T <= 4 ? 1 : T <= 8 ? 2 : 4;
-  // many sequences: a head's matrix whole in shared memory, eight or sixteen sequences a block (about one block per SM or more
-  // at 32 heads); padded rows of queries must keep 16-byte stores aligned
-  const int wide = T > 32 ? 16 : 8;
-  const bool wide_absorb = T > 16 && D % 4 == 0 && R % 8 == 0 && ((uintptr_t)w_uk & 15) == 0 && ((uintptr_t)qa & 15) == 0 &&
-                           absorb_wide_smem(wide, D, rank) <= WIDE_SMEM;
-  const bool wide_merge = T > 16 && ((uintptr_t)w_uv & 15) == 0 && (size_t)merge_wide_smem(wide, rank).total <= WIDE_SMEM;
+  // many sequences: a head's matrix whole in shared memory; padded rows of queries must keep 16-byte stores aligned
+  const int absorb_tt = wide_sequences(T, H, (size_t)D * rank * 2), merge_tt = wide_sequences(T, H, (size_t)V * rank * 2);
+  const bool wide_absorb = absorb_tt && D % 4 == 0 && R % 8 == 0 && ((uintptr_t)w_uk & 15) == 0 && ((uintptr_t)qa & 15) == 0 &&
+                           absorb_wide_smem(absorb_tt, D, rank) <= WIDE_SMEM;
+  const bool wide_merge = merge_tt && ((uintptr_t)w_uv & 15) == 0 && (size_t)merge_wide_smem(merge_tt, rank).total <= WIDE_SMEM;
   if (!wide_configured()) return IERT_CUDA_ERROR;
 #define ABSORB_WIDE(TQ, TT)                                                                                                        \
   launch_dep(latent_absorb_wide_kernel<TQ, TT>, dim3((T + TT - 1) / TT, Hpad), dim3(WIDE_THREADS), absorb_wide_smem(TT, D, rank), stream, (const TQ*)q, \
@@ -773,8 +790,8 @@ IERT_API int iert_latent_attention_decode_tc(const void* q, int q_f32, long long
   launch_dep(latent_absorb_q_kernel<TQ, TT>, dim3((T + TT - 1) / TT, Hpad), dim3(ABSORB_THREADS), (size_t)TT * (D + 4 * rank) * sizeof(float), \
              stream, (const TQ*)q, ldq, (const __nv_bfloat16*)w_uk, (__nv_bfloat16*)qa, H, Hpad, D, R, rank, inv_freq, rot_mul, pairing, *batch)
   if (wide_absorb) {
-    if (q_f32) { if (wide == 8) ABSORB_WIDE(float, 8); else ABSORB_WIDE(float, 16); }
-    else { if (wide == 8) ABSORB_WIDE(__nv_bfloat16, 8); else ABSORB_WIDE(__nv_bfloat16, 16); }
+    if (q_f32) { if (absorb_tt == 8) ABSORB_WIDE(float, 8); else ABSORB_WIDE(float, 16); }
+    else { if (absorb_tt == 8) ABSORB_WIDE(__nv_bfloat16, 8); else ABSORB_WIDE(__nv_bfloat16, 16); }
   } else if (q_f32) { if (tt == 1) ABSORB(float, 1); else if (tt == 2) ABSORB(float, 2); else ABSORB(float, 4); }
   else { if (tt == 1) ABSORB(__nv_bfloat16, 1); else if (tt == 2) ABSORB(__nv_bfloat16, 2); else ABSORB(__nv_bfloat16, 4); }
 #undef ABSORB
@@ -797,7 +814,7 @@ IERT_API int iert_latent_attention_decode_tc(const void* q, int q_f32, long long
   launch_dep(latent_merge_wide_kernel<TT>, dim3((T + TT - 1) / TT, H, (V + 127) / 128), dim3(WIDE_THREADS), (size_t)merge_wide_smem(TT, rank).total, stream, \
              (const float*)part_m, (const float*)part_l, (const float*)part_acc, splits, Hpad, rank, sink, gate, (const __nv_bfloat16*)w_uv, \
              (__nv_bfloat16*)out, *batch, H, V)
-  if (wide_merge && wide == 8) MERGE_WIDE(8);
+  if (wide_merge && merge_tt == 8) MERGE_WIDE(8);
   else if (wide_merge) MERGE_WIDE(16);
   else if (tt == 1) MERGE(1);
   else if (tt == 2) MERGE(2);

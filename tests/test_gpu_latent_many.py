@@ -24,6 +24,8 @@ def context(rt, kind, q_lens, pos0, slots):
 @pytest.mark.parametrize("batch", [16, 17, 32, 33, 50])
 @pytest.mark.parametrize("heads,dim,rot,vdim,rank,sink", [(5, 36, 16, 40, 64, False), (32, 128, 64, 128, 512, False), (3, 64, 32, 136, 96, False),
                                                           (4, 64, 0, 64, 128, True), (17, 20, 8, 24, 520 - 8, False),
+                                                          (64, 16, 8, 24, 40, False), (70, 32, 16, 136, 16, False), (40, 64, 32, 64, 256, False),
+                                                          (9, 128, 16, 128, 256, False), (4, 128, 64, 128, 128, False),
                                                           (4, 32, 16, 32, 16, False), (3, 16, 8, 24, 24, False), (20, 32, 0, 32, 32, True),
                                                           (4, 16, 8, 16, 40, False), (33, 64, 16, 136, 56, False)])
 def test_against_the_plain_kernels(batch, heads, dim, rot, vdim, rank, sink):
