@@ -18,6 +18,7 @@ def _slots(head_dim: int) -> int:
 _MAX_SPLITS = 16
 # what a cut by length costs a batch that fills the device, in page loads: at all, and for every round of the even step's CTAs
 CUT_COSTS, CUT_COSTS_A_ROUND = 24, 11
+CUT_SAVES_ROUND = 20         # page loads that a mostly empty last round must leave idle
 
 
 def decode_splits(n_tokens: int, kv_heads: int, group: int, head_dim: int) -> int:
@@ -36,9 +37,10 @@ def wants_length_cut(pos0, kv_heads: int, group: int, window, page_tokens: int, 
     if the longest sequence reads over 1.3 times the average number of pages (an even cut ends when its CTAs do).
     Where the batch alone fills the device, an even step needs neither parts nor a merge and takes about as long as its longest
     sequence or its share of all pages, whichever is more; a cut takes the share, a grid of eight parts per sequence (most of them empty)
-    and the merge: yes if the longest sequence has more pages beyond the share than that costs.  Measured at 32 heads over 8, even / cut,
+    and the merge: yes if the longest sequence has more pages beyond the share than that costs, or if a last round of CTAs that is mostly
+    empty leaves the slots idle for 20 page loads or more.  Measured at 32 heads over 8, even / cut,
     us a layer: 64 sequences of 200 to 256 positions 55 / 77, of 100 to 2,048 90 / 102, of 100 to 8,192 242 / 224, one of 8,000 among 63 of 200
-    126 / 91, two of 3,000 77 / 84; 48 of 2,100 111 / 114, of 100 to 4,096 125 / 115 (even by this rule), two of 3,000 among 46 of 200 75 / 72; 128 of 100 to
+    126 / 91, two of 3,000 77 / 84; 40 of 2,100 108 / 106, 48 of 2,100 111 / 114, of 100 to 4,096 125 / 115, two of 3,000 among 46 of 200 75 / 72; 128 of 100 to
     4,096 214 / 232, four of 1,500 among 124 of 500 95 / 135; 20 of 100 to 2,048 56 / 60, of 100 to 8,192 132 / 107."""
     n = len(pos0)
     if n < 2:
@@ -54,8 +56,10 @@ def wants_length_cut(pos0, kv_heads: int, group: int, window, page_tokens: int, 
     slots = _slots(head_dim)
     if 2 * n * per_sequence <= slots:
         return longest * n > 1.3 * total
-    rounds = n * per_sequence / slots
-    return longest - total * per_sequence / slots >= CUT_COSTS + CUT_COSTS_A_ROUND * rounds
+    rounds, share = n * per_sequence / slots, total * per_sequence / slots
+    if rounds > 1 and -(-n * per_sequence // slots) >= 1.4 * rounds and share * (-(-n * per_sequence // slots) / rounds - 1) >= CUT_SAVES_ROUND:
+        return True
+    return longest - share >= CUT_COSTS + CUT_COSTS_A_ROUND * rounds
 
 
 def decode_parts(n_tokens: int, kv_heads: int, group: int, unequal: bool, head_dim: int):
