@@ -2,8 +2,9 @@
 file has it (reference layout: src/ops/matmul.rs:1-3).  Not a registered part: mixers,
 feed-forwards and the output head use it for their matrix products.
 
-float32 runs use the kernel that splits fp32 numbers into three bf16 parts for the tensor cores (an error no
-larger than that of fp32 multiply-adds: csrc/gemm_f32_tc.cu) or, for short inner axes, the plain fp32 kernel
+float32 runs use the kernel that splits fp32 numbers into three bf16 parts for the tensor cores (an error below
+that of one fp32 sum of the same length, and the same within a few per cent where all but a few products are zero:
+csrc/gemm_f32_tc.cu) or, for short inner axes, the plain fp32 kernel
 (every multiply-add in 32-bit).  bfloat16 runs use the tcgen05 tensor-core kernel.  A runtime that asks for
 plain kernels only gets the plain kernel in both.
 """

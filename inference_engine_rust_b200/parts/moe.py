@@ -8,11 +8,12 @@ Run as two products over all experts at once: the experts' gate and up matrices 
 [expert 0 | expert 1 | ... | shared]; the block of an expert the token did not choose is multiplied by
 0 (by its routing weight otherwise) before the down product, which then sums exactly the chosen experts'
 outputs and the shared one and adds them to the residual.  The products are the same projection kernels
-the dense feed-forward uses, the step stays free of host decisions (CUDA graphs), and the result does
-not depend on what else is in the batch; the price is that every expert's product is computed for every
+the dense feed-forward uses, the step stays free of host decisions (CUDA graphs), and a token's result does
+not depend on what the other tokens are; the price is that every expert's product is computed for every
 token.  One-token steps and short prompts pay it gladly (all experts' weights are read anyway); longer prompts sort
 their (token, choice) pairs by expert on the device and run each expert's products over its own rows alone
-(`_forward_grouped`), the sums of a token's choices being added to the residual in order.
+(`_forward_grouped`), the sums of a token's choices being added to the residual in order.  The step's number of tokens picks the form, and
+the forms round differently: a prompt's result may differ in its last bits with how many tokens are batched beside it.
 
 `GroupedMoE` (kind "grouped_moe") is the same with another router and another expert: scores are the softmax over ALL
 router outputs, the choice is made on score + a stored `correction`, restricted to the `keep` best of `groups` equal
