@@ -357,7 +357,7 @@ struct StageStore {
   }
 };
 
-// FACTORS (gated launches): a factor per token and block of columns (p.ep).  A form of its own, since the dense feed-forwards have none:
+// FACTORS (gated launches, if p.ep asks for it): a factor per token and block of columns (p.ep).  A form of its own, since the dense feed-forwards have none:
 // with the factors' loads and the unrolled epilogue in their kernel, and the number of token tiles in a register instead of the parameters,
 // they took up to 1.7 us longer (64 tokens x 28,672 x 4,096 45.7 us, so 47.4).
 template <int BT, bool GATED, bool GROUPED = false, bool FACTORS = false>
@@ -406,7 +406,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   if (threadIdx.x == 0) pdl_launch_dependents();
   if (threadIdx.x == 0) IERT_TRACE(0);                       // start
   if (GROUPED) pdl_wait();                                   // the table of row tiles comes from a kernel in front
-  const int group_tiles = GROUPED ? p.groups[0] : 0;
+  // (without groups read from the parameters where it is needed; the form with factors holds it and keeps all 32 of them in registers so)
+  const int held_tiles = GROUPED ? p.groups[0] : FACTORS ? p.t_tiles : 0;
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -418,10 +419,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       uint32_t phase = 0;
       bool ok = true, dep_ready = GROUPED;
       int pend_kb[12], pend_t0[12];
-      WorkIter it(p, GROUPED ? group_tiles : p.t_tiles);
+      WorkIter it(p, GROUPED || FACTORS ? held_tiles : p.t_tiles);
       int tile, split, n_parts, kb0, kb1;
       while (ok && it.next(tile, split, n_parts, kb0, kb1)) {
-        const TilePlace at = tile_place<BT, GROUPED>(p, tile, group_tiles);
+        const TilePlace at = tile_place<BT, GROUPED>(p, tile, held_tiles);
         const int t0 = at.t0, w_row = at.w_row, w_col = at.w_col;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!dep_ready && issued == stages) {
@@ -471,7 +472,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
-      WorkIter it(p, GROUPED ? group_tiles : p.t_tiles);
+      WorkIter it(p, GROUPED || FACTORS ? held_tiles : p.t_tiles);
       int tile, split, n_parts, kb0, kb1;
       while (ok && it.next(tile, split, n_parts, kb0, kb1)) {
         if (!wait_or_abort(&acc_empty[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
@@ -521,10 +522,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     bool ok = true;
     StageStore stage_out{&map_o, out_s + q * 8192, lane, 0, 0};
     if (GATED && p.tma_store && threadIdx.x == 64) tma_prefetch_desc(&map_o);
-    WorkIter it(p, GROUPED ? group_tiles : p.t_tiles);
+    WorkIter it(p, GROUPED || FACTORS ? held_tiles : p.t_tiles);
     int tile, split, n_parts, kb0, kb1;
     while (ok && it.next(tile, split, n_parts, kb0, kb1)) {
-      const TilePlace at = tile_place<BT, GROUPED>(p, tile, group_tiles);
+      const TilePlace at = tile_place<BT, GROUPED>(p, tile, held_tiles);
       const int n_idx = at.n_idx, n0 = at.n0, t0 = at.t0, t_end = at.t_end;
       const int n = n0 + n_local;
       const int t_valid = min(BT, t_end - t0);
@@ -532,7 +533,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       constexpr int N_FACTORS = FACTORS && !GATED && BT <= 32 ? BT : 1;
       float factor[N_FACTORS];
       const float* factor_col = nullptr;
-      if (FACTORS && !GATED && q < 2) {
+      if (FACTORS && !GATED && p.mode == MODE_GATED_SILU && p.ep.scale && q < 2) {
         factor_col = p.ep.scale + (long long)t0 * p.ep.ld_scale + epilogue_block(n0 + n_local, p.ep);
 #pragma unroll
         for (int j = 0; j < N_FACTORS; ++j) factor[j] = j < t_valid ? factor_col[(long long)j * p.ep.ld_scale] : 0.f;
@@ -674,7 +675,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         // that belong to them.  The up warps hand their values over through shared memory, the
         // gate warps write silu(gate) * up, 64 consecutive outputs of a token per pair of warps.
         float* xch = reinterpret_cast<float*>(xch_s);                 // [16 tokens][64]
-        auto sixteen = [&](int c) {
+        if constexpr (FACTORS) {                     // unrolled: the factors are in registers
+#pragma unroll
+        for (int c = 0; c < BT; c += 16) {
+          if (c >= t_valid) break;                   // uniform over the four warps
           float v[16];
           tmem_ld16(taddr + c, v);
           if (q >= 2) {
@@ -690,20 +694,38 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 if (c + j < t_valid) {
                   const float r = scaled ? rstd_s[c + j] : 1.0f;
                   float act = silu_mul(v[j] * r, xch[j * 64 + n_local] * r);
-                  if (FACTORS) act *= N_FACTORS > 1 ? factor[(c + j) % N_FACTORS] : factor_col[(long long)(c + j) * p.ep.ld_scale];
+                  if (factor_col) act *= N_FACTORS > 1 ? factor[(c + j) % N_FACTORS] : factor_col[(long long)(c + j) * p.ep.ld_scale];
                   ((__nv_bfloat16*)p.out)[(long long)(t0 + c + j) * p.ldo + i] = __float2bfloat16_rn(act);
                 }
             }
           }
           asm volatile("bar.sync 1, 128;" ::: "memory");
-        };
-        if constexpr (FACTORS) {                     // unrolled: the factors are in registers
-#pragma unroll
-          for (int c = 0; c < BT; c += 16)
-            if (c < t_valid) sixteen(c);             // uniform over the four warps
+        }
         } else {
 #pragma unroll 1
-          for (int c = 0; c < t_valid; c += 16) sixteen(c);
+        for (int c = 0; c < BT; c += 16) {
+          if (c >= t_valid) break;
+          float v[16];
+          tmem_ld16(taddr + c, v);
+          if (q >= 2) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) xch[j * 64 + (n_local - 64)] = v[j];
+          }
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+          if (q < 2) {
+            const int i = n0 + n_local;              // n0 counts gate rows here (64 per tile)
+            if (i < p.N) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                if (c + j < t_valid) {
+                  const float r = scaled ? rstd_s[c + j] : 1.0f;
+                  float act = silu_mul(v[j] * r, xch[j * 64 + n_local] * r);
+                  ((__nv_bfloat16*)p.out)[(long long)(t0 + c + j) * p.ldo + i] = __float2bfloat16_rn(act);
+                }
+            }
+          }
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+        }
         }
       }
       // Many tokens, residual add, whole tile: 32 tokens per pass, so that twice as many reads of
@@ -1293,7 +1315,7 @@ int gemm_tc_impl(const void* x, long long ldx, const void* w, long long ldw, voi
   }
   switch (bt) {
     case 16: return launch<16, false>(mw, mx, p, grid, stream);
-    case 32: return launch<32, false>(mw, mx, p, grid, stream);
+    case 32: return launch<32, false, false, true>(mw, mx, p, grid, stream);      // (as the gated launches, see there)
     case 64: return launch<64, false>(mw, mx, p, grid, stream);
     case 128: return launch<128, false>(mw, mx, p, grid, stream, p.tma_out ? &mo : nullptr);
     default: return launch<256, false>(mw, mx, p, grid, stream, p.tma_out ? &mo : nullptr);
@@ -1387,7 +1409,9 @@ int gemm_tc_gated_impl(const void* x, long long ldx, const void* w, long long ld
     const int grid = p.n_tiles < slots ? p.n_tiles : slots;
     switch (wbt) {
       case 16: return ep ? launch<16, false, false, true>(mw, mx, p, grid, stream) : launch<16, false>(mw, mx, p, grid, stream);
-      case 32: return ep ? launch<32, false, false, true>(mw, mx, p, grid, stream) : launch<32, false>(mw, mx, p, grid, stream);
+      // (one kernel for both products and all launches of 17 to 32 tokens: dense ones lose nothing to the factors' form there, and a mixture's
+      // step of 32 tokens whose products are different kernels took 91.7 us, so 86.3)
+      case 32: return launch<32, false, false, true>(mw, mx, p, grid, stream);
       default: return ep ? launch<64, false, false, true>(mw, mx, p, grid, stream) : launch<64, false>(mw, mx, p, grid, stream);
     }
   }
