@@ -742,7 +742,7 @@ def delta_recur(qkv, beta, decay, state, s_off: int, o, G: int, D: int, H: int, 
     (`recurrent_scratch_floats`): prompts may go several tokens at a time."""
     _check_lib(_recurrent_lib(D).iert_delta_recur(qkv.data_ptr(), beta.data_ptr(), decay.data_ptr(), state.data_ptr(),
                                                   state.stride(0), s_off, o.data_ptr(), _ptr(scratch), G, H, V, byref(batch), stream),
-               "delta_recur", 2 if scratch is not None and batch.n_tokens >= 16 * batch.n_seqs and D in (64, 128) else 1)
+               "delta_recur", 2 if scratch is not None and batch.n_tokens >= max(32, 16 * batch.n_seqs) and D in (64, 128) else 1)
 
 
 def mlstm_recur(proj, gates, bi, bf, cap: float, state, s_off: int, n_off: int, m_off: int, coef, o, D: int, H: int, V: int,

@@ -168,56 +168,233 @@ __global__ void __launch_bounds__(256 + LOADERS) delta_recur_kernel(DeltaArgs a,
   }
 }
 
-// ---- prompts: eight tokens at a time ---------------------------------------------------------------------------------
+// ---- prompts: sixteen tokens at a time, on the tensor cores ------------------------------------------------------------
 // Token after token, a step's time is the latency of its chain (dot product, shuffles, update: about 680 cycles a token), not its
-// work.  Over a chunk of c = 8 tokens with decays g and G_i = g_1 .. g_i, the state in front of the chunk S and u_i as above:
+// work.  Over a chunk of 16 tokens with decays g and G_i = g_1 .. g_i, the state in front of the chunk S and u_i as above:
 //
-//   S_i = G_i S + sum_{j <= i} (G_i / G_j) k_j u_j      so      u_i = beta_i (v_i - G_i k_i.S - sum_{j < i} (G_i / G_j) (k_i.k_j) u_j)
-//   o_i = G_i q_i.S + sum_{j <= i} (G_i / G_j) (q_i.k_j) u_j
+//   S_i = G_i S + sum_{j <= i} (G_i / G_j) k_j u_j      so      u_i + sum_{j < i} A_ij u_j = x_i = beta_i (v_i - G_i k_i.S),
+//   A_ij = beta_i (G_i / G_j) (k_i.k_j)                          u = T x,  T = (1 + A)^-1  (lower triangular)
+//   o_i = G_i q_i.S + sum_{j <= i} P_ij u_j,  P_ij = (G_i / G_j) (q_i.k_j)
 //
-// The sixteen dot products k_i.S, q_i.S of a column are independent: all their partial sums are formed first and then added
-// over the 16 lanes of the column together, each lane ending with one of them (15 shuffles instead of 64); what is left of
-// the chain is eight steps of one broadcast and one multiply-add.  The tokens' products k_i.k_j, q_i.k_j (the same for all
-// columns) with the ratios (products of the decays between, never quotients) come from a kernel in front, which has a block per
-// chunk and key head; a loader warp brings everything through a ring of four chunks.  Everything is fp32.
-// A thread owns DIM / 16 rows of FOUR columns, so that a token's k and q, read from shared memory, serve four columns (with two
-// columns and twice the warps: 448 us against 404 over 2,048 tokens, 32 heads of 128 x 128).  Two rows share an
-// instruction: 344 us.
+// T and P (the same for all columns; ratios are products of the decays between, never quotients) come from a kernel in front with a
+// block per chunk and key head.  What is left is products of matrices: k.S, q.S, T x, P u and the update k^T u, on mma.sync m16n8k16.
+// The state is kept transposed, S^T [16 columns x rows], in the accumulator layout of one warp: as the left operand of k.S and
+// q.S it needs no exchange between lanes, and x and u come out as left operands of the next product.
+//
+// Everything stays fp32: an operand is the sum of three bf16 numbers (the nearest, the nearest to the remainder, the rest), a
+// product is the six partial products of weight 2^-16 and more, the largest in an accumulator of its own and no accumulator over
+// more than DIM / 2 numbers; these sums are added to fp32 registers by rounded additions (the three products left out come to 2^-24).
+// mma.sync runs at 1,020 multiply-adds per clock and SM here, so six products are worth 170 against 124 for FFMA, and there are
+// no dot products to add over lanes (15 shuffles per sum of 16 lanes before).
+//
+// A block owns 32 columns: four warps compute, each 16 columns x half of the rows (the halves of k.S and q.S are exchanged through
+// shared memory), four bring q, k, v and the coefficients and split them.  2,048 tokens, 32 heads of 128 x 128 (128 blocks): 200 to
+// 212 us; eight tokens at a time with FFMA, a thread holding 8 rows of four columns, took 344.  What bounds it is the chain
+// k.S - x - u - S of a warp, about 2,900 clocks a chunk: its 162 mma.sync take 10 to 12 clocks each beside ldmatrix, and nothing else of
+// that warp's scheduler has as much to do.  Other splits were no faster: q.S and P u in warps of their own with the state's parts
+// through shared memory 222, quarters of the rows in twice the warps 261 (236 with the column groups half a chunk apart).
 #define IERT_CHUNKED (DIM == 64 || DIM == 128)                // (larger sizes would not fit the registers)
 #if IERT_CHUNKED
-constexpr int CT = 8, CG = 4, CL = 16, CWORK = 128, CCOLS = CWORK / CL * CG;
-constexpr int CP = DIM / CL / 2;                              // pairs of rows per lane
-constexpr int RING = 4;                                       // chunks in shared memory
-// per token and head: 8 coefficients of earlier u in u_i, 8 in o_i, then G_i, G_8 / G_i, beta_i, G_8
-constexpr int COEF = 20;
+constexpr int CT = 16, CCOLS = 32, RING = 4;                  // tokens of a chunk, columns of a block, chunks in shared memory
+constexpr int CLOAD = 128;                                    // loading threads
+constexpr int OPROW = DIM + 8;                                // numbers from row to row of an operand tile: 8 rows meet no bank twice
+constexpr int VROW = CCOLS + 4;
+// per token and head: 16 of T, 16 of P, then beta_i, G_i, G_16 / G_i, and G_16 at the chunk's first token
+constexpr int COEF = 36, CROW = 40;
+constexpr int TPROW = 24;                                     // rows of 16 coefficients as operands
 
-// A lane's rows 64 x + 4 r .. + 3 of a vector in shared memory.
-__device__ __forceinline__ void own_rows(float2 (&v)[CP], const float* src, int r) {
+template <bool FIRST>      // d = a b (+ d)
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  if (FIRST)
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+  else
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// (Volatile, so that they stay behind the barriers in front of them; the tiles are other threads' writes, so this thread's own accesses may move past.)
+template <bool TRANS>
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16* p) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  if (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+
+// Two numbers as pairs of bf16 numbers p[0] + p[1] + p[2]; every remainder is exact.
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  float2 d;
+  asm("sub.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return d;
+}
+__device__ __forceinline__ void split2(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+  auto nearest = [](float2 f) {
+    const __nv_bfloat162 two = __floats2bfloat162_rn(f.x, f.y);
+    return *reinterpret_cast<const uint32_t*>(&two);
+  };
+  auto wide = [](uint32_t p) { return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u)); };
+  float2 f = make_float2(x, y);
+  p0 = nearest(f);
+  f = sub2(f, wide(p0));
+  p1 = nearest(f);
+  p2 = nearest(sub2(f, wide(p1)));
+}
+// Two neighbouring accumulator tiles [16 x 8] as the three parts of a left operand [16 x 16].
+struct Left { uint32_t p[3][4]; };
+__device__ __forceinline__ void left_of(Left& a, const float (&t0)[4], const float (&t1)[4]) {
+  split2(t0[0], t0[1], a.p[0][0], a.p[1][0], a.p[2][0]);
+  split2(t0[2], t0[3], a.p[0][1], a.p[1][1], a.p[2][1]);
+  split2(t1[0], t1[1], a.p[0][2], a.p[1][2], a.p[2][2]);
+  split2(t1[2], t1[3], a.p[0][3], a.p[1][3], a.p[2][3]);
+}
+// A product's sums: the main one (first parts), first with second parts, and the rest.  (Sums of their own so that a product does not wait for the
+// one in front of it: an mma.sync is issued every 8 clocks and takes 21.)
+struct Sums {
+  float m[4], a[4], b[4];
+  __device__ __forceinline__ float2 two(int i) const {
+    return add2(make_float2(m[2 * i], m[2 * i + 1]), add2(make_float2(a[2 * i], a[2 * i + 1]), make_float2(b[2 * i], b[2 * i + 1])));
+  }
+  __device__ __forceinline__ void all(float (&o)[4]) const {
+    const float2 x = two(0), y = two(1);
+    o[0] = x.x; o[1] = x.y; o[2] = y.x; o[3] = y.y;
+  }
+};
+// The six products of a left operand with two right operands (tiles of 8 outputs), r[part][4] as ldmatrix brings them.
+template <bool FIRST>
+__device__ __forceinline__ void six_by_two(Sums& s0, Sums& s1, const Left& l, const uint32_t (&r)[3][4]) {
+  mma16816<FIRST>(s0.b, l.p[0], r[2][0], r[2][1]); mma16816<FIRST>(s1.b, l.p[0], r[2][2], r[2][3]);
+  mma16816<FIRST>(s0.a, l.p[0], r[1][0], r[1][1]); mma16816<FIRST>(s1.a, l.p[0], r[1][2], r[1][3]);
+  mma16816<false>(s0.b, l.p[2], r[0][0], r[0][1]); mma16816<false>(s1.b, l.p[2], r[0][2], r[0][3]);
+  mma16816<FIRST>(s0.m, l.p[0], r[0][0], r[0][1]); mma16816<FIRST>(s1.m, l.p[0], r[0][2], r[0][3]);
+  mma16816<false>(s0.b, l.p[1], r[1][0], r[1][1]); mma16816<false>(s1.b, l.p[1], r[1][2], r[1][3]);
+  mma16816<false>(s0.a, l.p[1], r[0][0], r[0][1]); mma16816<false>(s1.a, l.p[1], r[0][2], r[0][3]);
+}
+// Three parts of an operand tile whose rows are tokens, as two right operands.  TRANS: the tokens are summed over (k^T u); else they are
+// the outputs (k.S).  `tile`: part 0, first row, first column.
+template <bool TRANS>
+__device__ __forceinline__ void right_of(uint32_t (&r)[3][4], const __nv_bfloat16* tile, int ld, int lane) {
+  const int row = TRANS ? (lane & 7) + (((lane >> 3) & 1) << 3) : (lane & 7) + ((lane >> 4) << 3);
+  const int col = TRANS ? (lane >> 4) * 8 : ((lane >> 3) & 1) * 8;
 #pragma unroll
-  for (int x = 0; x < CP / 2; ++x) {
-    const float4 f = *reinterpret_cast<const float4*>(src + 64 * x + 4 * r);
-    v[2 * x] = make_float2(f.x, f.y);
-    v[2 * x + 1] = make_float2(f.z, f.w);
+  for (int p = 0; p < 3; ++p) ldsm4<TRANS>(r[p], tile + (p * CT + row) * ld + col);
+}
+// Rows of coefficients of eight tokens (`tile`: part 0, first row) as a right operand, and the sums over the chunk's tokens of coefficient times x.
+struct Rows { uint32_t p[3][2]; };
+__device__ __forceinline__ void rows_of(Rows& b, const __nv_bfloat16* tile, int lane) {
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(tile + (p * CT + (lane & 7)) * TPROW + ((lane >> 3) & 1) * 8);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(b.p[p][0]), "=r"(b.p[p][1]) : "r"(at));
   }
 }
-// The rows 64 x + 4 r .. + 3 of four columns of the state, from memory and back.
-__device__ __forceinline__ void load_rows(float2 (&S)[CP][CG], const float* Sg, int V, int r, bool live) {
+__device__ __forceinline__ void six_of_rows(float (&o)[4], const Left& l, const Rows& b) {
+  float m[4], s0[4], s1[4];
+  mma16816<true>(m, l.p[0], b.p[0][0], b.p[0][1]);
+  mma16816<true>(s0, l.p[0], b.p[2][0], b.p[2][1]);
+  mma16816<true>(s1, l.p[0], b.p[1][0], b.p[1][1]);
+  mma16816<false>(s0, l.p[2], b.p[0][0], b.p[0][1]);
+  mma16816<false>(s1, l.p[1], b.p[0][0], b.p[0][1]);
+  mma16816<false>(s0, l.p[1], b.p[1][0], b.p[1][1]);
 #pragma unroll
-  for (int i = 0; i < CP; ++i) {
-    const float* p = Sg + (size_t)((i / 2) * 64 + 4 * r + (i % 2) * 2) * V;
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 u = live ? *reinterpret_cast<const float4*>(p) : z, v = live ? *reinterpret_cast<const float4*>(p + V) : z;
-    S[i][0] = make_float2(u.x, v.x); S[i][1] = make_float2(u.y, v.y); S[i][2] = make_float2(u.z, v.z); S[i][3] = make_float2(u.w, v.w);
+  for (int e = 0; e < 4; ++e) o[e] = m[e] + (s1[e] + s0[e]);
+}
+// sum_{j <= t} coef[t][j] x_j for this lane's tokens t = t0 + 2 (lane % 4) + {0, 1} and both rows of its tiles, where an infinity or a NaN
+// among the x must not reach the tokens in front of it (whose coefficients are zeros).
+__device__ __noinline__ float4 causal_sum(const float4 x0, const float4 x1, const float* coef, int ld, int t0) {
+  const int lane = threadIdx.x & 31, t = t0 + 2 * (lane & 3);
+  const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+  float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < CT; ++j) {
+    const int from = (lane & ~3) | ((j & 7) >> 1);
+    const float a = __shfl_sync(0xffffffffu, x[4 * (j >> 3) + (j & 1)], from), b = __shfl_sync(0xffffffffu, x[4 * (j >> 3) + 2 + (j & 1)], from);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (j <= t + i) {
+        const float f = coef[(t + i) * ld + j];
+        o[i] = fmaf(f, a, o[i]);
+        o[2 + i] = fmaf(f, b, o[2 + i]);
+      }
+  }
+  return make_float4(o[0], o[1], o[2], o[3]);
+}
+__device__ __forceinline__ bool any_not_finite(const float (&x)[2][4]) {
+  float z = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) z = fmaf(x[0][i], 0.f, fmaf(x[1][i], 0.f, z));
+  return __any_sync(0xffffffffu, z != 0.f);          // (a NaN is not equal to 0)
+}
+
+// A warp's part of the state: columns col, col + 8 (of the block's, by lane), rows 8 i + 2 (lane % 4) + {0, 1} of its share.
+template <int NT>
+__device__ __forceinline__ void load_state(float (&S)[NT][4], const float* Sg, int V, int row0, int col, int lane) {
+#pragma unroll
+  for (int i = 0; i < NT; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int d = row0 + 8 * i + 2 * (lane & 3) + (e & 1), j = col + 8 * (e >> 1);
+      S[i][e] = j < V ? Sg[(size_t)d * V + j] : 0.f;
+    }
+}
+template <int NT>
+__device__ __forceinline__ void store_state(const float (&S)[NT][4], float* Sg, int V, int row0, int col, int lane) {
+#pragma unroll
+  for (int i = 0; i < NT; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int d = row0 + 8 * i + 2 * (lane & 3) + (e & 1), j = col + 8 * (e >> 1);
+      if (j < V) Sg[(size_t)d * V + j] = S[i][e];
+    }
+}
+// (k or q).S over this warp's rows of S: `tile` their part 0, first token.
+template <int NK>
+__device__ __forceinline__ void state_product(Sums& s0, Sums& s1, const Left (&st)[NK], const __nv_bfloat16* tile, int lane) {
+  uint32_t r[2][3][4];
+  right_of<false>(r[0], tile, OPROW, lane);
+#pragma unroll
+  for (int i = 0; i < NK; ++i) {
+    if (i + 1 < NK) right_of<false>(r[(i + 1) & 1], tile + 16 * (i + 1), OPROW, lane);
+    if (i == 0) six_by_two<true>(s0, s1, st[i], r[i & 1]);
+    else six_by_two<false>(s0, s1, st[i], r[i & 1]);
   }
 }
-__device__ __forceinline__ void store_rows(const float2 (&S)[CP][CG], float* Sg, int V, int r) {
+// S <- scale S + k^T u over the chunk's tokens, two tiles of rows at a time; scale(i): the factors of tile i's rows of this lane; `tile`: as above.
+// The parts of the new S, for the chunk behind, are made while the next tiles' products run.
+template <int NT, int NK, typename Scale>
+__device__ __forceinline__ void update_state(float (&S)[NT][4], Left (&st)[NK], const Left& u, const __nv_bfloat16* tile, int lane, Scale scale) {
+  uint32_t r[2][3][4];
 #pragma unroll
-  for (int i = 0; i < CP; ++i) {
-    float* p = Sg + (size_t)((i / 2) * 64 + 4 * r + (i % 2) * 2) * V;
-    *reinterpret_cast<float4*>(p) = make_float4(S[i][0].x, S[i][1].x, S[i][2].x, S[i][3].x);
-    *reinterpret_cast<float4*>(p + V) = make_float4(S[i][0].y, S[i][1].y, S[i][2].y, S[i][3].y);
+  for (int i = 0; i < NT; i += 2) {
+    if (i == 0) right_of<true>(r[0], tile, OPROW, lane);
+    if (i + 2 < NT) right_of<true>(r[(i / 2 + 1) & 1], tile + 8 * (i + 2), OPROW, lane);
+    Sums s0, s1;
+    six_by_two<true>(s0, s1, u, r[(i / 2) & 1]);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float2 f = fma2(make_float2(S[i][2 * e], S[i][2 * e + 1]), scale(i), s0.two(e));
+      const float2 g = fma2(make_float2(S[i + 1][2 * e], S[i + 1][2 * e + 1]), scale(i + 1), s1.two(e));
+      S[i][2 * e] = f.x; S[i][2 * e + 1] = f.y;
+      S[i + 1][2 * e] = g.x; S[i + 1][2 * e + 1] = g.y;
+    }
+    left_of(st[i / 2], S[i], S[i + 1]);
   }
 }
+__device__ __forceinline__ void group_sync(int group, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(2 + group), "r"(threads) : "memory"); }
+__device__ __forceinline__ void loaders_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CLOAD) : "memory"); }
 
 __device__ __forceinline__ void copy16(void* dst, const void* src, bool in) {      // zeros where there is nothing to read
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
@@ -225,7 +402,8 @@ __device__ __forceinline__ void copy16(void* dst, const void* src, bool in) {   
 template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
-// The chunk that block `x` of a grid over all sequences' chunks looks after: first token and end of the sequence; false: none.
+// The chunk of CT tokens that block `x` of a grid over all sequences' chunks looks after: first token and end of the sequence; false: none.
+template <int CT>
 __device__ __forceinline__ bool chunk_of(const IertBatchView& b, int x, int& tc, int& t1) {
   for (int s = 0; s < b.n_seqs; ++s) {
     const int lo = b.cu_q[s], hi = b.cu_q[s + 1], n = (hi - lo + CT - 1) / CT;
@@ -239,73 +417,97 @@ __device__ __forceinline__ bool chunk_of(const IertBatchView& b, int x, int& tc,
   return false;
 }
 
-// Block (chunk, key head): a thread per product of two of the chunk's tokens, then per coefficient of each head that shares them.
+// Block (chunk, key head): a thread per product of two of the chunk's tokens (q_i.k_j for j <= i, k_i.k_j else), then, eight heads
+// that share them at a time, a thread per head and column of A, P and T.  (A thread per entry that multiplied its own decays took 40 us
+// for 2,048 tokens, 8 key heads and 32 heads: 25 now.)
 // (No early start for the kernel behind: its blocks want an SM each, and would be packed in pairs beside this kernel's.)
-__global__ void __launch_bounds__(128) delta_coef_kernel(DeltaArgs a, float* __restrict__ coef, IertBatchView b) {
-  __shared__ __align__(16) float k_s[CT][DIM + 4], q_s[CT][DIM + 4];
-  __shared__ float dot_s[2 * CT][CT], g_s[CT], beta_s[CT];
+__global__ void __launch_bounds__(CT * CT, 4) delta_coef_kernel(DeltaArgs a, float* __restrict__ coef, IertBatchView b) {
+  constexpr int HEADS = 8;
+  __shared__ __align__(16) float k_s[CT][DIM + 4], q_s[CT][DIM + 4], A_s[HEADS][CT][CT];
+  __shared__ float dot_s[CT][CT + 1], g_s[HEADS][CT], beta_s[HEADS][CT];
   pdl_wait();
   int tc, t1;
-  if (!chunk_of(b, blockIdx.x, tc, t1)) return;
+  if (!chunk_of<CT>(b, blockIdx.x, tc, t1)) return;
   const int g = blockIdx.y, GD = a.G * DIM, C = 2 * GD + a.H * a.V, n = min(CT, t1 - tc), rep = a.H / a.G;
-  for (int x = threadIdx.x; x < CT * DIM / 4; x += 128) {
+  for (int x = threadIdx.x; x < CT * DIM / 4; x += CT * CT) {
     const int t = x / (DIM / 4), d = 4 * (x % (DIM / 4));
     const float* row = a.qkv + (size_t)(tc + min(t, n - 1)) * C + g * DIM + d;
     *reinterpret_cast<float4*>(&q_s[t][d]) = *reinterpret_cast<const float4*>(row);
     *reinterpret_cast<float4*>(&k_s[t][d]) = *reinterpret_cast<const float4*>(row + GD);
   }
-  __syncthreads();
-  const int row = threadIdx.x / CT, j = threadIdx.x % CT, i = row % CT;      // row i of u, or row 8 + i of o
-  const bool used = j < i + (row >= CT ? 1 : 0);
-  if (used) {
-    const float* x = row < CT ? k_s[i] : q_s[i];
-    const float* y = k_s[j];
-    float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
+  const int hh = threadIdx.x / CT, j = threadIdx.x % CT;
+  for (int h0 = g * rep; h0 < (g + 1) * rep; h0 += HEADS) {
+    const int h = h0 + hh;
+    const bool mine = hh < min(HEADS, (g + 1) * rep - h0);
+    if (mine) {
+      const bool in = j < n;
+      beta_s[hh][j] = in ? a.beta[(size_t)(tc + j) * a.H + h] : 0.f;
+      g_s[hh][j] = in ? a.decay[(size_t)(tc + j) * a.H + h] : 1.f;
+    }
+    __syncthreads();
+    if (h0 == g * rep) {
+      const float* x = j <= hh ? q_s[hh] : k_s[hh];            // (here hh and j are two tokens)
+      const float* y = k_s[j];
+      float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
 #pragma unroll 8
-    for (int d = 0; d < DIM; d += 4) {
-      const float4 u = *reinterpret_cast<const float4*>(x + d), v = *reinterpret_cast<const float4*>(y + d);
-      d0 = fmaf(u.x, v.x, d0); d1 = fmaf(u.y, v.y, d1); d2 = fmaf(u.z, v.z, d2); d3 = fmaf(u.w, v.w, d3);
-    }
-    dot_s[row][j] = (d0 + d1) + (d2 + d3);
-  }
-  for (int h = g * rep; h < (g + 1) * rep; ++h) {
-    __syncthreads();
-    if (threadIdx.x < CT) {
-      const bool in = (int)threadIdx.x < n;
-      beta_s[threadIdx.x] = in ? a.beta[(size_t)(tc + threadIdx.x) * a.H + h] : 0.f;
-      g_s[threadIdx.x] = in ? a.decay[(size_t)(tc + threadIdx.x) * a.H + h] : 1.f;
-    }
-    __syncthreads();
-    if (i < n) {
-      float* out = coef + ((size_t)(tc + i) * a.H + h) * COEF;
-      float ratio = 1.f;
-      for (int m = j + 1; m <= i; ++m) ratio *= g_s[m];
-      const float v = used ? dot_s[row][j] * ratio : 0.f;
-      out[(row >= CT ? CT : 0) + j] = row < CT ? -beta_s[i] * v : v;
-      if (row < CT && j < 4) {
-        float to = 1.f, from = 1.f;
-        for (int m = 0; m <= i; ++m) to *= g_s[m];
-        for (int m = i + 1; m < CT; ++m) from *= g_s[m];
-        out[2 * CT + j] = j == 0 ? to : j == 1 ? from : j == 2 ? beta_s[i] : to * from;
+      for (int d = 0; d < DIM; d += 4) {
+        const float4 u = *reinterpret_cast<const float4*>(x + d), v = *reinterpret_cast<const float4*>(y + d);
+        d0 = fmaf(u.x, v.x, d0); d1 = fmaf(u.y, v.y, d1); d2 = fmaf(u.z, v.z, d2); d3 = fmaf(u.w, v.w, d3);
       }
+      dot_s[hh][j] = (d0 + d1) + (d2 + d3);
+      __syncthreads();
     }
+    float* out = coef + ((size_t)tc * a.H + h) * COEF;         // (rows of tokens: a.H * COEF apart)
+    const size_t row = (size_t)a.H * COEF;
+    if (mine) {
+      float ratio = 1.f;                                       // g_(j+1) .. g_i
+#pragma unroll
+      for (int i = 0; i < CT; ++i) {
+        if (i > j) ratio *= g_s[hh][i];
+        A_s[hh][j][i] = j < i ? beta_s[hh][i] * (ratio * dot_s[j][i]) : 0.f;
+        if (i < n) {
+          out[i * row + CT + j] = j <= i ? ratio * dot_s[i][j] : 0.f;
+          if (j == 0) out[i * row + 2 * CT + 1] = g_s[hh][0] * ratio;
+        }
+      }
+      if (j < n) {
+        out[j * row + 2 * CT] = beta_s[hh][j];
+        out[j * row + 2 * CT + 2] = ratio;
+      }
+      if (j == 0) out[2 * CT + 3] = g_s[hh][0] * ratio;
+    }
+    __syncthreads();
+    if (mine) {                                      // (1 + A) t = the j-th unit vector
+      float t[CT];
+#pragma unroll
+      for (int m = 0; m < CT; ++m) t[m] = m == j ? 1.f : 0.f;
+#pragma unroll
+      for (int m = 0; m < CT - 1; ++m) {
+        float col[CT];
+#pragma unroll
+        for (int x = (m + 1) / 4 * 4; x < CT; x += 4) *reinterpret_cast<float4*>(col + x) = *reinterpret_cast<const float4*>(&A_s[hh][m][x]);
+#pragma unroll
+        for (int x = m + 1; x < CT; ++x) t[x] = m >= j ? fmaf(-col[x], t[m], t[x]) : t[x];   // (a token's NaN stays behind it)
+      }
+#pragma unroll
+      for (int m = 0; m < CT; ++m)
+        if (m < n) out[m * row + j] = t[m];
+    }
+    __syncthreads();
   }
 }
 
-// Sum over the 16 lanes of a column of 2 * HALF values per column: the lanes whose bit MASK is set keep the upper half.
-template <int HALF, int MASK>
-__device__ __forceinline__ void halve(float (&v)[16][CG], bool upper) {
-#pragma unroll
-  for (int m = 0; m < HALF; ++m)
-#pragma unroll
-    for (int c = 0; c < CG; ++c) {
-      const float send = upper ? v[m][c] : v[m + HALF][c], keep = upper ? v[m + HALF][c] : v[m][c];
-      v[m][c] = keep + __shfl_xor_sync(0xffffffffu, send, MASK);
-    }
-}
+constexpr int DWORK = 128;           // computing threads: two column groups x two halves of the rows
+struct DeltaShared {
+  float v[RING][CT][VROW], c[RING][CT][CROW];
+  __nv_bfloat16 op[2][2][3][CT][OPROW];              // q, k in three parts
+  __nv_bfloat16 tp[2][2][3][CT][TPROW];              // T, P in three parts
+  float4 xk[4][2][32], xq[4][32];                    // a warp's half of the sums k.S, q.S for its partner
+};
 
-__global__ void __launch_bounds__(CWORK + 32) delta_chunk_kernel(DeltaArgs a, const float* __restrict__ coef, IertBatchView b) {
-  __shared__ __align__(16) float k_s[RING][CT][DIM], q_s[RING][CT][DIM], v_s[RING][CT][CCOLS], c_s[RING][CT][COEF];
+__global__ void __launch_bounds__(DWORK + CLOAD, 1) delta_chunk_kernel(DeltaArgs a, const float* __restrict__ coef, IertBatchView b) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  DeltaShared& sh = *reinterpret_cast<DeltaShared*>(smem_raw);
   pdl_wait();
   const int s = blockIdx.x, head = blockIdx.y, c0 = blockIdx.z * CCOLS;
   const int slot = b.slot_ids[s];
@@ -313,109 +515,160 @@ __global__ void __launch_bounds__(CWORK + 32) delta_chunk_kernel(DeltaArgs a, co
   if (slot < 0 || t1 <= t0) return;
   const int n_chunks = (t1 - t0 + CT - 1) / CT;
 
-  if (threadIdx.x >= CWORK) {
-    // ---------------- loader: one warp, three chunks ahead ----------------
-    const int lane = threadIdx.x - CWORK, g = head / (a.H / a.G), GD = a.G * DIM, C = 2 * GD + a.H * a.V;
+  if (threadIdx.x >= DWORK) {
+    // ---------------- loaders: q and k through registers, split a chunk ahead; v and the coefficients three chunks ahead ----------------
+    constexpr int ITER = CT * (DIM / 4) / CLOAD, STEP = CLOAD / (DIM / 4);      // a thread's rows of q: every STEP-th
+    const int lt = threadIdx.x - DWORK, g = head / (a.H / a.G), GD = a.G * DIM, C = 2 * GD + a.H * a.V;
+    const int tq = lt / (DIM / 4), dq = 4 * (lt % (DIM / 4)), tv = lt / (CCOLS / 4), ev = 4 * (lt % (CCOLS / 4));
+    const bool in_v = c0 + ev < a.V;
+    const float* pq = a.qkv + (size_t)(t0 + tq) * C + g * DIM + dq;
+    const float* pv = a.qkv + (size_t)(t0 + tv) * C + 2 * GD + (in_v ? head * a.V + c0 + ev : 0);
+    const float* pc = coef + ((size_t)t0 * a.H + head) * COEF;
+    float4 f[2 * ITER];
+    auto fetch = [&](int n) {
+      const int left = t1 - (t0 + n * CT);
+      const float* x = pq + (size_t)n * CT * C;
+#pragma unroll
+      for (int it = 0; it < ITER; ++it) {
+        const bool in = tq + it * STEP < left;
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        f[it] = in ? *reinterpret_cast<const float4*>(x + (size_t)(it * STEP) * C) : z;
+        f[ITER + it] = in ? *reinterpret_cast<const float4*>(x + (size_t)(it * STEP) * C + GD) : z;
+      }
+    };
     auto ask = [&](int n) {
       if (n < n_chunks) {
-        const int tc = t0 + n * CT, buf = n % RING;
-#pragma unroll
-        for (int t = 0; t < CT; ++t) {
-          const bool in = tc + t < t1;
-          const size_t tok = in ? tc + t : t0;
-          const float* row = a.qkv + tok * C;
-          if (lane < DIM / 4) {
-            copy16(&q_s[buf][t][4 * lane], row + g * DIM + 4 * lane, in);
-            copy16(&k_s[buf][t][4 * lane], row + GD + g * DIM + 4 * lane, in);
-          }
-          if (lane < CCOLS / 4) {
-            const bool col = c0 + 4 * lane < a.V;
-            copy16(&v_s[buf][t][4 * lane], row + 2 * GD + (col ? head * a.V + c0 + 4 * lane : 0), in && col);
-          } else if (lane < CCOLS / 4 + COEF / 4) {
-            const int x = 4 * (lane - CCOLS / 4);
-            copy16(&c_s[buf][t][x], coef + (tok * a.H + head) * COEF + x, in);
-          }
+        const int left = t1 - (t0 + n * CT), buf = n % RING;
+        copy16(&sh.v[buf][tv][ev], tv < left ? pv + (size_t)n * CT * C : a.qkv, tv < left && in_v);
+        for (int y = lt; y < CT * COEF / 4; y += CLOAD) {
+          const int t = y / (COEF / 4), e = 4 * (y % (COEF / 4));
+          copy16(&sh.c[buf][t][e], t < left ? pc + (size_t)(n * CT + t) * a.H * COEF + e : coef, t < left);
         }
       }
       copies_commit();
     };
+    auto put4 = [](const float4& x, __nv_bfloat16* dst, int part) {
+      uint2 p[3];
+      split2(x.x, x.y, p[0].x, p[1].x, p[2].x);
+      split2(x.z, x.w, p[0].y, p[1].y, p[2].y);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(dst + i * part) = p[i];
+    };
+    auto split = [&](int n) {
+      const int out = n & 1, t = lt / 8, e = 4 * (lt % 8);
+      const float4 tp = *reinterpret_cast<const float4*>(&sh.c[n % RING][t][e]);        // T, then P
+#pragma unroll
+      for (int it = 0; it < 2 * ITER; ++it) put4(f[it], &sh.op[out][it / ITER][0][tq + it % ITER * STEP][dq], CT * OPROW);
+      put4(tp, &sh.tp[out][e / CT][0][t][e % CT], CT * TPROW);
+    };
+    fetch(0);
     for (int n = 0; n < RING - 1; ++n) ask(n);
     copies_wait<RING - 2>();
+    loaders_sync();                      // every loader's copies of chunk 0
+    split(0);
+    fetch(1);
     __syncthreads();
     for (int n = 0; n < n_chunks; ++n) {
-      ask(n + RING - 1);                 // its place was read before the last barrier
-      copies_wait<RING - 2>();           // chunk n + 1 has arrived
+      copies_wait<RING - 3>();           // chunk n + 1 has arrived ...
+      loaders_sync();                    // ... for all loaders
+      if (n + 1 < n_chunks) split(n + 1);
+      fetch(n + 2);                      // (beyond the last chunk: nothing)
+      ask(n + RING - 1);                 // its place was read by the workers before the last barrier
       __syncthreads();
     }
     return;
   }
 
-  // ---------------- workers ----------------
-  const int r = threadIdx.x % CL, grp = threadIdx.x / CL, j0 = c0 + grp * CG;
-  const bool live = j0 < a.V;
-  const int i_own = r & (CT - 1), limit = r < CT ? r : i_own + 1;
-  float* Sg = a.state + (size_t)slot * a.state_stride + a.s_off + (size_t)head * DIM * a.V + j0;
-  float2 S[CP][CG];
-  load_rows(S, Sg, a.V, r, live);
+  // ---------------- workers: warp = (16 columns, half of the rows) ----------------
+  constexpr int HROWS = DIM / 2, NT = HROWS / 8, NK = HROWS / 16;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = warp >> 1, half = warp & 1, q4 = lane & 3, r8 = lane >> 2;
+  const int row0 = half * HROWS, col_s = group * 16 + r8, col = c0 + col_s, tok = 8 * half + 2 * q4;
+  float* Sg = a.state + (size_t)slot * a.state_stride + a.s_off + (size_t)head * DIM * a.V;
+  float* out = a.o + (size_t)(t0 + tok) * a.H * a.V + (size_t)head * a.V + col;
+  float S[NT][4];
+  Left st[NK];
+  load_state(S, Sg, a.V, row0, col, lane);
+#pragma unroll
+  for (int i = 0; i < NK; ++i) left_of(st[i], S[2 * i], S[2 * i + 1]);
   __syncthreads();
   for (int n = 0; n < n_chunks; ++n) {
-    const int buf = n % RING;
-    float2 kk[CT][CP];
-    float v[16][CG];
+    const int buf = n & 1, ring = n % RING;
+    const __nv_bfloat16* qo = &sh.op[buf][0][0][0][row0];
+    const __nv_bfloat16* ko = &sh.op[buf][1][0][0][row0];
+    const float(*co)[CROW] = sh.c[ring];
+    // tokens 8 i + 2 q4 + {0, 1} are this lane's: v, beta and G, the weight in the next S
+    float v[2][4], from[2][2];
+    float2 bg[2][2];
 #pragma unroll
-    for (int t = 0; t < CT; ++t) {
-      float2 qq[CP];
-      own_rows(kk[t], k_s[buf][t], r);
-      own_rows(qq, q_s[buf][t], r);
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int c = 0; c < CG; ++c) {
-        float2 dk = make_float2(0.f, 0.f), dq = dk;
-#pragma unroll
-        for (int i = 0; i < CP; ++i) { dk = fma2(S[i][c], kk[t][i], dk); dq = fma2(S[i][c], qq[i], dq); }
-        v[t][c] = dk.x + dk.y;
-        v[CT + t][c] = dq.x + dq.y;
+      for (int h = 0; h < 2; ++h) {
+        const int t = 8 * i + 2 * q4 + h;
+        bg[i][h] = *reinterpret_cast<const float2*>(&co[t][2 * CT]);
+        from[i][h] = co[t][2 * CT + 2];
+        v[i][h] = sh.v[ring][t][col_s];
+        v[i][2 + h] = sh.v[ring][t][col_s + 8];
       }
+    const float G16 = co[0][2 * CT + 3];
+    Sums k0, k1, q0, q1;
+    state_product(k0, k1, st, ko, lane);
+    Rows T0, T1, P;
+    rows_of(T0, &sh.tp[buf][0][0][0][0], lane);
+    rows_of(T1, &sh.tp[buf][0][0][8][0], lane);
+    rows_of(P, &sh.tp[buf][1][0][8 * half][0], lane);
+    float x[2][4];
+    k0.all(x[0]);
+    k1.all(x[1]);
+    sh.xk[warp][0][lane] = make_float4(x[0][0], x[0][1], x[0][2], x[0][3]);
+    sh.xk[warp][1][lane] = make_float4(x[1][0], x[1][1], x[1][2], x[1][3]);
+    state_product(q0, q1, st, qo, lane);
+    group_sync(group, DWORK / 2);
+    // x = beta (v - G k.S)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float4 o = sh.xk[warp ^ 1][i][lane];
+      const float p[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[i][e] = bg[i][e & 1].x * fmaf(-bg[i][e & 1].y, x[i][e] + p[e], v[i][e]);
     }
-    halve<8, 8>(v, r & 8);
-    halve<4, 4>(v, r & 4);
-    halve<2, 2>(v, r & 2);
-    halve<1, 1>(v, r & 1);               // lane r: k_r.S (r < 8) or q_(r - 8).S of the four columns
-    const float4 sc = *reinterpret_cast<const float4*>(&c_s[buf][i_own][2 * CT]);
-    const float G = sc.x, beta = sc.z;
-    const float4 vt = *reinterpret_cast<const float4*>(&v_s[buf][i_own][grp * CG]);
-    const float vv[CG] = {vt.x, vt.y, vt.z, vt.w};
-    float co[CT], x[CG], u[CT][CG];
-    *reinterpret_cast<float4*>(co) = *reinterpret_cast<const float4*>(&c_s[buf][i_own][r & CT]);
-    *reinterpret_cast<float4*>(co + 4) = *reinterpret_cast<const float4*>(&c_s[buf][i_own][(r & CT) + 4]);
+    float u[2][4], w[2][4];
+    Left l;
+    left_of(l, x[0], x[1]);
+    six_of_rows(u[0], l, T0);
+    six_of_rows(u[1], l, T1);
+    // S <- G_16 S + k^T (G_16 / G_j) u_j
 #pragma unroll
-    for (int c = 0; c < CG; ++c) x[c] = r < CT ? beta * (vv[c] - G * v[0][c]) : G * v[0][c];
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < CT; ++j)
-#pragma unroll
-      for (int c = 0; c < CG; ++c) {
-        u[j][c] = __shfl_sync(0xffffffffu, x[c], j, CL);
-        if (j < limit) x[c] = fmaf(co[j], u[j][c], x[c]);
-      }
-    if (live && r >= CT && t0 + n * CT + i_own < t1)
-      *reinterpret_cast<float4*>(a.o + (size_t)(t0 + n * CT + i_own) * a.H * a.V + (size_t)head * a.V + j0) = make_float4(x[0], x[1], x[2], x[3]);
-    const float2 G8 = make_float2(c_s[buf][0][2 * CT + 3], c_s[buf][0][2 * CT + 3]);
-#pragma unroll
-    for (int i = 0; i < CP; ++i)
-#pragma unroll
-      for (int c = 0; c < CG; ++c) S[i][c] = mul2(S[i][c], G8);
-#pragma unroll
-    for (int j = 0; j < CT; ++j) {
-      const float f = c_s[buf][j][2 * CT + 1];
-#pragma unroll
-      for (int c = 0; c < CG; ++c) {
-        const float2 uw = make_float2(f * u[j][c], f * u[j][c]);
-#pragma unroll
-        for (int i = 0; i < CP; ++i) S[i][c] = fma2(kk[j][i], uw, S[i][c]);
-      }
+      for (int e = 0; e < 4; ++e) w[i][e] = u[i][e] * from[i][e & 1];
+    left_of(l, w[0], w[1]);
+    update_state(S, st, l, ko, lane, [G16](int) { return make_float2(G16, G16); });
+    // o = G q.S + P u
+    float own[4], other[4], o[4];        // this half of q.S for the eight tokens whose read-out this warp ends with, and for the partner's
+    if (half) { q1.all(own); q0.all(other); }
+    else { q0.all(own); q1.all(other); }
+    sh.xq[warp][lane] = make_float4(other[0], other[1], other[2], other[3]);
+    left_of(l, u[0], u[1]);
+    six_of_rows(o, l, P);
+    if (any_not_finite(u)) {             // (where x has one, u of the tokens in front of it is lost in the product with T too)
+      const float4 x0 = make_float4(x[0][0], x[0][1], x[0][2], x[0][3]), x1 = make_float4(x[1][0], x[1][1], x[1][2], x[1][3]);
+      const float4 u0 = causal_sum(x0, x1, &co[0][0], CROW, 0), u1 = causal_sum(x0, x1, &co[0][0], CROW, 8);
+      const float4 f = causal_sum(u0, u1, &co[0][CT], CROW, 8 * half);
+      o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = f.w;
     }
+    group_sync(group, DWORK / 2);
+    const float4 f = sh.xq[warp ^ 1][lane];
+    const float p[4] = {f.x, f.y, f.z, f.w};
+    const int left = t1 - (t0 + n * CT) - tok;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float G = half ? bg[1][e & 1].y : bg[0][e & 1].y;
+      if ((e & 1) < left && col + 8 * (e >> 1) < a.V) out[(size_t)(e & 1) * a.H * a.V + 8 * (e >> 1)] = fmaf(G, own[e] + p[e], o[e]);
+    }
+    out += (size_t)CT * a.H * a.V;
     __syncthreads();
   }
-  if (live) store_rows(S, Sg, a.V, r);
+  store_state(S, Sg, a.V, row0, col, lane);
 }
 #endif
 
@@ -760,21 +1013,325 @@ __global__ void __launch_bounds__(256 + LOADERS) wkv_recur_kernel(WkvArgs a, Ier
   }
 }
 
-#if DIM == 64               // (at 128 the ring would not fit beside the scaled rows in the shared memory that needs no opt-in)
-// Prompts, eight tokens at a time, as for the delta rule above.  With W_i = w_1 .. w_i (per row of S) the state in front of the
+#if DIM == 64
+// Prompts of 48 tokens a sequence and more, sixteen at a time, as for the delta rule above.  With W_i = w_1 .. w_i (per row of S) the state in front of the
 // chunk S gives
 //   o_i = (W_(i-1) r_i).S + sum_{j < i} (sum_d r_i k_j w_(j+1) .. w_(i-1)) v_j + (r_i.(u k_i)) v_i
-//   S  <- W_8 S + sum_j (w_(j+1) .. w_8 k_j) v_j^T
-// There is no chain inside a chunk at all.  The products of two tokens (decays multiplied, never divided) come from a kernel in
-// front with a block per chunk and head; here a loader thread per row of S brings the rows through a ring and scales them.
+//   S  <- W_16 S + sum_j (w_(j+1) .. w_16 k_j) v_j^T
+// There is no chain inside a chunk at all.  The products of two tokens come from a kernel in front with a block per chunk and head;
+// here the loaders bring the rows through a ring, scale them by the decays between (products, never quotients) and split them.
+// 2,048 tokens, 64 heads of 64 x 64 (128 blocks): 103 us; eight tokens at a time with FFMA 252.
+
+// pairs[token][head][16]: row i of the chunk's products with the tokens j <= i.  Thread (half of the chunk, row d of S): row d's share
+// of the pairs inside a half, then summed over the rows; the pairs across the halves are products of r_i w_8 .. w_(i-1) with
+// k_j w_(j+1) .. w_7, a dot product of 64 by each of 64 threads.
+__global__ void __launch_bounds__(2 * DIM) wkv_pairs_kernel(WkvArgs a, float* __restrict__ pairs, IertBatchView b) {
+  constexpr int HT = CT / 2;
+  __shared__ float sum_s[2][DIM / 32][36];
+  __shared__ __align__(16) float x_s[2][HT][DIM + 4];
+  pdl_wait();                                                    // (no early start for the kernel behind, as above)
+  int tc, t1;
+  if (!chunk_of<CT>(b, blockIdx.x, tc, t1)) return;
+  const int head = blockIdx.y, side = threadIdx.x / DIM, d = threadIdx.x % DIM, lane = d & 31, HD = a.H * DIM, n = min(CT, t1 - tc);
+  const float bonus = a.u[head * DIM + d];
+  float r[HT], k[HT], w[HT];
+#pragma unroll
+  for (int t = 0; t < HT; ++t) {
+    const size_t tok = tc + min(side * HT + t, n - 1);
+    const float* row = a.x + tok * a.ld + head * DIM + d;
+    r[t] = row[0];
+    k[t] = row[HD];
+    w[t] = a.decay[tok * HD + head * DIM + d];
+  }
+  if (side == 0) {
+    float e = 1.f;
+#pragma unroll
+    for (int t = HT - 1; t >= 0; --t) { x_s[0][t][d] = k[t] * e; e *= w[t]; }
+  } else {
+    float e = 1.f;
+#pragma unroll
+    for (int t = 0; t < HT; ++t) { x_s[1][t][d] = r[t] * e; e *= w[t]; }
+  }
+  float p[36];                                                   // pair (i, j <= i) at i (i + 1) / 2 + j
+#pragma unroll
+  for (int j = 0; j < HT; ++j) {
+    p[j * (j + 1) / 2 + j] = r[j] * (bonus * k[j]);
+    float e = k[j];
+#pragma unroll
+    for (int i = j + 1; i < HT; ++i) {
+      p[i * (i + 1) / 2 + j] = r[i] * e;
+      e *= w[i];
+    }
+  }
+  // over the warp's rows: 32 of the sums spread over the lanes, the other four by full butterflies
+#pragma unroll
+  for (int half = 16; half > 0; half >>= 1) {
+    const bool upper = lane & half;
+#pragma unroll
+    for (int m = 0; m < half; ++m) {
+      const float send = upper ? p[m] : p[m + half], keep = upper ? p[m + half] : p[m];
+      p[m] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+    }
+  }
+#pragma unroll
+  for (int m = 32; m < 36; ++m) p[m] = warp_sum(p[m]);
+  sum_s[side][d / 32][lane] = p[0];
+  if (lane < 4) sum_s[side][d / 32][32 + lane] = lane == 0 ? p[32] : lane == 1 ? p[33] : lane == 2 ? p[34] : p[35];
+  __syncthreads();
+  // (64 threads: the entries across the halves, and zeros behind the diagonal; 64: those of both halves)
+  const int i = d / HT, j = d % HT;
+  float* row = pairs + ((size_t)(tc + i) * a.H + head) * CT + j;
+  const size_t half_on = (size_t)HT * a.H * CT;
+  if (side == 0) {
+    float t0 = 0.f, t1_ = 0.f;
+#pragma unroll
+    for (int x = 0; x < DIM; x += 4) {
+      const float4 u = *reinterpret_cast<const float4*>(&x_s[1][i][x]), v = *reinterpret_cast<const float4*>(&x_s[0][j][x]);
+      t0 = fmaf(u.x, v.x, t0); t1_ = fmaf(u.y, v.y, t1_); t0 = fmaf(u.z, v.z, t0); t1_ = fmaf(u.w, v.w, t1_);
+    }
+    if (HT + i < n) row[half_on] = t0 + t1_;
+    if (i < n) row[HT] = 0.f;
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (h * HT + i < n) {
+        float t = 0.f;
+        if (j <= i) {
+          t = sum_s[h][0][i * (i + 1) / 2 + j];
+#pragma unroll
+          for (int x = 1; x < DIM / 32; ++x) t += sum_s[h][x][i * (i + 1) / 2 + j];
+        }
+        row[h * (half_on + HT)] = t;
+      }
+  }
+}
+
+// What the four warps of a column group bring to a sum, added in an order that is the same for all four.
+__device__ __forceinline__ void sum_of_four(float (&o)[4], const float4 (*x)[2][32], int part, int tile, int lane) {
+  const float4 a = x[part ^ 1][tile][lane], b = x[part ^ 2][tile][lane], c = x[part ^ 3][tile][lane];
+  o[0] = (o[0] + a.x) + (b.x + c.x); o[1] = (o[1] + a.y) + (b.y + c.y);
+  o[2] = (o[2] + a.z) + (b.z + c.z); o[3] = (o[3] + a.w) + (b.w + c.w);
+}
+
+constexpr int PROW = 20, WWORK = 256;           // computing threads: two column groups x four quarters of the rows
+struct WkvShared {
+  float raw[RING][3][CT][DIM];                       // r, k, w as they are in memory
+  float v[RING][CT][VROW], p[RING][CT][PROW];
+  __nv_bfloat16 op[2][2][3][CT][OPROW];              // scaled r, k in three parts
+  __nv_bfloat16 tp[2][3][CT][TPROW];                 // the products of tokens in three parts
+  float wc[2][DIM];
+  float4 xo[8][2][32];                               // a warp's share of r.S
+};
+
+// PER_SM: blocks that share an SM (80 registers a thread then: 139 us for the one prompt above; 256 blocks and more are faster so, 64 prompts of
+// 64 tokens 1,091 us a layer against 1,156).
+template <int PER_SM>
+__global__ void __launch_bounds__(WWORK + CLOAD, PER_SM) wkv_chunk_kernel(WkvArgs a, const float* __restrict__ pairs, IertBatchView b) {
+  static_assert(DIM == 64 && CLOAD == 128, "a loader warp per 64 rows of r or k and half of the tokens");
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  WkvShared& sh = *reinterpret_cast<WkvShared*>(smem_raw);
+  pdl_wait();
+  const int s = blockIdx.x, head = blockIdx.y, c0 = blockIdx.z * CCOLS;
+  const int slot = b.slot_ids[s];
+  const int t0 = b.cu_q[s], t1 = b.cu_q[s + 1];
+  if (slot < 0 || t1 <= t0) return;
+  const int n_chunks = (t1 - t0 + CT - 1) / CT, HD = a.H * DIM;
+  const int lane = threadIdx.x & 31;
+
+  if (threadIdx.x >= WWORK) {
+    // ---------------- loaders: three chunks ahead; a warp scales eight tokens of r or of k, a lane two rows of S ----------------
+    constexpr int HT = CT / 2, ITER = CT * (DIM / 4) / CLOAD, STEP = CLOAD / (DIM / 4);
+    const int lt = threadIdx.x - WWORK;
+    const int tq = lt / (DIM / 4), dq = 4 * (lt % (DIM / 4)), tv = lt / (CCOLS / 4), ev = 4 * (lt % (CCOLS / 4)), tp = lt / 4, ep = 4 * (lt % 4);
+    const bool in_v = c0 + ev < a.V, of_k = (lt >> 5) & 1;
+    const int first = (lt >> 6) * HT, d = 2 * lane;              // this warp's tokens, this lane's rows
+    const bool both = first == (of_k ? 0 : HT);                  // the decays of the other half come first
+    const float* px = a.x + (size_t)(t0 + tq) * a.ld + head * DIM + dq;
+    const float* pw = a.decay + (size_t)(t0 + tq) * HD + head * DIM + dq;
+    const float* pv = a.x + (size_t)(t0 + tv) * a.ld + 2 * HD + (in_v ? head * a.V + c0 + ev : 0);
+    const float* pp = pairs + ((size_t)(t0 + tp) * a.H + head) * CT + ep;
+    auto ask = [&](int n) {
+      if (n < n_chunks) {
+        const int left = t1 - (t0 + n * CT), buf = n % RING;
+        const float* x = px + (size_t)n * CT * a.ld;
+        const float* w = pw + (size_t)n * CT * HD;
+#pragma unroll
+        for (int it = 0; it < ITER; ++it) {
+          const int t = tq + it * STEP;
+          const bool in = t < left;
+          const float* row = in ? x + (size_t)(it * STEP) * a.ld : a.x;
+          copy16(&sh.raw[buf][0][t][dq], row, in);
+          copy16(&sh.raw[buf][1][t][dq], in ? row + HD : row, in);
+          copy16(&sh.raw[buf][2][t][dq], in ? w + (size_t)(it * STEP) * HD : a.decay, in);
+        }
+        copy16(&sh.v[buf][tv][ev], tv < left ? pv + (size_t)n * CT * a.ld : a.x, tv < left && in_v);
+        if (tp < CT) copy16(&sh.p[buf][tp][ep], tp < left ? pp + (size_t)n * CT * a.H * CT : pairs, tp < left);
+      }
+      copies_commit();
+    };
+    auto scale = [&](int n) {                                    // a token beyond the sequence: zeros, decay 1
+      const int buf = n % RING, out = n & 1, left = t1 - (t0 + n * CT);
+      // in the order in which the decays are multiplied: from the first token on for r, from the last one back for k
+      auto token = [&](int half, int i) { return half + (of_k ? HT - 1 - i : i); };
+      auto decay = [&](int t) { return t < left ? *reinterpret_cast<const float2*>(&sh.raw[buf][2][t][d]) : make_float2(1.f, 1.f); };
+      float2 f = make_float2(1.f, 1.f), x[HT], w[HT];            // (every load before the first store: they would wait for one another)
+#pragma unroll
+      for (int i = 0; i < HT; ++i) {
+        x[i] = *reinterpret_cast<const float2*>(&sh.raw[buf][of_k][token(first, i)][d]);
+        w[i] = decay(token(first, i));
+      }
+      if (both) {
+#pragma unroll
+        for (int i = 0; i < HT; ++i) f = mul2(f, decay(token(HT - first, i)));
+      }
+      const float4 y = *reinterpret_cast<const float4*>(&sh.p[buf][tp % CT][ep]);
+#pragma unroll
+      for (int i = 0; i < HT; ++i) {
+        const float2 z = mul2(x[i], f);
+        f = mul2(f, w[i]);
+        uint32_t p[3];
+        split2(z.x, z.y, p[0], p[1], p[2]);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) *reinterpret_cast<uint32_t*>(&sh.op[out][of_k][m][token(first, i)][d]) = p[m];
+      }
+      if (both && !of_k) *reinterpret_cast<float2*>(&sh.wc[out][d]) = f;
+      if (tp < CT) {
+        uint2 p[3];
+        split2(y.x, y.y, p[0].x, p[1].x, p[2].x);
+        split2(y.z, y.w, p[0].y, p[1].y, p[2].y);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) *reinterpret_cast<uint2*>(&sh.tp[out][m][tp][ep]) = p[m];
+      }
+    };
+    for (int n = 0; n < RING - 1; ++n) ask(n);
+    copies_wait<RING - 2>();
+    loaders_sync();                      // every loader's copies of chunk 0
+    scale(0);
+    __syncthreads();
+    for (int n = 0; n < n_chunks; ++n) {
+      copies_wait<RING - 3>();           // chunk n + 1 has arrived ...
+      loaders_sync();                    // ... for all loaders
+      if (n + 1 < n_chunks) scale(n + 1);
+      ask(n + RING - 1);                 // its place: read by the workers before the last barrier, scaled from two chunks ago
+      __syncthreads();
+    }
+    return;
+  }
+
+  // ---------------- workers: warp = (16 columns, a quarter of the rows) ----------------
+  constexpr int QROWS = DIM / 4, NT = QROWS / 8, NK = QROWS / 16;
+  const int warp = threadIdx.x >> 5, group = warp >> 2, part = warp & 3, q4 = lane & 3, r8 = lane >> 2;
+  const int row0 = part * QROWS, col_s = group * 16 + r8, col = c0 + col_s;
+  const bool reads = part < 2;           // two of the four read out, eight tokens each
+  const int tok = 8 * part + 2 * q4;
+  float* Sg = a.state + (size_t)slot * a.state_stride + a.s_off + (size_t)head * DIM * a.V;
+  float* out = a.o + (size_t)(t0 + tok) * a.H * a.V + (size_t)head * a.V + col;
+  float S[NT][4];
+  Left st[NK];
+  load_state(S, Sg, a.V, row0, col, lane);
+#pragma unroll
+  for (int i = 0; i < NK; ++i) left_of(st[i], S[2 * i], S[2 * i + 1]);
+  __syncthreads();
+  for (int n = 0; n < n_chunks; ++n) {
+    const int buf = n & 1, ring = n % RING;
+    float v[2][4], y[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[i][e] = sh.v[ring][8 * i + 2 * q4 + (e & 1)][col_s + 8 * (e >> 1)];
+    {
+      Sums s0, s1;
+      state_product(s0, s1, st, &sh.op[buf][0][0][0][row0], lane);
+      s0.all(y[0]);
+      s1.all(y[1]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (i != part) sh.xo[warp][i][lane] = make_float4(y[i][0], y[i][1], y[i][2], y[i][3]);
+    }
+    Left vl;
+    left_of(vl, v[0], v[1]);
+    const float* wc = &sh.wc[buf][row0 + 2 * q4];
+    update_state(S, st, vl, &sh.op[buf][1][0][0][row0], lane, [wc](int i) { return *reinterpret_cast<const float2*>(wc + 8 * i); });
+    group_sync(group, WWORK / 2);
+    if (reads) {
+      Rows P;
+      rows_of(P, &sh.tp[buf][0][8 * part][0], lane);
+      float o[4], rs[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) rs[e] = part ? y[1][e] : y[0][e];
+      sum_of_four(rs, sh.xo + 4 * group, part, part, lane);
+      six_of_rows(o, vl, P);
+      if (any_not_finite(v)) {
+        const float4 f = causal_sum(make_float4(v[0][0], v[0][1], v[0][2], v[0][3]), make_float4(v[1][0], v[1][1], v[1][2], v[1][3]), &sh.p[ring][0][0], PROW, 8 * part);
+        o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = f.w;
+      }
+      const int left = t1 - (t0 + n * CT) - tok;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if ((e & 1) < left && col + 8 * (e >> 1) < a.V) out[(size_t)(e & 1) * a.H * a.V + 8 * (e >> 1)] = rs[e] + o[e];
+      out += (size_t)CT * a.H * a.V;
+    }
+    __syncthreads();
+  }
+  store_state(S, Sg, a.V, row0, col, lane);
+}
+
+// The same for sequences of few tokens, eight at a time with FFMA: a thread owns DIM / 16 rows of four columns of S, two rows an instruction, and the
+// sums of a token over the 16 lanes of a column are added together.  Such a step is many short chains, which want many small blocks on
+// an SM and little padding (layers at 4,096, eight / sixteen at a time, us: 128 sequences of 8 tokens 476 / 561, of 16 707 / 776, of 32 1,207 / 1,250;
+// 16 sequences of 24 262 / 270, of 48 306 / 305; 4 of 128 275 / 273, one of 2,048 688 / 570).
+namespace eight {
+constexpr int CT = 8, CG = 4, CL = 16, CWORK = 128, CCOLS = CWORK / CL * CG;
+constexpr int CP = DIM / CL / 2;                              // pairs of rows per lane
+
+// A lane's rows 64 x + 4 r .. + 3 of a vector in shared memory.
+__device__ __forceinline__ void own_rows(float2 (&v)[CP], const float* src, int r) {
+#pragma unroll
+  for (int x = 0; x < CP / 2; ++x) {
+    const float4 f = *reinterpret_cast<const float4*>(src + 64 * x + 4 * r);
+    v[2 * x] = make_float2(f.x, f.y);
+    v[2 * x + 1] = make_float2(f.z, f.w);
+  }
+}
+// The rows 64 x + 4 r .. + 3 of four columns of the state, from memory and back.
+__device__ __forceinline__ void load_rows(float2 (&S)[CP][CG], const float* Sg, int V, int r, bool live) {
+#pragma unroll
+  for (int i = 0; i < CP; ++i) {
+    const float* p = Sg + (size_t)((i / 2) * 64 + 4 * r + (i % 2) * 2) * V;
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 u = live ? *reinterpret_cast<const float4*>(p) : z, v = live ? *reinterpret_cast<const float4*>(p + V) : z;
+    S[i][0] = make_float2(u.x, v.x); S[i][1] = make_float2(u.y, v.y); S[i][2] = make_float2(u.z, v.z); S[i][3] = make_float2(u.w, v.w);
+  }
+}
+__device__ __forceinline__ void store_rows(const float2 (&S)[CP][CG], float* Sg, int V, int r) {
+#pragma unroll
+  for (int i = 0; i < CP; ++i) {
+    float* p = Sg + (size_t)((i / 2) * 64 + 4 * r + (i % 2) * 2) * V;
+    *reinterpret_cast<float4*>(p) = make_float4(S[i][0].x, S[i][1].x, S[i][2].x, S[i][3].x);
+    *reinterpret_cast<float4*>(p + V) = make_float4(S[i][0].y, S[i][1].y, S[i][2].y, S[i][3].y);
+  }
+}
+
+// Sum over the 16 lanes of a column of 2 * HALF values per column: the lanes whose bit MASK is set keep the upper half.
+template <int HALF, int MASK>
+__device__ __forceinline__ void halve(float (&v)[16][CG], bool upper) {
+#pragma unroll
+  for (int m = 0; m < HALF; ++m)
+#pragma unroll
+    for (int c = 0; c < CG; ++c) {
+      const float send = upper ? v[m][c] : v[m + HALF][c], keep = upper ? v[m + HALF][c] : v[m][c];
+      v[m][c] = keep + __shfl_xor_sync(0xffffffffu, send, MASK);
+    }
+}
+
 constexpr int WLOAD = DIM;
 
 // pairs[token][head][8]: row i of the chunk's products with the tokens j <= i.  Thread d: row d's share, then summed over the rows.
 __global__ void __launch_bounds__(DIM) wkv_pairs_kernel(WkvArgs a, float* __restrict__ pairs, IertBatchView b) {
   __shared__ float sum_s[DIM / 32][36];
-  pdl_wait();                                                    // (no early start for the kernel behind, as above)
+  pdl_wait();                                                    // (no early start for the kernel behind, as for the delta rule)
   int tc, t1;
-  if (!chunk_of(b, blockIdx.x, tc, t1)) return;
+  if (!chunk_of<CT>(b, blockIdx.x, tc, t1)) return;
   const int head = blockIdx.y, d = threadIdx.x, lane = d & 31, HD = a.H * DIM, n = min(CT, t1 - tc);
   const float bonus = a.u[head * DIM + d];
   float r[CT], k[CT], w[CT];
@@ -949,19 +1506,21 @@ __global__ void __launch_bounds__(CWORK + WLOAD) wkv_chunk_kernel(WkvArgs a, con
   }
   if (live) store_rows(S, Sg, a.V, r);
 }
+}  // namespace eight
 #endif
 
 // Lanes per column: the fewest that give the device about eight warps per SM (at most 32), and columns per
 // CTA so that a CTA has up to 256 computing threads.  (Measured at 32 heads of 128 x 128, one prompt of 2,048
 // tokens: 8 lanes per column 1.08 ms, 16 lanes 0.91 ms, 32 lanes 1.42 ms per layer.)
 #if IERT_CHUNKED
-// Prompts go eight tokens at a time; steps of few tokens per sequence token after token: a chunk costs what eight tokens cost, the kernel
-// in front is one launch more, and such a step is bound by reading and writing the state.  Where the line lies (layers at 4,096, sequences of
+// Prompts go sixteen (eight) tokens at a time; steps of few tokens per sequence token after token: a chunk costs what all its tokens cost, the
+// kernel in front is one launch more, and such a step is bound by reading and writing the state.  Where the line lies (layers at 4,096, sequences of
 // equal length, chunks / token after token, us):
-//   delta rule, 16 tokens a sequence: one sequence 56 / 54, eight 133 / 132, 32 314 / 313, 128 930 / 961; four tokens 51 / 46, 93 / 85,
-//   201 / 173, 577 / 493; twelve 55 / 52, 124 / 117, 280 / 255, 882 / 817; 64 87 / 93, 254 / 282, 693 / 763;
-//   decays per channel: one sequence of 4 to 32 tokens 71 / 70 to 109 / 110, two of 8 82 / 81, four of 8 110 / 113, eight of 4 114 / 118 and of
-//   16 138 / 165, 32 of 4 170 / 185.
+//   delta rule, 16 tokens a sequence: two sequences 75 / 78, four 87 / 90, 16 188 / 206, 64 430 / 515, 128 797 / 986; 17 tokens 79 / 80, 102 / 98,
+//   198 / 198, 546 / 557, 1,003 / 1,011; one sequence of 17 70 / 67, of 24 71 / 70, of 32 73 / 75, of 128 104 / 131; 64 tokens 106 / 135, 165 / 190,
+//   318 / 418, 1,062 / 1,455;
+//   decays per channel (eight at a time): one sequence of 4 to 32 tokens 71 / 70 to 109 / 110, two of 8 82 / 81, four of 8 110 / 113, eight of
+//   4 114 / 118 and of 16 138 / 165, 32 of 4 170 / 185.
 bool chunked(const IertBatchView* b, int tokens_a_sequence, int tokens) {
   const char* off = getenv("IERT_RECURRENT_LANES");                  // (a forced number of lanes asks for the other kernels)
   return !(off && atoi(off) >= 1) && b->n_tokens >= tokens && b->n_tokens >= (long long)tokens_a_sequence * b->n_seqs;
@@ -997,7 +1556,7 @@ IERT_API int iert_recurrent_dim() { return DIM; }
   }
 
 // Scratch (floats) of the recurrences over n_tokens tokens and H heads: the products of tokens with one another.
-IERT_API long long iert_recurrent_scratch_floats(int n_tokens, int H) { return (long long)n_tokens * H * 20; }
+IERT_API long long iert_recurrent_scratch_floats(int n_tokens, int H) { return (long long)n_tokens * H * 36; }
 
 // scratch: as many floats as above, or null (then tokens go one after another)
 IERT_API int iert_delta_recur(const float* qkv, const float* beta, const float* decay, float* state,
@@ -1006,11 +1565,14 @@ IERT_API int iert_delta_recur(const float* qkv, const float* beta, const float* 
   if (batch->n_seqs <= 0 || batch->n_tokens <= 0) return IERT_OK;
   if (G <= 0 || H <= 0 || H % G || V <= 0 || H > 65535) return IERT_BAD_ARGUMENT;
 #if IERT_CHUNKED
-  if (scratch && chunked(batch, 16, 16) && V % 4 == 0 && (2 * G * DIM + H * V) % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
+  if (scratch && chunked(batch, 16, 32) && V % 4 == 0 && (2 * G * DIM + H * V) % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
       (((uintptr_t)qkv | (uintptr_t)state | (uintptr_t)o | (uintptr_t)scratch) & 15) == 0) {
     DeltaArgs a = {qkv, beta, decay, state, state_stride, s_off, o, G, H, V, CCOLS};
-    launch_dep(delta_coef_kernel, dim3(batch->n_tokens / CT + batch->n_seqs, G), dim3(128), 0, stream, a, scratch, *batch);
-    launch_dep(delta_chunk_kernel, dim3(batch->n_seqs, H, (V + CCOLS - 1) / CCOLS), dim3(CWORK + 32), 0, stream, a, (const float*)scratch, *batch);
+    if (cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaShared)) != cudaSuccess)
+      return iert_check_launch("delta_recur attribute");
+    launch_dep(delta_coef_kernel, dim3(batch->n_tokens / CT + batch->n_seqs, G), dim3(CT * CT), 0, stream, a, scratch, *batch);
+    launch_dep(delta_chunk_kernel, dim3(batch->n_seqs, H, (V + CCOLS - 1) / CCOLS), dim3(DWORK + CLOAD), sizeof(DeltaShared), stream, a,
+               (const float*)scratch, *batch);
     return iert_check_launch("delta_recur");
   }
 #endif
@@ -1032,8 +1594,18 @@ IERT_API int iert_wkv_recur(const float* x, long long ld, const float* decay, co
   if (scratch && chunked(batch, 4, 32) && V % 4 == 0 && ld % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 &&
       (((uintptr_t)x | (uintptr_t)decay | (uintptr_t)state | (uintptr_t)o | (uintptr_t)scratch) & 15) == 0) {
     WkvArgs a = {x, ld, decay, u, state, state_stride, s_off, o, H, V, CCOLS};
-    launch_dep(wkv_pairs_kernel, dim3(batch->n_tokens / CT + batch->n_seqs, H), dim3(DIM), 0, stream, a, scratch, *batch);
-    launch_dep(wkv_chunk_kernel, dim3(batch->n_seqs, H, (V + CCOLS - 1) / CCOLS), dim3(CWORK + WLOAD), 0, stream, a, (const float*)scratch, *batch);
+    const dim3 columns(batch->n_seqs, H, (V + CCOLS - 1) / CCOLS);
+    if (chunked(batch, 48, 48)) {
+      auto* kernel = (long long)columns.x * columns.y * columns.z > iert_sm_count_cached() ? wkv_chunk_kernel<2> : wkv_chunk_kernel<1>;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WkvShared)) != cudaSuccess)
+        return iert_check_launch("wkv_recur attribute");
+      launch_dep(wkv_pairs_kernel, dim3(batch->n_tokens / CT + batch->n_seqs, H), dim3(2 * DIM), 0, stream, a, scratch, *batch);
+      launch_dep(kernel, columns, dim3(WWORK + CLOAD), sizeof(WkvShared), stream, a, (const float*)scratch, *batch);
+    } else {
+      static_assert(eight::CCOLS == CCOLS, "the same grid");
+      launch_dep(eight::wkv_pairs_kernel, dim3(batch->n_tokens / eight::CT + batch->n_seqs, H), dim3(DIM), 0, stream, a, scratch, *batch);
+      launch_dep(eight::wkv_chunk_kernel, columns, dim3(eight::CWORK + eight::WLOAD), 0, stream, a, (const float*)scratch, *batch);
+    }
     return iert_check_launch("wkv_recur");
   }
 #endif
