@@ -178,6 +178,7 @@ def _declare(lib) -> None:
         "iert_moe_gather": [P, LL, P, P, c_int, P, c_int, S],
         "iert_moe_combine": [P, P, P, c_int, c_int, P, LL, c_int, S],
         "iert_gemm_tc_grouped_gated": [P, LL, P, LL, P, LL, c_int, c_int, P, c_int, c_int, c_int, c_int, P, POINTER(GatedAct), P, S],
+        "iert_gemm_tc_batched": [P, LL, c_int, P, LL, P, c_int, LL, c_int, c_int, c_int, c_int, P, S],
         "iert_gemm_tc_grouped": [P, LL, P, LL, P, LL, c_int, c_int, P, c_int, c_int, c_int, P, S],
         "iert_router_grouped": [P, LL, LL, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
                                 c_int, c_int, P, c_int, P, P, P, P, c_int, LL, P, LL, c_int, S],
@@ -439,6 +440,20 @@ def gemm_tc(x, w, out, M: int, mode: int, err, stream, force_bt: int = 0, force_
     if status == 1:
         return False
     check(status, "gemm_tc")
+    return True
+
+
+def gemm_tc_batched(x, w, out, M: int, batches: int, err, stream) -> bool:
+    """out[:M, b N : (b + 1) N] = x[b, :M] @ w[b N : (b + 1) N].T for x [batches, rows, K] and w [batches * N, K] in one launch, for prompts of
+    more than 256 rows and N in multiples of 256.  Returns False, having launched nothing, otherwise."""
+    K = w.shape[1]
+    if x.stride(0) % x.stride(1):
+        return False
+    status = core().iert_gemm_tc_batched(x.data_ptr(), x.stride(1), x.stride(0) // x.stride(1), w.data_ptr(), w.stride(0), out.data_ptr(),
+                                         dtype_code(out.dtype), out.stride(0), M, w.shape[0] // batches, K, batches, err.data_ptr(), stream)
+    if status == 1:
+        return False
+    check(status, "gemm_tc_batched")
     return True
 
 

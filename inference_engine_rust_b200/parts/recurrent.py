@@ -188,11 +188,14 @@ class Wkv(Mixer):
 
     def load(self, t: Mapping[str, torch.Tensor]) -> None:
         self.mu = _f32(torch.stack([t[f"mu.{m}"] for m in self.MIXES], dim=0))
-        self.proj = [Linear(t[m], self.rt) for m in ("r", "k", "v", "g")]
+        # one matrix by rows: a prompt's four products are one launch
+        stacked = torch.cat([t[m].to(self.rt.dtype) for m in ("r", "k", "v", "g")], dim=0)
+        self.stacked = stacked if stacked.dtype == torch.bfloat16 else None
+        self.proj = [Linear(w, self.rt) for w in stacked.chunk(4)]
         self.L = t["w1"].shape[0]
         if t["w2"].shape[1] != self.L:
             raise ValueError(f"wkv: w1 has {self.L} rows but w2 has {t['w2'].shape[1]} columns")
-        self.w1 = Linear(_stack(self.rt, [t["w1"]], 4), self.rt)
+        self.w1 = Linear(_stack(self.rt, [t["w1"]], 4), self.rt, narrow=True)
         self.w2t = _f32(t["w2"].to(torch.float32).t())
         self.w0, self.u, self.norm = _f32(t["w0"]), _f32(t["u"]), _f32(t["norm"])
         self.o = Linear(t["o"], self.rt)
@@ -209,8 +212,9 @@ class Wkv(Mixer):
         mixed = ws.take("wkv.mixed", (len(self.MIXES), T, self.hidden_size), rt.dtype)
         B.token_shift(xn, state, self.s_floats, self.mu, mixed, ctx.batch, ctx.stream)
         x = ws.take("wkv.proj", (T, 4 * hd), torch.float32)
-        for i, lin in enumerate(self.proj):
-            lin.apply(mixed[i], x[:, i * hd:(i + 1) * hd], T, ctx.stream)
+        if self.stacked is None or not rt.fast or not B.gemm_tc_batched(mixed[:4], self.stacked, x, T, 4, rt.err, ctx.stream):
+            for i, lin in enumerate(self.proj):
+                lin.apply(mixed[i], x[:, i * hd:(i + 1) * hd], T, ctx.stream)
         z = ws.take("wkv.lora", (T, self.w1.out_features), torch.float32)
         self.w1.apply(mixed[4], z, T, ctx.stream)
         decay = ws.take("wkv.decay", (T, hd), torch.float32)
