@@ -19,6 +19,7 @@ import numpy as np
 import torch
 
 from ..cache import PAGE_TOKENS, Cache, CacheError, CacheFull
+from ..cache.staging import PinnedRing
 from ..csrc import bindings as B
 from ..parts.base import HostCopyUnavailable, StepContext
 from .model import Model
@@ -33,34 +34,6 @@ class DeviceFault(RuntimeError):
 
 
 Want = Union[str, Sequence[Sequence[int]], None]
-
-
-class _Staging:
-    """Pinned host buffers for a step's integer metadata, used in rotation so that a buffer
-    is rewritten only after its copy to the device has finished."""
-
-    def __init__(self, device, depth: int = 4):
-        self.device = device
-        self.depth = depth
-        self.host: List[Optional[torch.Tensor]] = [None] * depth
-        self.events: List[Optional[torch.cuda.Event]] = [None] * depth
-        self.turn = 0
-
-    def next(self, n_ints: int) -> Tuple[torch.Tensor, int]:
-        i = self.turn
-        self.turn = (self.turn + 1) % self.depth
-        if self.events[i] is not None:
-            self.events[i].synchronize()
-        buf = self.host[i]
-        if buf is None or buf.numel() < n_ints:
-            buf = torch.empty(max(n_ints, 4096), dtype=torch.int32, pin_memory=True)
-            self.host[i] = buf
-        return buf, i
-
-    def sent(self, i: int) -> None:
-        ev = self.events[i] or torch.cuda.Event()
-        ev.record()
-        self.events[i] = ev
 
 
 @contextlib.contextmanager
@@ -177,7 +150,7 @@ class Engine:
                            max_seq_len=min(max_seq_len, spec.max_position),
                            max_sequences=max_sequences, dtype=self.rt.dtype, device=self.rt.device,
                            page_tokens=page_tokens, poison=poison_cache)
-        self._staging = _Staging(self.rt.device)
+        self._staging = PinnedRing()
         self._meta_dev: Optional[torch.Tensor] = None
         self.steps_run = 0
         self.h2d_bytes_last_step = 0
@@ -303,7 +276,7 @@ class Engine:
         n, T, R = len(slots), int(cu[-1]), len(rows)
         for slot, p, q in zip(slots, pos0, q_lens):
             self.cache.reserve(slot, p + q)
-        self.cache.upload()
+        self.cache.upload(wait=False)
         if kind == "decode" and self.use_graphs and R in (0, n) and rows == list(range(R)):
             logits = self._step_graph(slots, pos0, tokens, R, device_tokens)
         elif (kind == "prompt" and self.use_graphs and T <= PROMPT_GRAPH_MAX_TOKENS and n <= PROMPT_GRAPH_MAX_SEQUENCES
