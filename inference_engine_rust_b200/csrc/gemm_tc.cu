@@ -57,7 +57,9 @@ constexpr int THREADS = 192;
 constexpr int W_STAGE_BYTES = TILE_N * TILE_K * 2;
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
 constexpr int OUT_STAGE_BYTES = 32 * TILE_N * 4;   // residual add by TMA: 32 tokens x 128 outputs fp32, two of them
-constexpr int XCH_BYTES = 16 * 64 * 4 + 16 + 256;   // weight-major gated tile: 16 tokens x 64 up values, aligned; 64 row scales
+// weight-major gated tile of BT tokens: 16 tokens x 64 values (twice: more than 16 tokens), aligned; 64 row scales
+constexpr int xch_floats(int bt) { return (bt > 16 ? 2 : 1) * 16 * 64; }
+constexpr int xch_bytes(int bt) { return xch_floats(bt) * 4 + 16 + 256; }
 
 enum : int { MODE_STORE = 0, MODE_ADD_RESIDUAL = 1, MODE_GATED_SILU = 2 };
 
@@ -164,11 +166,11 @@ __device__ __forceinline__ void write_out4(const GemmParams& p, int tok, int n, 
 
 // Split-K: rows t_first, t_first + 4, ... < t_end of a tile's partial products (one [BT][TILE_N]
 // fp32 block per split at `base`) added in split order and written out; 32 threads share a row, each
-// four columns (c4).  Four rows and four splits are in flight per thread and pass, and a residual is
+// four columns (c4).  R rows and U splits are in flight per thread and pass, and a residual is
 // read together with the first partials, so that a pass costs one round trip to the L2: with 64
 // rows per split a row-at-a-time loop spent 30 us here.
-template <int BT>
-__device__ __forceinline__ void reduce_partial_rows(const GemmParams& p, const float* base, int t_first, int t_end,
+template <int BT, int R, int U>
+__device__ __forceinline__ void reduce_rows_by(const GemmParams& p, const float* base, int t_first, int t_end,
                                                     int t0, int n, int c4, int n_idx, const float* rstd) {
   const bool vec_res = p.mode == MODE_ADD_RESIDUAL && p.out_dtype == IERT_F32 && n + 4 <= p.N && (p.ldo & 3) == 0 &&
                        ((uintptr_t)p.out & 15) == 0;
@@ -181,33 +183,33 @@ __device__ __forceinline__ void reduce_partial_rows(const GemmParams& p, const f
         g[i] = p.ahead.weight_dtype == IERT_F32 ? ((const float*)p.ahead.weight)[n + i]
                                                 : __bfloat162float(((const __nv_bfloat16*)p.ahead.weight)[n + i]);
   }
-  for (int t = t_first; t < t_end; t += 16) {
-    float4 acc[4], res[4];
+  for (int t = t_first; t < t_end; t += 4 * R) {
+    float4 acc[R], res[R];
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
+    for (int h = 0; h < R; ++h) {
       acc[h] = make_float4(0.f, 0.f, 0.f, 0.f);
       res[h] = (vec_res && t + 4 * h < t_end)
                    ? *reinterpret_cast<const float4*>((const float*)p.out + (long long)(t0 + t + 4 * h) * p.ldo + n)
                    : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    for (int s0 = 0; s0 < p.splits; s0 += 4) {
-      float4 v[4][4];
+    for (int s0 = 0; s0 < p.splits; s0 += U) {
+      float4 v[R][U];
 #pragma unroll
-      for (int h = 0; h < 4; ++h)
+      for (int h = 0; h < R; ++h)
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < U; ++u)
           v[h][u] = (s0 + u < p.splits && t + 4 * h < t_end)
                         ? __ldcg(reinterpret_cast<const float4*>(base + ((size_t)(s0 + u) * BT + t + 4 * h) * TILE_N) + c4)
                         : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int h = 0; h < 4; ++h)
+      for (int h = 0; h < R; ++h)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < U; ++u) {
           acc[h].x += v[h][u].x; acc[h].y += v[h][u].y; acc[h].z += v[h][u].z; acc[h].w += v[h][u].w;
         }
     }
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
+    for (int h = 0; h < R; ++h) {
       if (t + 4 * h >= t_end) break;                     // the same for the 32 threads that share the row
       const int row = t + 4 * h;
       if (rstd) {                                        // the input rows' 1 / rms (see IertRowScale)
@@ -248,6 +250,13 @@ __device__ __forceinline__ void reduce_partial_rows(const GemmParams& p, const f
       }
     }
   }
+}
+// (More than four splits: two rows and all of up to eight splits at once.  Four and four then took a second trip for the same rows.)
+template <int BT>
+__device__ __forceinline__ void reduce_partial_rows(const GemmParams& p, const float* base, int t_first, int t_end,
+                                                    int t0, int n, int c4, int n_idx, const float* rstd) {
+  if (BT > 16 && p.splits > 4) reduce_rows_by<BT, 2, 8>(p, base, t_first, t_end, t0, n, c4, n_idx, rstd);
+  else reduce_rows_by<BT, 4, 4>(p, base, t_first, t_end, t0, n, c4, n_idx, rstd);
 }
 
 // A CTA's list of work, the same for its three roles: items (tile, part of k) strided over the
@@ -385,7 +394,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   int* ticket_s = (int*)(tmem_slot + 2);
-  uint8_t* xch_s = (uint8_t*)(((uintptr_t)(tmem_slot + 4) + 15) & ~(uintptr_t)15);   // 4 KB, weight-major gated only
+  uint8_t* xch_s = (uint8_t*)(((uintptr_t)(tmem_slot + 4) + 15) & ~(uintptr_t)15);   // 8 KB, weight-major gated only
   // 2 x 16 KB: staging of the residual add by TMA, or of the token-major stores (four warps, two boxes of 4 KB each)
   uint8_t* out_s = GATED ? (uint8_t*)(((uintptr_t)(tmem_slot + 4) + 1023) & ~(uintptr_t)1023)
                          : (uint8_t*)(((uintptr_t)(tmem_slot + 4) + 127) & ~(uintptr_t)127);
@@ -511,7 +520,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // ---------------- epilogue: 4 warps, warp w reads TMEM lanes 32*(w%4).. ----------------
     pdl_wait();
     // [64] row scales: behind the gated tile's exchange buffer, or in its place for a plain launch
-    float* rstd_s = reinterpret_cast<float*>(p.mode == MODE_GATED_SILU ? xch_s + 16 * 64 * 4 : xch_s);
+    float* rstd_s = reinterpret_cast<float*>(p.mode == MODE_GATED_SILU ? xch_s + xch_floats(BT) * 4 : xch_s);
     const bool scaled = !GATED && BT <= 64 && p.scale.sumsq != nullptr;
     if (scaled) {                          // the rows' 1 / rms, while the weights stream
       row_scales_from_parts(p.scale, p.M < BT ? p.M : BT, rstd_s, (int)threadIdx.x - 64, 128);
@@ -523,6 +532,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     uint32_t acc_phase = 0;
     bool ok = true;
     StageStore stage_out{&map_o, out_s + q * 8192, lane, 0, 0};
+    int xch_turn = 0;                      // weight-major gated tiles: the exchange buffer whose turn it is
     if (GATED && p.tma_store && threadIdx.x == 64) tma_prefetch_desc(&map_o);
     WorkIter it(p, GROUPED || FACTORS ? held_tiles : p.t_tiles);
     int tile, split, n_parts, kb0, kb1;
@@ -531,14 +541,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       const int n_idx = at.n_idx, n0 = at.n0, t0 = at.t0, t_end = at.t_end;
       const int n = n0 + n_local;
       const int t_valid = min(BT, t_end - t0);
-      // (weight-major gated tiles: the columns' factors are asked for while the weights stream)
-      constexpr int N_FACTORS = FACTORS && !GATED && BT <= 32 ? BT : 1;
+      // (weight-major gated tiles: the columns' factors are asked for while the weights stream; a warp finishes eight of 16 tokens, see below)
+      constexpr int N_FACTORS = !FACTORS || GATED || BT > 32 ? 1 : BT > 16 ? BT / 2 : BT;
       float factor[N_FACTORS];
       const float* factor_col = nullptr;
-      if (FACTORS && !GATED && p.mode == MODE_GATED_SILU && p.ep.scale && q < 2) {
-        factor_col = p.ep.scale + (long long)t0 * p.ep.ld_scale + epilogue_block(n0 + n_local, p.ep);
+      if (FACTORS && !GATED && p.mode == MODE_GATED_SILU && p.ep.scale) {
+        const int first = BT > 16 && q >= 2 ? 8 : 0;
+        factor_col = p.ep.scale + (long long)(t0 + first) * p.ep.ld_scale + epilogue_block(n0 + (n_local & 63), p.ep);
 #pragma unroll
-        for (int j = 0; j < N_FACTORS; ++j) factor[j] = j < t_valid ? factor_col[(long long)j * p.ep.ld_scale] : 0.f;
+        for (int j = 0; j < N_FACTORS; ++j) {
+          const int t = BT > 16 ? j / 8 * 16 + j % 8 : j;
+          factor[j] = t + first < t_valid ? factor_col[(long long)t * p.ep.ld_scale] : 0.f;
+        }
       }
       if (!wait_or_abort(&acc_full[acc], acc_phase, abort_flag)) { ok = false; break; }
       if (threadIdx.x == 64) IERT_TRACE(5);                    // the accumulator is complete
@@ -674,61 +688,49 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       }
       if (!GATED && p.mode == MODE_GATED_SILU) {
         // Weight-major gated tile: TMEM lanes 0-63 hold 64 gate rows, lanes 64-127 the up rows
-        // that belong to them.  The up warps hand their values over through shared memory, the
-        // gate warps write silu(gate) * up, 64 consecutive outputs of a token per pair of warps.
-        float* xch = reinterpret_cast<float*>(xch_s);                 // [16 tokens][64]
+        // that belong to them.  With more than 16 tokens, of 16 the gate warps finish the first eight and the up warps the others: they hand each
+        // other what they lack through shared memory, two buffers in turn, and write 64 consecutive outputs of a token per pair
+        // of warps.  (With the gate warps alone at work 64 tokens took 5.4 us behind the last MMA, a step of 64 tokens 354 us with this and the store
+        // below as they were, 330 now.)
+        constexpr bool BOTH = BT > 16;
+        const int row = n_local & 63, own = BOTH && q >= 2 ? 8 : 0, i = n0 + row;             // n0 counts gate rows here (64 per tile)
+        __nv_bfloat16* o = (__nv_bfloat16*)p.out + (long long)(t0 + own) * p.ldo + i;
+        auto chunk = [&](int c) {
+          float* xch = reinterpret_cast<float*>(xch_s) + xch_turn * (16 * 64);        // [16 tokens][64]
+          if (BOTH) xch_turn ^= 1;
+          float v[16];
+          tmem_ld16(taddr + c, v);
+          if (BOTH) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) xch[(8 - own + j) * 64 + row] = q >= 2 ? v[j] : v[8 + j];
+          } else if (q >= 2) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) xch[j * 64 + row] = v[j];
+          }
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+          if (i < p.N && (BOTH || q < 2)) {
+#pragma unroll
+            for (int j = 0; j < (BOTH ? 8 : 16); ++j) {
+              if (c + own + j < t_valid) {
+                const float r = scaled ? rstd_s[c + own + j] : 1.0f;
+                const float mine = (BOTH && q >= 2 ? v[(8 + j) & 15] : v[j]) * r, other = xch[(own + j) * 64 + row] * r;
+                float act = BOTH && q >= 2 ? silu_mul(other, mine) : silu_mul(mine, other);
+                if (FACTORS && factor_col)
+                  act *= N_FACTORS > 1 ? factor[(c / (BOTH ? 2 : 1) + j) % N_FACTORS] : factor_col[(long long)(c + j) * p.ep.ld_scale];
+                o[(long long)(c + j) * p.ldo] = __float2bfloat16_rn(act);
+              }
+            }
+          }
+        };
         if constexpr (FACTORS) {                     // unrolled: the factors are in registers
 #pragma unroll
-        for (int c = 0; c < BT; c += 16) {
-          if (c >= t_valid) break;                   // uniform over the four warps
-          float v[16];
-          tmem_ld16(taddr + c, v);
-          if (q >= 2) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) xch[j * 64 + (n_local - 64)] = v[j];
-          }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          if (q < 2) {
-            const int i = n0 + n_local;              // n0 counts gate rows here (64 per tile)
-            if (i < p.N) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                if (c + j < t_valid) {
-                  const float r = scaled ? rstd_s[c + j] : 1.0f;
-                  float act = silu_mul(v[j] * r, xch[j * 64 + n_local] * r);
-                  if (factor_col) act *= N_FACTORS > 1 ? factor[(c + j) % N_FACTORS] : factor_col[(long long)(c + j) * p.ep.ld_scale];
-                  ((__nv_bfloat16*)p.out)[(long long)(t0 + c + j) * p.ldo + i] = __float2bfloat16_rn(act);
-                }
-            }
-          }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-        }
+          for (int c = 0; c < BT; c += 16)
+            if (c < t_valid) chunk(c);               // uniform over the four warps
         } else {
 #pragma unroll 1
-        for (int c = 0; c < BT; c += 16) {
-          if (c >= t_valid) break;
-          float v[16];
-          tmem_ld16(taddr + c, v);
-          if (q >= 2) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) xch[j * 64 + (n_local - 64)] = v[j];
-          }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          if (q < 2) {
-            const int i = n0 + n_local;              // n0 counts gate rows here (64 per tile)
-            if (i < p.N) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                if (c + j < t_valid) {
-                  const float r = scaled ? rstd_s[c + j] : 1.0f;
-                  float act = silu_mul(v[j] * r, xch[j * 64 + n_local] * r);
-                  ((__nv_bfloat16*)p.out)[(long long)(t0 + c + j) * p.ldo + i] = __float2bfloat16_rn(act);
-                }
-            }
-          }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
+          for (int c = 0; c < t_valid; c += 16) chunk(c);
         }
-        }
+        if (!BOTH) asm volatile("bar.sync 1, 128;" ::: "memory");                     // (one buffer: the next tile's values may come now)
       }
       // Many tokens, residual add, whole tile: 32 tokens per pass, so that twice as many reads of
       // the residual are in flight per round trip (the last tile's epilogue is not hidden behind
@@ -783,6 +785,33 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             if (mine) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) o[(long long)j * p.ldo] = r[j] + v[j];
+            }
+          }
+          wide_done = true;
+        }
+      }
+      // Plain store of a one-token step: the tokens' rows by one pointer that goes on, nothing to decide per output.  (64 tokens x 32,000 fp32: 5.1 us
+      // behind the last MMA by the general loop below.)
+      if constexpr (!GATED && BT <= 64) {
+        if (p.mode == MODE_STORE && !part && !epilogue_on(p.ep)) {
+          const bool f32 = p.out_dtype == IERT_F32;
+          float* of = (float*)p.out + (long long)t0 * p.ldo + n;
+          __nv_bfloat16* ob = (__nv_bfloat16*)p.out + (long long)t0 * p.ldo + n;
+#pragma unroll 1
+          for (int c = 0; c < BT; c += 16) {
+            if (c >= t_valid) break;
+            float v[16];
+            tmem_ld16(taddr + c, v);
+            if (n < p.N) {
+              if (f32) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j, of += p.ldo)
+                  if (c + j < t_valid) *of = v[j];
+              } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j, ob += p.ldo)
+                  if (c + j < t_valid) *ob = __float2bfloat16_rn(v[j]);
+              }
             }
           }
           wide_done = true;
@@ -1066,13 +1095,13 @@ int sm_count() {
 // Dynamic shared memory of a launch: ring, alignment slack, barriers; the weight-major gated tile
 // adds its exchange buffer, the residual add by TMA its two staging buffers.  The one formula for
 // the launch and for the estimate of how many CTAs an SM holds (ctas_per_sm_of).
-constexpr size_t dynamic_smem_bytes(int stages, int stage_bytes, bool gated_weight_major, bool tma_out, bool row_scales = false) {
-  return (size_t)stages * stage_bytes + 1024 + 256 + (gated_weight_major ? XCH_BYTES : row_scales ? 256 + 16 : 0) +
+constexpr size_t dynamic_smem_bytes(int stages, int stage_bytes, int exchange_bytes, bool tma_out, bool row_scales = false) {
+  return (size_t)stages * stage_bytes + 1024 + 256 + (exchange_bytes ? exchange_bytes : row_scales ? 256 + 16 : 0) +
          (tma_out ? 2 * OUT_STAGE_BYTES + 1024 : 0);
 }
 
 // Is there shared memory beside the ring for the token-major stores' staging?
-bool room_for_staging(int stages, int stage_bytes) { return dynamic_smem_bytes(stages, stage_bytes, false, true) <= 227 * 1024; }
+bool room_for_staging(int stages, int stage_bytes) { return dynamic_smem_bytes(stages, stage_bytes, 0, true) <= 227 * 1024; }
 
 #ifdef IERT_GEMM_TRACE
 int g_trace_meta[TRACE_LAUNCHES][8];
@@ -1092,7 +1121,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, GemmParams p, int grid,
   tm[0] = g_trace_next++; tm[1] = p.M; tm[2] = p.N; tm[3] = p.K; tm[4] = grid; tm[5] = BT; tm[6] = p.splits; tm[7] = p.mode;
 #endif
   constexpr int STAGE_BYTES = (GATED ? 2 : 1) * W_STAGE_BYTES + BT * TILE_K * 2;
-  const size_t smem = dynamic_smem_bytes(p.stages, STAGE_BYTES, !GATED && p.mode == MODE_GATED_SILU, p.tma_out != 0 || p.tma_store != 0,
+  const size_t smem = dynamic_smem_bytes(p.stages, STAGE_BYTES, !GATED && p.mode == MODE_GATED_SILU ? xch_bytes(BT) : 0, p.tma_out != 0 || p.tma_store != 0,
                                          p.scale.sumsq != nullptr);
   static bool configured = false;
   if (!configured) {
@@ -1115,7 +1144,7 @@ int ctas_per_sm_of(int stages) {
   if (stages < 0 || stages > 12) return 0;
   if (!cached[stages]) {
     // (a plain weight-major launch: no exchange buffer, no TMA-out staging; only such launches reduce cooperatively)
-    const size_t smem = dynamic_smem_bytes(stages, W_STAGE_BYTES + BT * TILE_K * 2, false, false, true);   // (the larger of the two plain layouts)
+    const size_t smem = dynamic_smem_bytes(stages, W_STAGE_BYTES + BT * TILE_K * 2, 0, false, true);   // (the larger of the two plain layouts)
     int n = 0, dev = 0, smem_sm = 0, regs_sm = 0;
     cudaFuncAttributes a;
     if (cudaGetDevice(&dev) == cudaSuccess && cudaFuncGetAttributes(&a, gemm_tc_kernel<BT, false>) == cudaSuccess &&
@@ -1429,9 +1458,9 @@ int gemm_tc_gated_impl(const void* x, long long ldx, const void* w, long long ld
     p.ws = nullptr; p.counters = nullptr; p.err = err;
     if (scale) p.scale = *scale;
     const int stage_bytes = W_STAGE_BYTES + wbt * TILE_K * 2;
-    int stages = force_stages ? force_stages : (113 * 1024 - 2048 - XCH_BYTES) / stage_bytes;
+    int stages = force_stages ? force_stages : (113 * 1024 - 2048 - xch_bytes(wbt)) / stage_bytes;
     if (stages > 12) stages = 12;
-    if (stages < 2 || (size_t)stages * stage_bytes + 1280 + XCH_BYTES > 227 * 1024) return IERT_BAD_ARGUMENT;
+    if (stages < 2 || (size_t)stages * stage_bytes + 1280 + xch_bytes(wbt) > 227 * 1024) return IERT_BAD_ARGUMENT;
     p.stages = stages;
     CUtensorMap mw, mx;
     if (!tensor_map(w, (long long)up_rows + inter, K, ldw, TILE_N / 2, &mw) || !tensor_map(x, M, K, ldx, wbt, &mx)) return IERT_BAD_ARGUMENT;
