@@ -539,49 +539,60 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     }
   }
   const __nv_bfloat16* tok_row = p.qkv + (size_t)t * ((size_t)(p.heads + 2 * c.kv_heads) * HD);
-  auto rotate_into = [&](const __nv_bfloat16* src, __nv_bfloat16* dst, int k) {
-    const int i0 = p.pairing == IERT_PAIR_HALF ? k : 2 * k;
-    const int i1 = p.pairing == IERT_PAIR_HALF ? k + half : 2 * k + 1;
-    const float a = __bfloat162float(src[i0]), bb = __bfloat162float(src[i1]);
-    dst[i0] = __float2bfloat16_rn(a * cs_tab[k] - bb * cs_tab[half + k]);
-    dst[i1] = __float2bfloat16_rn(a * cs_tab[half + k] + bb * cs_tab[k]);
-  };
+  // the page that the new row goes to is known before the row is
+  const bool writes_row = own_new_row && slice == 0;
+  const int own_page = writes_row ? c.page_table[(size_t)slot * c.table_width + iert_table_entry(c, pos / PAGE)] : -1;
   pdl_wait();
-  {
-    const __nv_bfloat16* q = tok_row + (size_t)head0 * HD;
-    if (p.rope) {
-      consumer_sync();                                   // the angle table is complete
-      for (int i = threadIdx.x; i < ROWS * (HD / 2); i += THREADS) {
-        const int r = i / (HD / 2), k = i % (HD / 2);
-        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(q_tile + r * ROW_BYTES);
-        if (r >= n_g) { dst[2 * k] = __float2bfloat16_rn(0.f); dst[2 * k + 1] = __float2bfloat16_rn(0.f); }
-        else if (k < half) rotate_into(q + r * HD, dst, k);
-        else { const int d = p.rotary_dim + 2 * (k - half); dst[d] = q[r * HD + d]; dst[d + 1] = q[r * HD + d + 1]; }
-      }
-    } else {
-      constexpr int CHUNKS = HD / 8;
-      for (int i = threadIdx.x; i < ROWS * CHUNKS; i += THREADS) {
-        const int r = i / CHUNKS, cc = i % CHUNKS;
-        const uint4 val = r < n_g ? *reinterpret_cast<const uint4*>(q + r * HD + cc * 8) : make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(q_tile + r * ROW_BYTES + cc * 16) = val;
-      }
+  const __nv_bfloat16* q = tok_row + (size_t)head0 * HD;
+  if (p.rope) {
+    // every load of the queries and of the new row is issued before the first is used: they are all that a CTA waits for here, and with
+    // one round trip for every 128 pairs and two more behind them eight sequences of 2,070 positions took 15.3 us a layer, so 13.5; 64 of 290
+    // positions 23, so 22.  Query rows that no head has are left as they are: their scores and sums are never written.
+    constexpr int ITER = (8 * (HD / 2) + THREADS - 1) / THREADS;
+    __nv_bfloat16 qa[ITER], qb[ITER], kv4[4];
+    auto first = [&](int k) { return k < half ? (p.pairing == IERT_PAIR_HALF ? k : 2 * k) : p.rotary_dim + 2 * (k - half); };
+    auto second = [&](int k) { return k < half && p.pairing == IERT_PAIR_HALF ? k + half : first(k) + 1; };
+#pragma unroll
+    for (int it = 0; it < ITER; ++it) {
+      const int i = threadIdx.x + it * THREADS, r = i / (HD / 2), k = i % (HD / 2);
+      if (r < n_g) { qa[it] = q[r * HD + first(k)]; qb[it] = q[r * HD + second(k)]; }
     }
-  }
-  if (own_new_row) {
-    const __nv_bfloat16* kn = tok_row + (size_t)(p.heads + kvh) * HD;
-    const __nv_bfloat16* vn = tok_row + (size_t)(p.heads + c.kv_heads + kvh) * HD;
-    for (int k = threadIdx.x; k < HD / 2; k += THREADS) {
-      if (k < half) rotate_into(kn, new_kv, k);
-      else { const int d = p.rotary_dim + 2 * (k - half); new_kv[d] = kn[d]; new_kv[d + 1] = kn[d + 1]; }
-      new_kv[HD + 2 * k] = vn[2 * k];
-      new_kv[HD + 2 * k + 1] = vn[2 * k + 1];
+    const int own_k = threadIdx.x;
+    static_assert(HD / 2 <= THREADS, "a pair of the new row a thread");
+    if (own_new_row && own_k < HD / 2) {
+      const __nv_bfloat16* kn = tok_row + (size_t)(p.heads + kvh) * HD;
+      const __nv_bfloat16* vn = tok_row + (size_t)(p.heads + c.kv_heads + kvh) * HD;
+      kv4[0] = kn[first(own_k)]; kv4[1] = kn[second(own_k)];
+      kv4[2] = vn[2 * own_k]; kv4[3] = vn[2 * own_k + 1];
+    }
+    consumer_sync();                                     // the angle table is complete
+    auto rotate = [&](__nv_bfloat16 x, __nv_bfloat16 y, __nv_bfloat16* dst, int k) {
+      const float a = __bfloat162float(x), bb = __bfloat162float(y);
+      dst[first(k)] = k < half ? __float2bfloat16_rn(a * cs_tab[k] - bb * cs_tab[half + k]) : x;
+      dst[second(k)] = k < half ? __float2bfloat16_rn(a * cs_tab[half + k] + bb * cs_tab[k]) : y;
+    };
+#pragma unroll
+    for (int it = 0; it < ITER; ++it) {
+      const int i = threadIdx.x + it * THREADS, r = i / (HD / 2), k = i % (HD / 2);
+      if (r < n_g) rotate(qa[it], qb[it], reinterpret_cast<__nv_bfloat16*>(q_tile + r * ROW_BYTES), k);
+    }
+    if (own_new_row && own_k < HD / 2) {
+      rotate(kv4[0], kv4[1], new_kv, own_k);
+      new_kv[HD + 2 * own_k] = kv4[2];
+      new_kv[HD + 2 * own_k + 1] = kv4[3];
+    }
+  } else {
+    constexpr int CHUNKS = HD / 8;
+    for (int i = threadIdx.x; i < ROWS * CHUNKS; i += THREADS) {
+      const int r = i / CHUNKS, cc = i % CHUNKS;
+      const uint4 val = r < n_g ? *reinterpret_cast<const uint4*>(q + r * HD + cc * 8) : make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4*>(q_tile + r * ROW_BYTES + cc * 16) = val;
     }
   }
   consumer_sync();
-  if (own_new_row && slice == 0) {
-    const int page = c.page_table[(size_t)slot * c.table_width + iert_table_entry(c, pos / PAGE)];
-    if (page >= 0 && page < c.n_pages) {
-      const size_t off = ((((size_t)page * c.kv_heads + kvh) * PAGE) + pos % PAGE) * HD;
+  if (writes_row) {
+    if (own_page >= 0 && own_page < c.n_pages) {
+      const size_t off = ((((size_t)own_page * c.kv_heads + kvh) * PAGE) + pos % PAGE) * HD;
       for (int d = threadIdx.x; d < HD; d += THREADS) {
         ((__nv_bfloat16*)c.k)[off + d] = new_kv[d];
         ((__nv_bfloat16*)c.v)[off + d] = new_kv[HD + d];
@@ -716,23 +727,36 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   if (tq == 0) { ml_s[(warp * 8 + g) * 2] = m_row; ml_s[(warp * 8 + g) * 2 + 1] = l_row; }
   consumer_sync();
   const bool direct = p.splits == 1 && p.sink == nullptr;
-  for (int r = 0; r < n_g && r < 8; ++r) {
+  // four numbers of a head a thread
+  for (int i = threadIdx.x; i < n_g * (HD / 4); i += THREADS) {
+    const int r = i / (HD / 4), d = 4 * (i % (HD / 4));
     float mm = -INFINITY;
+#pragma unroll
     for (int w = 0; w < WARPS; ++w) mm = fmaxf(mm, ml_s[(w * 8 + r) * 2]);
     float wgt[WARPS], ll = 0.f;
+#pragma unroll
     for (int w = 0; w < WARPS; ++w) {
       const float mw = ml_s[(w * 8 + r) * 2];
       wgt[w] = mw == -INFINITY ? 0.f : exp2f(mw - mm);
       ll += wgt[w] * ml_s[(w * 8 + r) * 2 + 1];
     }
     const float inv = ll > 0.f ? 1.0f / ll : 0.f;
-    for (int d = threadIdx.x; d < HD; d += THREADS) {
-      float acc = 0.f;
-      for (int w = 0; w < WARPS; ++w) acc += wgt[w] * o_s[(w * 8 + r) * HD + d];
-      if (direct) p.out[((size_t)t * p.heads + head0 + r) * HD + d] = __float2bfloat16_rn(acc * inv);
-      else po[(size_t)r * p.splits * HD + d] = acc;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+      const float4 x = *reinterpret_cast<const float4*>(&o_s[(w * 8 + r) * HD + d]);
+      acc.x += wgt[w] * x.x; acc.y += wgt[w] * x.y; acc.z += wgt[w] * x.z; acc.w += wgt[w] * x.w;
     }
-    if (!direct && threadIdx.x == 0) { pml[(size_t)r * p.splits * 2] = mm; pml[(size_t)r * p.splits * 2 + 1] = ll; }
+    if (direct) {
+      uint2 out;
+      *reinterpret_cast<__nv_bfloat162*>(&out.x) = __floats2bfloat162_rn(acc.x * inv, acc.y * inv);
+      *reinterpret_cast<__nv_bfloat162*>(&out.y) = __floats2bfloat162_rn(acc.z * inv, acc.w * inv);
+      *reinterpret_cast<uint2*>(p.out + ((size_t)t * p.heads + head0 + r) * HD + d) = out;
+    } else {
+      float* dst = po + (size_t)r * p.splits * HD + d;
+      dst[0] = acc.x; dst[1] = acc.y; dst[2] = acc.z; dst[3] = acc.w;
+      if (d == 0) { pml[(size_t)r * p.splits * 2] = mm; pml[(size_t)r * p.splits * 2 + 1] = ll; }
+    }
   }
 }
 #endif  // HEAD_DIM % 64 == 0
@@ -834,7 +858,7 @@ int launch_decode(const void* qkv, void* out, const IertBatchView* batch, const 
   static const bool use_tma = [] { const char* e = getenv("IERT_DECODE_TMA"); return !(e && e[0] == '0'); }();
   CUtensorMap map_k, map_v;
   const long long cache_rows = (long long)cache->n_pages * cache->kv_heads * PAGE;
-  if (use_tma && tma_host::tensor_map_2d(cache->k, cache_rows, HD, HD, PAGE, &map_k) &&
+  if (use_tma && ((uintptr_t)out & 7) == 0 && tma_host::tensor_map_2d(cache->k, cache_rows, HD, HD, PAGE, &map_k) &&
       tma_host::tensor_map_2d(cache->v, cache_rows, HD, HD, PAGE, &map_v)) {
     const size_t ring = 2 * NSTAGE * (size_t)TMA_TILE_BYTES;
     size_t smem_tma = ring + ROWS * ROW_BYTES + 8 * (size_t)HD + 1024;      // (+ alignment of the ring)
