@@ -169,6 +169,7 @@ def _declare(lib) -> None:
         "iert_token_shift": [P, c_int, LL, P, LL, LL, P, c_int, c_int, P, POINTER(BatchView), S],
         "iert_wkv_decay": [P, LL, c_int, P, P, c_int, P, P, c_int, LL, c_int, P, LL, LL, POINTER(BatchView), S],
         "iert_wkv_finish": [P, P, LL, P, c_float, c_float, P, c_int, POINTER(BatchView), c_int, c_int, S],
+        "iert_latent_decode_tc_rows": [c_int, c_int, c_int, c_int, c_int],
         "iert_latent_decode_tc_plan": [c_int, c_int, c_int, c_int, c_int, POINTER(c_int), POINTER(c_int)],
         "iert_router_topk": [P, LL, LL, P, c_int, c_int, c_int, P, c_int, P, P, S],
         "iert_moe_scale": [P, c_int, LL, P, c_int, c_int, c_int, c_int, S],
@@ -858,6 +859,11 @@ def latent_decode_tc_plan(n_seqs: int, H: int, rank: int, rot_dim: int, table_wi
     return hpad.value, splits.value
 
 
+def latent_decode_tc_rows(n_seqs: int, H: int, rank: int, rot_dim: int, splits: int) -> int:
+    """Partial results of a sequence that `latent_attention_decode_tc` makes use of (the second size of its scratch, at least `splits`)."""
+    return core().iert_latent_decode_tc_rows(n_seqs, H, rank, rot_dim, splits)
+
+
 def latent_attention_decode_tc(q, w_uk, w_uv, out, batch: BatchView, kv: KvView, H: int, D: int, V: int, scale: float, sink,
                                hpad: int, splits: int, qa, part_m, part_l, part_acc, err, stream, rot_dim: int = 0,
                                gate=None, inv_freq=None, rot_mul: float = 1.0, pairing: int = PAIR_HALF) -> bool:
@@ -871,12 +877,12 @@ def latent_attention_decode_tc(q, w_uk, w_uv, out, batch: BatchView, kv: KvView,
     if not getattr(fn, "_declared", False):
         fn.argtypes = [c_void_p, c_int, c_longlong, c_void_p, c_float, c_int, c_void_p, c_void_p, c_void_p, POINTER(BatchView),
                        POINTER(KvView), c_int, c_int,
-                       c_int, c_int, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                       c_int, c_int, c_float, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                        c_void_p]
         fn.restype = c_int
         fn._declared = True
     status = fn(q.data_ptr(), 1 if q.dtype == torch.float32 else 0, q.stride(0), _ptr(inv_freq), rot_mul, pairing, w_uk.data_ptr(), w_uv.data_ptr(), out.data_ptr(), byref(batch), byref(kv), H, D,
-                rot_dim, V, scale, _ptr(sink), _ptr(gate), hpad, splits, qa.data_ptr(), part_m.data_ptr(), part_l.data_ptr(), part_acc.data_ptr(),
+                rot_dim, V, scale, _ptr(sink), _ptr(gate), hpad, splits, part_m.shape[1] if part_m.dim() == 3 else splits, qa.data_ptr(), part_m.data_ptr(), part_l.data_ptr(), part_acc.data_ptr(),
                 err.data_ptr(), stream)
     if status == 1:
         return False

@@ -712,7 +712,7 @@ bool umma_enabled() {
 // latent_decode_umma.cu
 int latent_umma_heads(int H, int rank, int R);
 int launch_latent_decode_umma(const void* qa, const IertBatchView* batch, const IertKvView* kv, int H, int Hpad, int R, float scale,
-                              int splits, float* part_m, float* part_l, float* part_acc, int* err, cudaStream_t stream);
+                              int splits, int rows, float* part_m, float* part_l, float* part_acc, int* err, cudaStream_t stream);
 
 // Heads padded to whole MMA tiles (16, or 32 from 17 heads on), and how many runs of tiles a sequence is cut into.
 // `table_width`: pages of the longest walk.
@@ -742,17 +742,22 @@ IERT_API int iert_latent_decode_tc_plan(int n_seqs, int H, int rank, int R, int 
   return IERT_OK;
 }
 
+// Partial results of a sequence to make room for beside `splits` runs: some more let the kernel cut a step of several sequences by length.
+IERT_API int iert_latent_decode_tc_rows(int n_seqs, int H, int rank, int R, int splits) {
+  return umma_enabled() && latent_umma_heads(H, rank, R) && n_seqs >= 8 && splits <= 8 ? splits + 4 : splits;
+}
+
 // The wide merge's shared memory for `tt` sequences a block (bytes).
 IERT_API int iert_latent_merge_wide_smem(int tt, int rank) { return merge_wide_smem(tt, rank).total; }
 
 // q [T, ldq] (H*(D+R) per token, one token per sequence: per head D unrotated and R rotated numbers), bf16 with the rotated
 // numbers turned already, or with q_f32 != 0 fp32 as projected (turned here by inv_freq, rot_mul and pairing); the cache's
 // rows are rank + R wide (latent | rotated key part); w_uk [H*D, rank], w_uv [H*V, rank] bf16 row-major; gate: fp32 [T, H]
-// or null.  qa: scratch bf16 [T, Hpad, rank + R]; part_m, part_l: fp32 [T, splits, Hpad]; part_acc: fp32 [T, splits, Hpad, rank];
-// out bf16 [T, H*V].  Hpad and splits as iert_latent_decode_tc_plan gives them.
+// or null.  qa: scratch bf16 [T, Hpad, rank + R]; part_m, part_l: fp32 [T, rows, Hpad]; part_acc: fp32 [T, rows, Hpad, rank];
+// out bf16 [T, H*V].  Hpad and splits as iert_latent_decode_tc_plan gives them, rows >= splits (more: see latent_decode_umma.cu).
 IERT_API int iert_latent_attention_decode_tc(const void* q, int q_f32, long long ldq, const float* inv_freq, float rot_mul, int pairing, const void* w_uk, const void* w_uv, void* out,
                                              const IertBatchView* batch, const IertKvView* kv, int H, int D, int R, int V,
-                                             float scale, const float* sink, const float* gate, int Hpad, int splits,
+                                             float scale, const float* sink, const float* gate, int Hpad, int splits, int rows,
                                              void* qa, float* part_m, float* part_l, float* part_acc, int* err,
                                              cudaStream_t stream) {
   const int T = batch->n_tokens, width = kv->head_dim, rank = width - R;
@@ -760,7 +765,7 @@ IERT_API int iert_latent_attention_decode_tc(const void* q, int q_f32, long long
   const bool umma = umma_enabled() && latent_umma_heads(H, rank, R) && ((uintptr_t)qa & 15) == 0 && ((uintptr_t)kv->k & 15) == 0;
   if (!umma && (rank % 32 || R % 16 || rank < 32)) return IERT_BAD_ARGUMENT;
   if (T != batch->n_seqs || kv->dtype != IERT_BF16 || kv->kv_heads != 1 || kv->page_tokens != BK || rank % 8 || R < 0 ||
-      width > 640 || rank < 8 || rank > MAX_NTW * 32 || H <= 0 || Hpad % 16 || Hpad < H || Hpad > 65535 || splits < 1 || splits > 64 ||
+      width > 640 || rank < 8 || rank > MAX_NTW * 32 || H <= 0 || Hpad % 16 || Hpad < H || Hpad > 65535 || splits < 1 || rows < splits || rows > 64 ||
       D <= 0 || 4 * (D + 4 * rank) > 12000 || V <= 0 || (q_f32 && R > 0 && !inv_freq))
     return IERT_BAD_ARGUMENT;
   const int mt = Hpad % 32 == 0 ? 2 : 1;
@@ -796,23 +801,23 @@ IERT_API int iert_latent_attention_decode_tc(const void* q, int q_f32, long long
   else { if (tt == 1) ABSORB(__nv_bfloat16, 1); else if (tt == 2) ABSORB(__nv_bfloat16, 2); else ABSORB(__nv_bfloat16, 4); }
 #undef ABSORB
 #undef ABSORB_WIDE
-  dim3 grid(T, splits, Hpad / (mt * 16));
+  const dim3 grid(T, rows, Hpad / (mt * 16));         // (mma.sync: as many runs as there is room for)
   if (umma) {
-    const int st = launch_latent_decode_umma(qa, batch, kv, H, Hpad, R, scale, splits, part_m, part_l, part_acc, err, stream);
+    const int st = launch_latent_decode_umma(qa, batch, kv, H, Hpad, R, scale, splits, rows, part_m, part_l, part_acc, err, stream);
     if (st != IERT_OK) return IERT_CUDA_ERROR;       // (the sizes were checked above)
   } else if (mt == 2)
     launch_dep(latent_decode_tc_kernel<2>, grid, dim3(THREADS), smem, stream, (const __nv_bfloat16*)qa, *batch, *kv, Hpad, R,
-               scale, splits, part_m, part_l, part_acc, err);
+               scale, rows, part_m, part_l, part_acc, err);
   else
     launch_dep(latent_decode_tc_kernel<1>, grid, dim3(THREADS), smem, stream, (const __nv_bfloat16*)qa, *batch, *kv, Hpad, R,
-               scale, splits, part_m, part_l, part_acc, err);
+               scale, rows, part_m, part_l, part_acc, err);
 #define MERGE(TT)                                                                                                                  \
   launch_dep(latent_decode_merge_kernel<__nv_bfloat16, TT>, dim3((T + TT - 1) / TT, H, V >= 64 && T <= 8 ? 2 : 1), dim3(MERGE_THREADS),                       \
-             (size_t)TT * (rank + 64) * sizeof(float), stream, (const float*)part_m, (const float*)part_l, (const float*)part_acc, splits, \
+             (size_t)TT * (rank + 64) * sizeof(float), stream, (const float*)part_m, (const float*)part_l, (const float*)part_acc, rows, \
              Hpad, rank, sink, gate, (const __nv_bfloat16*)w_uv, (__nv_bfloat16*)out, *batch, H, V)
 #define MERGE_WIDE(TT)                                                                                                             \
   launch_dep(latent_merge_wide_kernel<TT>, dim3((T + TT - 1) / TT, H, (V + 127) / 128), dim3(WIDE_THREADS), (size_t)merge_wide_smem(TT, rank).total, stream, \
-             (const float*)part_m, (const float*)part_l, (const float*)part_acc, splits, Hpad, rank, sink, gate, (const __nv_bfloat16*)w_uv, \
+             (const float*)part_m, (const float*)part_l, (const float*)part_acc, rows, Hpad, rank, sink, gate, (const __nv_bfloat16*)w_uv, \
              (__nv_bfloat16*)out, *batch, H, V)
   if (wide_merge && merge_tt == 8) MERGE_WIDE(8);
   else if (wide_merge) MERGE_WIDE(16);

@@ -10,7 +10,12 @@
 //   page meets, live in TMEM: 128 lanes hold 128 / NH copies of the NH heads, every warp of the softmax finds all heads in
 //   its own 32 lanes and takes 16 of the page's 64 keys.  Their way there is through the last stage of the page ring,
 //   which is filled with pages once they have moved on.
-//   grid (sequences, runs of pages, groups of NH heads); a CTA walks its run of the sequence's pages.
+//   grid (runs of pages, 1, groups of NH heads); a CTA walks its run of a sequence's pages.  Sequences are cut evenly, `splits` runs each, or
+//   (where there is room for more partial results) by length: runs of the fewest pages that let all of them have an SM at once, which every CTA
+//   works out from the lengths.  The pages' bytes bound a step whose sequences are alike, whatever the cut (3,104 pages of 64 x 576 numbers
+//   55 us, about two pages in flight an SM); an even cut is worse where its longest run has over three times an SM's share of all pages
+//   (layers with 32 heads, even / by length, us: 63 sequences of 300 and one of 4,000 positions 139 / 115, 28 of 500 and four of 4,000
+//   105 / 97; 100 of 400 to 1,300 160 / 165, 64 of 2,048 to 4,096 150 / 150).
 //   warp 4      TMA producer: the queries once, then pages into a ring of `stages`; the first pages, unless one is the
 //               newest, are asked for before the wait on the kernel in front.
 //   warp 5      MMA issuer: the scores of the next page as soon as it has landed, the weighted sum of this one as soon as
@@ -39,7 +44,7 @@ constexpr uint32_t POLL_LIMIT = 1u << 25;      // polls that do not suspend the 
 constexpr int MAX_STAGES = 4;
 
 struct LatentUmmaParams {
-  int Hpad, H, rank, nbox, qcols, mblocks, splits, stages;
+  int Hpad, H, rank, nbox, qcols, mblocks, splits, rows, ctas, stages;       // rows: partial results a sequence has room for
   uint32_t tmem_cols;
   float scale_log2e;
   float* part_m;
@@ -114,18 +119,93 @@ latent_decode_umma_kernel(const __grid_constant__ CUtensorMap map_c, const __gri
   volatile int* armed = abort_flag + 1;                  // pages the producer has asked for; -1: not even the queries
   volatile int* stop = armed + 1;                        // [2]: the flag as warp 0 saw it in front of a barrier, so that all agree
 
-  const int s = blockIdx.x, split = blockIdx.y, rows0 = blockIdx.z * NH;
+  const int cta = blockIdx.x, rows0 = blockIdx.z * NH;
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);          // known to be the same for the whole warp
+  // one token per sequence: its own row is in the cache
+  auto pages_of = [&](int i) { return b.slot_ids[i] < 0 ? 0 : iert_page_walk(kv, b.pos0[i], BK).n; };
+  int s = cta % b.n_seqs, part = cta / b.n_seqs, parts = p.splits;
+  if (p.ctas > 0) {                                      // (the same numbers in every CTA)
+    int* red = reinterpret_cast<int*>(wmax);             // [2][8]
+    // sums and the largest over the sequences' runs of at most `most` pages
+    auto count = [&](int most, int& longest) {
+      int runs = 0, top = 0;
+      for (int i = tid; i < b.n_seqs; i += THREADS) {
+        const int n = pages_of(i);
+        runs += (n + most - 1) / most;
+        top = max(top, n);
+      }
+      runs = __reduce_add_sync(0xffffffffu, runs);
+      top = __reduce_max_sync(0xffffffffu, top);
+      if (lane == 0) { red[warp] = runs; red[8 + warp] = top; }
+      __syncthreads();
+      runs = top = 0;
+      for (int w = 0; w < THREADS / 32; ++w) { runs += red[w]; top = max(top, red[8 + w]); }
+      __syncthreads();
+      longest = top;
+      return runs;
+    };
+    int longest = 0;
+    const int total = count(1, longest);
+    const int even_run = (longest + p.splits - 1) / p.splits;
+    const bool worth = (long long)even_run * p.ctas > 3ll * total;
+    // the fewest pages a run with which there are no more runs than SMs and partial results
+    int low = max(max((total + p.ctas - 1) / p.ctas, (longest + p.rows - 1) / p.rows), 1), high = max(longest, low);
+    if (!worth || count(high, longest) > p.ctas) high = 0;         // (too many sequences for one wave)
+    while (low < high) {
+      const int mid = (low + high) / 2;
+      if (count(mid, longest) <= p.ctas) high = mid;
+      else low = mid + 1;
+    }
+    if (high > 0 && high < even_run) {
+      // the sequence that run `cta` belongs to
+      if (warp == 0) {
+        int before = 0, found = -1, first_run = 0, n_runs = 0;
+        for (int base = 0; found < 0 && base < b.n_seqs; base += 32) {
+          const int runs = base + lane < b.n_seqs ? (pages_of(base + lane) + high - 1) / high : 0;
+          int end = runs;
+#pragma unroll
+          for (int o = 1; o < 32; o *= 2) {
+            const int x = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += x;
+          }
+          const unsigned hit = __ballot_sync(0xffffffffu, before + end > cta);
+          if (hit) {
+            const int who = __ffs(hit) - 1;
+            found = base + who;
+            first_run = before + __shfl_sync(0xffffffffu, end - runs, who);
+            n_runs = __shfl_sync(0xffffffffu, runs, who);
+          }
+          before += __shfl_sync(0xffffffffu, end, 31);
+        }
+        if (lane == 0) { red[0] = found; red[1] = first_run; red[2] = n_runs; }
+      }
+      __syncthreads();
+      s = red[0];
+      part = cta - red[1];
+      parts = red[2];
+      __syncthreads();
+      if (s < 0) { pdl_wait(); return; }                 // no run left for this CTA
+    }
+  }
+  if (part >= parts) { pdl_wait(); return; }
   const int slot = b.slot_ids[s];
   if (slot < 0) { pdl_wait(); return; }
-  const int pos = b.pos0[s];                             // one token per sequence: its own row is in the cache
+  const int pos = b.pos0[s];
   const IertPageWalk walk = iert_page_walk(kv, pos, BK);
-  const int t_lo = (int)((long long)split * walk.n / p.splits), t_hi = (int)((long long)(split + 1) * walk.n / p.splits);
+  const int t_lo = (int)((long long)part * walk.n / parts), t_hi = (int)((long long)(part + 1) * walk.n / parts);
   const int n_tiles = t_hi - t_lo;
-  const size_t part_row0 = ((size_t)s * p.splits + split) * p.Hpad + rows0;
+  const size_t part_row0 = ((size_t)s * p.rows + part) * p.Hpad + rows0;
+  auto clear_rest = [&](int threads) {                   // what nobody writes: partials that the merge skips
+    for (int i = tid; part == 0 && i < (p.rows - parts) * NH; i += threads) {
+      const size_t row = ((size_t)s * p.rows + parts + i / NH) * p.Hpad + rows0 + i % NH;
+      p.part_m[row] = -INFINITY;
+      p.part_l[row] = 0.f;
+    }
+  };
   if (n_tiles <= 0) {                                    // an empty run: a partial that the merge skips
     pdl_wait();
+    clear_rest(THREADS);
     if (tid < NH) { p.part_m[part_row0 + tid] = -INFINITY; p.part_l[part_row0 + tid] = 0.f; }
     return;
   }
@@ -257,6 +337,7 @@ latent_decode_umma_kernel(const __grid_constant__ CUtensorMap map_c, const __gri
   } else {
     // ---------------- softmax: lane = head (lane % NH), warp = 16 keys of the page ----------------
     pdl_wait();
+    clear_rest(SOFT);
     const uint32_t lane_bits = (uint32_t)(warp * 32) << 16;
     const int hl = lane % NH;
     if (!wait_bar(q_full, 0, abort_flag)) { ok = false; *abort_flag = 1; }
@@ -418,10 +499,10 @@ int latent_umma_heads(int H, int rank, int R) {
   return nh;
 }
 
-// qa bf16 [T, Hpad, width]; part_m, part_l fp32 [T, splits, Hpad]; part_acc fp32 [T, splits, Hpad, rank] (rows of heads below
-// H are written).  One token per sequence; a cache of bf16 rows `width` = rank + R wide, pages of 64.
+// qa bf16 [T, Hpad, width]; part_m, part_l fp32 [T, rows, Hpad]; part_acc fp32 [T, rows, Hpad, rank] (rows of heads below
+// H are written), rows >= splits: with more of them the sequences may be cut by length.  One token per sequence; a cache of bf16 rows `width` = rank + R wide, pages of 64.
 int launch_latent_decode_umma(const void* qa, const IertBatchView* batch, const IertKvView* kv, int H, int Hpad, int R, float scale,
-                              int splits, float* part_m, float* part_l, float* part_acc, int* err, cudaStream_t stream) {
+                              int splits, int rows, float* part_m, float* part_l, float* part_acc, int* err, cudaStream_t stream) {
   const int T = batch->n_tokens, width = kv->head_dim, rank = width - R;
   const int nh = latent_umma_heads(H, rank, R);
   if (!nh || Hpad % nh || ((uintptr_t)qa & 15) || ((uintptr_t)kv->k & 15)) return IERT_BAD_ARGUMENT;
@@ -448,7 +529,10 @@ int launch_latent_decode_umma(const void* qa, const IertBatchView* batch, const 
     }
     configured = true;
   }
-  const dim3 grid(T, splits, Hpad / nh);
+  const int groups = Hpad / nh, sms = iert_sm_count_cached();
+  p.rows = rows;
+  p.ctas = rows > splits && groups <= sms ? sms / groups : 0;
+  const dim3 grid(T * splits > p.ctas ? T * splits : p.ctas, 1, groups);
   if (nh == 16) launch_dep(latent_decode_umma_kernel<16>, grid, dim3(THREADS), smem, stream, map_c, map_q, p, *batch, *kv);
   else launch_dep(latent_decode_umma_kernel<32>, grid, dim3(THREADS), smem, stream, map_c, map_q, p, *batch, *kv);
   return cudaGetLastError() == cudaSuccess ? IERT_OK : IERT_CUDA_ERROR;

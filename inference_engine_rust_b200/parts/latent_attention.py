@@ -141,6 +141,21 @@ class LatentAttention(Mixer):
     def cache_request(self) -> KVRequest:
         return KVRequest(kv_heads=1, head_dim=self.kv_rank + self.R, window=self.window, values=False)
 
+    def cut_by_length_key(self):
+        return ("latent", self.H, self.kv_rank, self.R, self.window)
+
+    def cut_by_length(self, pos0, cache_view) -> bool:
+        """Where the longest run of an even cut has over three times an SM's share of the step's pages (the kernel's own rule)."""
+        if cache_view is None or not self.rt.fast or self.rt.dtype != torch.bfloat16:
+            return False
+        group, page = cache_view.group, cache_view.group.page_tokens
+        width = min(group.table_width, group.ring_pages + 1) if not self.plain_form else group.table_width
+        hpad, splits = B.latent_decode_tc_plan(len(pos0), self.H, self.kv_rank, self.R, width)
+        if B.latent_decode_tc_rows(len(pos0), self.H, self.kv_rank, self.R, splits) == splits:
+            return False
+        pages = [p // page + 1 - (max(p + 1 - self.window, 0) // page if self.window else 0) for p in pos0]
+        return -(-max(pages) // splits) * (B.sm_count() // max(1, hpad // 32)) > 3 * sum(pages)
+
     def weight_bytes(self) -> int:
         if not self.plain_form:
             return self.proj.nbytes() + (self.uq.nbytes() if self.uq is not None else 0) + self.w_uk.numel() * self.w_uk.element_size() * 2 + self.o.nbytes()
@@ -195,10 +210,11 @@ class LatentAttention(Mixer):
             if rt.fast and c_ext.dtype == torch.bfloat16 and ctx.kind == "decode":
                 group = cache_view.group
                 hpad, splits = B.latent_decode_tc_plan(ctx.n_seqs, H, rank, R, min(group.table_width, group.ring_pages + 1))
+                rows = B.latent_decode_tc_rows(ctx.n_seqs, H, rank, R, splits) if ctx.unequal_lengths else splits
                 qa = ws.take("latent.qa", (T, hpad, rank + R), torch.bfloat16)
-                part_m = ws.take("latent.part_m", (T, splits, hpad), torch.float32)
-                part_l = ws.take("latent.part_l", (T, splits, hpad), torch.float32)
-                part_acc = ws.take("latent.part_acc", (T, splits, hpad, rank), torch.float32)
+                part_m = ws.take("latent.part_m", (T, rows, hpad), torch.float32)
+                part_l = ws.take("latent.part_l", (T, rows, hpad), torch.float32)
+                part_acc = ws.take("latent.part_acc", (T, rows, hpad, rank), torch.float32)
                 done = B.latent_attention_decode_tc(q_raw, self.w_uk, self.w_uv, out, ctx.batch, kv, H, D, V, self.scale, None,
                                                     hpad, splits, qa, part_m, part_l, part_acc, rt.err, ctx.stream,
                                                     rot_dim=R, gate=gate, inv_freq=self.inv_freq, rot_mul=self.rot_mul,
@@ -239,10 +255,11 @@ class LatentAttention(Mixer):
             if rt.fast and q.dtype == torch.bfloat16 and ctx.kind == "decode":
                 hpad, splits = B.latent_decode_tc_plan(ctx.n_seqs, H, self.kv_rank, 0, cache_view.group.table_width)
                 rank = self.kv_rank
+                rows = B.latent_decode_tc_rows(ctx.n_seqs, H, rank, 0, splits) if ctx.unequal_lengths else splits
                 qa = ws.take("latent.qa", (T, hpad, rank), torch.bfloat16)
-                part_m = ws.take("latent.part_m", (T, splits, hpad), torch.float32)
-                part_l = ws.take("latent.part_l", (T, splits, hpad), torch.float32)
-                part_acc = ws.take("latent.part_acc", (T, splits, hpad, rank), torch.float32)
+                part_m = ws.take("latent.part_m", (T, rows, hpad), torch.float32)
+                part_l = ws.take("latent.part_l", (T, rows, hpad), torch.float32)
+                part_acc = ws.take("latent.part_acc", (T, rows, hpad, rank), torch.float32)
                 done = B.latent_attention_decode_tc(q, self.w_uk, self.w_uv, out, ctx.batch, kv, H, D, V, self.scale,
                                                     self.sink, hpad, splits, qa, part_m, part_l, part_acc, rt.err, ctx.stream)
             if not done:
