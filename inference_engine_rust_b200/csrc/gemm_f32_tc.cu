@@ -13,13 +13,15 @@
 // 14,336: 1.6e-7 / 2.2e-6.  Sums that are short because nearly all of a row is zero have the same error in both: one number in a row
 // 2.6e-8 / 2.5e-8, eight 5.5e-8 / 5.3e-8 (with the two next products as well 2.5e-8 and 5.5e-8, and a tenth more time).
 //
-// Measured (gemm_plain.cu in brackets): 333 tokens x 28,672 x 4,096 0.81 ms (4.43), 333 x 4,096 x 14,336 0.43 ms (2.46), one token
+// Measured (gemm_plain.cu in brackets): 333 tokens x 28,672 x 4,096 0.72 ms (4.43), 333 x 4,096 x 14,336 0.39 ms (2.46), one token
 // x 28,672 x 4,096 0.27 ms (0.96), x 4,096 x 14,336 0.12 ms (2.38).  What bounds it is the chain of a block (copy, split, MMAs, read
-// back: about 2,400 cycles for 128 tokens); the six products alone are 768.  An 8 x 8 register tile of fp32 multiply-adds reached
+// back: about 2,000 cycles for 128 tokens); the six products alone are 768.  The weights' parts in tensor memory instead of shared memory (96 tokens
+// a tile then) were no faster, 778 us for the first of these, nor tokens split by a kernel in front, 903.  An 8 x 8 register tile of fp32 multiply-adds reached
 // 2.1 ms on the first of these sizes: shared memory returns one operand word per lane and cycle, which that tile needs in full.
 //
-// Roles: TMA brings fp32 tiles of 32 k into a ring; warps 8-15 split them into swizzled operand tiles, two to four blocks deep; a lane
-// of warp 0 asks for the tiles and issues the 12 MMAs of a block (128 weight rows on the M side, BT tokens on the N side); warps 0-7 add every second
+// Roles: TMA brings fp32 tiles of 32 k into a ring; warps 8-15 split them into swizzled operand tiles, two to four blocks deep; warp 16 asks for the
+// tiles and issues the 12 MMAs of a block (128 weight rows on the M side, BT tokens on the N side), converged, one lane acting (a lane of
+// warp 0 did so between its additions, each MMA's operands moved to uniform registers one by one: 839 us where this takes 742); warps 0-7 add every second
 // block's sums (64 k) to their registers while the next one's MMAs run.  A matrix with few rows is split over k between the
 // CTAs of a cluster (by the matrix's shape alone, so that a row's result does not depend on how many rows the call has), which
 // add their parts in order through distributed shared memory: no scratch, no counters.  An output that is not finite (an
@@ -34,7 +36,7 @@ using namespace sm100;
 
 namespace {
 
-constexpr int TILE_N = 128, BLOCK_K = 32, THREADS = 16 * 32;
+constexpr int TILE_N = 128, BLOCK_K = 32, THREADS = 17 * 32;
 constexpr int W_PART_BYTES = TILE_N * BLOCK_K * 2, W_STAGE_BYTES = TILE_N * BLOCK_K * 4;
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
 
@@ -132,9 +134,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
                                                                  const __grid_constant__ CUtensorMap map_x, const F32Params p) {
   using P = Plan<BT>;
   constexpr int X_PART_BYTES = BT * BLOCK_K * 2;
-  constexpr uint32_t ACC_COLS = 4 * BT;                                       // two buffers of (small products, main products)
+  // two buffers of (small products, main products)
+  constexpr uint32_t ACC_COLS = BT <= 16 ? 64 : BT <= 32 ? 128 : BT <= 64 ? 256 : 512;
   constexpr uint32_t IDESC = instr_desc_bf16(TILE_N, BT);
-  constexpr int W_ITEMS = TILE_N / 64, X_ITEMS = BT >= 64 ? BT / 64 : 1;     // rows a converter thread looks after
+  constexpr int W_ITEMS = TILE_N / 64, X_ITEMS = (BT + 63) / 64;     // rows a converter thread looks after
   constexpr int CPT = BT / 2;                                                 // outputs of an accumulating thread
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -176,7 +179,54 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
     tma_load_2d(ring + s * P::STAGE_BYTES + W_STAGE_BYTES, &map_x, &st_full[s], (kb0 + b) * BLOCK_K, t0);
   };
 
-  if (warp >= 8) {
+  if (warp == 16) {
+    // ---------------- tiles and MMAs ----------------
+    const uint32_t leader = elect_leader();
+    int asked = min(n_kb, P::STAGES);
+    if (lane == 0) {
+      tma_prefetch_desc(&map_w);
+      tma_prefetch_desc(&map_x);
+      for (int b = 0; b < asked; ++b) load_w(b);                               // the weights do not depend on the kernel in front
+      pdl_wait();
+      for (int b = 0; b < asked; ++b) load_x(b);
+    }
+    __syncwarp();
+    // a wait of the whole warp: what one lane sees, all act on
+    auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag)) != 0; };
+    int buf = 0;
+    uint32_t o_phase = 0;
+    for (int q = 0; ok && 2 * q < n_kb; ++q) {
+      // the MMAs of blocks 2 q and 2 q + 1: the main product x0 w0 in a sum of its own, the five small ones in another
+      if (!warp_wait(&acc_empty[q & 1], ((q >> 1) & 1) ^ 1)) { ok = false; break; }
+      const uint32_t d = tmem_base + (uint32_t)((q & 1) * 2 * BT);
+      for (int b = 2 * q; b < min(2 * q + 2, n_kb); ++b) {
+        if (!warp_wait(&op_full[buf], o_phase)) { ok = false; break; }
+        if (asked < n_kb) {                                                    // block b has left its place in the ring
+          if (lane == 0) { load_w(asked); load_x(asked); }
+          ++asked;
+          __syncwarp();
+        }
+        tc_fence_after();
+        const uint32_t wa = smem_addr(smem + buf * P::BUF_BYTES), xa = wa + 3 * W_PART_BYTES;
+        constexpr int WP[6] = {2, 0, 1, 1, 0, 0}, XP[6] = {0, 2, 1, 0, 1, 0};  // (part of w, part of x)
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+          const uint64_t da = smem_desc_k64(wa + WP[m] * W_PART_BYTES), db = smem_desc_k64(xa + XP[m] * X_PART_BYTES);
+#pragma unroll
+          for (int ks = 0; ks < BLOCK_K / 16; ++ks)
+            mma_ss(leader, d + (m == 5 ? BT : 0), da + 2 * ks, db + 2 * ks, IDESC, ((b & 1) || (m != 0 && m != 5) || ks > 0) ? 1u : 0u);
+        }
+        mma_commit(leader, &op_empty[buf]);
+        if (++buf == P::BUFS) { buf = 0; o_phase ^= 1; }
+      }
+      if (ok) mma_commit(leader, &acc_full[q & 1]);
+    }
+    if (!ok) {
+      *abort_flag = 1;
+      if (lane == 0)                                                           // copies under way land before the CTA ends
+        for (int b = max(0, asked - P::STAGES); b < asked; ++b) mbar_wait(&st_full[b % P::STAGES], (b / P::STAGES) & 1, WAIT_LIMIT);
+    }
+  } else if (warp >= 8) {
     // ---------------- converters ----------------
     const int ct = threadIdx.x - 8 * 32, row = ct >> 2, chunk = ct & 3;       // 64 rows x 4 runs of 8 k per pass
     // eight lanes read two rows of 128 bytes: odd rows take their second 16 bytes first, so that no two lanes meet in a bank
@@ -192,7 +242,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
       uint8_t* out = smem + buf * P::BUF_BYTES + out_off;
 #pragma unroll
       for (int i = 0; i < W_ITEMS + X_ITEMS; ++i) {
-        if (i >= W_ITEMS && BT < 64 && row >= BT) break;
+        if (i >= W_ITEMS && BT % 64 && row + 64 * (i - W_ITEMS) >= BT) break;
         const uint8_t* src = in + i * 64 * 128;                                // the tokens' rows follow the weights'
         const float4 u = *reinterpret_cast<const float4*>(src + half), v = *reinterpret_cast<const float4*>(src + (half ^ 16));
         float4 lo, hi;
@@ -213,55 +263,19 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
       if (++buf == P::BUFS) { buf = 0; o_phase ^= 1; }
     }
   } else {
-    // ---------------- MMA issue and accumulation: warp w reads TMEM lanes 32 (w % 4).., the columns of its half ----------------
+    // ---------------- accumulation: warp w reads TMEM lanes 32 (w % 4).., the columns of its half ----------------
     const int n_pairs = (n_kb + 1) / 2;
     float acc[CPT];
 #pragma unroll
     for (int j = 0; j < CPT; ++j) acc[j] = 0.f;
-    int asked = 0;
-    if (threadIdx.x == 0) {                        // one lane asks for the tiles and issues the MMAs
-      tma_prefetch_desc(&map_w);
-      tma_prefetch_desc(&map_x);
-      const int first = min(n_kb, P::STAGES);
-      for (; asked < first; ++asked) load_w(asked);                            // the weights do not depend on the kernel in front
-      pdl_wait();
-      for (int b = 0; b < first; ++b) load_x(b);
-    }
     pdl_wait();                                   // (the residual is read and written below)
     const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * CPT);
-    // the MMAs of blocks 2 q and 2 q + 1, by one lane: the main product x0 w0 in a sum of its own, the five small ones in another
-    int buf = 0;
-    uint32_t o_phase = 0;
-    auto issue = [&](int q) {
-      if (!wait_or_abort(&acc_empty[q & 1], ((q >> 1) & 1) ^ 1, abort_flag)) { ok = false; *abort_flag = 1; return; }
-      const uint32_t d = tmem_base + (uint32_t)((q & 1) * 2 * BT);
-      for (int b = 2 * q; b < min(2 * q + 2, n_kb); ++b) {
-        if (!wait_or_abort(&op_full[buf], o_phase, abort_flag)) { ok = false; *abort_flag = 1; return; }
-        if (asked < n_kb) { load_w(asked); load_x(asked); ++asked; }           // block b has left its place in the ring
-        tc_fence_after();
-        const uint32_t wa = smem_addr(smem + buf * P::BUF_BYTES), xa = wa + 3 * W_PART_BYTES;
-        constexpr int WP[6] = {2, 0, 1, 1, 0, 0}, XP[6] = {0, 2, 1, 0, 1, 0};  // (part of w, part of x)
-#pragma unroll
-        for (int m = 0; m < 6; ++m) {
-          const uint64_t da = smem_desc_k64(wa + WP[m] * W_PART_BYTES), db = smem_desc_k64(xa + XP[m] * X_PART_BYTES);
-#pragma unroll
-          for (int ks = 0; ks < BLOCK_K / 16; ++ks)
-            umma_bf16(d + (m == 5 ? BT : 0), da + 2 * ks, db + 2 * ks, IDESC, ((b & 1) || (m != 0 && m != 5) || ks > 0) ? 1u : 0u);
-        }
-        umma_commit(&op_empty[buf]);
-        if (++buf == P::BUFS) { buf = 0; o_phase ^= 1; }
-      }
-      umma_commit(&acc_full[q & 1]);
-    };
-    if (threadIdx.x == 0 && n_pairs > 0) issue(0);
     for (int q = 0; q < n_pairs; ++q) {
-      if (threadIdx.x == 0 && q + 1 < n_pairs) issue(q + 1);
-      __syncwarp();
       if (!wait_or_abort(&acc_full[q & 1], (q >> 1) & 1, abort_flag)) ok = false;
       if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
       tc_fence_after();
       const uint32_t src = taddr + (q & 1) * 2 * BT;
-      constexpr int STEP = CPT == 8 || CPT == 64 ? 8 : 16;
+      constexpr int STEP = CPT % 16 || CPT == 64 ? 8 : 16;
 #pragma unroll
       for (int c = 0; c < CPT; c += STEP) {
         float v[STEP], u[STEP];
@@ -280,8 +294,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[q & 1]);
     }
-    if (!ok && threadIdx.x == 0)                                              // copies under way land before the CTA ends
-      for (int b = max(0, asked - P::STAGES); b < asked; ++b) mbar_wait(&st_full[b % P::STAGES], (b / P::STAGES) & 1, WAIT_LIMIT);
     const int n_local = (warp & 3) * 32 + lane, c0 = (warp >> 2) * CPT;
 #pragma unroll
     for (int j = 0; j < CPT; ++j) {
@@ -375,7 +387,10 @@ IERT_API int iert_gemm_f32_tc(const float* x, const float* w, float* out, int M,
   // the splits follow from the matrix alone: as many as keep one token tile's CTAs within one per SM
   while (p.splits < 4 && 2 * p.splits * n_tiles <= iert_sm_count_cached() && p.kb_total / (2 * p.splits) >= 8) p.splits *= 2;
   p.kb_per_split = (p.kb_total + p.splits - 1) / p.splits;
-  const int bt = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+  // as few tiles of up to 128 tokens as there can be, of the fewest tokens (a row's result does not depend on the tile: 333 tokens in three of
+  // 112 instead of three of 128: x 28,672 x 4,096 742 -> 716 us, x 4,096 x 14,336 405 -> 387)
+  const int least = (M + 127) / 128, each = (M + least - 1) / least;
+  const int bt = each <= 16 ? 16 : each <= 32 ? 32 : each <= 64 ? 64 : (each + 15) / 16 * 16;
   p.t_tiles = (M + bt - 1) / bt;
   const long long tiles = (long long)n_tiles * p.t_tiles;
   if (tiles * p.splits > 0x7fffffff) return IERT_BAD_ARGUMENT;
@@ -383,6 +398,9 @@ IERT_API int iert_gemm_f32_tc(const float* x, const float* w, float* out, int M,
     case 16: return launch<16>(p, (int)tiles, stream);
     case 32: return launch<32>(p, (int)tiles, stream);
     case 64: return launch<64>(p, (int)tiles, stream);
+    case 80: return launch<80>(p, (int)tiles, stream);
+    case 96: return launch<96>(p, (int)tiles, stream);
+    case 112: return launch<112>(p, (int)tiles, stream);
     default: return launch<128>(p, (int)tiles, stream);
   }
 }
