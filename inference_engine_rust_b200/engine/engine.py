@@ -56,7 +56,7 @@ class _DecodeGraph:
     """A captured one-token step for `nb` sequences: its own metadata buffer, workspace and
     logits buffer (a graph replays fixed addresses), and the graph."""
 
-    def __init__(self, engine: "Engine", nb: int, unequal: bool = False):
+    def __init__(self, engine: "Engine", nb: int, cut_families: frozenset = frozenset()):
         rt, model = engine.rt, engine.model
         from ..parts.base import Workspace
         _, o_slot, _, o_seq, o_tok, o_rows, total = Engine._layout(nb, nb, nb)
@@ -75,7 +75,7 @@ class _DecodeGraph:
                 # the launches are replayed for other sequences: their host lists must not be read
                 ctx = engine._context("decode", self.meta, nb, nb, [1] * nb, HostCopyUnavailable("pos0"),
                                       HostCopyUnavailable("slots"))
-                ctx.unequal_lengths = unequal
+                ctx.cut_families = cut_families
                 model.forward(ctx, self.meta[o_tok:o_tok + nb], engine.cache,
                               self.meta[o_rows:o_rows + nb], nb, logits_out=self.logits)
             run()                                      # eager once: lazy set-up happens outside the capture
@@ -307,10 +307,10 @@ class Engine:
                            slot_ids_dev=meta[o_slot:o_slot + n], pos0_dev=meta[o_pos:o_pos + n],
                            cu_q_dev=meta[o_cu:o_cu + n + 1])
 
-    def _unequal(self, pos0) -> bool:
-        """Do the mixers want this one-token step cut by the sequences' lengths?  Steps of either
+    def _cut_families(self, pos0) -> frozenset:
+        """Which families of mixers want this one-token step cut by the sequences' lengths?  Steps of every
         kind replay a graph of their own."""
-        return len(pos0) >= 2 and self.model.cut_by_length(pos0, self.cache)
+        return self.model.cut_by_length(pos0, self.cache) if len(pos0) >= 2 else frozenset()
 
     @staticmethod
     def _place_device_tokens(dest: torch.Tensor, device_tokens) -> None:
@@ -345,7 +345,7 @@ class Engine:
             self._place_device_tokens(meta[o_tok:o_tok + T], device_tokens)
         self.h2d_bytes_last_step = total * 4
         ctx = self._context(kind, meta, n, T, q_lens, pos0, slots)
-        ctx.unequal_lengths = kind == "decode" and self._unequal(pos0)
+        ctx.cut_families = self._cut_families(pos0) if kind == "decode" else frozenset()
         return self.model.forward(ctx, meta[o_tok:o_tok + T], self.cache,
                                   meta[o_rows:o_rows + R] if R else None, R)
 
@@ -358,10 +358,10 @@ class Engine:
         nb = 1
         while nb < n:
             nb *= 2
-        unequal = self._unequal(pos0)
-        g = self._graphs.get((nb, unequal))
+        families = self._cut_families(pos0)
+        g = self._graphs.get((nb, families))
         if g is None:
-            g = self._graphs[(nb, unequal)] = _DecodeGraph(self, nb, unequal)
+            g = self._graphs[(nb, families)] = _DecodeGraph(self, nb, families)
         o_cu, o_slot, o_pos, o_seq, o_tok, o_rows, total = self._layout(nb, nb, nb)
         host, turn = self._staging.next(total)
         pad = nb - n

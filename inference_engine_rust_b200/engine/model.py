@@ -14,7 +14,7 @@ import torch
 from ..cache import CacheRequest
 from ..config.specs import ModelSpec
 from ..csrc import bindings as B
-from ..parts.base import Runtime, StepContext, first_norm_request_of, part_class
+from ..parts.base import Runtime, StepContext, cut_questions, first_norm_request_of, part_class
 from ..weights.loader import (RandomSource, TensorSpec, WeightError, check_source, fetch_many)
 
 
@@ -217,23 +217,23 @@ class Model:
         return total
 
     # ---- forward --------------------------------------------------------------------------
-    def cut_by_length(self, pos0, cache) -> bool:
-        """Does any mixer want this one-token step (positions of the live sequences) cut by length?
-        Each is asked with the view of the cache that its layer reads."""
+    def cut_by_length(self, pos0, cache) -> frozenset:
+        """The families of mixers (`Mixer.cut_family`) that want this one-token step (positions of the live sequences) cut by
+        length.  Each mixer is asked with the view of the cache that its layer reads."""
         if self._cut_askers is None:
-            # every mixer that has the (optional) method, one per `cut_by_length_key()` where mixers
-            # say that their answers are the same (layers of equal shape): asked every step
+            # every mixer that has the (optional) method, one per key where mixers say that their
+            # answers are the same (layers of equal shape): asked every step
             seen, self._cut_askers = set(), []
             for pos, e in enumerate(self.spec.schedule):
-                mixer = self._layer_parts[e.layer][1]
-                ask = getattr(mixer, "cut_by_length", None)
-                if ask is None:
-                    continue
-                key = getattr(mixer, "cut_by_length_key", lambda m=mixer: id(m))()
-                if key not in seen:
-                    seen.add(key)
-                    self._cut_askers.append((ask, self.spec.cache_entry(pos)))
-        return any(ask(pos0, cache.layer_view(entry)) for ask, entry in self._cut_askers)
+                for key, family, ask in cut_questions(self._layer_parts[e.layer][1]):
+                    if key not in seen:
+                        seen.add(key)
+                        self._cut_askers.append((family, ask, self.spec.cache_entry(pos)))
+        asked = set()
+        for family, ask, entry in self._cut_askers:
+            if family not in asked and ask(pos0, cache.layer_view(entry)):
+                asked.add(family)
+        return frozenset(asked)
 
     def forward(self, ctx: StepContext, tokens: torch.Tensor, cache, logit_rows: Optional[torch.Tensor],
                 n_logit_rows: int, logits_out: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
@@ -280,6 +280,7 @@ class Model:
             # no block prepares rows for a layer in front of which the start of a pass changes them
             last = pos + 1 == len(sched) or sched[pos + 1].pass_start is not None
             ctx.next_block = None if last else self.blocks[sched[pos + 1].layer]
+            ctx.answer_cut(self._layer_parts[e.layer][1])
             self.blocks[e.layer].forward(rows, ctx, view, e.writes_cache)
             if self.after_block is not None:
                 self.after_block(pos, rows, ctx)

@@ -141,6 +141,8 @@ class LatentAttention(Mixer):
     def cache_request(self) -> KVRequest:
         return KVRequest(kv_heads=1, head_dim=self.kv_rank + self.R, window=self.window, values=False)
 
+    cut_family = "latent"
+
     def cut_by_length_key(self):
         return ("latent", self.H, self.kv_rank, self.R, self.window)
 

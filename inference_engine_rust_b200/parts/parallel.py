@@ -14,7 +14,7 @@ import torch
 
 from ..config.specs import PartSpec
 from ..weights.loader import TensorSpec
-from .base import Mixer, Runtime, StepContext, part_class, register_part
+from .base import Mixer, Runtime, StepContext, cut_questions, part_class, register_part
 
 SIDES = ("left", "right")
 
@@ -48,14 +48,15 @@ class ParallelMixers(Mixer):
     def weight_bytes(self) -> int:
         return sum(m.weight_bytes() for m in self.subs if hasattr(m, "weight_bytes"))
 
-    def cut_by_length_key(self):
-        return ("parallel",) + tuple(getattr(m, "cut_by_length_key", lambda m=m: id(m))() for m in self.subs)
-
-    def cut_by_length(self, pos0, cache_view) -> bool:
-        return cache_view is not None and any(m.cut_by_length(pos0, v) for m, v in zip(self.subs, cache_view))
+    def cut_questions(self) -> list:
+        def of_side(i, ask):
+            return lambda pos0, cache_view: cache_view is not None and ask(pos0, cache_view[i])
+        return [(("parallel", i, key), family, of_side(i, ask))
+                for i, m in enumerate(self.subs) for key, family, ask in cut_questions(m)]
 
     def forward(self, xn, residual, ctx: StepContext, cache_view, writes_cache: bool) -> None:
         for m, view in zip(self.subs, cache_view):
+            ctx.answer_cut(m)
             m.forward(xn, residual, ctx, view, writes_cache)
 
 
