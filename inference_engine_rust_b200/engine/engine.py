@@ -307,10 +307,10 @@ class Engine:
                            slot_ids_dev=meta[o_slot:o_slot + n], pos0_dev=meta[o_pos:o_pos + n],
                            cu_q_dev=meta[o_cu:o_cu + n + 1])
 
-    def _cut_families(self, pos0) -> frozenset:
-        """Which families of mixers want this one-token step cut by the sequences' lengths?  Steps of every
-        kind replay a graph of their own."""
-        return self.model.cut_by_length(pos0, self.cache) if len(pos0) >= 2 else frozenset()
+    def _cut_families(self, pos0, n_seqs: int) -> frozenset:
+        """Which families of mixers want this one-token step, sized for `n_seqs` sequences, cut by the sequences' lengths?
+        Steps of every kind replay a graph of their own."""
+        return self.model.cut_by_length(pos0, self.cache, n_seqs) if len(pos0) >= 2 else frozenset()
 
     @staticmethod
     def _place_device_tokens(dest: torch.Tensor, device_tokens) -> None:
@@ -345,7 +345,7 @@ class Engine:
             self._place_device_tokens(meta[o_tok:o_tok + T], device_tokens)
         self.h2d_bytes_last_step = total * 4
         ctx = self._context(kind, meta, n, T, q_lens, pos0, slots)
-        ctx.cut_families = self._cut_families(pos0) if kind == "decode" else frozenset()
+        ctx.cut_families = self._cut_families(pos0, n) if kind == "decode" else frozenset()
         return self.model.forward(ctx, meta[o_tok:o_tok + T], self.cache,
                                   meta[o_rows:o_rows + R] if R else None, R)
 
@@ -358,7 +358,7 @@ class Engine:
         nb = 1
         while nb < n:
             nb *= 2
-        families = self._cut_families(pos0)
+        families = self._cut_families(pos0, nb)
         g = self._graphs.get((nb, families))
         if g is None:
             g = self._graphs[(nb, families)] = _DecodeGraph(self, nb, families)

@@ -217,9 +217,9 @@ class Model:
         return total
 
     # ---- forward --------------------------------------------------------------------------
-    def cut_by_length(self, pos0, cache) -> frozenset:
-        """The families of mixers (`Mixer.cut_family`) that want this one-token step (positions of the live sequences) cut by
-        length.  Each mixer is asked with the view of the cache that its layer reads."""
+    def cut_by_length(self, pos0, cache, n_seqs: Optional[int] = None) -> frozenset:
+        """The families of mixers (`Mixer.cut_family`) that want this one-token step (positions of the live sequences; `n_seqs`
+        with padding, by default without any) cut by length.  Each mixer is asked with the view of the cache that its layer reads."""
         if self._cut_askers is None:
             # every mixer that has the (optional) method, one per key where mixers say that their
             # answers are the same (layers of equal shape): asked every step
@@ -231,7 +231,7 @@ class Model:
                         self._cut_askers.append((family, ask, self.spec.cache_entry(pos)))
         asked = set()
         for family, ask, entry in self._cut_askers:
-            if family not in asked and ask(pos0, cache.layer_view(entry)):
+            if family not in asked and ask(pos0, cache.layer_view(entry), n_seqs or len(pos0)):
                 asked.add(family)
         return frozenset(asked)
 

@@ -265,6 +265,9 @@ class Mixer(Part):
     # mixers to which a cut costs and gives something else: one asked for by latent attention made grouped-query layers of the same
     # step slower (128 sequences, four of 1,500 positions: 95 us a layer evenly, 135 cut).
     cut_family = "attention"
+    # True: `cut_by_length` takes a third argument, the number of sequences that the step's launches are sized for (a captured
+    # step is padded to a power of two), which is what they plan by.
+    cut_by_batch = False
 
     def cache_request(self) -> CacheRequest:
         return None
@@ -284,8 +287,9 @@ class Mixer(Part):
 
 
 def cut_questions(mixer) -> list:
-    """(key, family, ask) of what a mixer of any registered class has to be asked before a one-token step: its (optional)
-    `cut_by_length`, or those of the mixers it is made of (a method `cut_questions`).  Questions of equal keys have the same answer."""
+    """(key, family, ask(pos0, cache_view, sequences the launches are sized for)) of what a mixer of any registered class has to be
+    asked before a one-token step: its (optional) `cut_by_length`, or those of the mixers it is made of (a method `cut_questions`).
+    Questions of equal keys have the same answer."""
     parts = getattr(mixer, "cut_questions", None)
     if parts is not None:
         return parts()
@@ -293,6 +297,8 @@ def cut_questions(mixer) -> list:
     if ask is None:
         return []
     key = getattr(mixer, "cut_by_length_key", lambda: id(mixer))()
+    if not getattr(mixer, "cut_by_batch", Mixer.cut_by_batch):
+        return [(key, getattr(mixer, "cut_family", Mixer.cut_family), lambda pos0, cache_view, n_seqs: ask(pos0, cache_view))]
     return [(key, getattr(mixer, "cut_family", Mixer.cut_family), ask)]
 
 

@@ -41,6 +41,26 @@ from .base import Mixer, Runtime, StepContext, part_class, register_part
 from .linear import Linear
 
 
+def length_cut_run(pages, splits: int, rows: int, ctas: int) -> int:
+    """Pages a run has at most where csrc/latent_decode_umma.cu, with room for `rows` partial results a sequence and `ctas` CTAs, cuts
+    sequences of these pages by length; 0 where it cuts each into `splits`.  (The kernel works the same out on the device.)"""
+    total, longest = sum(pages), max(pages)
+    even_run = -(-longest // splits)
+    if rows <= splits or ctas <= 0 or even_run * ctas <= 3 * total:
+        return 0
+    low = max(-(-total // ctas), -(-longest // rows), 1)
+    high = max(longest, low)
+    if len(pages) > ctas:                # (not even a run a sequence fits the device at once)
+        return 0
+    while low < high:
+        mid = (low + high) // 2
+        if sum(-(-n // mid) for n in pages) <= ctas:
+            high = mid
+        else:
+            low = mid + 1
+    return high if high < even_run else 0
+
+
 class LatentAttention(Mixer):
     graph_safe = True
     takes_out_scale = True
@@ -141,22 +161,24 @@ class LatentAttention(Mixer):
     def cache_request(self) -> KVRequest:
         return KVRequest(kv_heads=1, head_dim=self.kv_rank + self.R, window=self.window, values=False)
 
-    cut_family = "latent"
+    cut_family, cut_by_batch = "latent", True
 
     def cut_by_length_key(self):
         return ("latent", self.H, self.kv_rank, self.R, self.window)
 
-    def cut_by_length(self, pos0, cache_view) -> bool:
-        """Where the longest run of an even cut has over three times an SM's share of the step's pages (the kernel's own rule)."""
-        if cache_view is None or not self.rt.fast or self.rt.dtype != torch.bfloat16:
+    def cut_by_length(self, pos0, cache_view, n_seqs=None) -> bool:
+        """Will the kernel, launched for `n_seqs` sequences (by default as many as there are) and with room for it, cut these by length?"""
+        n_seqs = n_seqs or len(pos0)
+        if cache_view is None or not self.rt.fast or self.rt.dtype != torch.bfloat16 or n_seqs < 8:       # (fewer: never room)
             return False
         group, page = cache_view.group, cache_view.group.page_tokens
         width = min(group.table_width, group.ring_pages + 1) if not self.plain_form else group.table_width
-        hpad, splits = B.latent_decode_tc_plan(len(pos0), self.H, self.kv_rank, self.R, width)
-        if B.latent_decode_tc_rows(len(pos0), self.H, self.kv_rank, self.R, splits) == splits:
-            return False
+        hpad, splits = B.latent_decode_tc_plan(n_seqs, self.H, self.kv_rank, self.R, width)
+        rows, ctas = B.latent_decode_tc_rows(n_seqs, self.H, self.kv_rank, self.R, splits), B.sm_count() // (hpad // (32 if self.H > 16 else 16))
+        if rows == splits or not self.window and page * -(-(max(pos0) // page + 1) // splits) * ctas <= 3 * sum(pos0):
+            return False                 # (the second: a lower bound of the pages' sum already says no)
         pages = [p // page + 1 - (max(p + 1 - self.window, 0) // page if self.window else 0) for p in pos0]
-        return -(-max(pages) // splits) * (B.sm_count() // max(1, hpad // 32)) > 3 * sum(pages)
+        return length_cut_run(pages, splits, rows, ctas) > 0
 
     def weight_bytes(self) -> int:
         if not self.plain_form:

@@ -50,7 +50,7 @@ class ParallelMixers(Mixer):
 
     def cut_questions(self) -> list:
         def of_side(i, ask):
-            return lambda pos0, cache_view: cache_view is not None and ask(pos0, cache_view[i])
+            return lambda pos0, cache_view, n_seqs: cache_view is not None and ask(pos0, cache_view[i], n_seqs)
         return [(("parallel", i, key), family, of_side(i, ask))
                 for i, m in enumerate(self.subs) for key, family, ask in cut_questions(m)]
 
