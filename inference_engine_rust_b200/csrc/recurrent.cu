@@ -226,7 +226,10 @@ __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16* p) 
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
 
-// Two numbers as pairs of bf16 numbers p[0] + p[1] + p[2]; every remainder is exact.
+// Two numbers as pairs of bf16 numbers p[0] + p[1] + p[2]; every remainder is exact, but for bits below 2^-133, bf16's smallest number, which are
+// lost (an error of 2^-134 at most; fp32 keeps bits down to 2^-149).  The first two parts stop at bf16's largest finite number: what rounds beyond
+// it (3.39e38 and more) would leave a remainder of the other sign without end.  So an infinity is (largest, largest, infinity), whose products are
+// the infinities that they are in fp32, and a NaN stays one.
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
   float2 d;
   asm("sub.rn.f32x2 %0, %1, %2;"
@@ -246,11 +249,16 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t& p0, uint32_t&
     const __nv_bfloat162 two = __floats2bfloat162_rn(f.x, f.y);
     return *reinterpret_cast<const uint32_t*>(&two);
   };
+  auto nearest_finite = [](float2 f) {
+    uint32_t two;
+    asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(two) : "f"(f.y), "f"(f.x));
+    return two;
+  };
   auto wide = [](uint32_t p) { return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u)); };
   float2 f = make_float2(x, y);
-  p0 = nearest(f);
+  p0 = nearest_finite(f);
   f = sub2(f, wide(p0));
-  p1 = nearest(f);
+  p1 = nearest_finite(f);
   p2 = nearest(sub2(f, wide(p1)));
 }
 // Two neighbouring accumulator tiles [16 x 8] as the three parts of a left operand [16 x 16].
