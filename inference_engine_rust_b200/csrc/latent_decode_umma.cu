@@ -10,7 +10,7 @@
 //   page meets, live in TMEM: 128 lanes hold 128 / NH copies of the NH heads, every warp of the softmax finds all heads in
 //   its own 32 lanes and takes 16 of the page's 64 keys.  Their way there is through the last stage of the page ring,
 //   which is filled with pages once they have moved on.
-//   grid (runs of pages, 1, groups of NH heads); a CTA walks its run of a sequence's pages.  Sequences are cut evenly, `splits` runs each, or
+//   grid (sequences, runs of pages, groups of NH heads); a CTA walks its run of a sequence's pages.  Sequences are cut evenly, `splits` runs each, or
 //   (where there is room for more partial results) by length: runs of the fewest pages that let all of them have an SM at once, which every CTA
 //   works out from the lengths.  The pages' bytes bound a step whose sequences are alike, whatever the cut (3,104 pages of 64 x 576 numbers
 //   55 us, about two pages in flight an SM); an even cut is worse where its longest run has over three times an SM's share of all pages
@@ -67,7 +67,9 @@ __device__ __forceinline__ float ex2(float x) {
 }
 __device__ __forceinline__ void soft_sync() { asm volatile("bar.sync 1, %0;" ::"n"(SOFT) : "memory"); }
 
-template <int NH>
+// CUT: a launch with room for more partial results than `splits` runs need, whose sequences may be cut by length.  (A kernel of its own: with the
+// rule's code in front of it an even step of 16 sequences of 4,096 positions took 104.2 us a layer, without it 101.4.)
+template <int NH, bool CUT>
 __global__ void __launch_bounds__(THREADS, 1)
 latent_decode_umma_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_q, LatentUmmaParams p,
                           IertBatchView b, IertKvView kv) {
@@ -94,13 +96,14 @@ latent_decode_umma_kernel(const __grid_constant__ CUtensorMap map_c, const __gri
   volatile int* armed = abort_flag + 1;                  // pages the producer has asked for; -1: not even the queries
   volatile int* stop = armed + 1;                        // [2]: the flag as warp 0 saw it in front of a barrier, so that all agree
 
-  const int cta = blockIdx.x, rows0 = blockIdx.z * NH;
+  const int rows0 = blockIdx.z * NH;
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);          // known to be the same for the whole warp
-  // one token per sequence: its own row is in the cache
-  auto pages_of = [&](int i) { return b.slot_ids[i] < 0 ? 0 : iert_page_walk(kv, b.pos0[i], BK).n; };
-  int s = cta % b.n_seqs, part = cta / b.n_seqs, parts = p.splits;
-  if (p.ctas > 0) {                                      // (the same numbers in every CTA)
+  int s = CUT ? (int)blockIdx.x % b.n_seqs : blockIdx.x, part = CUT ? (int)blockIdx.x / b.n_seqs : blockIdx.y, parts = p.splits;
+  if (CUT && p.ctas > 0) {                               // (the same numbers in every CTA)
+    const int cta = blockIdx.x;
+    // one token per sequence: its own row is in the cache
+    auto pages_of = [&](int i) { return b.slot_ids[i] < 0 ? 0 : iert_page_walk(kv, b.pos0[i], BK).n; };
     int* red = reinterpret_cast<int*>(wmax);             // [2][8]
     // sums and the largest over the sequences' runs of at most `most` pages
     auto count = [&](int most, int& longest) {
@@ -163,16 +166,16 @@ latent_decode_umma_kernel(const __grid_constant__ CUtensorMap map_c, const __gri
       if (s < 0) { pdl_wait(); return; }                 // no run left for this CTA
     }
   }
-  if (part >= parts) { pdl_wait(); return; }
+  if (CUT && part >= parts) { pdl_wait(); return; }
   const int slot = b.slot_ids[s];
   if (slot < 0) { pdl_wait(); return; }
-  const int pos = b.pos0[s];
+  const int pos = b.pos0[s];                             // one token per sequence: its own row is in the cache
   const IertPageWalk walk = iert_page_walk(kv, pos, BK);
   const int t_lo = (int)((long long)part * walk.n / parts), t_hi = (int)((long long)(part + 1) * walk.n / parts);
   const int n_tiles = t_hi - t_lo;
-  const size_t part_row0 = ((size_t)s * p.rows + part) * p.Hpad + rows0;
+  const size_t part_row0 = ((size_t)s * (CUT ? p.rows : p.splits) + part) * p.Hpad + rows0;
   auto clear_rest = [&](int threads) {                   // what nobody writes: partials that the merge skips
-    for (int i = tid; part == 0 && i < (p.rows - parts) * NH; i += threads) {
+    for (int i = tid; CUT && part == 0 && i < (p.rows - parts) * NH; i += threads) {
       const size_t row = ((size_t)s * p.rows + parts + i / NH) * p.Hpad + rows0 + i % NH;
       p.part_m[row] = -INFINITY;
       p.part_l[row] = 0.f;
@@ -497,8 +500,13 @@ int launch_latent_decode_umma(const void* qa, const IertBatchView* batch, const 
   const size_t smem = fixed_smem(nh) + (size_t)p.stages * p.nbox * BOX;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(latent_decode_umma_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
-        cudaFuncSetAttribute(latent_decode_umma_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
+    bool good = true;
+    auto ask = [&](auto* k) { good = good && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess; };
+    ask(latent_decode_umma_kernel<16, false>);
+    ask(latent_decode_umma_kernel<32, false>);
+    ask(latent_decode_umma_kernel<16, true>);
+    ask(latent_decode_umma_kernel<32, true>);
+    if (!good) {
       cudaGetLastError();
       return IERT_CUDA_ERROR;
     }
@@ -507,8 +515,10 @@ int launch_latent_decode_umma(const void* qa, const IertBatchView* batch, const 
   const int groups = Hpad / nh, sms = iert_sm_count_cached();
   p.rows = rows;
   p.ctas = rows > splits && groups <= sms ? sms / groups : 0;
-  const dim3 grid(T * splits > p.ctas ? T * splits : p.ctas, 1, groups);
-  if (nh == 16) launch_dep(latent_decode_umma_kernel<16>, grid, dim3(THREADS), smem, stream, map_c, map_q, p, *batch, *kv);
-  else launch_dep(latent_decode_umma_kernel<32>, grid, dim3(THREADS), smem, stream, map_c, map_q, p, *batch, *kv);
+  const bool cut = rows > splits;
+  const dim3 grid = cut ? dim3(T * splits > p.ctas ? T * splits : p.ctas, 1, groups) : dim3(T, splits, groups);
+  auto* kernel = nh == 16 ? (cut ? latent_decode_umma_kernel<16, true> : latent_decode_umma_kernel<16, false>)
+                          : (cut ? latent_decode_umma_kernel<32, true> : latent_decode_umma_kernel<32, false>);
+  launch_dep(kernel, grid, dim3(THREADS), smem, stream, map_c, map_q, p, *batch, *kv);
   return cudaGetLastError() == cudaSuccess ? IERT_OK : IERT_CUDA_ERROR;
 }
