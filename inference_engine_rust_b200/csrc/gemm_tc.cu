@@ -166,11 +166,13 @@ __device__ __forceinline__ void write_out4(const GemmParams& p, int tok, int n, 
 
 // Split-K: rows t_first, t_first + 4, ... < t_end of a tile's partial products (one [BT][TILE_N]
 // fp32 block per split at `base`) added in split order and written out; 32 threads share a row, each
-// four columns (c4).  R rows and U splits are in flight per thread and pass, and a residual is
+// four columns (c4).  Four rows and four splits are in flight per thread and pass, and a residual is
 // read together with the first partials, so that a pass costs one round trip to the L2: with 64
-// rows per split a row-at-a-time loop spent 30 us here.
-template <int BT, int R, int U>
-__device__ __forceinline__ void reduce_rows_by(const GemmParams& p, const float* base, int t_first, int t_end,
+// rows per split a row-at-a-time loop spent 30 us here.  (A second form for more than four splits, two rows by eight splits, saved 0.3 us where
+// one product follows another of its kind, and cost 3 to 4 us a product in layers of other kernels, whose weights push this code out of the
+// caches: 26 KB more, fetched when the last accumulator is done.  Delta rule, six sequences of 64 tokens in all: 110 us a layer with it, 104 without.)
+template <int BT>
+__device__ __forceinline__ void reduce_partial_rows(const GemmParams& p, const float* base, int t_first, int t_end,
                                                     int t0, int n, int c4, int n_idx, const float* rstd) {
   const bool vec_res = p.mode == MODE_ADD_RESIDUAL && p.out_dtype == IERT_F32 && n + 4 <= p.N && (p.ldo & 3) == 0 &&
                        ((uintptr_t)p.out & 15) == 0;
@@ -183,33 +185,33 @@ __device__ __forceinline__ void reduce_rows_by(const GemmParams& p, const float*
         g[i] = p.ahead.weight_dtype == IERT_F32 ? ((const float*)p.ahead.weight)[n + i]
                                                 : __bfloat162float(((const __nv_bfloat16*)p.ahead.weight)[n + i]);
   }
-  for (int t = t_first; t < t_end; t += 4 * R) {
-    float4 acc[R], res[R];
+  for (int t = t_first; t < t_end; t += 16) {
+    float4 acc[4], res[4];
 #pragma unroll
-    for (int h = 0; h < R; ++h) {
+    for (int h = 0; h < 4; ++h) {
       acc[h] = make_float4(0.f, 0.f, 0.f, 0.f);
       res[h] = (vec_res && t + 4 * h < t_end)
                    ? *reinterpret_cast<const float4*>((const float*)p.out + (long long)(t0 + t + 4 * h) * p.ldo + n)
                    : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    for (int s0 = 0; s0 < p.splits; s0 += U) {
-      float4 v[R][U];
+    for (int s0 = 0; s0 < p.splits; s0 += 4) {
+      float4 v[4][4];
 #pragma unroll
-      for (int h = 0; h < R; ++h)
+      for (int h = 0; h < 4; ++h)
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int u = 0; u < 4; ++u)
           v[h][u] = (s0 + u < p.splits && t + 4 * h < t_end)
                         ? __ldcg(reinterpret_cast<const float4*>(base + ((size_t)(s0 + u) * BT + t + 4 * h) * TILE_N) + c4)
                         : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int h = 0; h < R; ++h)
+      for (int h = 0; h < 4; ++h)
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
+        for (int u = 0; u < 4; ++u) {
           acc[h].x += v[h][u].x; acc[h].y += v[h][u].y; acc[h].z += v[h][u].z; acc[h].w += v[h][u].w;
         }
     }
 #pragma unroll
-    for (int h = 0; h < R; ++h) {
+    for (int h = 0; h < 4; ++h) {
       if (t + 4 * h >= t_end) break;                     // the same for the 32 threads that share the row
       const int row = t + 4 * h;
       if (rstd) {                                        // the input rows' 1 / rms (see IertRowScale)
@@ -250,13 +252,6 @@ __device__ __forceinline__ void reduce_rows_by(const GemmParams& p, const float*
       }
     }
   }
-}
-// (More than four splits: two rows and all of up to eight splits at once.  Four and four then took a second trip for the same rows.)
-template <int BT>
-__device__ __forceinline__ void reduce_partial_rows(const GemmParams& p, const float* base, int t_first, int t_end,
-                                                    int t0, int n, int c4, int n_idx, const float* rstd) {
-  if (BT > 16 && p.splits > 4) reduce_rows_by<BT, 2, 8>(p, base, t_first, t_end, t0, n, c4, n_idx, rstd);
-  else reduce_rows_by<BT, 4, 4>(p, base, t_first, t_end, t0, n, c4, n_idx, rstd);
 }
 
 // A CTA's list of work, the same for its three roles: items (tile, part of k) strided over the
