@@ -71,19 +71,23 @@ def apply(linear, x, out, n_rows: int, mode: int, stream: int, ctx=None, epilogu
     if x.dtype != torch.bfloat16:
         return False
     # (a forced token tile keeps a prompt's plain store off the token-major kernel, which does not split the inner axis)
-    return B.gemm_tc(x, linear.weight, out, n_rows, mode, err, stream, force_bt=narrow_tile(linear, n_rows), epilogue=epilogue)
+    return B.gemm_tc(x, linear.weight, out, n_rows, mode, err, stream, force_bt=narrow_tile(linear, n_rows) if linear.narrow else 0,
+                     epilogue=epilogue)
 
 
 def narrow_tile(linear, n_rows: int) -> int:
     """Token tile of a prompt's product with few outputs (0: the kernel's own choice).  Its tiles are split over the inner axis; tiles of 64
-    tokens are more of them, with smaller partial results, as long as at least three parts of each fit the device (two CTAs an SM).  64 / 256
-    tokens a tile, us: 64 outputs of 4,096, 256 tokens 9.7 / 14.9, 512 9.9 / 15.1, 2,048 11.9 / 15.5, 4,096 14.6 / 16.7; 288 of 8,192, 256
-    tokens 13.6 / 17.1, 1,024 16.6 / 18.4, 2,048 23.8 / 23.5, 4,096 49.6 / 39.1 (the kernel's choice: 22.3 for the first of 2,048, 53 for the last)."""
+    tokens are more of them, with smaller partial results, as long as at least six parts of each fit the device (two CTAs an SM).  Up to 256
+    tokens that holds for one tile of weight rows only: beside others the launch's many CTAs keep the kernels behind it waiting.
+    Layers whole, tiles of 64 / otherwise, us: 64 outputs of 4,096 (delta rule), 180 tokens 135 / 137, 250 149 / 153, 600 212 / 217, 2,500 617 / 624,
+    4,096 962 / 952; 288 of 8,192 (selective scan), 130 tokens 146 / 141, 169 156 / 153, 256 188 / 188, 300 200 / 203, 600 287 / 292,
+    1,000 384 / 385, 1,600 576 / 569."""
     if not linear.narrow or n_rows <= 128:
         return 0
-    if 3 * -(-n_rows // 64) * -(-linear.out_features // 128) <= 2 * B.sm_count():
-        return 64
-    return 256 if n_rows > 256 else 0
+    weight_tiles = -(-linear.out_features // 128)
+    if n_rows <= 256:
+        return 64 if weight_tiles == 1 else 0
+    return 64 if 6 * -(-n_rows // 64) * weight_tiles <= 2 * B.sm_count() else 256
 
 
 def apply_gated(linear, x, act, n_rows: int, stream: int, fn=None, epilogue=None) -> bool:
