@@ -173,12 +173,23 @@ class LatentAttention(Mixer):
             return False
         group, page = cache_view.group, cache_view.group.page_tokens
         width = min(group.table_width, group.ring_pages + 1) if not self.plain_form else group.table_width
-        hpad, splits = B.latent_decode_tc_plan(n_seqs, self.H, self.kv_rank, self.R, width)
-        rows, ctas = B.latent_decode_tc_rows(n_seqs, self.H, self.kv_rank, self.R, splits), B.sm_count() // (hpad // (32 if self.H > 16 else 16))
-        if rows == splits or not self.window and page * -(-(max(pos0) // page + 1) // splits) * ctas <= 3 * sum(pos0):
-            return False                 # (the second: a lower bound of the pages' sum already says no)
+        splits, rows, ctas = self._cut_plan(n_seqs, width)
+        if rows == splits:
+            return False
+        longest = max(pos0)
+        if not (self.window and longest >= self.window) and page * -(-(longest // page + 1) // splits) * ctas <= 3 * sum(pos0):
+            return False                 # (a lower bound of the pages' sum already says no)
         pages = [p // page + 1 - (max(p + 1 - self.window, 0) // page if self.window else 0) for p in pos0]
         return length_cut_run(pages, splits, rows, ctas) > 0
+
+    def _cut_plan(self, n_seqs: int, width: int):
+        """(runs of an even cut, partial results a sequence has room for, CTAs that walk pages at once); asked every step, so kept."""
+        plans = self.__dict__.setdefault("_cut_plans", {})
+        if (n_seqs, width) not in plans:
+            hpad, splits = B.latent_decode_tc_plan(n_seqs, self.H, self.kv_rank, self.R, width)
+            rows = B.latent_decode_tc_rows(n_seqs, self.H, self.kv_rank, self.R, splits)
+            plans[n_seqs, width] = splits, rows, B.sm_count() // (hpad // (32 if self.H > 16 else 16))
+        return plans[n_seqs, width]
 
     def weight_bytes(self) -> int:
         if not self.plain_form:
