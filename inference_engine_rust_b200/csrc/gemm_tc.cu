@@ -389,7 +389,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   int* ticket_s = (int*)(tmem_slot + 2);
-  uint8_t* xch_s = (uint8_t*)(((uintptr_t)(tmem_slot + 4) + 15) & ~(uintptr_t)15);   // 8 KB, weight-major gated only
+  uint8_t* xch_s = (uint8_t*)(((uintptr_t)(tmem_slot + 4) + 15) & ~(uintptr_t)15);   // weight-major gated only: 8 KB, 4 up to 16 tokens
   // 2 x 16 KB: staging of the residual add by TMA, or of the token-major stores (four warps, two boxes of 4 KB each)
   uint8_t* out_s = GATED ? (uint8_t*)(((uintptr_t)(tmem_slot + 4) + 1023) & ~(uintptr_t)1023)
                          : (uint8_t*)(((uintptr_t)(tmem_slot + 4) + 127) & ~(uintptr_t)127);
@@ -540,7 +540,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       constexpr int N_FACTORS = !FACTORS || GATED || BT > 32 ? 1 : BT > 16 ? BT / 2 : BT;
       float factor[N_FACTORS];
       const float* factor_col = nullptr;
-      if (FACTORS && !GATED && p.mode == MODE_GATED_SILU && p.ep.scale) {
+      if (FACTORS && !GATED && p.mode == MODE_GATED_SILU && p.ep.scale && (BT > 16 || q < 2)) {
         const int first = BT > 16 && q >= 2 ? 8 : 0;
         factor_col = p.ep.scale + (long long)(t0 + first) * p.ep.ld_scale + epilogue_block(n0 + (n_local & 63), p.ep);
 #pragma unroll
