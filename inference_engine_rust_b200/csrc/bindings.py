@@ -731,6 +731,8 @@ def _recurrent_lib(dim: int):
         lib.iert_mlstm_recur.restype = c_int
         lib.iert_recurrent_scratch_floats.argtypes = [c_int, c_int]
         lib.iert_recurrent_scratch_floats.restype = LL
+        lib.iert_wkv_scratch_floats.argtypes = [c_int, c_int]
+        lib.iert_wkv_scratch_floats.restype = LL
         lib.iert_wkv_recur.argtypes = [P, LL, P, P, P, LL, LL, P, P, c_int, c_int, POINTER(BatchView), P]
         lib.iert_wkv_recur.restype = c_int
         if os.environ.get("IERT_PDL", "1") == "0":
@@ -749,8 +751,13 @@ def _check_lib(status: int, what: str, launches: int = 1) -> None:
 
 
 def recurrent_scratch_floats(D: int, n_tokens: int, H: int) -> int:
-    """Scratch that lets `delta_recur` and `wkv_recur` take a prompt several tokens at a time (fp32)."""
+    """Scratch that lets `delta_recur` take a prompt several tokens at a time (fp32; enough for `wkv_recur` too)."""
     return _recurrent_lib(D).iert_recurrent_scratch_floats(n_tokens, H)
+
+
+def wkv_scratch_floats(D: int, n_tokens: int, H: int) -> int:
+    """Scratch that lets `wkv_recur` take a prompt several tokens at a time (fp32)."""
+    return _recurrent_lib(D).iert_wkv_scratch_floats(n_tokens, H)
 
 
 def delta_recur(qkv, beta, decay, state, s_off: int, o, G: int, D: int, H: int, V: int, batch: BatchView, stream, scratch=None) -> None:
@@ -789,8 +796,8 @@ def wkv_decay(z, L: int, w2t, w0, decay, h, state, prev_off: int, batch: BatchVi
 
 def wkv_recur(x, decay, u, state, s_off: int, o, D: int, H: int, V: int, batch: BatchView, stream, scratch=None) -> None:
     """o_t = (S + diag(u) k_t v_t^T)^T r_t; S <- diag(w_t) S + k_t v_t^T over the step's tokens, from the fp32
-    projections x = [r | k | v | ...] and the decays w; S [H, D, V] per slot in `state` at `s_off`.  `scratch` as for
-    `delta_recur`."""
+    projections x = [r | k | v | ...] and the decays w; S [H, D, V] per slot in `state` at `s_off`.  `scratch`
+    (`wkv_scratch_floats`): prompts may go several tokens at a time."""
     _check_lib(_recurrent_lib(D).iert_wkv_recur(x.data_ptr(), x.stride(0), decay.data_ptr(), u.data_ptr(), state.data_ptr(),
                                                 state.stride(0), s_off, o.data_ptr(), _ptr(scratch), H, V, byref(batch), stream),
                "wkv_recur", 2 if scratch is not None and batch.n_tokens >= max(32, 4 * batch.n_seqs) and D == 64 else 1)

@@ -1563,8 +1563,10 @@ IERT_API int iert_recurrent_dim() { return DIM; }
     default: { constexpr int RR = 32; CALL; } break;                 \
   }
 
-// Scratch (floats) of the recurrences over n_tokens tokens and H heads: the products of tokens with one another.
+// Scratch (floats) of the recurrences over n_tokens tokens and H heads: the products of tokens with one another, for the delta rule with what
+// else its chunks need; for the decay per key channel a row of products alone.
 IERT_API long long iert_recurrent_scratch_floats(int n_tokens, int H) { return (long long)n_tokens * H * 36; }
+IERT_API long long iert_wkv_scratch_floats(int n_tokens, int H) { return (long long)n_tokens * H * 16; }      // (eight of them: chunks of eight tokens)
 
 // scratch: as many floats as above, or null (then tokens go one after another)
 IERT_API int iert_delta_recur(const float* qkv, const float* beta, const float* decay, float* state,

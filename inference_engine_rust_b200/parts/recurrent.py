@@ -222,7 +222,7 @@ class Wkv(Mixer):
         decay = ws.take("wkv.decay", (T, hd), torch.float32)
         B.wkv_decay(z, self.L, self.w2t, self.w0, decay, xn, state, self.s_floats, ctx.batch, ctx.stream)
         o = ws.take("wkv.readout", (T, hd), torch.float32)
-        scratch = ws.take("wkv.pairs", (B.recurrent_scratch_floats(D, T, H),), torch.float32)
+        scratch = ws.take("wkv.pairs", (B.wkv_scratch_floats(D, T, H),), torch.float32)
         B.wkv_recur(x, decay, self.u, state, 0, o, D, H, D, ctx.batch, ctx.stream, scratch=scratch)
         out = ws.take("wkv.out", (T, hd), rt.dtype)
         B.wkv_finish(o, x[:, 3 * hd:], self.norm, self.eps, self.out_scale, out, ctx.batch, H, D, ctx.stream)

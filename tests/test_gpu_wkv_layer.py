@@ -49,6 +49,28 @@ def test_many_blocks(monkeypatch):
         assert off(got, want) <= 1.25 * off(plain, want) + 2.0 ** -25
 
 
+@pytest.mark.parametrize("lens", [[65, 100], [48], [47, 17], [33, 1, 0, 9]])       # (sixteen tokens at a time, and eight)
+def test_scratch_is_as_large_as_asked_for(lens):
+    from inference_engine_rust_b200.csrc import bindings as B
+    D = V = 64
+    H, T, g = 3, sum(lens), torch.Generator(device=DEV).manual_seed(len(lens))
+    x = torch.randn((T, 3 * H * D), generator=g, device=DEV)
+    decay = torch.exp(-torch.exp(torch.rand((T, H * D), generator=g, device=DEV) * 6 - 6))
+    u = torch.randn((H, D), generator=g, device=DEV)
+    state = torch.randn((len(lens), H * D * V), generator=g, device=DEV)
+    view, keep = batch(lens, list(range(len(lens))))
+    n, res = B.wkv_scratch_floats(D, T, H), []
+    assert n == 16 * T * H <= B.recurrent_scratch_floats(D, T, H)
+    for room in (n, B.recurrent_scratch_floats(D, T, H)):
+        scratch = torch.full((room + 4096,), 7.0, device=DEV)       # (room behind it, so that a write too far is seen and harms nothing)
+        s, o = state.clone(), torch.zeros((T, H * V), device=DEV)
+        B.wkv_recur(x, decay, u, s, 0, o, D, H, V, view, B.stream_ptr(), scratch=scratch)
+        torch.cuda.synchronize()
+        assert (scratch[n:] == 7.0).all()
+        res.append((o, s))
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+
+
 @pytest.mark.parametrize("lens,together", [([300], True), ([200, 57], True), ([256], False)])
 def test_four_projections_in_one_launch(monkeypatch, lens, together):
     from inference_engine_rust_b200.cache import Cache
