@@ -1028,7 +1028,7 @@ __global__ void __launch_bounds__(256 + LOADERS) wkv_recur_kernel(WkvArgs a, Ier
 //   S  <- W_16 S + sum_j (w_(j+1) .. w_16 k_j) v_j^T
 // There is no chain inside a chunk at all.  The products of two tokens come from a kernel in front with a block per chunk and head;
 // here the loaders bring the rows through a ring, scale them by the decays between (products, never quotients) and split them.
-// 2,048 tokens, 64 heads of 64 x 64 (128 blocks): 103 us; eight tokens at a time with FFMA 252.
+// 2,048 tokens, 64 heads of 64 x 64 (128 blocks): 109 us, and 28 of the kernel in front; eight tokens at a time with FFMA 252 in all.
 
 // pairs[token][head][16]: row i of the chunk's products with the tokens j <= i.  Thread (half of the chunk, row d of S): row d's share
 // of the pairs inside a half, then summed over the rows; the pairs across the halves are products of r_i w_8 .. w_(i-1) with
@@ -1131,8 +1131,9 @@ struct WkvShared {
   float4 xo[8][2][32];                               // a warp's share of r.S
 };
 
-// PER_SM: blocks that share an SM (80 registers a thread then: 139 us for the one prompt above; 256 blocks and more are faster so, 64 prompts of
-// 64 tokens 1,091 us a layer against 1,156).
+// PER_SM: blocks that share an SM (80 registers a thread with two, each then slower: 139 us for the one prompt above).  Two are for more blocks than
+// two waves of one an SM; this kernel and the one in front, two / one, us: 152 blocks (2,048 tokens of 76 heads) 271 / 248, 256 (two prompts of 1,024, 64
+// heads) 156 / 149, 384 (three of 100) 41.8 / 43.8, 1,024 (eight of 48) 45.5 / 52.4.
 template <int PER_SM>
 __global__ void __launch_bounds__(WWORK + CLOAD, PER_SM) wkv_chunk_kernel(WkvArgs a, const float* __restrict__ pairs, IertBatchView b) {
   static_assert(DIM == 64 && CLOAD == 128, "a loader warp per 64 rows of r or k and half of the tokens");
@@ -1606,7 +1607,7 @@ IERT_API int iert_wkv_recur(const float* x, long long ld, const float* decay, co
     WkvArgs a = {x, ld, decay, u, state, state_stride, s_off, o, H, V, CCOLS};
     const dim3 columns(batch->n_seqs, H, (V + CCOLS - 1) / CCOLS);
     if (chunked(batch, 48, 48)) {
-      auto* kernel = (long long)columns.x * columns.y * columns.z > iert_sm_count_cached() ? wkv_chunk_kernel<2> : wkv_chunk_kernel<1>;
+      auto* kernel = (long long)columns.x * columns.y * columns.z > 2 * iert_sm_count_cached() ? wkv_chunk_kernel<2> : wkv_chunk_kernel<1>;
       if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WkvShared)) != cudaSuccess)
         return iert_check_launch("wkv_recur attribute");
       launch_dep(wkv_pairs_kernel, dim3(batch->n_tokens / CT + batch->n_seqs, H), dim3(2 * DIM), 0, stream, a, scratch, *batch);

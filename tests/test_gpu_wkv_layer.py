@@ -10,16 +10,16 @@ pytestmark = pytest.mark.gpu
 
 
 def test_many_blocks(monkeypatch):
-    """Two prompts of 64 heads are 256 blocks, two an SM; one of them alone has an SM for each block and the same bits."""
+    """Three prompts of 64 heads are 384 blocks, two an SM; one of them alone has an SM for each block and the same bits."""
     from inference_engine_rust_b200.csrc import bindings as B
     D = V = 64
-    H, lens = 64, [50, 61]
-    assert 2 * H * len(lens) > B.sm_count() >= 2 * H
+    H, lens = 64, [50, 61, 48]
+    assert 2 * H * len(lens) > 2 * B.sm_count() >= 2 * H
     T, g = sum(lens), torch.Generator(device=DEV).manual_seed(3)
     x = torch.randn((T, 3 * H * D), generator=g, device=DEV)
     decay = torch.exp(-torch.exp(torch.rand((T, H * D), generator=g, device=DEV) * 6 - 6))
     u = torch.randn((H, D), generator=g, device=DEV)
-    state = torch.randn((2, H * D * V), generator=g, device=DEV)
+    state = torch.randn((3, H * D * V), generator=g, device=DEV)
 
     def run(lens, first):
         view, keep = batch(lens, list(range(len(lens))))
@@ -34,7 +34,7 @@ def test_many_blocks(monkeypatch):
     (o, s), (o1, s1) = both_ways(monkeypatch, run(lens, 0), state)
     r, k, v = (x[:, i * H * D:(i + 1) * H * D].double().view(T, H, -1) for i in range(3))
     w = decay.double().view(T, H, D)
-    want_o, want_s, at = torch.zeros((T, H, V), dtype=torch.float64, device=DEV), state.double().view(2, H, D, V).clone(), 0
+    want_o, want_s, at = torch.zeros((T, H, V), dtype=torch.float64, device=DEV), state.double().view(3, H, D, V).clone(), 0
     for i, m in enumerate(lens):
         for t in range(at, at + m):
             kv = k[t][:, :, None] * v[t][:, None]
