@@ -60,7 +60,6 @@ def test_launches_with_room_for_a_cut(heads, rank, lens, cut):
     from inference_engine_rust_b200.config.specs import PartSpec
     from inference_engine_rust_b200.csrc import bindings as B
     from inference_engine_rust_b200.parts import Runtime, part_class
-    from inference_engine_rust_b200.parts.latent_attention import length_cut_run
     p = {"hidden_size": 64, "heads": heads, "dim": 32, "vdim": 32, "kv_rank": rank, "q_rank": None, "scale": 0.2, "eps": 1e-5, "sink": False,
          "rot_dim": 16, "gate": "head", "position": PartSpec("rope", {"theta": 1e4, "rotary_dim": 16, "pairing": "interleaved"})}
     g = torch.Generator(device=DEV).manual_seed(len(lens) + heads)
@@ -80,7 +79,10 @@ def test_launches_with_room_for_a_cut(heads, rank, lens, cut):
     hpad, splits = B.latent_decode_tc_plan(batch, heads, rank, 16, max(pages))
     rows = B.latent_decode_tc_rows(batch, heads, rank, 16, splits)
     assert rows > splits
-    assert (length_cut_run(pages, splits, rows, B.sm_count() // (hpad // (32 if heads > 16 else 16))) > 0) == cut
+    # the kernel's rule: the fewest pages a run with which every run has a CTA and a partial result, if an even run is longer
+    ctas, even = B.sm_count() // (hpad // (32 if heads > 16 else 16)), -(-max(pages) // splits)
+    fits = [r for r in range(1, max(pages) + 1) if max(pages) <= r * rows and sum(-(-n // r) for n in pages) <= ctas]
+    assert (even * ctas > 3 * sum(pages) and bool(fits) and fits[0] < even) == cut
     assert part.cut_by_length(lens, cache.layer_view(0)) == cut
     out = []
     for by_length in (True, False):
