@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(256 + LOADERS) delta_recur_kernel(DeltaArgs a,
 // A block owns 32 columns: four warps compute, each 16 columns x half of the rows (the halves of k.S and q.S are exchanged through
 // shared memory), four bring q, k, v and the coefficients and split them.  2,048 tokens, 32 heads of 128 x 128 (128 blocks): 200 to
 // 212 us; eight tokens at a time with FFMA, a thread holding 8 rows of four columns, took 344.  What bounds it is the chain
-// k.S - x - u - S of a warp, about 2,900 clocks a chunk: its 162 mma.sync take 10 to 12 clocks each beside ldmatrix, and nothing else of
+// k.S - x - u - S of a warp, about 2,500 cycles a chunk, in half of which the tensor pipe is active (162 mma.sync of 8 cycles): nothing else of
 // that warp's scheduler has as much to do.  Other splits were no faster: q.S and P u in warps of their own with the state's parts
 // through shared memory 222, quarters of the rows in twice the warps 261 (236 with the column groups half a chunk apart).
 #define IERT_CHUNKED (DIM == 64 || DIM == 128)                // (larger sizes would not fit the registers)
